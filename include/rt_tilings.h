@@ -493,8 +493,9 @@ RT_API rt_status rt_dm_sampler_engine_info(rt_dm_sampler* s, int64_t* out4);
 /* Launch shape of the sampler's next runs (no counterpart in the reference: its kernels use
    one compile-time block shape, BLOCK_DIM 8 in src/Domino/dominokernel.cuh:4): engine (0
    automatic, 1 per-half-sweep kernels, 2 the run kernel, 3 k_persist, 4 the bit-plane
-   kernel), bands (CTAs, 0: one per SM) and threads per band (a multiple of 32 up to 1024,
-   0: 1024) of the run kernel.
+   kernel), bands (CTAs, 0: one per SM; with engine 0 or 4, 1..16 bands are the CTAs of one
+   thread-block cluster that holds the whole tiling, where it fits) and threads per band (a
+   multiple of 32 up to 1024, 0: 1024) of the run kernel.
    Results do not depend on the shape: every draw is keyed by its site.  Without this call,
    and with rt_walk_opts.engine 0, the autotuner's table (rt_tune_load) chooses when it has an
    entry.  out6 of rt_dm_sampler_launch_info = {engine, units, bands, units per thread,

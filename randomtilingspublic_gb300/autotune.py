@@ -25,9 +25,10 @@ THREADS = (512, 640, 768, 896, 960, 992, 1024)
 
 def candidates(sms: int) -> list[tuple[int, int, int]]:
     """(engine, bands, threads): the per-half-sweep kernels, k_persist, the run kernel over
-    bands and threads per band, and the bit-plane kernel (TinyMT only; its threads follow from
-    its plan) over bands."""
-    out = [(1, 0, 0), (3, 0, 0)]
+    bands and threads per band, the bit-plane kernel (TinyMT only; its threads follow from
+    its plan) over bands, and its form in one thread-block cluster (engine 0 with the
+    cluster's CTAs as bands)."""
+    out = [(1, 0, 0), (3, 0, 0), (0, 1, 0), (0, 4, 0), (0, 16, 0)]
     for bands in sorted({sms, (3 * sms) // 4, sms // 2}, reverse=True):
         out.append((4, bands, 0))
         for threads in THREADS:
@@ -57,6 +58,10 @@ def measure(rt, n, chains, rng, tmax, tmin, shape, half_sweeps: int = 256, reps:
         except rt.RTError:
             return None
         engine, bands, threads = shape
+        if engine == 0:  # the cluster form, reported as the bit-plane kernel
+            if info["engine"] != 4 or info["bands"] > bands:
+                return None
+            engine = 4
         if info["engine"] != engine or (engine == 2 and info["threads"] != threads):
             return None
         used = (engine, info["bands"], threads) if engine in (2, 4) else shape

@@ -238,6 +238,7 @@ __global__ void k_diff(DmView v, int a, int b, unsigned long long* out) {
   } while (0)
 
 DmSampler::~DmSampler() {
+  cluster.reset();
   bits.reset();  // the engines free their plan buffers on the stream before the stream goes
   runs.reset();
   persist.reset();
@@ -558,24 +559,24 @@ rt_status DmSampler::sync() {
 rt_status DmSampler::use_persistent(bool* yes) {
   *yes = false;
   resident = 0;
+  in_cluster = false;
   // The engine: opts.engine when set, else the sampler's explicit launch shape, else the
   // autotuner's entry for this side, chain count and mode, else automatic.
-  int engine = opts.engine;
-  const bool explicit_engine = engine != 0 || launch_engine != 0;
+  const bool explicit_engine = opts.engine != 0 || launch_engine != 0;
+  int engine = opts.engine != 0 ? opts.engine : launch_engine;
   eff_bands = launch_bands;
   eff_threads = launch_threads;
   tuned = false;
-  if (engine == 0 && launch_engine != 0) {
-    engine = launch_engine;
-  } else if (engine == 0 && launch_bands == 0 && launch_threads == 0) {
+  const bool ask_table = !explicit_engine && launch_bands == 0 && launch_threads == 0;
+  auto take_entry = [&](int skip) {
     int e = 0, b = 0, t = 0;
-    if (tune_lookup(RT_MODEL_DOMINO, N, active, opts.rng_mode, &e, &b, &t)) {
-      engine = e;
-      eff_bands = b;
-      eff_threads = t;
-      tuned = true;
-    }
-  }
+    tuned = tune_lookup(RT_MODEL_DOMINO, N, active, opts.rng_mode, skip, &e, &b, &t);
+    engine = tuned ? e : 0;
+    eff_bands = tuned ? b : 0;
+    eff_threads = tuned ? t : 0;
+    return tuned;
+  };
+  if (ask_table) take_entry(0);
   if (engine == 1 || opts.rng_mode == RT_RNG_MTGP) return RT_OK;
   if (plan_dirty) {
     if (rt_status st = fetch_candidates()) return st;
@@ -585,16 +586,43 @@ rt_status DmSampler::use_persistent(bool* yes) {
       return fail(RT_ERR_INVALID_ARGUMENT, "persistent engine needs consistent loaded tilings");
     return RT_OK;
   }
-  // Engine 0: the bit-plane kernel, else the run kernel, else k_persist; 4: the bit-plane
-  // kernel alone; 2: the run kernel, else k_persist; 3: k_persist alone.
-  if (plan_dirty ||
-      (runs && (runs->nch != active || runs->bands_asked != eff_bands || runs->threads_asked != eff_threads)) ||
-      (persist && persist->nch != active) || (bits && bits->nch != active)) {
+  if (plan_dirty) {
+    cluster.reset();
     bits.reset();
     runs.reset();
     persist.reset();
   }
   plan_dirty = false;
+  // The bit-plane kernel in one thread-block cluster: where 1..16 bands are asked for (they are
+  // the cluster's CTAs), or automatically up to the size at which more SMs pay for the slower
+  // exchange (cl_auto_words).  A table entry that asks for it gives way to the next where the
+  // domain does not fit.
+  const bool fast = opts.rng_mode == RT_RNG_FAST;
+  for (int skip = 0; (engine == 0 || (engine == 4 && !(fast && explicit_engine))) && eff_bands <= kClMaxCtas &&
+                     (eff_bands > 0 || engine == 0);) {
+    if (cluster && (cluster->nch != active || cluster->bands_asked != eff_bands)) cluster.reset();
+    if (!cluster) {
+      cluster = std::make_unique<ClusterEngine>();
+      if (rt_status st = cluster->prepare(*this)) return st;
+    }
+    if (cluster->ready && (launch_bands > 0 || cluster->plan.words <= cl_auto_words(fast, active))) {
+      resident = 4;
+      in_cluster = true;
+      *yes = true;
+      return RT_OK;
+    }
+    if (!tuned) break;
+    take_entry(++skip);
+  }
+  // Engine 0: the bit-plane kernel, else the run kernel, else k_persist; 4: the bit-plane
+  // kernel alone; 2: the run kernel, else k_persist; 3: k_persist alone.
+  if ((runs && (runs->nch != active || runs->bands_asked != eff_bands || runs->threads_asked != eff_threads)) ||
+      (persist && persist->nch != active) || (bits && bits->nch != active)) {
+    bits.reset();
+    runs.reset();
+    persist.reset();
+  }
+  if (engine == 1) return RT_OK;
   std::string why;
   if (engine == 0 || engine == 4) {
     if (!bits) {
@@ -637,6 +665,9 @@ rt_status DmSampler::use_persistent(bool* yes) {
 }
 
 rt_status DmSampler::check_resident_error() {
+  if (cluster) {
+    if (rt_status st = cluster->check_error(*this)) return st;
+  }
   if (bits) {
     if (rt_status st = bits->check_error(*this)) return st;
   }
@@ -650,6 +681,7 @@ rt_status DmSampler::check_resident_error() {
 }
 
 rt_status DmSampler::launch_resident(const uint8_t* colours, int64_t steps, uint64_t fast_seed, int64_t h0) {
+  if (in_cluster) return cluster->launch(*this, colours, steps, fast_seed, h0);
   if (resident == 4) return bits->launch(*this, colours, steps);
   if (resident == 2) return runs->launch(*this, colours, steps, fast_seed, h0);
   return persist->launch(*this, colours, steps, fast_seed, h0);
@@ -766,7 +798,11 @@ RT_API rt_status rt_dm_sampler_engine_info(rt_dm_sampler* s, int64_t* out4) {
   bool pers = false;
   if (rt_status st = d.use_persistent(&pers)) return st;
   int64_t units = 0, bands = 0, k = 0;
-  if (pers && d.resident == 4) {
+  if (pers && d.in_cluster) {
+    units = d.cluster->plan.draw_cells;
+    bands = d.cluster->plan.ctas;
+    k = d.cluster->plan.slots;
+  } else if (pers && d.resident == 4) {
     units = d.bits->plan.draw_cells;
     bands = (int64_t)d.bits->plan.bands.size();
     k = kBitSlots;
@@ -805,7 +841,8 @@ RT_API rt_status rt_dm_sampler_launch_info(rt_dm_sampler* s, int64_t* out6) {
   if (rt_status st = rt_dm_sampler_engine_info(s, e4)) return st;
   DmSampler& d = *s->impl;
   for (int k = 0; k < 4; ++k) out6[k] = e4[k];
-  out6[4] = (e4[0] == 4)   ? (int64_t)d.bits->plan.warps * 32
+  out6[4] = d.in_cluster   ? (int64_t)d.cluster->plan.threads()
+            : (e4[0] == 4) ? (int64_t)d.bits->plan.warps * 32
             : (e4[0] == 2) ? d.runs->plan.threads
                            : (e4[0] == 3 ? (int64_t)kPersistThreads : 0);
   out6[5] = d.tuned ? 1 : 0;
@@ -961,7 +998,11 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
         for (int k = att + q; k >= 0; --k) epochs[(size_t)q].push_back({ep_seed[(size_t)k], &colours_of(k)});
       cudaEventRecord(s->ev0, s->stream);
       int ran = 0;
-      if (s->resident == 4) {
+      if (s->in_cluster) {
+        if (rt_status st =
+                s->cluster->cftp(*s, att, n, epochs, first_steps, (uint64_t)driver_seed, &ran, &coalesced))
+          return st;
+      } else if (s->resident == 4) {
         if (rt_status st = s->bits->cftp(*s, n, epochs, &ran, &coalesced)) return st;
       } else if (rt_status st = s->runs->cftp(*s, att, n, epochs, first_steps, (uint64_t)driver_seed, &ran, &coalesced)) {
         return st;

@@ -5,7 +5,9 @@
 // Text format, one entry per line ('#' starts a comment):
 //   <model> <n_lo> <n_hi> <chains> <rng> <engine> <bands> <threads> [<us per half-sweep>]
 // model: domino; rng: tinymt | fast; engine: 1 per-half-sweep kernels, 2 the run kernel,
-// 3 k_persist, 4 the bit-plane kernel; bands, threads: 0 for the engine's default.
+// 3 k_persist, 4 the bit-plane kernel (1..16 bands: the CTAs of one thread-block cluster);
+// bands, threads: 0 for the engine's default.  The first entry whose range holds the side
+// counts; a cluster entry whose domain does not fit one gives way to the next that matches.
 #include <cstdlib>
 #include <fstream>
 #include <mutex>
@@ -57,7 +59,7 @@ rt_status parse_table(const std::string& path, std::vector<TuneEntry>* out) {
 
 }  // namespace
 
-bool tune_lookup(int model, int n_side, int chains, int rng, int* engine, int* bands, int* threads) {
+bool tune_lookup(int model, int n_side, int chains, int rng, int skip, int* engine, int* bands, int* threads) {
   std::lock_guard<std::mutex> lock(g_tune_mu);
   if (!g_tune_env_read) {
     g_tune_env_read = true;
@@ -68,7 +70,7 @@ bool tune_lookup(int model, int n_side, int chains, int rng, int* engine, int* b
     }
   }
   for (const TuneEntry& e : g_tune)
-    if (e.model == model && e.rng == rng && e.chains == chains && n_side >= e.n_lo && n_side <= e.n_hi) {
+    if (e.model == model && e.rng == rng && e.chains == chains && n_side >= e.n_lo && n_side <= e.n_hi && skip-- == 0) {
       *engine = e.engine;
       *bands = e.bands;
       *threads = e.threads;
@@ -106,7 +108,7 @@ RT_API rt_status rt_tune_lookup(int32_t model, int32_t n_side, int32_t chains, i
   clear_error();
   if (!out3) return fail(RT_ERR_INVALID_ARGUMENT, "tune lookup: NULL out");
   int e = 0, b = 0, t = 0;
-  if (!tune_lookup(model, n_side, chains, rng_mode, &e, &b, &t))
+  if (!tune_lookup(model, n_side, chains, rng_mode, 0, &e, &b, &t))
     return fail(RT_ERR_INVALID_ARGUMENT, "tune lookup: no entry");
   out3[0] = e;
   out3[1] = b;
