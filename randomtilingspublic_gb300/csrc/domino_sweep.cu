@@ -245,7 +245,7 @@ DmSampler::~DmSampler() {
   for (void* p : {(void*)tmt, (void*)tmt_params, mtgp, (void*)base, (void*)scratch, (void*)counter, (void*)d_scan,
                   (void*)d_cand})
     dev_free(p, stream);
-  for (void* p : {(void*)d_dom, (void*)d_cls, (void*)d_h, (void*)d_hflags})
+  for (void* p : {(void*)d_dom, (void*)d_hf, (void*)d_h, (void*)d_hflags})
     if (p) cudaFree(p);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
@@ -525,13 +525,12 @@ rt_status DmSampler::set_domain(const int32_t* domain, int m_side) {
   const size_t NN = (size_t)N * N;
   if (!d_dom) {
     RT_CUDA(cudaMalloc(&d_dom, (size_t)M * M * sizeof(int32_t)));
-    RT_CUDA(cudaMalloc(&d_cls, NN * sizeof(int32_t)));
+    RT_CUDA(cudaMalloc(&d_hf, NN));
     RT_CUDA(cudaMalloc(&d_h, NN * sizeof(int32_t)));
     RT_CUDA(cudaMalloc(&d_hflags, 16 * sizeof(unsigned)));
   }
   RT_CUDA(cudaMemcpyAsync(d_dom, domain, (size_t)M * M * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-  RT_CUDA(cudaMemsetAsync(d_hflags, 0, 16 * sizeof(unsigned), stream));
-  if (rt_status st = dm_classes_device(d_dom, M, d_cls, d_hflags + 8, stream)) return st;
+  if (rt_status st = dm_hf_domain(d_dom, M, d_hf, stream)) return st;
   RT_CUDA(cudaStreamSynchronize(stream));
   return RT_OK;
 }
@@ -543,11 +542,11 @@ rt_status DmSampler::accumulate_heights(int ch, long long* sums, int32_t* height
   k_merge<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(v, ch, scratch);
   launches++;
   if (rt_status st = check_launch()) return st;
-  if (rt_status st = dm_heights_device(scratch, d_cls, d_dom, N, hf_start, d_h, d_hflags, stream)) return st;
+  int32_t* const h = heights ? heights : d_h;
+  if (rt_status st = dm_heights_device(scratch, d_hf, N, hf_start, h, d_hflags, stream)) return st;
   if (sums) {
-    if (rt_status st = dm_heights_accumulate(d_h, N, sums, stream)) return st;
+    if (rt_status st = dm_heights_accumulate(h, N, sums, stream)) return st;
   }
-  if (heights) RT_CUDA(cudaMemcpyAsync(heights, d_h, (size_t)N * N * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
   return RT_OK;
 }
 

@@ -43,10 +43,10 @@ __device__ __forceinline__ uint8_t dm_flip(uint32_t e, uint32_t u, uint32_t lo_u
 rt_status mtgp_rotate(const DmView& v, int t, const DmRule& rule, void* states, cudaStream_t stream);
 
 // Device height functions (domino_thurston.cu).
-rt_status dm_heights_device(const int32_t* d_t, const int32_t* d_cls, const int32_t* d_dom, int N, int start,
-                            int32_t* d_h, unsigned* d_flags, cudaStream_t st);
+rt_status dm_heights_device(const int32_t* d_t, const uint8_t* d_dom, int N, int start, int32_t* d_h, unsigned* d_flags,
+                            cudaStream_t st);
 rt_status dm_heights_accumulate(const int32_t* d_h, int N, long long* sums, cudaStream_t st);
-rt_status dm_classes_device(const int32_t* d_dom, int M, int32_t* d_cls, unsigned* d_count, cudaStream_t st);
+rt_status dm_hf_domain(const int32_t* d_dom, int M, uint8_t* d_out, cudaStream_t st);
 int dm_first_boundary_vertex(const int32_t* domain, int M);
 
 struct DmSampler {
@@ -106,7 +106,8 @@ struct DmSampler {
   // added to running sums.
   rt_status set_domain(const int32_t* domain, int m_side);
   rt_status accumulate_heights(int ch, long long* sums, int32_t* heights);
-  int32_t *d_dom = nullptr, *d_cls = nullptr, *d_h = nullptr;
+  int32_t *d_dom = nullptr, *d_h = nullptr;
+  uint8_t* d_hf = nullptr;  // vertex and edge flags of the domain (dm_hf_domain)
   unsigned* d_hflags = nullptr;
   int hf_start = -1;
   rt_status store(int ch, int32_t* tiling);

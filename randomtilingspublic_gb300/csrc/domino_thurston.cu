@@ -101,59 +101,156 @@ __global__ void __launch_bounds__(kTile * kTile) k_th_relax_tile(ThArgs a, unsig
 
 // Height function of a tiling (TilingToHeightfunc, DominoTiler.cpp:555-593): from the start
 // vertex (height 0), heights spread across every edge no domino covers (its bit clear at the
-// vertex it leaves) that touches the domain, by +-1 (th_step).  For a tiling the heights do
-// not depend on the path, so each unassigned vertex takes the value from its first assigned
-// neighbour; one tile at a time in shared memory until the tile stops changing.
-__device__ __forceinline__ bool th_touches(const int32_t* dom, int M, int ui, int uj, int nb) {
-  const int ai = ui + c_dirs[nb].fa_i, aj = uj + c_dirs[nb].fa_j, bi = ui + c_dirs[nb].fb_i, bj = uj + c_dirs[nb].fb_j;
-  const bool fa = ai >= 0 && aj >= 0 && ai < M && aj < M && dom[ai * M + aj];
-  const bool fb = bi >= 0 && bj >= 0 && bi < M && bj < M && dom[bi * M + bj];
-  return fa || fb;
+// vertex it leaves) that touches the domain, by +-1 (th_step).  Across an edge inside a domino
+// the height changes by -3 times that step: three sides of the same square lead around it, none
+// of them covered.  So every edge that touches the domain links its ends with a known
+// difference, and a line of linked vertices is known as soon as one of them is: a scan, not a
+// walk.  Passes over all columns and all rows alternate until nothing is left (an Aztec diamond:
+// the start's row, the columns, the rows).
+// Bound: the bytes of a pass, in L2.  One vertex per thread and round in 32 x 32 tiles, as this was
+// before, moved the front by one tile per pass: 128 passes and 5.0 ms at order 1024; three passes
+// over the 4.2 M vertices take 0.25 ms.
+enum : uint8_t { kHfVertex = 1, kHfRight = 2, kHfDown = 4 };
+
+// Per vertex: does it touch the domain, and do its edges to the right and down.
+__global__ void k_hf_domain(const int32_t* d, int M, uint8_t* out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y, N = M + 1;
+  if (j >= N) return;
+  auto sq = [&](int a, int b) { return a >= 0 && b >= 0 && a < M && b < M && d[(size_t)a * M + b] != 0; };
+  const bool nw = sq(i - 1, j - 1), ne = sq(i - 1, j), sw = sq(i, j - 1), se = sq(i, j);
+  out[(size_t)i * N + j] = (uint8_t)((nw || ne || sw || se ? kHfVertex : 0) | (ne || se ? kHfRight : 0) |
+                                     (sw || se ? kHfDown : 0));
 }
 
-__global__ void __launch_bounds__(kTile * kTile) k_hf_tile(const int32_t* t, const int32_t* cls, const int32_t* dom,
-                                                           int32_t* h, int N, unsigned* changed) {
-  pdl_begin();
-  __shared__ int32_t sh[kTile + 2][kTile + 2];
-  __shared__ int8_t st[kTile + 2][kTile + 2];
-  __shared__ int8_t sc[kTile + 2][kTile + 2];
-  const int M = N - 1, tx = threadIdx.x, ty = threadIdx.y;
-  const int j0 = blockIdx.x * kTile - 1, i0 = blockIdx.y * kTile - 1;
-  for (int k = ty * kTile + tx; k < (kTile + 2) * (kTile + 2); k += kTile * kTile) {
-    const int r = k / (kTile + 2), c = k % (kTile + 2), i = i0 + r, j = j0 + c;
-    const bool in = i >= 0 && j >= 0 && i < N && j < N;
-    sh[r][c] = in ? h[i * N + j] : kUnset;
-    st[r][c] = in ? (int8_t)t[i * N + j] : (int8_t)0;
-    sc[r][c] = in ? (int8_t)cls[i * N + j] : (int8_t)0;
-  }
-  __syncthreads();
-  const int r = ty + 1, c = tx + 1, i = i0 + r, j = j0 + c;
-  const bool open = i < N && j < N && sc[r][c] > 0;
-  constexpr int kOpp[4] = {1, 0, 3, 2};
-  bool any = false;
-  for (int round = 0; round < 2 * kTile * kTile; ++round) {
-    int32_t val = kUnset;
-    if (open && sh[r][c] == kUnset) {
+// A step along a line as a map of the height before it: a constant, or a difference.
+struct HfMap {
+  int32_t v;
+  bool fixed;
+};
+__device__ __forceinline__ HfMap hf_then(HfMap a, HfMap b) {  // a, then b
+  if (b.fixed) return b;
+  if (a.fixed && a.v == kUnset) return a;
+  return HfMap{a.v + b.v, a.fixed};
+}
+__device__ __forceinline__ int32_t hf_apply(HfMap f, int32_t x) { return f.fixed ? f.v : (x == kUnset ? kUnset : x + f.v); }
+
+// The difference along the edge from (i, j) to the right (bit 8) or down (bit 2).
+__device__ __forceinline__ int32_t hf_delta(int mask, bool right, int i, int j) {
+  const int s = th_step(i, j, right ? 2 : 0);
+  return (mask & (right ? 8 : 2)) ? -3 * s : s;
+}
+
+// Rows: a warp per row, four vertices a lane, forward then back.  left (when given) counts the
+// vertices of the domain still unset, changed is set when a height was.
+constexpr int kHfPer = 4;
+__global__ void __launch_bounds__(256) k_hf_rows(const int32_t* t, const uint8_t* dom, int32_t* h, int N, int row0,
+                                                 int rows, unsigned* changed, unsigned* left) {
+  const int r = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int i = row0 + r;
+  const int32_t* tr = t + (size_t)i * N;
+  const uint8_t* dr = dom + (size_t)i * N;
+  int32_t* hr = h + (size_t)i * N;
+  const int blocks = (N + 32 * kHfPer - 1) / (32 * kHfPer);
+  bool moved = false;
+  unsigned unset = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    int32_t carry = kUnset;
+    for (int q = 0; q < blocks; ++q) {
+      const int j0 = (pass ? blocks - 1 - q : q) * 32 * kHfPer + (pass ? 31 - lane : lane) * kHfPer;
+      HfMap f[kHfPer], all{0, false};
+      int32_t old[kHfPer];
 #pragma unroll
-      for (int nbv = 0; nbv < 4; ++nbv) {
-        const int ur = r + c_dirs[nbv].di, uc = c + c_dirs[nbv].dj;
-        if (sc[ur][uc] == 0 || sh[ur][uc] == kUnset) continue;
-        const int nb = kOpp[nbv];  // the step from u back to v
-        if (st[ur][uc] & c_dirs[nb].bit) continue;
-        const int ui = i + c_dirs[nbv].di, uj = j + c_dirs[nbv].dj;
-        if (!th_touches(dom, M, ui, uj, nb)) continue;
-        val = sh[ur][uc] + th_step(ui, uj, nb);
-        break;
+      for (int k = 0; k < kHfPer; ++k) {
+        const int j = j0 + (pass ? kHfPer - 1 - k : k);
+        old[k] = j < N ? hr[j] : kUnset;
+        f[k] = HfMap{kUnset, true};
+        if (old[k] != kUnset) {
+          f[k].v = old[k];
+        } else if (pass == 0 ? (j > 0 && j < N && (dr[j - 1] & kHfRight)) : (j + 1 < N && (dr[j] & kHfRight))) {
+          const int e = pass == 0 ? j - 1 : j;  // the edge's left end
+          const int32_t d = hf_delta(tr[e], true, i, e);
+          f[k] = HfMap{pass == 0 ? d : -d, false};
+        }
+        all = hf_then(all, f[k]);
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const HfMap before{__shfl_up_sync(~0u, all.v, o), (bool)__shfl_up_sync(~0u, (int)all.fixed, o)};
+        if (lane >= o) all = hf_then(before, all);
+      }
+      const int32_t mine = hf_apply(all, carry);  // after this lane's vertices
+      int32_t x = __shfl_up_sync(~0u, mine, 1);
+      if (lane == 0) x = carry;
+      carry = __shfl_sync(~0u, mine, 31);
+#pragma unroll
+      for (int k = 0; k < kHfPer; ++k) {
+        const int j = j0 + (pass ? kHfPer - 1 - k : k);
+        x = hf_apply(f[k], x);
+        if (j < N && old[k] == kUnset) {
+          if (x != kUnset) hr[j] = x, moved = true;
+          else if (pass && (dr[j] & kHfVertex)) ++unset;
+        }
       }
     }
-    const bool moved = val != kUnset;
-    __syncthreads();
-    if (moved) sh[r][c] = val;
-    any = any || moved;
-    if (!__syncthreads_or(moved)) break;
+    __syncwarp();  // this lane reads other lanes' heights on the way back
   }
-  if (open && any) h[i * N + j] = sh[r][c];
-  if (__syncthreads_or(any) && tx == 0 && ty == 0) *changed = 1u;
+  if (__any_sync(~0u, moved) && lane == 0) *changed = 1u;
+  unset = __reduce_add_sync(~0u, unset);
+  if (left && lane == 0 && unset) atomicAdd(left, unset);
+}
+
+// Columns: a CTA per 32 columns, each warp a chunk of rows; the chunks' maps are joined in shared
+// memory, then each warp fills its chunk, forward and back.
+__global__ void __launch_bounds__(1024) k_hf_cols(const int32_t* t, const uint8_t* dom, int32_t* h, int N,
+                                                  unsigned* changed) {
+  __shared__ int32_t sv[2][32][33];
+  __shared__ bool sf[2][32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+  const int per = (N + 31) / 32, i0 = w * per, i1 = min(N, i0 + per);
+  const bool in = j < N;
+  auto at = [&](int i) { return (size_t)i * N + j; };
+  // the map from the vertex above (below) to vertex (i, j)
+  auto down = [&](int i, int32_t old) -> HfMap {
+    if (old != kUnset) return HfMap{old, true};
+    if (i > 0 && (dom[at(i - 1)] & kHfDown)) return HfMap{hf_delta(t[at(i - 1)], false, i - 1, j), false};
+    return HfMap{kUnset, true};
+  };
+  auto up = [&](int i, int32_t old) -> HfMap {
+    if (old != kUnset) return HfMap{old, true};
+    if (i + 1 < N && (dom[at(i)] & kHfDown)) return HfMap{-hf_delta(t[at(i)], false, i, j), false};
+    return HfMap{kUnset, true};
+  };
+  HfMap fd{0, false}, fu{0, false};
+  if (in) {
+#pragma unroll 4
+    for (int i = i0; i < i1; ++i) {
+      const int32_t old = h[at(i)];
+      fd = hf_then(fd, down(i, old));
+      fu = hf_then(up(i, old), fu);  // from below: the lowest row's map comes first
+    }
+  }
+  sv[0][w][lane] = fd.v, sf[0][w][lane] = fd.fixed;
+  sv[1][w][lane] = fu.v, sf[1][w][lane] = fu.fixed;
+  __syncthreads();
+  if (!in) return;
+  int32_t x = kUnset, y = kUnset;  // the heights before the chunk, from above and from below
+  for (int q = 0; q < w; ++q) x = hf_apply(HfMap{sv[0][q][lane], sf[0][q][lane]}, x);
+  for (int q = 31; q > w; --q) y = hf_apply(HfMap{sv[1][q][lane], sf[1][q][lane]}, y);
+  bool moved = false;
+#pragma unroll 4
+  for (int i = i0; i < i1; ++i) {
+    const int32_t old = h[at(i)];
+    x = hf_apply(down(i, old), x);
+    if (old == kUnset && x != kUnset) h[at(i)] = x, moved = true;
+  }
+#pragma unroll 4
+  for (int i = i1 - 1; i >= i0; --i) {
+    const int32_t old = h[at(i)];
+    y = hf_apply(up(i, old), y);
+    if (old == kUnset && y != kUnset) h[at(i)] = y, moved = true;
+  }
+  if (moved) *changed = 1u;
 }
 
 __global__ void k_fill_unset(int32_t* h, int64_t nn, int start) {
@@ -226,25 +323,24 @@ __global__ void k_th_tiling(const int32_t* h, const int32_t* d, int N, int32_t* 
 
 }  // namespace
 
-// Device height function of the host-layout tiling d_t (N x N) for the domain whose vertex
-// classes are d_cls, starting at vertex `start` (height 0).  d_h receives the heights
-// (INT32_MAX where unset); d_flags needs 8 words.
-rt_status dm_heights_device(const int32_t* d_t, const int32_t* d_cls, const int32_t* d_dom, int N, int start,
-                            int32_t* d_h, unsigned* d_flags, cudaStream_t st) {
+// Device height function of the host-layout tiling d_t (N x N) for the domain whose vertex and
+// edge flags are d_dom (dm_hf_domain), starting at vertex `start` (height 0).  d_h receives the
+// heights (INT32_MAX where unset); d_flags needs 4 words.
+rt_status dm_heights_device(const int32_t* d_t, const uint8_t* d_dom, int N, int start, int32_t* d_h, unsigned* d_flags,
+                            cudaStream_t st) {
   const int64_t NN = (int64_t)N * N;
-  // every vertex unset, the start vertex at 0
   k_fill_unset<<<(unsigned)((NN + 255) / 256), 256, 0, st>>>(d_h, NN, start);
-  constexpr int kBatch = 8;
-  const dim3 tgrid((N + kTile - 1) / kTile, (N + kTile - 1) / kTile), tblock(kTile, kTile);
-  for (int64_t passes = 0;; passes += kBatch) {
-    if (passes > NN + kBatch) return fail(RT_ERR_TIMEOUT, "height function: propagation did not converge");
-    cudaMemsetAsync(d_flags, 0, kBatch * sizeof(unsigned), st);
-    for (int k = 0; k < kBatch; ++k) pdl_launch(k_hf_tile, tgrid, tblock, st, d_t, d_cls, d_dom, d_h, N, d_flags + k);
-    unsigned last = 1;
-    cudaMemcpyAsync(&last, d_flags + kBatch - 1, sizeof last, cudaMemcpyDeviceToHost, st);
+  k_hf_rows<<<1, 256, 0, st>>>(d_t, d_dom, d_h, N, start / N, 1, d_flags + 3, nullptr);
+  for (int64_t passes = 0;; ++passes) {
+    if (passes > NN) return fail(RT_ERR_TIMEOUT, "height function: propagation did not converge");
+    cudaMemsetAsync(d_flags, 0, 3 * sizeof(unsigned), st);  // columns changed, rows changed, vertices left
+    k_hf_cols<<<(unsigned)((N + 31) / 32), 1024, 0, st>>>(d_t, d_dom, d_h, N, d_flags);
+    k_hf_rows<<<(unsigned)((N + 7) / 8), 256, 0, st>>>(d_t, d_dom, d_h, N, 0, N, d_flags + 1, d_flags + 2);
+    unsigned f[3] = {1, 1, 1};
+    cudaMemcpyAsync(f, d_flags, sizeof f, cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("height function: ") + cudaGetErrorString(e));
-    if (!last) return RT_OK;
+    if (f[2] == 0 || (!f[0] && !f[1])) return RT_OK;  // all set, or what is left is not linked to the start
   }
 }
 
@@ -255,11 +351,11 @@ rt_status dm_heights_accumulate(const int32_t* d_h, int N, long long* sums, cuda
   return e == cudaSuccess ? RT_OK : fail(RT_ERR_CUDA, std::string("height sums: ") + cudaGetErrorString(e));
 }
 
-rt_status dm_classes_device(const int32_t* d_dom, int M, int32_t* d_cls, unsigned* d_count, cudaStream_t st) {
+rt_status dm_hf_domain(const int32_t* d_dom, int M, uint8_t* d_out, cudaStream_t st) {
   const int N = M + 1;
-  k_th_classes<<<dim3((N + 127) / 128, N), 128, 0, st>>>(d_dom, M, d_cls, d_count);
+  k_hf_domain<<<dim3((N + 127) / 128, N), 128, 0, st>>>(d_dom, M, d_out);
   const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? RT_OK : fail(RT_ERR_CUDA, std::string("vertex classes: ") + cudaGetErrorString(e));
+  return e == cudaSuccess ? RT_OK : fail(RT_ERR_CUDA, std::string("vertex flags: ") + cudaGetErrorString(e));
 }
 
 // First boundary vertex in row-major order (the reference's start vertex), or -1.
@@ -433,13 +529,14 @@ RT_API rt_status rt_domino_heightfunc_device(const int32_t* tiling, const int32_
   }
   cudaStream_t st = (cudaStream_t)cuda_stream;
   const size_t NN = (size_t)N * N;
-  int32_t *d_t = nullptr, *d_cls = nullptr, *d_dom = nullptr, *d_h = nullptr;
+  int32_t *d_t = nullptr, *d_dom = nullptr, *d_h = nullptr;
+  uint8_t* d_hf = nullptr;
   unsigned* d_flags = nullptr;
   auto cleanup = [&]() {
-    for (void* p : {(void*)d_t, (void*)d_cls, (void*)d_dom, (void*)d_h, (void*)d_flags})
+    for (void* p : {(void*)d_t, (void*)d_hf, (void*)d_dom, (void*)d_h, (void*)d_flags})
       if (p) cudaFree(p);
   };
-  if (cudaMalloc(&d_t, NN * 4) != cudaSuccess || cudaMalloc(&d_cls, NN * 4) != cudaSuccess ||
+  if (cudaMalloc(&d_t, NN * 4) != cudaSuccess || cudaMalloc(&d_hf, NN) != cudaSuccess ||
       cudaMalloc(&d_dom, (size_t)M * M * 4) != cudaSuccess || cudaMalloc(&d_h, NN * 4) != cudaSuccess ||
       cudaMalloc(&d_flags, 16 * sizeof(unsigned)) != cudaSuccess) {
     cudaGetLastError();
@@ -448,9 +545,8 @@ RT_API rt_status rt_domino_heightfunc_device(const int32_t* tiling, const int32_
   }
   cudaMemcpyAsync(d_t, tiling, NN * 4, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_dom, domain, (size_t)M * M * 4, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(d_flags, 0, 16 * sizeof(unsigned), st);
-  rt_status status = dm_classes_device(d_dom, M, d_cls, d_flags + 8, st);
-  if (status == RT_OK) status = dm_heights_device(d_t, d_cls, d_dom, N, start, d_h, d_flags, st);
+  rt_status status = dm_hf_domain(d_dom, M, d_hf, st);
+  if (status == RT_OK) status = dm_heights_device(d_t, d_hf, N, start, d_h, d_flags, st);
   if (status == RT_OK) {
     cudaMemcpyAsync(out, d_h, NN * 4, cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);

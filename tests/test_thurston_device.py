@@ -90,3 +90,41 @@ def test_sampler_height_sums_equal_host_sums(rt):
     torch.cuda.synchronize()
     assert np.array_equal(sums.cpu().numpy(), host)
     s.close()
+
+
+def _brick_domain(cells):
+    """Domain and tiling of aligned horizontal dominoes: cells[r, c] puts one on squares
+    (r + 1, 2 c + 2) and (r + 1, 2 c + 3)."""
+    rows, cols = cells.shape
+    M = max(rows, 2 * cols) + 4
+    d = np.zeros((M, M), np.int32)
+    t = np.zeros((M + 1, M + 1), np.int32)
+    for r, c in zip(*np.nonzero(cells)):
+        i, j = r + 1, 2 * c + 2
+        d[i, j] = d[i, j + 1] = 1
+        t[i, j + 1] |= 2      # the edge inside the domino, seen from above
+        t[i + 1, j + 1] |= 1  # and from below
+    return d.ravel(), t.ravel()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,kind", [(1, 1, "full"), (1, 70, "full"), (140, 1, "full"), (33, 16, "full"),
+                                            (41, 30, "serpentine"), (37, 33, "sparse"), (64, 64, "sparse"),
+                                            (20, 20, "apart")])
+def test_device_heights_on_winding_and_broken_domains(rt, rows, cols, kind):
+    """Lines of linked vertices broken in every way: a passage that turns back on itself, holes,
+    pieces that touch in a corner or not at all (their heights stay unset, as on the host)."""
+    rng = np.random.default_rng(rows * 1000 + cols)
+    cells = np.ones((rows, cols), bool)
+    if kind == "serpentine":
+        cells[1::2] = False
+        cells[1::4, -1] = True
+        cells[3::4, 0] = True
+    elif kind == "sparse":
+        cells = rng.random((rows, cols)) < 0.6
+        cells[0, 0] = True
+    elif kind == "apart":
+        cells[rows // 2] = False
+    d, t = _brick_domain(cells)
+    D = rt.DominoTiler
+    assert np.array_equal(D.TilingToHeightfuncDevice(t, d), D.TilingToHeightfunc(t, d))
