@@ -11,6 +11,7 @@
 // site of the chosen class whose cycle has one half covered flips with probability 1/2.
 // Same-class cycles are edge-disjoint (the reference's colourings), and two cycles that can
 // flip together share no vertex, so byte read-modify-writes never race.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <curand_kernel.h>
 
@@ -141,6 +142,494 @@ __global__ void k_td_step_fast(uint8_t* D, int M, TdStep s, uint64_t seed, uint3
   }
 }
 
+// ---- the cluster kernel ------------------------------------------------------------------------
+//
+// The dimers as bit planes: per vertex row three planes of 32-bit words (H, L, R), bit k of word w
+// for column 32 w + k.  A step is then a handful of logic operations per word: the cycles of 32
+// sites have their halves covered where the AND of 2-4 shifted plane words is set, the class is a
+// periodic mask, and a flip toggles 4-8 shifted words.  Same-class cycles share no edge, so the
+// words are read and toggled (shared-memory XOR) within one step without order, and one barrier
+// separates steps.
+//
+// The rows live in the shared memory of one thread-block cluster.  A CTA owns the sites of rows
+// [r0, r1) and holds rows r0 - 2 .. r1 (all that its cycles reach); a toggle of a row that a
+// neighbour holds too goes to both copies (XOR through distributed shared memory).
+//
+// Draws.  Fast mode: only quads of columns with a site that can flip need their Philox block, so
+// the step first lists those (about a tenth of them), then draws for the list.  TinyMT: every
+// site's generator is in a register of the lane of its column, a ballot gives a word's acceptance
+// bits, and a step's draws are made between arrival and wait of the barrier before it.
+//
+// Bound: the dependent instructions of a step's two passes and the cluster barrier between steps
+// (its release waits for the toggles across the seams): a third of the issue slots are used.
+// Rhombus 512, fast mode: 2.6 us a step; with one launch per step and a byte per vertex 5.3 us on the
+// device and 7.8 in the call, whose launches the host could not issue faster.
+constexpr int kTdClCtas = 16;
+constexpr int kTdFastThreads = 1024, kTdTmtThreads = 512;  // TinyMT: up to 128 registers a thread
+constexpr int kTdClSlots = 16;                             // TinyMT words a warp
+
+struct TdClArgs {
+  uint8_t* D;  // M x M dimer bytes
+  int M, ctas, f;              // f: the first row of sites
+  int row_start[kTdClCtas + 1];
+  int w0, words;               // words that hold sites
+  uint4* tmt;                  // generators between launches
+  const uint4* tmt_params;
+  uint32_t seed;
+  bool first, last;
+  const uint8_t* sched;        // packed TdStep per step
+  int steps, list_cap;
+  uint64_t fast_seed;
+  uint32_t stream;
+  int64_t h0;
+};
+
+inline uint8_t td_pack_step(const TdStep& s) {
+  return (uint8_t)(s.type | s.r1 << 2 | s.r2 << 4 | s.p1 << 5 | s.p2 << 7);
+}
+__device__ __forceinline__ TdStep td_unpack_step(uint32_t v) {
+  return TdStep{(int)(v & 3u), (int)((v >> 2) & 3u), (int)((v >> 4) & 1u), (int)((v >> 5) & 3u), (int)((v >> 7) & 1u)};
+}
+
+// The cycles of c_cycles, edge by edge: f(half, da, db, plane).
+template <int V>
+struct TdI {
+  static constexpr int v = V;
+};
+template <int kHalf, int kDa, int kDb, int kP, class F>
+__device__ __forceinline__ void td_edge(F& f) {
+  f(TdI<kHalf>{}, TdI<kDa>{}, TdI<kDb>{}, TdI<kP>{});
+}
+template <int C, class F>
+__device__ __forceinline__ void td_edges(F f) {
+  constexpr int H = 0, L = 1, R = 2;
+  if constexpr (C == 0) {
+    td_edge<0, -1, 0, R>(f), td_edge<0, 0, 0, R>(f);
+    td_edge<1, -1, 1, L>(f), td_edge<1, 0, 0, L>(f);
+  } else if constexpr (C == 1) {
+    td_edge<0, -1, 0, H>(f), td_edge<0, 0, -1, H>(f);
+    td_edge<1, 0, 0, R>(f), td_edge<1, 0, -1, R>(f);
+  } else if constexpr (C == 2) {
+    td_edge<0, -1, 0, H>(f), td_edge<0, 0, 0, H>(f);
+    td_edge<1, 0, 1, L>(f), td_edge<1, 0, 0, L>(f);
+  } else if constexpr (C == 3) {
+    td_edge<0, -1, 0, H>(f), td_edge<0, 0, 1, R>(f), td_edge<0, 1, 0, L>(f);
+    td_edge<1, 0, 0, L>(f), td_edge<1, -1, 1, H>(f), td_edge<1, 1, 0, R>(f);
+  } else if constexpr (C == 4) {
+    td_edge<0, 0, -1, H>(f), td_edge<0, 0, 1, L>(f), td_edge<0, -1, 0, R>(f);
+    td_edge<1, 0, -1, R>(f), td_edge<1, 0, 0, H>(f), td_edge<1, -1, 1, L>(f);
+  } else if constexpr (C == 5) {
+    td_edge<0, -1, 0, L>(f), td_edge<0, -2, 1, H>(f), td_edge<0, 0, 1, L>(f), td_edge<0, 0, -1, H>(f);
+    td_edge<1, -2, 0, H>(f), td_edge<1, -1, 1, R>(f), td_edge<1, 0, 0, H>(f), td_edge<1, 0, -1, R>(f);
+  } else if constexpr (C == 6) {
+    td_edge<0, -1, 0, R>(f), td_edge<0, 0, 1, L>(f), td_edge<0, 1, -1, R>(f), td_edge<0, 0, -1, L>(f);
+    td_edge<1, -1, 1, L>(f), td_edge<1, 0, 0, H>(f), td_edge<1, 1, -1, L>(f), td_edge<1, -1, -1, H>(f);
+  } else {
+    td_edge<0, -1, 0, R>(f), td_edge<0, -1, 1, H>(f), td_edge<0, 1, 0, R>(f), td_edge<0, 0, -1, H>(f);
+    td_edge<1, -1, 1, L>(f), td_edge<1, 0, 1, R>(f), td_edge<1, 1, 0, L>(f), td_edge<1, 0, -1, R>(f);
+  }
+}
+// The sites of class s among columns 32 w .. 32 w + 31 of row a (td_in_class); a3, w3: a and w mod 3.
+__device__ __forceinline__ uint32_t td_class_mask(const TdStep& s, int a, int a3, int w3) {
+  auto every3 = [](int x) -> uint32_t { return 0x49249249u << (x - (x >= 3 ? 3 : 0) - (x >= 6 ? 3 : 0)); };  // x < 9
+  auto parity = [](int p) -> uint32_t { return p ? 0xaaaaaaaau : 0x55555555u; };  // (32 w is even, and 32 = 2 mod 3)
+  if (s.type == 0) {
+    if (s.r1 == 0) return (a & 1) == s.r2 ? ~0u : 0u;
+    return parity(s.r1 == 1 ? s.r2 : (s.r2 ^ a) & 1);
+  }
+  if (s.type == 1) return every3(s.r1 + a3 + w3);
+  if (s.r1 == 0) return a3 == s.p1 ? parity(s.p2) : 0u;
+  if (s.r1 == 1) return (a & 1) == s.p2 ? every3(s.p1 + w3) : 0u;
+  return every3(s.p1 + w3 + (a3 ? 3 - a3 : 0)) & parity(s.p2);
+}
+
+__device__ __forceinline__ uint32_t td_remote(const void* p, int rank) {
+  uint32_t r;
+  const uint32_t x = (uint32_t)__cvta_generic_to_shared(p);
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(rank));
+  return r;
+}
+
+// K: TinyMT words a warp (0: fast mode).
+template <int K, bool kParams>
+__global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cluster(const __grid_constant__ TdClArgs a) {
+  extern __shared__ __align__(16) uint32_t tsm[];
+  __shared__ int s_count[2];
+  __shared__ uint32_t s_mask[2][18];
+  constexpr bool kFast = K == 0;
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
+  const int rank = (int)cooperative_groups::this_cluster().block_rank();
+  const int r0 = a.row_start[rank], r1 = a.row_start[rank + 1], rows = r1 - r0, words = a.words, Wp = words + 2;
+  // Window row y is vertex row r0 - 2 + y; word x is column word w0 - 1 + x; planes H, L, R, -.
+  uint32_t* const planes = tsm;
+  uint32_t* const list = tsm + (size_t)(rows + 3) * Wp * 4;
+  auto word = [&](int y, int x, int p) -> uint32_t& { return planes[(y * Wp + x) * 4 + p]; };
+  for (int it = warp; it < (rows + 3) * Wp; it += nwarps) {
+    const int y = it / Wp, x = it - y * Wp, row = r0 - 2 + y, col = 32 * (a.w0 - 1 + x) + lane;
+    const uint32_t v = row >= 0 && row < a.M && col >= 0 && col < a.M ? a.D[(size_t)row * a.M + col] : 0u;
+    const uint32_t h = __ballot_sync(~0u, v & kH), l = __ballot_sync(~0u, v & kL), r = __ballot_sync(~0u, v & kR);
+    if (lane < 4) word(y, x, lane) = lane == 0 ? h : lane == 1 ? l : lane == 2 ? r : 0u;
+  }
+  if (tid < 2) s_count[tid] = 0;
+  const uint32_t self = (uint32_t)__cvta_generic_to_shared(planes);
+  const uint32_t up = rank > 0 ? td_remote(planes, rank - 1) : 0u;
+  const uint32_t dn = rank + 1 < a.ctas ? td_remote(planes, rank + 1) : 0u;
+  const int rows_up = rank > 0 ? r0 - a.row_start[rank - 1] : 0;
+  // XOR (predicated, not branched) into this CTA's copy; where the row is held twice (kSeam), into
+  // the neighbour's too: window rows 0 .. 2 are r0 - 2 and r0 - 1, owned above, and r0, held above;
+  // rows `rows` .. rows + 2 are r1 - 2 and r1 - 1, held below, and r1, owned below.
+  auto toggle_word = [&](auto seam, int y, int x, int p, uint32_t m) {
+    const uint32_t at = (uint32_t)((y * Wp + x) * 4 + p) * 4u;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q red.shared.xor.b32 [%0], %1;\n\t}" ::"r"(self + at),
+                 "r"(m)
+                 : "memory");
+    if constexpr (decltype(seam)::v) {
+      if (m && rank > 0 && y <= 2)
+        asm volatile("red.shared::cluster.xor.b32 [%0], %1;" ::"r"(up + at + (uint32_t)(rows_up * Wp * 16)), "r"(m) : "memory");
+      if (m && rank + 1 < a.ctas && y >= rows)
+        asm volatile("red.shared::cluster.xor.b32 [%0], %1;" ::"r"(dn + at - (uint32_t)(rows * Wp * 16)), "r"(m) : "memory");
+    }
+  };
+  // Sites of the word at `at` whose cycle has a half covered.
+  const int pitch = Wp * 4;
+  auto covered = [&](auto c, const uint32_t* at) -> uint32_t {
+    uint32_t half[2] = {~0u, ~0u};
+    td_edges<decltype(c)::v>([&](auto hf, auto da, auto db, auto p) {
+      constexpr int d = decltype(db)::v;
+      const uint32_t* q = at + decltype(da)::v * pitch + decltype(p)::v;
+      const uint32_t v = *q;
+      if constexpr (d == 0) half[decltype(hf)::v] &= v;
+      else if constexpr (d == 1) half[decltype(hf)::v] &= __funnelshift_r(v, q[4], 1);
+      else half[decltype(hf)::v] &= __funnelshift_l(q[-4], v, 1);
+    });
+    return half[0] | half[1];
+  };
+  auto toggle_in = [&](auto seam, auto c, int y, int x, uint32_t m) {
+    td_edges<decltype(c)::v>([&](auto, auto da, auto db, auto p) {
+      constexpr int d = decltype(db)::v, pl = decltype(p)::v;
+      const int yy = y + decltype(da)::v;
+      if constexpr (d == 0) {
+        toggle_word(seam, yy, x, pl, m);
+      } else if constexpr (d == 1) {
+        toggle_word(seam, yy, x, pl, m << 1);
+        toggle_word(seam, yy, x + 1, pl, m >> 31);
+      } else {
+        toggle_word(seam, yy, x, pl, m >> 1);
+        toggle_word(seam, yy, x - 1, pl, m << 31);
+      }
+    });
+  };
+  // Flips the sites m of row r0 + i, word x (a cycle spans window rows i .. i + 3).
+  auto toggle = [&](auto c, int i, int x, uint32_t m) {
+    if (i > 2 && i < rows - 3) toggle_in(TdI<0>{}, c, i + 2, x, m);
+    else toggle_in(TdI<1>{}, c, i + 2, x, m);
+  };
+  auto by_cycle = [](int c, auto f) {  // c is the same for the whole grid
+    switch (c) {
+      case 0: f(TdI<0>{}); break;
+      case 1: f(TdI<1>{}); break;
+      case 2: f(TdI<2>{}); break;
+      case 3: f(TdI<3>{}); break;
+      case 4: f(TdI<4>{}); break;
+      case 5: f(TdI<5>{}); break;
+      case 6: f(TdI<6>{}); break;
+      default: f(TdI<7>{}); break;
+    }
+  };
+  // An item: row r0 + i, word x; its first plane word and its entry of the class masks.
+  struct Item {
+    int i, x, mask;
+    const uint32_t* at;
+  };
+  auto item_at = [&](int it) -> Item {
+    const int i = it / words, x = 1 + it - i * words;
+    return Item{i, x, ((r0 + i) % 6) * 3 + (a.w0 - 1 + x) % 3, planes + ((i + 2) * Wp + x) * 4};
+  };
+  // Its sites that can flip in this step.  (A cycle with a half covered has all its vertices covered,
+  // so it lies inside the array.)
+  auto sites = [&](int c, int b, const Item& e) -> uint32_t {
+    uint32_t m = s_mask[b][e.mask];
+    if (m) by_cycle(c, [&](auto cc) { m &= covered(cc, e.at); });
+    return m;
+  };
+  // The class masks of a step by (row mod 6, word mod 3), lane l of a warp the l-th.
+  auto make_masks = [&](uint32_t packed, int b) {
+    if (lane < 18) s_mask[b][lane] = td_class_mask(td_unpack_step(packed), lane / 3, lane / 3 % 3, lane % 3);
+  };
+  const int items = rows * words;
+
+  // TinyMT: slot k of a warp is item warp + k * nwarps; lane l keeps the generator of its column l.
+  uint4 gen[kFast ? 1 : K];
+  uint32_t acc = 0u;  // lane k: the acceptance word of slot k
+  auto gen_index = [&](int k, bool* valid) -> int64_t {
+    const int it = warp + k * nwarps, row = r0 + it / words, col = 32 * (a.w0 + it % words) + lane;
+    *valid = it < items && col < a.M;
+    return (int64_t)row * a.M + col;
+  };
+  if constexpr (!kFast) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      bool v;
+      const int64_t g = gen_index(k, &v);
+      gen[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (!v) continue;
+      if (a.first) {
+        const uint4 p = kParams ? a.tmt_params[g] : make_uint4(kTmtMat1, kTmtMat2, kTmtTmat, 0);
+        gen[k] = tmt_seed(a.seed + (uint32_t)g, p.x, p.y, p.z);
+      } else {
+        gen[k] = a.tmt[g];
+      }
+    }
+  }
+  auto draw = [&] {
+    if constexpr (!kFast) {
+      uint32_t mine = 0u;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        uint4 p = make_uint4(kTmtMat1, kTmtMat2, kTmtTmat, 0);
+        if (kParams) {
+          bool v;
+          const int64_t g = gen_index(k, &v);
+          p = __ldg(&a.tmt_params[v ? g : 0]);
+        }
+        // the 23-bit draw is below 2^22: the top bit of the tempered word is clear
+        const uint32_t ok = __ballot_sync(~0u, (int)tmt_next_t0_mad(gen[k], p.x, p.y, p.z) >= 0);
+        mine = lane == k ? ok : mine;
+      }
+      acc = mine;
+    }
+  };
+  const Item first = item_at(min(kFast ? tid : warp + lane * nwarps, items - 1));  // this thread's item in every step
+  if (a.steps > 0) draw();
+  uint32_t step = a.steps > 0 ? __ldg(&a.sched[0]) : 0u, next = a.steps > 1 ? __ldg(&a.sched[1]) : 0u;
+  if (warp == nwarps - 1) make_masks(step, 0);
+  cooperative_groups::this_cluster().sync();  // the windows are loaded
+  for (int s = 0; s < a.steps; ++s) {
+    const int c = td_cycle_of(td_unpack_step(step));
+    step = next;
+    next = s + 2 < a.steps ? __ldg(&a.sched[s + 2]) : 0u;
+    if constexpr (kFast) {
+      // the quads with a site that can flip: (row << 20) | (quad << 4) | sites
+      int* const count = &s_count[s & 1];
+      for (int it0 = warp * 32; it0 < items; it0 += T) {
+        const Item e = it0 < T ? first : item_at(min(it0 + lane, items - 1));
+        const uint32_t m = it0 + lane < items ? sites(c, s & 1, e) : 0u;
+        uint32_t quads = (m | (m >> 1) | (m >> 2) | (m >> 3)) & 0x11111111u;
+        int at = __popc(quads);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int before = __shfl_up_sync(~0u, at, o);
+          if (lane >= o) at += before;
+        }
+        int base = 0;
+        if (lane == 31 && at) base = atomicAdd(count, at);
+        base = __shfl_sync(~0u, base, 31);
+        uint32_t* to = list + base + at - __popc(quads);
+        const uint32_t tag = (uint32_t)e.i << 20 | (uint32_t)e.x << 7;
+        for (; quads; quads &= quads - 1) {
+          const int k = __ffs((int)quads) - 1;
+          *to++ = tag | (uint32_t)k << 2 | ((m >> k) & 15u);
+        }
+      }
+      __syncthreads();
+      const int n = *count;
+      if (tid == 0) s_count[(s + 1) & 1] = 0;
+      if (warp == nwarps - 1) make_masks(step, (s + 1) & 1);
+      for (int e = tid; e < n; e += T) {
+        const uint32_t v = list[e];
+        const int i = (int)(v >> 20), qx = (int)((v >> 4) & 0xffffu), x = qx >> 3, k = qx & 7;
+        const uint4 d = fast_quad(a.fast_seed, a.stream, a.h0 + s, (uint32_t)(r0 + i), (uint32_t)(8 * (a.w0 - 1) + qx));
+        const uint32_t ok = (~d.x >> 31) | ((~d.y >> 31) << 1) | ((~d.z >> 31) << 2) | ((~d.w >> 31) << 3);
+        const uint32_t m = (v & ok & 15u) << (4 * k);
+        if (m) by_cycle(c, [&](auto cc) { toggle(cc, i, x, m); });
+      }
+    } else {
+      if (warp == nwarps - 1) make_masks(step, (s + 1) & 1);
+      const int it = warp + lane * nwarps;
+      if (lane < K && it < items) {
+        const uint32_t m = sites(c, s & 1, first) & acc;
+        if (m) by_cycle(c, [&](auto cc) { toggle(cc, first.i, first.x, m); });
+      }
+      __syncwarp();
+    }
+    const bool more = s + 1 < a.steps;
+    if (a.ctas == 1) {
+      if (more) draw();
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      if (more) draw();
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+  }
+  for (int it = warp; it < rows * words; it += nwarps) {
+    const int i = it / words, x = 1 + it - i * words, col = 32 * (a.w0 - 1 + x) + lane;
+    if (col >= a.M) continue;
+    uint32_t v = 0;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) v |= ((word(i + 2, x, p) >> lane) & 1u) << p;
+    a.D[(size_t)(r0 + i) * a.M + col] = (uint8_t)v;
+  }
+  if constexpr (!kFast) {
+    if (a.last) return;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      bool v;
+      const int64_t g = gen_index(k, &v);
+      if (v) a.tmt[g] = gen[k];
+    }
+  }
+}
+
+// ---- between the reference's tiling format and the dimer bytes, on the device ---------------------
+
+// What k_td_pack finds: bit 0 of flags a state that is not a dimer configuration's, bit 1 two dimers
+// at a vertex, bit 2 a dimer that leaves the array; the rows and columns of the covered vertices; their number by (row, column) mod 6.
+struct TdScan {
+  unsigned flags;
+  int row_lo, row_hi, col_lo, col_hi;
+  unsigned long long by_residue[36];
+};
+
+__device__ __forceinline__ uint32_t td_byte(const int32_t* t, int N, int M, int a, int b) {
+  if (a < 0 || b < 0 || a >= M || b >= M) return 0u;
+  const int eR = t[(size_t)(2 * a + 1) * N + 2 * b + 1], eH = t[(size_t)(2 * a) * N + 2 * b + 1];
+  return ((eR & 4) ? kH : 0) | ((eR & 8) ? kL : 0) | ((eH & 4) ? kR : 0);
+}
+
+// td_from_tiling, and the checks of a walk's input (td_to_tiling gives the tiling back, at most
+// one dimer at a vertex).
+__global__ void k_td_pack(const int32_t* t, int N, uint8_t* D, TdScan* scan) {
+  __shared__ unsigned hist[36];
+  __shared__ int s_lo, s_hi;  // this block's covered columns
+  const int M = N / 2, b = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
+  for (int k = threadIdx.x; k < 36; k += blockDim.x) hist[k] = 0u;
+  if (threadIdx.x == 0) s_lo = M, s_hi = -1;
+  __syncthreads();
+  if (b < M) {
+    auto bit = [&](int y, int x, uint32_t k) -> int { return (td_byte(t, N, M, y, x) & k) ? 1 : 0; };
+    const uint32_t v = td_byte(t, N, M, a, b);
+    D[(size_t)a * M + b] = (uint8_t)v;
+    const int h = (v & kH) ? 1 : 0, l = (v & kL) ? 1 : 0, r = (v & kR) ? 1 : 0;
+    const int nR = bit(a - 1, b, kR), nH = bit(a - 1, b, kH), wH = bit(a, b - 1, kH), wR = bit(a, b - 1, kR);
+    const int eL = bit(a, b + 1, kL), neL = bit(a - 1, b + 1, kL);
+    unsigned flags = 0;
+    if (t[(size_t)(2 * a) * N + 2 * b + 1] != nR + 2 * neL + 4 * r + 8 * l) flags |= 1u;
+    if (t[(size_t)(2 * a + 1) * N + 2 * b] != nH + 2 * r + 4 * wH + 8 * wR) flags |= 1u;
+    if (t[(size_t)(2 * a + 1) * N + 2 * b + 1] != nH + 2 * eL + 4 * h + 8 * l) flags |= 1u;
+    const int cover = h + l + r + wH + bit(a + 1, b, kL) + bit(a + 1, b - 1, kR);
+    if (cover > 1) flags |= 2u;
+    if ((a == 0 && (l || r)) || (b == M - 1 && (h || r))) flags |= 4u;
+    if (flags) atomicOr(&scan->flags, flags);
+    if (cover) {
+      atomicMin(&s_lo, b);
+      atomicMax(&s_hi, b);
+      atomicAdd(&hist[(a % 6) * 6 + b % 6], 1u);
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 36; k += blockDim.x)
+    if (hist[k]) atomicAdd(&scan->by_residue[k], (unsigned long long)hist[k]);
+  if (threadIdx.x == 0 && s_hi >= 0) {
+    atomicMin(&scan->row_lo, a);
+    atomicMax(&scan->row_hi, a);
+    atomicMin(&scan->col_lo, s_lo);
+    atomicMax(&scan->col_hi, s_hi);
+  }
+}
+
+// td_to_tiling on the device (the (even, even) entries stay).
+__global__ void k_td_unpack(const uint8_t* D, int N, int32_t* t) {
+  const int M = N / 2, b = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
+  if (b >= M) return;
+  auto bit = [&](int y, int x, int k) -> int {
+    return (y >= 0 && x >= 0 && y < M && x < M && (D[(size_t)y * M + x] & k)) ? 1 : 0;
+  };
+  const int nH = bit(a - 1, b, kH), r = bit(a, b, kR), l = bit(a, b, kL);
+  t[(size_t)(2 * a) * N + 2 * b + 1] = bit(a - 1, b, kR) + 2 * bit(a - 1, b + 1, kL) + 4 * r + 8 * l;
+  t[(size_t)(2 * a + 1) * N + 2 * b] = nH + 2 * r + 4 * bit(a, b - 1, kH) + 8 * bit(a, b - 1, kR);
+  t[(size_t)(2 * a + 1) * N + 2 * b + 1] = nH + 2 * bit(a, b + 1, kL) + 4 * bit(a, b, kH) + 8 * l;
+}
+
+struct TdClPlan {
+  bool ok = false;
+  int ctas = 0, threads = 0, K = 0, w0 = 0, words = 0, list_cap = 0;
+  int row_start[kTdClCtas + 1] = {};
+  size_t smem = 0;
+  void* kernel = nullptr;
+};
+
+void* td_cluster_kernel(bool fast, bool params, int K) {
+  if (fast) return (void*)k_td_cluster<0, false>;
+  switch (K) {
+    case 1: return params ? (void*)k_td_cluster<1, true> : (void*)k_td_cluster<1, false>;
+    case 2: return params ? (void*)k_td_cluster<2, true> : (void*)k_td_cluster<2, false>;
+    case 4: return params ? (void*)k_td_cluster<4, true> : (void*)k_td_cluster<4, false>;
+    case 8: return params ? (void*)k_td_cluster<8, true> : (void*)k_td_cluster<8, false>;
+    default: return params ? (void*)k_td_cluster<16, true> : (void*)k_td_cluster<16, false>;
+  }
+}
+
+// Words of sites up to which one CTA is faster than a cluster and its barrier.
+constexpr int kTdOneCta = 64;
+
+TdClPlan td_cluster_plan(const TdScan& sc, bool fast, bool params) {
+  TdClPlan p;
+  if (sc.row_hi < sc.row_lo || sc.flags) return p;
+  const int rows = sc.row_hi - sc.row_lo + 1;
+  p.w0 = sc.col_lo / 32;
+  p.words = sc.col_hi / 32 - p.w0 + 1;
+  p.ctas = (int64_t)rows * p.words <= kTdOneCta ? 1 : std::max(1, std::min(kTdClCtas, rows / 3));
+  int rows_max = 0;
+  for (int k = 0; k <= p.ctas; ++k) p.row_start[k] = sc.row_lo + (int)((int64_t)rows * k / p.ctas);
+  for (int k = 0; k < p.ctas; ++k) rows_max = std::max(rows_max, p.row_start[k + 1] - p.row_start[k]);
+  const int64_t items = (int64_t)rows_max * p.words;
+  p.smem = (size_t)(rows_max + 3) * (p.words + 2) * 16;
+  if (fast) {
+    p.list_cap = (int)std::min<int64_t>(items * 8, 1 << 20);
+    p.smem += (size_t)p.list_cap * sizeof(uint32_t);
+    p.threads = items > 128 ? kTdFastThreads : 256;
+    if (rows_max > 4095 || p.words + 2 > 8191) return p;
+  } else {
+    const int64_t K = (items + kTdTmtThreads / 32 - 1) / (kTdTmtThreads / 32);
+    if (K > kTdClSlots) return p;
+    p.K = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+    p.threads = K <= 1 ? (int)items * 32 : kTdTmtThreads;
+  }
+  p.kernel = td_cluster_kernel(fast, params, p.K);
+  if (p.smem > 200 * 1024) return p;
+  if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return p;
+  }
+  p.ok = true;
+  return p;
+}
+
+struct TdClLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  TdClLaunch(const TdClPlan& p, cudaStream_t st) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)p.ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)p.ctas);
+    cfg.blockDim = dim3((unsigned)p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+  }
+  bool fits(const TdClPlan& p) {
+    int clusters = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, p.kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
+  }
+};
+
 // Philox4x32-10 on the host (the fast-mode step schedule).
 void philox_host(uint32_t c[4], uint32_t k0, uint32_t k1) {
   for (int r = 0; r < 10; ++r) {
@@ -199,6 +688,20 @@ std::vector<int> td_cover(const uint8_t* D, int M) {
       if (v & kR) add(a, b), add(a - 1, b + 1);
     }
   return c;
+}
+
+// The checks of k_td_pack on the host, for an input refused before a missing device is.
+rt_status td_check_host(const int32_t* tiling, int N) {
+  const int M = N / 2;
+  std::vector<uint8_t> D((size_t)M * M);
+  td_from_tiling(tiling, N, D.data());
+  std::vector<int32_t> back(tiling, tiling + (size_t)N * N);
+  td_to_tiling(D.data(), N, back.data());
+  if (!std::equal(back.begin(), back.end(), tiling))
+    return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: tiling states are not those of a dimer configuration");
+  for (int v : td_cover(D.data(), M))
+    if (v > 1) return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: two dimers share a vertex");
+  return RT_OK;
 }
 
 }  // namespace
@@ -438,44 +941,61 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   if (o.tinymt_params && o.rng_mode != RT_RNG_TINYMT)
     return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: a TinyMT parameter table needs the TinyMT mode");
   const int N = n_side, M = N / 2;
-  std::vector<uint8_t> D((size_t)M * M);
-  td_from_tiling(tiling, N, D.data());
-  {
-    // the state must be a dimer covering of its vertex set, and must round-trip
-    std::vector<int32_t> back((size_t)N * N, 0);
-    for (size_t p = 0; p < back.size(); ++p) back[p] = tiling[p];
-    td_to_tiling(D.data(), N, back.data());
-    for (size_t p = 0; p < back.size(); ++p)
-      if (back[p] != tiling[p]) return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: tiling states are not those of a dimer configuration");
-    for (int v : td_cover(D.data(), M))
-      if (v > 1) return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: two dimers share a vertex");
-  }
   int devs = 0;
   if (cudaGetDeviceCount(&devs) != cudaSuccess || devs == 0) {
     cudaGetLastError();
+    if (rt_status cs = td_check_host(tiling, N)) return cs;
     return fail(RT_ERR_CUDA, "no CUDA device: the sweep has no CPU fallback");
   }
-  // flip attempts: sites of each class whose cycle anchor is a covered vertex
-  std::vector<int> cover = td_cover(D.data(), M);
   cudaStream_t st = (cudaStream_t)o.cuda_stream;
+  const bool fast = o.rng_mode == RT_RNG_FAST;
+  const size_t cells = (size_t)N * N;
+  int32_t* d_t = nullptr;
   uint8_t* dD = nullptr;
+  TdScan* d_scan = nullptr;
+  uint8_t* d_sched = nullptr;
   uint4 *tmt = nullptr, *tmt_params = nullptr;
   void* mtgp = nullptr;
   const MtgpGrid mg = mtgp_grid(M, M);
   auto cleanup = [&]() {
-    if (dD) cudaFree(dD);
-    if (tmt) cudaFree(tmt);
+    for (void* q : {(void*)d_t, (void*)dD, (void*)d_scan, (void*)d_sched, (void*)tmt, mtgp}) dev_free(q, st);
     if (tmt_params) cudaFree(tmt_params);
-    if (mtgp) cudaFree(mtgp);
   };
-  if (cudaMalloc(&dD, D.size()) != cudaSuccess ||
-      (o.rng_mode == RT_RNG_TINYMT && cudaMalloc(&tmt, (size_t)M * M * sizeof(uint4)) != cudaSuccess) ||
-      (o.rng_mode == RT_RNG_MTGP && cudaMalloc(&mtgp, mtgp_state_bytes(mg.count())) != cudaSuccess)) {
-    cudaGetLastError();
+  auto out_of_memory = [&]() {
     cleanup();
     return fail(RT_ERR_OUT_OF_MEMORY, "bibone walk: device allocation failed");
+  };
+  if (dev_alloc(&d_t, cells * sizeof(int32_t), st) || dev_alloc(&dD, (size_t)M * M, st) ||
+      dev_alloc(&d_scan, sizeof(TdScan), st))
+    return out_of_memory();
+  TdScan scan{};
+  scan.row_lo = scan.col_lo = M;
+  scan.row_hi = scan.col_hi = -1;
+  cudaMemcpyAsync(d_t, tiling, cells * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(d_scan, &scan, sizeof scan, cudaMemcpyHostToDevice, st);
+  const dim3 g_all((M + 127) / 128, M), g_quad(((M + 3) / 4 + 31) / 32, (M + 7) / 8);
+  k_td_pack<<<g_all, 128, 0, st>>>(d_t, N, dD, d_scan);
+  cudaMemcpyAsync(&scan, d_scan, sizeof scan, cudaMemcpyDeviceToHost, st);
+  const cudaError_t pe = cudaStreamSynchronize(st);
+  if (pe != cudaSuccess) {
+    cleanup();
+    return fail(RT_ERR_CUDA, std::string("bibone walk: ") + cudaGetErrorString(pe));
   }
-  cudaMemcpyAsync(dD, D.data(), D.size(), cudaMemcpyHostToDevice, st);
+  if (scan.flags & 3u) {
+    cleanup();
+    return fail(RT_ERR_INVALID_ARGUMENT, (scan.flags & 1u) ? "bibone walk: tiling states are not those of a dimer configuration"
+                                                           : "bibone walk: two dimers share a vertex");
+  }
+  TdClPlan plan;
+  if (o.rng_mode != RT_RNG_MTGP && steps > 0) plan = td_cluster_plan(scan, fast, o.tinymt_params != nullptr);
+  TdClLaunch launch(plan, st);
+  const bool in_cluster = plan.ok && launch.fits(plan);
+  constexpr int64_t chunk_max = (int64_t)1 << 20;  // steps of a cluster launch
+  if ((o.rng_mode == RT_RNG_TINYMT && (!in_cluster || steps > chunk_max) &&
+       dev_alloc(&tmt, (size_t)M * M * sizeof(uint4), st)) ||
+      (in_cluster && dev_alloc(&d_sched, (size_t)steps, st)) ||
+      (o.rng_mode == RT_RNG_MTGP && dev_alloc(&mtgp, mtgp_state_bytes(mg.count()), st)))
+    return out_of_memory();
   if (o.rng_mode == RT_RNG_TINYMT) {
     if (rt_status ps = tmt_param_table(o, (int64_t)M * M, &tmt_params, st)) {
       cleanup();
@@ -501,7 +1021,7 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  if (o.rng_mode == RT_RNG_TINYMT) {
+  if (o.rng_mode == RT_RNG_TINYMT && !in_cluster) {
     const int64_t count = (int64_t)M * M;
     k_td_seed<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(tmt, tmt_params, count, (uint32_t)seed);
   } else if (o.rng_mode == RT_RNG_MTGP) {
@@ -513,9 +1033,37 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
       return ms;
     }
   }
+  std::vector<uint8_t> packed;
+  if (in_cluster) {
+    packed.resize((size_t)steps);
+    for (int64_t h = 0; h < steps; ++h) packed[(size_t)h] = td_pack_step(sched[(size_t)h]);
+    cudaMemcpyAsync(d_sched, packed.data(), packed.size(), cudaMemcpyHostToDevice, st);
+  }
+  cudaError_t le = cudaSuccess;
   cudaEventRecord(e0, st);
-  const dim3 g_all((M + 127) / 128, M), g_quad(((M + 3) / 4 + 31) / 32, (M + 7) / 8);
-  for (int64_t h = 0; h < steps; ++h) {
+  for (int64_t s0 = 0; in_cluster && s0 < steps && le == cudaSuccess; s0 += chunk_max) {
+    TdClArgs a{};
+    a.D = dD;
+    a.M = M;
+    a.ctas = plan.ctas;
+    std::copy(plan.row_start, plan.row_start + kTdClCtas + 1, a.row_start);
+    a.w0 = plan.w0;
+    a.words = plan.words;
+    a.tmt = tmt;
+    a.tmt_params = tmt_params;
+    a.seed = (uint32_t)seed;
+    a.first = s0 == 0;
+    a.steps = (int)std::min(chunk_max, steps - s0);
+    a.last = s0 + a.steps >= steps;
+    a.sched = d_sched + s0;
+    a.list_cap = plan.list_cap;
+    a.fast_seed = (uint64_t)seed;
+    a.stream = o.fast_stream;
+    a.h0 = s0;
+    void* args[] = {&a};
+    le = cudaLaunchKernelExC(&launch.cfg, plan.kernel, args);
+  }
+  for (int64_t h = 0; !in_cluster && h < steps; ++h) {
     if (o.rng_mode == RT_RNG_TINYMT)
       pdl_launch(k_td_step_tmt, g_all, dim3(128), st, dD, tmt, (const uint4*)tmt_params, M, sched[(size_t)h]);
     else if (o.rng_mode == RT_RNG_MTGP)
@@ -525,8 +1073,9 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
       pdl_launch(k_td_step_fast, g_quad, dim3(32, 8), st, dD, M, sched[(size_t)h], (uint64_t)seed, o.fast_stream, h);
   }
   cudaEventRecord(e1, st);
-  cudaError_t le = cudaGetLastError();
-  cudaMemcpyAsync(D.data(), dD, D.size(), cudaMemcpyDeviceToHost, st);
+  k_td_unpack<<<g_all, 128, 0, st>>>(dD, N, d_t);
+  if (le == cudaSuccess) le = cudaGetLastError();
+  if (le == cudaSuccess) cudaMemcpyAsync(tiling, d_t, cells * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
   const cudaError_t se = cudaStreamSynchronize(st);
   float ms = 0.f;
   if (se == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -535,18 +1084,18 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   cleanup();
   if (le != cudaSuccess || se != cudaSuccess)
     return fail(RT_ERR_CUDA, std::string("bibone walk: ") + cudaGetErrorString(le != cudaSuccess ? le : se));
-  td_to_tiling(D.data(), N, tiling);
   if (stats) {
     std::memset(stats, 0, sizeof *stats);
-    // per class, the sites whose anchor vertex is covered
+    // per class, the sites whose anchor vertex is covered: the classes have periods 2 and 3
     int64_t attempts = 0;
     std::vector<int64_t> per_class(3 * 3 * 2 * 3 * 2, -1);
     for (const TdStep& s : sched) {
       const size_t key = (((size_t)s.type * 3 + s.r1) * 2 + s.r2) * 6 + (s.type == 2 ? s.p1 * 2 + s.p2 : 0);
       if (per_class[key] < 0) {
         int64_t c = 0;
-        for (int a = 0; a < M; ++a)
-          for (int b = 0; b < M; ++b) c += cover[(size_t)a * M + b] && td_in_class(s, a, b);
+        for (int a = 0; a < 6; ++a)
+          for (int b = 0; b < 6; ++b)
+            if (td_in_class(s, a, b)) c += (int64_t)scan.by_residue[a * 6 + b];
         per_class[key] = c;
       }
       attempts += per_class[key];
