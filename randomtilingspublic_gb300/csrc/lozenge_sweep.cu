@@ -14,6 +14,7 @@
 #include <curand_kernel.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -21,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "lozenge_bits.h"
 #include "lozenge_resident.h"
 #include "pdl.cuh"
 #include "rng.cuh"
@@ -169,6 +171,46 @@ __global__ void k_lz_update_w(LzView v, int r) {
   }
 }
 
+// Scan of a host-layout tiling in device memory.  scan[0]: bit 0 a value above 63, bit 1 an edge whose
+// two endpoints disagree (or that leaves the array), bit 2 a vertex that can flip beside one that the
+// reference never rebuilds.  cand: each row's first and last slot of such a vertex (all six triangles
+// around it covered).  scan[1 + c]: their number in colour c = (j - i) mod 3.
+__global__ void k_lz_scan(const int32_t* t, int N, int* cand, unsigned long long* scan, int count) {
+  __shared__ unsigned inside[3];
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y, M = N / 3;
+  if (threadIdx.x < 3) inside[threadIdx.x] = 0u;
+  __syncthreads();
+  unsigned f = 0;
+  int lo = INT_MAX, hi = -1;
+  if (j < N) {
+    auto at = [&](int y, int x) -> int { return y >= 0 && x >= 0 && y < N && x < N ? t[(size_t)y * N + x] : 0; };
+    const int v = at(i, j);
+    if ((uint32_t)v > 63u) f |= 1u;
+    if (((v >> 3) & 1) != ((at(i, j + 1) >> 2) & 1) || ((v >> 1) & 1) != ((at(i - 1, j + 1) >> 4) & 1) ||
+        (v & 1) != ((at(i - 1, j) >> 5) & 1) || ((v >> 2) & 1) != ((at(i, j - 1) >> 3) & 1) ||
+        ((v >> 4) & 1) != ((at(i + 1, j - 1) >> 1) & 1) || ((v >> 5) & 1) != (at(i + 1, j) & 1))
+      f |= 2u;
+    // triangles A(y, x) of (y, x), (y, x+1), (y-1, x+1) and B(y, x) of (y, x), (y-1, x), (y-1, x+1)
+    auto A = [&](int y, int x) { return (at(y, x) & 10) || (at(y, x + 1) & 1); };
+    auto B = [&](int y, int x) { return (at(y, x) & 3) || (at(y - 1, x) & 8); };
+    if (A(i, j) && B(i, j) && A(i, j - 1) && A(i + 1, j - 1) && B(i + 1, j - 1) && B(i + 1, j)) {
+      lo = hi = j / 3;
+      if (i < 2 || i > N - 3 || (j - 1) / 3 < 1 || j < 4 || (j + 1) / 3 > M - 2) f |= 4u;
+      if (count) atomicAdd(&inside[((j - i) % 3 + 3) % 3], 1u);
+    }
+  }
+  f = __reduce_or_sync(0xffffffffu, f);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    if (f) atomicOr(reinterpret_cast<unsigned*>(&scan[0]), f);
+    if (lo != INT_MAX) atomicMin(&cand[i], lo);
+    if (hi >= 0) atomicMax(&cand[N + i], hi);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3 && inside[threadIdx.x]) atomicAdd(&scan[1 + threadIdx.x], (unsigned long long)inside[threadIdx.x]);
+}
+
 __global__ void k_lz_split(LzView v, int ch, const int32_t* t) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
   if (j >= v.N) return;
@@ -276,15 +318,18 @@ struct LzSampler {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::unique_ptr<LzResidentState> res;  // the resident engine for `res_nch` swept chains
   int res_nch = 0;
+  std::unique_ptr<LbState> bits;  // the bit-plane engine for its nch swept chains
+  int* d_cand = nullptr;          // [2][N]: first (INT_MAX: none) and last slot that can flip, over the loaded chains
+  unsigned long long* d_scan = nullptr;
+  bool consistent = true, border = false, cand_dirty = true;
+  std::vector<int> cand_lo, cand_hi;
 
   ~LzSampler() {
     res.reset();
-    if (base) cudaFree(base);
-    if (tmt) cudaFree(tmt);
+    bits.reset();
+    for (void* p : {(void*)base, (void*)tmt, mtgp, (void*)scratch, (void*)counter, (void*)d_cand, (void*)d_scan})
+      dev_free(p, stream);
     if (tmt_params) cudaFree(tmt_params);
-    if (mtgp) cudaFree(mtgp);
-    if (scratch) cudaFree(scratch);
-    if (counter) cudaFree(counter);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (own_stream && stream) cudaStreamDestroy(stream);
@@ -331,15 +376,25 @@ struct LzSampler {
     }
     LZ_CUDA(cudaEventCreate(&s->ev0));
     LZ_CUDA(cudaEventCreate(&s->ev1));
-    LZ_CUDA(cudaMalloc(&s->base, s->chain_stride * chains));
+    // pool allocations, ordered on the sampler's stream (device_pool.cpp)
+    if (rt_status st = dev_alloc(&s->base, s->chain_stride * chains, s->stream)) return st;
     LZ_CUDA(cudaMemsetAsync(s->base, 0, s->chain_stride * chains, s->stream));
-    LZ_CUDA(cudaMalloc(&s->scratch, (size_t)s->N * s->N * sizeof(int32_t)));
-    LZ_CUDA(cudaMalloc(&s->counter, sizeof(unsigned long long)));
+    if (rt_status st = dev_alloc(&s->scratch, (size_t)s->N * s->N * sizeof(int32_t), s->stream)) return st;
+    if (rt_status st = dev_alloc(&s->counter, sizeof(unsigned long long), s->stream)) return st;
+    if (rt_status st = dev_alloc(&s->d_scan, 4 * sizeof(unsigned long long), s->stream)) return st;
+    if (rt_status st = dev_alloc(&s->d_cand, 2 * (size_t)s->N * sizeof(int), s->stream)) return st;
+    {
+      std::vector<int> init(2 * (size_t)s->N, -1);
+      std::fill(init.begin(), init.begin() + s->N, INT_MAX);
+      LZ_CUDA(cudaMemcpyAsync(s->d_cand, init.data(), init.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
+    }
     if (o.rng_mode == RT_RNG_TINYMT) {
-      LZ_CUDA(cudaMalloc(&s->tmt, (size_t)s->N * s->M * sizeof(uint4)));
+      if (rt_status st = dev_alloc(&s->tmt, (size_t)s->N * s->M * sizeof(uint4), s->stream)) return st;
       if (rt_status st = tmt_param_table(o, (int64_t)s->N * s->M, &s->tmt_params, s->stream)) return st;
     }
-    if (o.rng_mode == RT_RNG_MTGP) LZ_CUDA(cudaMalloc(&s->mtgp, mtgp_state_bytes(mtgp_grid(s->N, s->M).count())));
+    if (o.rng_mode == RT_RNG_MTGP) {
+      if (rt_status st = dev_alloc(&s->mtgp, mtgp_state_bytes(mtgp_grid(s->N, s->M).count()), s->stream)) return st;
+    }
     *out = std::move(s);
     return RT_OK;
   }
@@ -361,19 +416,61 @@ struct LzSampler {
     *out = res.get();
     return RT_OK;
   }
-  rt_status resident_error() { return res ? lz_resident_error(*res, stream) : RT_OK; }
+  rt_status resident_error() {
+    if (bits) {
+      if (rt_status st = lb_error(*bits, stream)) return st;
+    }
+    return res ? lz_resident_error(*res, stream) : RT_OK;
+  }
+  // The bit-plane engine for the swept chains (engine 0) where it holds the size and the tilings'
+  // edges agree; NULL: the resident or per-step kernels.
+  rt_status bit_engine(LbState** out) {
+    *out = nullptr;
+    if (opts.engine != 0 || opts.rng_mode == RT_RNG_MTGP || !consistent || border) return RT_OK;
+    if (cand_dirty) {
+      std::vector<int> both(2 * (size_t)N);
+      LZ_CUDA(cudaMemcpyAsync(both.data(), d_cand, both.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
+      LZ_CUDA(cudaStreamSynchronize(stream));
+      cand_lo.assign(both.begin(), both.begin() + N);
+      cand_hi.assign(both.begin() + N, both.end());
+      for (int& v : cand_lo) v = v == INT_MAX ? -1 : v;
+      cand_dirty = false;
+      bits.reset();
+    }
+    if (!bits || bits->nch != active) {
+      bits = std::make_unique<LbState>();
+      bits->nch = active;
+      bits->plan = lb_plan(geom(), LzResidentRule{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn}, cand_lo, cand_hi,
+                           opts.rng_mode == RT_RNG_TINYMT, tmt_params != nullptr);
+    }
+    if (bits->plan.ok) *out = bits.get();
+    return RT_OK;
+  }
   rt_status check() {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     return RT_OK;
   }
   rt_status load(int ch, const int32_t* t) {
-    for (size_t p = 0; p < (size_t)N * N; ++p)
-      if ((uint32_t)t[p] > 63u) return fail(RT_ERR_INVALID_ARGUMENT, "lozenge tiling values must be edge masks in [0, 63]");
+    LZ_CUDA(cudaMemcpyAsync(scratch, t, (size_t)N * N * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+    LZ_CUDA(cudaMemsetAsync(d_scan, 0, 4 * sizeof(unsigned long long), stream));
+    k_lz_scan<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(scratch, N, d_cand, d_scan, ch == 0);
+    unsigned long long h[4] = {0, 0, 0, 0};
+    LZ_CUDA(cudaMemcpyAsync(h, d_scan, sizeof h, cudaMemcpyDeviceToHost, stream));
+    LZ_CUDA(cudaStreamSynchronize(stream));
+    if (h[0] & 1u) return fail(RT_ERR_INVALID_ARGUMENT, "lozenge tiling values must be edge masks in [0, 63]");
+    consistent = consistent && !(h[0] & 2u);
+    border = border || (h[0] & 4u);
+    cand_dirty = true;
     if (ch == 0) {
       // Interior vertices per colour (all six triangles covered): the flip attempts of one step.
-      std::vector<int32_t> dom((size_t)2 * (N - 1) * (N - 1)), cls((size_t)N * N);
-      if (rt_lozenge_tiling_to_domain(t, N, dom.data()) == RT_OK &&
+      for (int c = 0; c < 3; ++c) interior[c] = (int64_t)h[1 + c];
+      std::vector<int32_t> dom, cls;
+      if (h[0] & 2u) {  // not a tiling: as the host's walk over its domain counts
+        dom.resize((size_t)2 * (N - 1) * (N - 1));
+        cls.resize((size_t)N * N);
+      }
+      if (!dom.empty() && rt_lozenge_tiling_to_domain(t, N, dom.data()) == RT_OK &&
           rt_lozenge_domain_to_vertices(dom.data(), N - 1, cls.data()) == RT_OK) {
         for (int c = 0; c < 3; ++c) interior[c] = 0;
         for (int i = 0; i < N; ++i)
@@ -382,7 +479,6 @@ struct LzSampler {
       }
       clear_error();
     }
-    LZ_CUDA(cudaMemcpyAsync(scratch, t, (size_t)N * N * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
     k_lz_split<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(view(), ch, scratch);
     return check();
   }
@@ -426,6 +522,15 @@ struct LzSampler {
       }
       return check();
     }
+    LbState* lb = nullptr;
+    if (rt_status st = bit_engine(&lb)) return st;
+    if (lb) {
+      const LzResidentRule rr{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn};
+      if (rt_status st = lb_run(*lb, geom(), base, rr, true, tmt, tmt_params, d_cand, colours, steps, 0, 0, 0, stream))
+        return st;
+      for (int64_t s = 0; s < steps; ++s) steps_by_colour[colours[s]]++;
+      return RT_OK;
+    }
     LzResidentState* rs = nullptr;
     if (rt_status st = resident(&rs)) return st;
     if (rs) {
@@ -445,6 +550,16 @@ struct LzSampler {
     return check();
   }
   rt_status run_fast(uint64_t seed_value, int64_t h0, int64_t steps) {
+    LbState* lb = nullptr;
+    if (rt_status st = bit_engine(&lb)) return st;
+    if (lb) {
+      const LzResidentRule rr{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn};
+      if (rt_status st = lb_run(*lb, geom(), base, rr, false, nullptr, nullptr, d_cand, nullptr, steps, seed_value,
+                                opts.fast_stream, h0, stream))
+        return st;
+      for (int64_t s = 0; s < steps; ++s) steps_by_colour[(((h0 + s) % 3) + 3) % 3]++;
+      return RT_OK;
+    }
     LzResidentState* rs = nullptr;
     if (rt_status st = resident(&rs)) return st;
     if (rs) {
