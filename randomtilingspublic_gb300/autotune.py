@@ -25,10 +25,10 @@ THREADS = (512, 640, 768, 896, 960, 992, 1024)
 
 def candidates(sms: int) -> list[tuple[int, int, int]]:
     """(engine, bands, threads): the per-half-sweep kernels, k_persist, the run kernel over
-    bands and threads per band, the bit-plane kernel (TinyMT only; its threads follow from
-    its plan) over bands, and its form in one thread-block cluster (engine 0 with the
-    cluster's CTAs as bands)."""
-    out = [(1, 0, 0), (3, 0, 0), (0, 1, 0), (0, 4, 0), (0, 16, 0)]
+    bands and threads per band, the band form of the bit-plane kernel with polled
+    deltas (engine 4, TinyMT only), and the bit-plane kernel in one thread-block cluster or
+    with one band per SM (engine 0 with the bands asked for)."""
+    out = [(1, 0, 0), (3, 0, 0), (0, 1, 0), (0, 4, 0), (0, 16, 0), (0, sms, 0)]
     for bands in sorted({sms, (3 * sms) // 4, sms // 2}, reverse=True):
         out.append((4, bands, 0))
         for threads in THREADS:
@@ -58,8 +58,8 @@ def measure(rt, n, chains, rng, tmax, tmin, shape, half_sweeps: int = 256, reps:
         except rt.RTError:
             return None
         engine, bands, threads = shape
-        if engine == 0:  # the cluster form, reported as the bit-plane kernel
-            if info["engine"] != 4 or info["bands"] > bands:
+        if engine == 0:  # the cluster and grid forms, reported as the bit-plane kernel
+            if info["engine"] != 4 or info["bands"] > bands or (bands > 16) != (info["bands"] > 16):
                 return None
             engine = 4
         if info["engine"] != engine or (engine == 2 and info["threads"] != threads):

@@ -40,16 +40,13 @@
 #include <vector>
 
 #include "domino_cluster.h"
+#include "domino_planes.cuh"
 #include "domino_sweep.h"
 #include "rng.cuh"
 
 namespace rt {
 
 namespace {
-
-constexpr int kClPad = 16;  // words of the scratch word and its neighbours
-
-enum : int { kClTmt = 0, kClTmtParams = 1, kClFast = 2 };
 
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -82,36 +79,6 @@ __device__ __forceinline__ void cl_bar_expect_if(bool on, uint32_t bar, uint32_t
       "r"(bytes), "r"((uint32_t)on)
       : "memory");
 }
-__device__ __forceinline__ uint32_t cl_lds(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint2 cl_lds2(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint4 cl_lds4(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(a)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ void cl_sts(uint32_t a, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void cl_xor(uint32_t a, uint32_t v) {
-  asm volatile("red.shared.xor.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void cl_xor_if(uint32_t a, uint32_t v) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p red.shared.xor.b32 [%0], %1;\n\t}" ::"r"(a), "r"(v)
-               : "memory");
-}
-// The CTA's barrier, met by the update warps and the draw warps at places of their own.
-__device__ __forceinline__ void cl_cta_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
 // Bounded wait for the phase of the given parity; false when it gave up.
 __device__ __forceinline__ bool cl_bar_wait(uint32_t addr, uint32_t parity, long max_spin) {
   for (long it = 0; it <= max_spin; ++it) {
@@ -124,11 +91,6 @@ __device__ __forceinline__ bool cl_bar_wait(uint32_t addr, uint32_t parity, long
     if (done) return true;
   }
   return false;
-}
-
-// Bits a, b, c, d from the least significant up.
-__device__ __forceinline__ uint32_t cl_nibble(bool a, bool b, bool c, bool d) {
-  return (a ? 1u : 0u) | (b ? 2u : 0u) | (c ? 4u : 0u) | (d ? 8u : 0u);
 }
 
 // kSlots: words per draw warp (TinyMT: their generators are in registers); UI: words and chains
@@ -203,23 +165,8 @@ __global__ void __launch_bounds__(cl_max_threads(kMode == kClFast, KS), 1) k_clu
       sslot[(first + at / per) * KS + at % per] = make_uint2(((uint32_t)i << 16) | (uint32_t)w, valid);
     }
   }
-  // The CTA's window of the chains at src as planes (one warp per row and word: lane l reads
-  // cell 32 w + l of both colours).
   auto load_band = [&](const uint8_t* src) {
-    for (int it = warp; it < R * wn; it += nwarps) {
-      const int ri = it / wn, wi = it - ri * wn;
-      const int i = r0 - 1 + ri, w = wlo + wi, m = 32 * w + lane;
-      const bool in = i >= 0 && w >= 0 && m < a.P;
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        const uint8_t* row = src + (size_t)c * a.chain_stride + (size_t)i * a.P;
-        const uint32_t b0 = in ? row[m] : 0u, b1 = in ? row[a.colour_stride + m] : 0u;
-        const uint32_t bo = (i & 1) ? b1 : b0;  // the colour whose cells sit at odd lattice columns
-        const uint32_t vd0 = __ballot_sync(~0u, (b0 >> 1) & 1u), vd1 = __ballot_sync(~0u, (b1 >> 1) & 1u);
-        const uint32_t he = __ballot_sync(~0u, (bo >> 2) & 1u), ho = __ballot_sync(~0u, (bo >> 3) & 1u);
-        if (lane < 4) *PL(ri, lane, wi, c) = lane == 0 ? vd0 : lane == 1 ? vd1 : lane == 2 ? he : ho;
-      }
-    }
+    cl_load_window<NCH>(sm, src, a.chain_stride, a.colour_stride, a.P, r0 - 1, R, wlo, wn);
   };
   const bool cftp = a.attempts > 0;
   if (!cftp) load_band(a.base);
@@ -315,8 +262,6 @@ __global__ void __launch_bounds__(cl_max_threads(kMode == kClFast, KS), 1) k_clu
       tm = p.z;
     }
   };
-  // The moves of a run, one pair of words per slot: bit k of x (y) is set where cell k, in state 3
-  // (12) at the start of the run, is in state 3 at its end.  They do not depend on the state.
   auto draw_run = [&](uint32_t run, int64_t h, uint32_t reseed_to, uint2* out) {
     const uint4 rl = srule[par | ((int)(run >> 31) << 1)];
     if constexpr (!kFast) {
@@ -330,57 +275,12 @@ __global__ void __launch_bounds__(cl_max_threads(kMode == kClFast, KS), 1) k_clu
           if (v) gen[s] = tmt_seed(reseed_to + (uint32_t)g, m1, m2, tm);
         }
       }
-      const int L = (int)(run & 0x3fffffffu);
-      // Every lane composes the moves of all its warp's words (two logic operations a word) where
-      // registers allow it, else lane s those of slot s (two selects more).
-      constexpr bool kAll = KS <= 4;
-      uint32_t x[kAll ? KS : 1], y[kAll ? KS : 1];
-#pragma unroll
-      for (int s = 0; s < (kAll ? KS : 1); ++s) x[s] = 0xffffffffu, y[s] = 0u;
-      for (int hh = 0; hh < L; ++hh) {
-        uint32_t um = 0u, dm = 0u;
-#pragma unroll
-        for (int s = 0; s < KS; ++s) {
-          uint32_t m1, m2, tm;
-          params_of(s, m1, m2, tm);
-          const uint32_t t0 = tmt_next_t0_mad(gen[s], m1, m2, tm);
-          const uint32_t bu = __ballot_sync(~0u, t0 < rl.x);
-          const uint32_t bd = __ballot_sync(~0u, t0 - rl.y < rl.z);
-          if constexpr (kAll) {
-            x[s] ^= (x[s] & bu) | (~x[s] & bd);
-            y[s] ^= (y[s] & bu) | (~y[s] & bd);
-          } else {
-            um = lane == s ? bu : um;
-            dm = lane == s ? bd : dm;
-          }
-        }
-        if constexpr (!kAll) {
-          x[0] ^= (x[0] & um) | (~x[0] & dm);
-          y[0] ^= (y[0] & um) | (~y[0] & dm);
-        }
-      }
-      if constexpr (kAll) {
-#pragma unroll
-        for (int s = 0; s < KS; ++s)
-          if (lane == s) out[warp * KS + s] = make_uint2(x[s], y[s]);
-      } else {
-        if (lane < KS) out[warp * KS + lane] = make_uint2(x[0], y[0]);
-      }
+      cl_moves_tmt<KS>(gen, rl, (int)(run & 0x3fffffffu), out + warp * KS, params_of);
     } else {
 #pragma unroll
       for (int g = 0; g < KS / 4; ++g) {
         if (g > 0 && g >= groups) break;
-        const uint4 d = fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]);
-        // Four tests each way as one nibble, two lanes' nibbles as one byte of the word's moves.
-        const uint32_t u = cl_nibble(d.x < rl.x, d.y < rl.x, d.z < rl.x, d.w < rl.x);
-        const uint32_t v = cl_nibble(d.x - rl.y < rl.z, d.y - rl.y < rl.z, d.z - rl.y < rl.z, d.w - rl.y < rl.z);
-        const uint32_t mine = (u ^ 15u) | (v << 16);
-        const uint32_t pair = mine | (__shfl_down_sync(~0u, mine, 1) << 4);
-        if (!(lane & 1)) {
-          uint8_t* to = reinterpret_cast<uint8_t*>(out + warp * KS + 4 * g + (lane >> 3)) + ((lane & 7) >> 1);
-          to[0] = (uint8_t)pair;
-          to[4] = (uint8_t)(pair >> 16);
-        }
+        cl_moves_fast(a.seed, a.stream, h, f_row[g], f_quad[g], rl, out + warp * KS + 4 * g);
       }
     }
   };
@@ -532,31 +432,8 @@ __global__ void __launch_bounds__(cl_max_threads(kMode == kClFast, KS), 1) k_clu
     }
     __syncthreads();  // s_differ read before the next attempt's flags
   }
-  // CTA rows of both colours back to the chains as edge masks: cells m in [1, cols] of the
-  // window's words (the others keep their bytes, as the reference never rebuilds them).
   __syncthreads();
-  for (int it = warp; it < (R - 1) * (wn - 2) * 2; it += nwarps) {
-    const int t = it & 1, q = it >> 1;
-    const int ri = 1 + q / (wn - 2), wi = 1 + q % (wn - 2);
-    const int i = r0 - 1 + ri, w = wlo + wi, m = 32 * w + lane;
-    if (m < 1 || m > a.cols || m >= a.P) continue;
-    const bool aligned = ((i + 1 - t) & 1) != 0;
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) {
-      const uint32_t up = (*PL(ri - 1, 1 - t, wi, c) >> lane) & 1u, dn = (*PL(ri, t, wi, c) >> lane) & 1u;
-      const uint32_t he = (*PL(ri, 2, wi, c) >> lane) & 1u;
-      uint32_t lft, rgt;
-      if (aligned) {
-        lft = he;
-        rgt = (*PL(ri, 3, wi, c) >> lane) & 1u;
-      } else {
-        lft = lane ? (*PL(ri, 3, wi, c) >> (lane - 1)) & 1u : *PL(ri, 3, wi - 1, c) >> 31;
-        rgt = he;
-      }
-      a.base[(size_t)c * a.chain_stride + (size_t)t * a.colour_stride + (size_t)i * a.P + m] =
-          (uint8_t)(up | (dn << 1) | (lft << 2) | (rgt << 3));
-    }
-  }
+  cl_store_window<NCH>(sm, a.base, a.chain_stride, a.colour_stride, a.P, a.cols, r0 - 1, R, wlo, wn);
   if constexpr (!kFast) {
 #pragma unroll
     for (int s = 0; s < KS; ++s) {
@@ -603,12 +480,12 @@ int cl_ctas_for(int64_t words, bool fast) {
 
 }  // namespace
 
-// Measured on a GB300 (us per half-sweep, cluster against the best band shape).  TinyMT: order 64
-// 0.27 / 0.81, 100 0.36 / 0.82, 200 0.88 / 1.07, 220 (the largest its 8 words per draw warp hold)
-// 0.89 / 1.08: wherever it fits.  Fast mode: order 100 0.52 / 1.6, 250 1.03 / 1.48 (one chain),
-// 1.20 / 1.62 (two), 300 1.36 / 1.56 (one); the draws of 16 SMs then take longer than the bands'
-// exchange.
-int64_t cl_auto_words(bool fast, int nch) { return fast ? (nch == 1 ? 3400 : 2600) : 2048; }
+// Measured on a GB300, us per half-sweep, cluster / one band per SM (domino_grid.cu).  TinyMT: order 64
+// 0.30 / 0.53, 100 0.37 / 0.51, 120 (686 words) 0.44 / 0.46, 130 (779) 0.65 / 0.56.  Fast mode:
+// order 100 0.60 / 0.94, 220 (1915) 0.95 / 1.13, 250 (2442) 1.03 / 1.15 with one chain and 1.21 / 1.15
+// with two, 260 (2615) 1.12 / 1.07.  Beyond, the draws of 16 SMs take longer than the exchange of
+// 152 bands through L2.
+int64_t cl_auto_words(bool fast) { return fast ? 2400 : 700; }
 
 void ClPlan::build(const std::vector<int>& lo, const std::vector<int>& hi, int N, int nch, bool fast, int ctas_asked) {
   ok = false;

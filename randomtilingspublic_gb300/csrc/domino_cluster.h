@@ -63,7 +63,7 @@ struct ClPlan {
 };
 
 // Words per half-sweep up to which the automatic choice is the cluster.
-int64_t cl_auto_words(bool fast, int nch);
+int64_t cl_auto_words(bool fast);
 
 struct ClusterEngine {
   ClPlan plan;

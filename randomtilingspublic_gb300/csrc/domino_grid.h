@@ -1,0 +1,51 @@
+// Grid engine of the domino sweep (see domino_grid.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "domino_rules.h"
+#include "rt_internal.h"
+
+namespace rt {
+
+struct DmSampler;
+
+constexpr int kGrMaxBands = 160;
+
+struct GrPlan {
+  bool ok = false;
+  std::string why;
+  int bands = 0, slots = 0, draw_warps = 0, update_warps = 0, per_lane = 1;  // slots: words per draw warp
+  int row_start[kGrMaxBands + 1] = {};
+  int windows[2 * kGrMaxBands] = {};  // each band's first window word and window words
+  int xlo = 0, xn = 0;                // first word and words of an exchange row
+  int64_t words = 0, draw_cells = 0;
+  size_t smem_bytes = 0;
+  int threads() const { return 32 * (draw_warps + update_warps); }
+  // From each colour-array row's first and last flip-candidate column (-1: none).
+  void build(const std::vector<int>& lo, const std::vector<int>& hi, int N, int nch, bool fast, int bands_max);
+};
+
+struct GridEngine {
+  GrPlan plan;
+  bool ready = false;
+  int nch = 0, bands_asked = 0;
+  void* kernel = nullptr;
+  cudaStream_t stream = nullptr;
+  int* d_rows = nullptr;       // the plan's row_start and windows, then the error word
+  uint64_t* d_xbuf = nullptr;  // tagged words
+  size_t xbuf_bytes = 0;
+  uint32_t* d_runs = nullptr;
+  int64_t runs_cap = 0;
+  bool pending_error_check = false;
+
+  ~GridEngine();
+  rt_status prepare(DmSampler& s);
+  rt_status launch(DmSampler& s, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed, int64_t h0);
+  rt_status check_error(DmSampler& s);
+};
+
+}  // namespace rt

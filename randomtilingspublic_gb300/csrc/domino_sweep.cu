@@ -239,6 +239,7 @@ __global__ void k_diff(DmView v, int a, int b, unsigned long long* out) {
 
 DmSampler::~DmSampler() {
   cluster.reset();
+  grid.reset();
   bits.reset();  // the engines free their plan buffers on the stream before the stream goes
   runs.reset();
   persist.reset();
@@ -558,7 +559,7 @@ rt_status DmSampler::sync() {
 rt_status DmSampler::use_persistent(bool* yes) {
   *yes = false;
   resident = 0;
-  in_cluster = false;
+  in_cluster = on_grid = false;
   // The engine: opts.engine when set, else the sampler's explicit launch shape, else the
   // autotuner's entry for this side, chain count and mode, else automatic.
   const bool explicit_engine = opts.engine != 0 || launch_engine != 0;
@@ -587,6 +588,7 @@ rt_status DmSampler::use_persistent(bool* yes) {
   }
   if (plan_dirty) {
     cluster.reset();
+    grid.reset();
     bits.reset();
     runs.reset();
     persist.reset();
@@ -604,7 +606,7 @@ rt_status DmSampler::use_persistent(bool* yes) {
       cluster = std::make_unique<ClusterEngine>();
       if (rt_status st = cluster->prepare(*this)) return st;
     }
-    if (cluster->ready && (launch_bands > 0 || cluster->plan.words <= cl_auto_words(fast, active))) {
+    if (cluster->ready && (launch_bands > 0 || cluster->plan.words <= cl_auto_words(fast))) {
       resident = 4;
       in_cluster = true;
       *yes = true;
@@ -612,6 +614,21 @@ rt_status DmSampler::use_persistent(bool* yes) {
     }
     if (!tuned) break;
     take_entry(++skip);
+  }
+  // The bit-plane kernel on every SM: where the table asks for engine 4 or bands are asked for, and
+  // automatically in TinyMT mode (in fast mode without a table the run kernel stays the choice).
+  if ((engine == 0 || engine == 4) && !explicit_engine && (!fast || tuned || eff_bands > 0)) {
+    if (grid && (grid->nch != active || grid->bands_asked != eff_bands)) grid.reset();
+    if (!grid) {
+      grid = std::make_unique<GridEngine>();
+      if (rt_status st = grid->prepare(*this)) return st;
+    }
+    if (grid->ready) {
+      resident = 4;
+      on_grid = true;
+      *yes = true;
+      return RT_OK;
+    }
   }
   // Engine 0: the bit-plane kernel, else the run kernel, else k_persist; 4: the bit-plane
   // kernel alone; 2: the run kernel, else k_persist; 3: k_persist alone.
@@ -667,6 +684,9 @@ rt_status DmSampler::check_resident_error() {
   if (cluster) {
     if (rt_status st = cluster->check_error(*this)) return st;
   }
+  if (grid) {
+    if (rt_status st = grid->check_error(*this)) return st;
+  }
   if (bits) {
     if (rt_status st = bits->check_error(*this)) return st;
   }
@@ -681,6 +701,7 @@ rt_status DmSampler::check_resident_error() {
 
 rt_status DmSampler::launch_resident(const uint8_t* colours, int64_t steps, uint64_t fast_seed, int64_t h0) {
   if (in_cluster) return cluster->launch(*this, colours, steps, fast_seed, h0);
+  if (on_grid) return grid->launch(*this, colours, steps, fast_seed, h0);
   if (resident == 4) return bits->launch(*this, colours, steps);
   if (resident == 2) return runs->launch(*this, colours, steps, fast_seed, h0);
   return persist->launch(*this, colours, steps, fast_seed, h0);
@@ -801,6 +822,10 @@ RT_API rt_status rt_dm_sampler_engine_info(rt_dm_sampler* s, int64_t* out4) {
     units = d.cluster->plan.draw_cells;
     bands = d.cluster->plan.ctas;
     k = d.cluster->plan.slots;
+  } else if (pers && d.on_grid) {
+    units = d.grid->plan.draw_cells;
+    bands = d.grid->plan.bands;
+    k = d.grid->plan.slots;
   } else if (pers && d.resident == 4) {
     units = d.bits->plan.draw_cells;
     bands = (int64_t)d.bits->plan.bands.size();
@@ -841,6 +866,7 @@ RT_API rt_status rt_dm_sampler_launch_info(rt_dm_sampler* s, int64_t* out6) {
   DmSampler& d = *s->impl;
   for (int k = 0; k < 4; ++k) out6[k] = e4[k];
   out6[4] = d.in_cluster   ? (int64_t)d.cluster->plan.threads()
+            : d.on_grid    ? (int64_t)d.grid->plan.threads()
             : (e4[0] == 4) ? (int64_t)d.bits->plan.warps * 32
             : (e4[0] == 2) ? d.runs->plan.threads
                            : (e4[0] == 3 ? (int64_t)kPersistThreads : 0);
@@ -983,7 +1009,7 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   const int64_t kLaunchHalfSweeps = (int64_t)1 << 21;
   bool pers = false;
   if (rt_status st = s->use_persistent(&pers)) return st;
-  const bool one_launch = pers && (s->resident == 2 || s->resident == 4) && o.rng_mode != RT_RNG_MTGP;
+  const bool one_launch = pers && !s->on_grid && (s->resident == 2 || s->resident == 4) && o.rng_mode != RT_RNG_MTGP;
   int att = 0;
   bool coalesced = false;
   while (att < max_attempts && !coalesced) {

@@ -7,6 +7,7 @@
 
 #include "domino_bits.h"
 #include "domino_cluster.h"
+#include "domino_grid.h"
 #include "domino_persist.h"
 #include "domino_runs.h"
 #include "domino_rules.h"
@@ -79,12 +80,14 @@ struct DmSampler {
   bool border_candidates = false;  // a candidate borders a cell the reference never rebuilds
   bool plan_dirty = true;
   std::unique_ptr<ClusterEngine> cluster;  // the bit-plane kernel in one cluster (domino_cluster.cu)
+  std::unique_ptr<GridEngine> grid;        // the bit-plane kernel on every SM (domino_grid.cu)
   std::unique_ptr<BitEngine> bits;        // the bit-plane kernel (domino_bits.cu)
   std::unique_ptr<RunEngine> runs;        // the run-resident kernel (domino_runs.cu)
   std::unique_ptr<PersistEngine> persist;  // the per-half-sweep-exchange resident kernel
   int resident = 0;     // the resident kernel the next run uses: 2 run kernel, 3 k_persist,
                         // 4 bit-plane kernel, 0 none
-  bool in_cluster = false;  // resident 4: in one thread-block cluster (cluster), else bits
+  bool in_cluster = false;  // resident 4: in one thread-block cluster (cluster),
+  bool on_grid = false;     // or on every SM (grid), else bits
   int last_engine = 0;  // engine of the last run: 1 per-half-sweep kernels, 2-4 as resident
   // Launch shape: an explicit choice (rt_dm_sampler_set_launch; 0 = none), and the shape in
   // force, from that choice, else the autotuner's table, else the defaults (0).
