@@ -738,7 +738,8 @@ class SixVertexTiler:
     """Six-vertex model on an n x n grid (no counterpart in the reference; shaped like its
     per-model classes).  State: the (n+1) x (n+1) int32 height function; weights a, b, c;
     fast (Philox) random mode only, ``fast_stream`` selects an independent stream.  ``engine``:
-    0 automatic, 1 one kernel per sub-sweep, 2 the cluster-resident kernel."""
+    0 automatic, 1 one kernel per sub-sweep, 2 the resident kernel wherever it holds the chains
+    (refused where 16 CTAs could not)."""
 
     def __init__(self, a: float = 1.0, b: float = 1.0, c: float = 1.0, fast_stream: int = 0, engine: int = 0):
         self.abc = np.array([a, b, c], np.float64)

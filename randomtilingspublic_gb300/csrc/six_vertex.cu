@@ -17,7 +17,6 @@
 // bit b of data word w is point k = 32 w + b of the class row (x = 2k + px, y = 2r + py).
 // A thread owns one word: 32 points updated with bitwise logic, the random comparison done
 // bit-sliced from the most significant plane down and stopped once every lane is decided.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -85,62 +84,41 @@ struct SvRows {
   const uint32_t *H, *Vn, *Vs, *Dn, *Ds;
 };
 
-// Updates data word w (index idx = w + 1) of class row r in NCH chains that share the draws.
+// Planes 4 q .. 4 q + 3 (the most significant first) of the draws of word w of row r.
 __device__ __forceinline__ uint4 sv_block(uint32_t w, uint32_t r, int q, uint32_t c2, uint32_t c3, uint64_t seed) {
   return philox4x32_10(make_uint4(w | ((uint32_t)q << 24), r, c2, c3), (uint32_t)seed, (uint32_t)(seed >> 32));
 }
 
-// Blocks q < NPRE of the draws arrive precomputed in pre[] (they do not depend on the state).
-template <int NCH, int NPRE = 0>
-__device__ __forceinline__ void sv_update_word(const SvRows (&rows)[NCH], int idx, int px, int py, uint32_t imask,
-                                               uint32_t w, uint32_t r, const uint32_t (&leaf)[32][9], uint64_t seed,
-                                               uint32_t c2, uint32_t c3, const uint4* pre = nullptr) {
-  uint32_t f[NCH], flip[NCH], sup[NCH], mk[NCH][9], lt[NCH], und[NCH];
-  uint32_t any = 0;
-#pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    const SvRows& R = rows[c];
-    f[c] = R.F[idx];
-    const uint32_t wv = west_of(R.H, idx, px), ev = east_of(R.H, idx, px);
-    const uint32_t nv = R.Vn[idx], sv = R.Vs[idx];
-    flip[c] = ~(wv ^ ev) & ~(wv ^ nv) & ~(wv ^ sv) & imask;
-    sup[c] = (px ^ py) ? wv : ~wv;  // sigma of h' + 1 (neighbour parity 1 - (px ^ py))
-    const uint32_t e1a = ~(west_of(R.Dn, idx, px) ^ sup[c]), e1b = ~(east_of(R.Ds, idx, px) ^ sup[c]);
-    const uint32_t e2a = ~(east_of(R.Dn, idx, px) ^ sup[c]), e2b = ~(west_of(R.Ds, idx, px) ^ sup[c]);
-    const uint32_t a0 = ~(e1a | e1b), a1 = e1a ^ e1b, a2 = e1a & e1b;
-    const uint32_t b0 = ~(e2a | e2b), b1 = e2a ^ e2b, b2 = e2a & e2b;
-    mk[c][0] = a0 & b0, mk[c][1] = a0 & b1, mk[c][2] = a0 & b2;
-    mk[c][3] = a1 & b0, mk[c][4] = a1 & b1, mk[c][5] = a1 & b2;
-    mk[c][6] = a2 & b0, mk[c][7] = a2 & b1, mk[c][8] = a2 & b2;
-    lt[c] = 0;
-    und[c] = flip[c];
-    any |= flip[c];
-  }
-  if (!any) return;
+// Updates data word w (index idx = w + 1) of class row r.
+__device__ __forceinline__ void sv_update_word(const SvRows& R, int idx, int px, int py, uint32_t imask, uint32_t w,
+                                               uint32_t r, const uint32_t (&leaf)[32][9], uint64_t seed, uint32_t c2,
+                                               uint32_t c3) {
+  const uint32_t f = R.F[idx], wv = west_of(R.H, idx, px), ev = east_of(R.H, idx, px);
+  const uint32_t flip = ~(wv ^ ev) & ~(wv ^ R.Vn[idx]) & ~(wv ^ R.Vs[idx]) & imask;
+  if (!flip) return;
+  const uint32_t sup = (px ^ py) ? wv : ~wv;  // sigma of h' + 1 (neighbour parity 1 - (px ^ py))
+  const uint32_t e1a = ~(west_of(R.Dn, idx, px) ^ sup), e1b = ~(east_of(R.Ds, idx, px) ^ sup);
+  const uint32_t e2a = ~(east_of(R.Dn, idx, px) ^ sup), e2b = ~(west_of(R.Ds, idx, px) ^ sup);
+  const uint32_t a0 = ~(e1a | e1b), a1 = e1a ^ e1b, a2 = e1a & e1b;
+  const uint32_t b0 = ~(e2a | e2b), b1 = e2a ^ e2b, b2 = e2a & e2b;
+  const uint32_t mk[9] = {a0 & b0, a0 & b1, a0 & b2, a1 & b0, a1 & b1, a1 & b2, a2 & b0, a2 & b1, a2 & b2};
+  uint32_t lt = 0, und = flip;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    uint32_t open = 0;
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) open |= und[c];
-    if (!open) break;
-    const uint4 Rq = q < NPRE ? pre[q] : sv_block(w, r, q, c2, c3, seed);
+    if (!und) break;
+    const uint4 Rq = sv_block(w, r, q, c2, c3, seed);
     const uint32_t planes[4] = {Rq.x, Rq.y, Rq.z, Rq.w};
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int j = 31 - (4 * q + t);
+      uint32_t Tj = 0;  // bit j of each point's threshold
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        uint32_t Tj = 0;  // bit j of each point's threshold
-#pragma unroll
-        for (int m = 0; m < 9; ++m) Tj |= mk[c][m] & leaf[j][m];
-        lt[c] |= und[c] & ~planes[t] & Tj;
-        und[c] &= ~(planes[t] ^ Tj);
-      }
+      for (int m = 0; m < 9; ++m) Tj |= mk[m] & leaf[j][m];
+      lt |= und & ~planes[t] & Tj;
+      und &= ~(planes[t] ^ Tj);
     }
   }
-#pragma unroll
-  for (int c = 0; c < NCH; ++c)
-    if (flip[c]) rows[c].F[idx] = (f[c] & ~flip[c]) | (flip[c] & ~(lt[c] ^ sup[c]));
+  R.F[idx] = (f & ~flip) | (flip & ~(lt ^ sup));
 }
 
 __device__ __forceinline__ uint32_t interior_mask(int w, int k_lo, int k_hi) {
@@ -163,114 +141,355 @@ __global__ void __launch_bounds__(128) k_sv_sub(SvLaunch L) {
   const uint32_t* V = chain + (size_t)(cls ^ 2) * L.class_words;
   const uint32_t* D = chain + (size_t)(cls ^ 3) * L.class_words;
   const int rn = py ? r : r - 1, rs = py ? r + 1 : r;
-  const SvRows rows[1] = {{chain + (size_t)cls * L.class_words + (size_t)r * L.P,
+  const SvRows rows = {chain + (size_t)cls * L.class_words + (size_t)r * L.P,
                            chain + (size_t)(cls ^ 1) * L.class_words + (size_t)r * L.P, V + (size_t)rn * L.P,
-                           V + (size_t)rs * L.P, D + (size_t)rn * L.P, D + (size_t)rs * L.P}};
+                           V + (size_t)rs * L.P, D + (size_t)rn * L.P, D + (size_t)rs * L.P};
   const uint32_t c2 = (uint32_t)(uint64_t)L.s, c3 = ((uint32_t)((uint64_t)L.s >> 32) & 0xffffu) | (L.stream << 16);
-  sv_update_word<1>(rows, w + 1, px, py, imask, (uint32_t)w, (uint32_t)r, L.leaf, L.seed, c2, c3);
+  sv_update_word(rows, w + 1, px, py, imask, (uint32_t)w, (uint32_t)r, L.leaf, L.seed, c2, c3);
 }
 
-// Resident engine: one thread-block cluster holds NCH chains in shared memory, CTA `rank`
-// owning class rows [rank * rpc, rank * rpc + rpc) of all four classes; the one halo row
-// above and below is read from the neighbouring CTA's shared memory (distributed shared
-// memory).  A cluster barrier separates sub-sweeps; no other waits.
-struct SvClusterArgs {
-  uint32_t* base;
+// Resident engine: the chains in shared memory, a band of class rows per CTA.
+//
+// Bound: latency.  With one word a thread and a cluster barrier per sub-sweep a word took about 800 dependent
+// instructions (Philox, then planes against nine thresholds): n = 512 6.2 us per sweep (four sub-sweeps),
+// n = 48 with two chains 2.2 us.  Here
+//   * draw warps compute, phases ahead, what does not depend on the state: for every word the
+//     bits [u < T] of each distinct threshold T (nine; five where T depends on k1 + k2 only, as
+//     for a = b).  16 planes are compared at once, least significant first (one logic operation
+//     per plane and threshold for "less", one for "equal"); words with an undecided point, one
+//     warp in eight, look at more.  The update warps then select among the words: about 50
+//     operations a word;
+//   * a phase is the two sub-sweeps of one row parity.  They read rows of the other parity and
+//     their own row, so bands meet at most twice a sweep; a band also updates `depth` rows beyond
+//     its own on both sides, whose draws it makes itself, and meets its neighbours every `depth`
+//     sweeps only (rows as 64-bit words tagged with the period, through L2; every wait bounded).
+// Measured (GB300, a = b): n = 512 1.10 us per sweep, n = 101 0.86, n = 1024 1.84 (before, one launch per
+// sub-sweep: 8.3), n = 48 with two chains 0.80.  A warp's draws cost about 600 cycles of a scheduler in
+// Philox (the high halves of its products) and 360 (five thresholds) or 630 (nine) in the comparison; a
+// band's update alone takes about 0.65 us per sweep, an exchange 0.3-0.5 us.
+struct SvBandArgs {
+  const uint32_t* src;  // chain 0, chain c at + c * chain_words
+  uint32_t* dst;        // not src: a band may write back before another has loaded
   size_t chain_words, class_words;
-  int P, n, R, rpc;
-  uint32_t leaf[32][9];  // as SvLaunch::leaf
+  int P, n, R, words;   // words: data words of a row that can change
+  int bands, depth;     // sweeps between exchanges (each band owns at least depth rows)
+  int group;            // update threads per chain, a word each (a multiple of 32)
+  int batch;            // phases drawn at once
+  int items;            // most words of one sub-sweep in a band (a multiple of 4)
+  int rows;             // most rows of a band's window
+  uint32_t leaf[32][9];  // as SvLaunch::leaf; of the distinct thresholds only, in the order they are drawn
   uint64_t seed;
   uint32_t stream;
-  int64_t s0, count;
+  int64_t s0;           // first sub-sweep, a multiple of 4
+  int sweeps;
+  uint64_t* xbuf;       // [period parity][band][to above, to below][chain][row][class][word], tags cleared
+  int* error;
+  long max_spin;
 };
 
-template <int NCH>
-constexpr int sv_cluster_max_threads() {
-  return 512;
+constexpr int kSvDrawPlanes = 16;
+constexpr int kSvBandThreads = 640;
+
+// First row of band b of `bands` over the rows that can change.
+__host__ __device__ __forceinline__ int sv_band_row(int b, int bands, int rows) { return (int)((int64_t)b * rows / bands); }
+
+// Rows [lo, hi) that a band owning [r0, r1) updates in a phase of row parity py, `left` sweeps
+// before its next exchange (this one included).
+__host__ __device__ __forceinline__ void sv_phase_rows(int n, int r0, int r1, int py, int left, int* lo, int* hi) {
+  *lo = max(py ? 0 : 1, r0 - (left - 1));
+  *hi = min(py ? (n - 2) / 2 + 1 : (n - 1) / 2 + 1, py ? r1 + left - 1 : r1 + left);
+  if (*hi < *lo) *hi = *lo;
 }
 
-__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-// The class rows, words and interior columns of sub-sweep s restricted to rows [r0, r1).
-struct SvSub {
-  int px, py, cls, r_lo, r_hi, k_lo, k_hi, words;
-  uint32_t c2, c3;
-};
-
-__device__ __forceinline__ SvSub sv_sub_of(int64_t s, int n, int r0, int r1, uint32_t stream) {
-  SvSub u;
-  u.px = (int)(s & 1);
-  u.py = (int)((s >> 1) & 1);
-  u.cls = u.px | (u.py << 1);
-  u.r_lo = max(u.py ? 0 : 1, r0);
-  u.r_hi = min((n - 1 - u.py) / 2, r1 - 1);
-  u.k_lo = u.px ? 0 : 1;
-  u.k_hi = (n - 1 - u.px) / 2;
-  u.words = u.k_hi / 32 + 1;
-  u.c2 = (uint32_t)(uint64_t)s;
-  u.c3 = ((uint32_t)((uint64_t)s >> 32) & 0xffffu) | (stream << 16);
-  return u;
+// One plane of the bit-sliced comparison, from the least significant up: less = T ? ~p | less : ~p & less
+// and equal &= ~(p ^ T), one operation each (the compiler makes two of the first).
+__device__ __forceinline__ uint32_t sv_less(uint32_t less, uint32_t p, uint32_t T) {
+  uint32_t d;
+  constexpr int a = 0xf0, b = 0xcc, c = 0xaa;
+  asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(T), "r"(p), "r"(less), "n"(((a & (~b | c)) | (~a & ~b & c)) & 0xff));
+  return d;
+}
+__device__ __forceinline__ uint32_t sv_equal(uint32_t equal, uint32_t p, uint32_t T) {
+  uint32_t d;
+  constexpr int a = 0xf0, b = 0xcc, c = 0xaa;
+  asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(T), "r"(p), "r"(equal), "n"((c & ~(a ^ b)) & 0xff));
+  return d;
 }
 
-template <int NCH>
-__global__ void __launch_bounds__(sv_cluster_max_threads<NCH>()) k_sv_cluster(SvClusterArgs A) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ uint32_t sm[];  // [NCH][4][rpc][P]
-  const int rank = (int)cluster.block_rank(), C = (int)cluster.num_blocks();
-  const int r0 = rank * A.rpc, r1 = min(r0 + A.rpc, A.R), P = A.P;
-  const int own = max(r1 - r0, 0);
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int i = tid; i < NCH * 4 * own * P; i += nt) {
-    const int p = i % P, lr = (i / P) % own, cc = i / (P * own);  // cc = chain * 4 + class
-    sm[((size_t)cc * A.rpc + lr) * P + p] =
-        A.base[(size_t)(cc >> 2) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(r0 + lr) * P + p];
-  }
-  // shared memory of the CTAs above and below (rows r0 - 1 and r1 live there)
-  uint32_t* const up = rank > 0 ? cluster.map_shared_rank(sm, rank - 1) : sm;
-  uint32_t* const dn = rank + 1 < C ? cluster.map_shared_rank(sm, rank + 1) : sm;
-  const size_t plane = (size_t)A.rpc * P;  // words of one class of one chain
-  auto row = [&](int c, int cls, int r) -> uint32_t* {
-    uint32_t* b = r < r0 ? up + (size_t)(A.rpc - 1) * P : r >= r1 ? dn : sm + (size_t)(r - r0) * P;
-    return b + (size_t)(c * 4 + cls) * plane;
-  };
-  const int n = A.n;
-  constexpr int kPre = 2;
-  uint4 pre[kPre];
-  SvSub u = sv_sub_of(A.s0, n, r0, r1, A.stream);
-  if (tid < (u.r_hi - u.r_lo + 1) * u.words)
-    for (int q = 0; q < kPre; ++q) pre[q] = sv_block(tid % u.words, u.r_lo + tid / u.words, q, u.c2, u.c3, A.seed);
-  cluster.sync();
-  for (int64_t s = A.s0; s < A.s0 + A.count; ++s) {
-    const int items = (u.r_hi - u.r_lo + 1) * u.words;
-    for (int it = tid; it < items; it += nt) {
-      const int w = it % u.words, r = u.r_lo + it / u.words;
-      const uint32_t imask = interior_mask(w, u.k_lo, u.k_hi);
-      if (!imask) continue;
-      const int rn = u.py ? r : r - 1, rs = u.py ? r + 1 : r;
-      SvRows rows[NCH];
+// Bits [u < T[m]] of the 32 points of word w of row r in one sub-sweep, for M thresholds.
+template <int M>
+__device__ __forceinline__ void sv_draw_word(uint32_t* set, int item, int items, const uint32_t (&leaf)[32][9], uint32_t imask,
+                                             uint32_t w, uint32_t r, uint32_t c2, uint32_t c3, uint64_t seed) {
+  uint32_t planes[kSvDrawPlanes];
 #pragma unroll
-      for (int c = 0; c < NCH; ++c)
-        rows[c] = {row(c, u.cls, r), row(c, u.cls ^ 1, r), row(c, u.cls ^ 2, rn), row(c, u.cls ^ 2, rs),
-                   row(c, u.cls ^ 3, rn), row(c, u.cls ^ 3, rs)};
-      if (it == tid)
-        sv_update_word<NCH, kPre>(rows, w + 1, u.px, u.py, imask, (uint32_t)w, (uint32_t)r, A.leaf, A.seed, u.c2, u.c3, pre);
-      else
-        sv_update_word<NCH>(rows, w + 1, u.px, u.py, imask, (uint32_t)w, (uint32_t)r, A.leaf, A.seed, u.c2, u.c3);
-    }
-    // the next sub-sweep's first draws do not depend on the state: compute them while the
-    // other CTAs of the cluster reach the barrier
-    cluster_arrive_release();
-    u = sv_sub_of(s + 1, n, r0, r1, A.stream);
-    if (s + 1 < A.s0 + A.count && tid < (u.r_hi - u.r_lo + 1) * u.words)
-      for (int q = 0; q < kPre; ++q) pre[q] = sv_block(tid % u.words, u.r_lo + tid / u.words, q, u.c2, u.c3, A.seed);
-    cluster_wait_acquire();
+  for (int q = 0; q < kSvDrawPlanes / 4; ++q) {
+    const uint4 b = sv_block(w, r, q, c2, c3, seed);
+    planes[4 * q] = b.x, planes[4 * q + 1] = b.y, planes[4 * q + 2] = b.z, planes[4 * q + 3] = b.w;
   }
+  uint32_t lt[M], eq[M], open = 0;
+#pragma unroll
+  for (int m = 0; m < M; ++m) lt[m] = 0u, eq[m] = imask;
+#pragma unroll
+  for (int t = kSvDrawPlanes - 1; t >= 0; --t)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const uint32_t T = leaf[31 - t][m];
+      lt[m] = sv_less(lt[m], planes[t], T);
+      eq[m] = sv_equal(eq[m], planes[t], T);
+    }
+#pragma unroll
+  for (int m = 0; m < M; ++m) open |= eq[m];
+  for (int q = kSvDrawPlanes / 4; open && q < 8; ++q) {
+    const uint4 b = sv_block(w, r, q, c2, c3, seed);
+    const uint32_t more[4] = {b.x, b.y, b.z, b.w};
+    open = 0;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint32_t T = leaf[31 - 4 * q - t][m];
+        lt[m] |= eq[m] & ~more[t] & T;
+        eq[m] &= ~(more[t] ^ T);
+      }
+      open |= eq[m];
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < M; ++m) set[m * items + item] = lt[m];
+}
+
+// The drawn bit of each point's threshold, from the bits of its diagonal points that equal h' + 1: e1a,
+// e1b on the a/c diagonal, e2a, e2b on the b/c diagonal.  kSum: T depends on k1 + k2 only.
+template <bool kSum>
+__device__ __forceinline__ uint32_t sv_pick(const uint32_t (&drawn)[kSum ? 5 : 9], uint32_t e1a, uint32_t e1b,
+                                            uint32_t e2a, uint32_t e2b) {
+  if constexpr (kSum) {
+    const uint32_t x = e1a ^ e1b ^ e2a, y = (e1a & e1b) | (e2a & (e1a | e1b));  // e1a + e1b + e2a
+    const uint32_t one = x ^ e2b, z = x & e2b, two = y ^ z, four = y & z;
+    const uint32_t l01 = (one & drawn[1]) | (~one & drawn[0]), l23 = (one & drawn[3]) | (~one & drawn[2]);
+    const uint32_t low = (two & l23) | (~two & l01);
+    return (four & drawn[4]) | (~four & low);
+  } else {
+    const uint32_t a1 = e1a ^ e1b, a2 = e1a & e1b, b1 = e2a ^ e2b, b2 = e2a & e2b;
+    uint32_t k[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const uint32_t low = (b1 & drawn[3 * i + 1]) | (~b1 & drawn[3 * i]);
+      k[i] = (b2 & drawn[3 * i + 2]) | (~b2 & low);
+    }
+    const uint32_t low = (a1 & k[1]) | (~a1 & k[0]);
+    return (a2 & k[2]) | (~a2 & low);
+  }
+}
+
+__device__ __forceinline__ int sv_div(int a, float inv) { return (int)(((float)a + 0.5f) * inv); }  // a < 2^20
+
+template <int NCH, bool kSum>
+__global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_constant__ SvBandArgs A) {
+  constexpr int M = kSum ? 5 : 9;
+  // [NCH][4][rows][P] states; [2][batch][2][M][items] drawn bits; [depth + 1][2] rows of a phase
+  extern __shared__ __align__(16) uint32_t sm[];
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int n = A.n, P = A.P, words = A.words, band = blockIdx.x;
+  const int movable = (n - 1) / 2 + 1;  // rows that can change
+  const int r0 = sv_band_row(band, A.bands, movable), r1 = sv_band_row(band + 1, A.bands, movable);
+  const int w0 = max(r0 - A.depth, 0), w1 = min(r1 + A.depth, A.R);  // the window's rows
+  const int cs = A.rows * P;
+  uint32_t* const drawn = sm + ((NCH * 4 * cs + 3) & ~3);
+  const int sub_words = M * A.items, set_words = A.batch * 2 * sub_words;
+  int2* const phase_tab = reinterpret_cast<int2*>(drawn + 2 * set_words);  // [sweeps left][py]: first row, words
+  const float inv_words = 1.0f / (float)words;
+
+  for (int i = tid; i < NCH * 4 * (w1 - w0) * P; i += nt) {
+    const int p = i % P, lr = (i / P) % (w1 - w0), cc = i / (P * (w1 - w0));  // cc: chain * 4 + class
+    sm[cc * cs + lr * P + p] =
+        A.src[(size_t)(cc >> 2) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(w0 + lr) * P + p];
+  }
+
+  for (int i = tid; i < 2 * (A.depth + 1); i += nt) {
+    int lo, hi;
+    sv_phase_rows(n, r0, r1, i & 1, i >> 1, &lo, &hi);
+    phase_tab[i] = make_int2(lo, (hi - lo) * words);
+  }
+  __syncthreads();
+
+  const int updaters = NCH * A.group;
+  const bool updates = tid < updaters;
+  const int phases = 2 * A.sweeps, batches = (phases + A.batch - 1) / A.batch;
+  // Draws of batch b: tasks of 32 words in turn over the draw warps.
+  int ahead = 0, drawn_left = min(A.depth, A.sweeps);  // the sweep reached, and sweeps left before the exchange after it
+  int2 rows_of[2] = {phase_tab[2 * drawn_left], phase_tab[2 * drawn_left + 1]};
+  auto draw_batch = [&](int b) {
+    const int dw = warp - (updaters >> 5), ndw = (nt - updaters) >> 5;
+    uint32_t* const set = drawn + (b & 1) * set_words;
+    int turn = 0;
+    for (int q = 0; q < A.batch; ++q) {
+      const int f = b * A.batch + q;
+      if (f >= phases) break;
+      const int py = f & 1;
+      const int lo = py ? rows_of[1].x : rows_of[0].x, items = py ? rows_of[1].y : rows_of[0].y;
+      if (py && A.depth > 1) {
+        ++ahead;
+        drawn_left = drawn_left > 1 ? drawn_left - 1 : min(A.depth, A.sweeps - ahead);
+        rows_of[0] = phase_tab[2 * drawn_left], rows_of[1] = phase_tab[2 * drawn_left + 1];
+      }
+      for (int e0 = 0; e0 < 2 * items; e0 += 32, turn = turn + 1 == ndw ? 0 : turn + 1) {
+        if (turn != dw) continue;
+        const int e = e0 + lane;
+        if (e >= 2 * items) continue;
+        const int px = e >= items ? 1 : 0, it = e - px * items, rr = sv_div(it, inv_words), w = it - rr * words;
+        const uint64_t s = (uint64_t)(A.s0 + 2 * (int64_t)f + px);
+        const uint32_t imask = interior_mask(w, px ? 0 : 1, (n - 1 - px) / 2);
+        sv_draw_word<M>(set + (2 * q + px) * sub_words, it, A.items, A.leaf, imask, (uint32_t)w, (uint32_t)(lo + rr),
+                        (uint32_t)s, ((uint32_t)(s >> 32) & 0xffffu) | (A.stream << 16), A.seed);
+      }
+    }
+  };
+
+  const int chain = NCH == 2 && tid >= A.group ? 1 : 0, ut = tid - chain * A.group;
+  uint32_t* const S = sm + chain * 4 * cs;
+  auto group_sync = [&](int group) {
+    if (group == 32)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + chain), "r"(group) : "memory");
+  };
+  const int my_row = sv_div(ut, inv_words), my_word = ut - my_row * words;
+  const uint32_t my_mask[2] = {interior_mask(my_word, 1, (n - 1) / 2), interior_mask(my_word, 0, (n - 2) / 2)};
+  bool dead = false;  // a wait gave up: no further waits, the launch runs to its end
+  // Exchange: what each thread sends (its word, of the last sweep before an exchange) and receives (up to
+  // four words) is the same every period; -1: nothing.
+  const int per_side = A.depth * 4 * words;
+  const uint32_t xparity = (uint32_t)(A.bands * 2 * NCH * per_side);
+  auto slot = [&](int b, int dir) { return ((b * 2 + dir) * NCH + chain) * per_side; };
+  int send_up[2] = {-1, -1}, send_dn[2] = {-1, -1}, recv_from[4], recv_to[4];
+#pragma unroll
+  for (int py = 0; py < 2; ++py) {
+    const int2 ph = phase_tab[2 + py];
+    const int row = ph.x + my_row;
+    if (!updates || ut >= ph.y || row < r0 || row >= r1) continue;
+    if (band > 0 && row < r0 + A.depth) send_up[py] = slot(band, 0) + ((row - r0) * 4 + 2 * py) * words + my_word;
+    if (band + 1 < A.bands && row >= r1 - A.depth)
+      send_dn[py] = slot(band, 1) + ((row - (r1 - A.depth)) * 4 + 2 * py) * words + my_word;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int e = ut + i * A.group;
+    const int dir = e >= per_side ? 1 : 0, x = e - dir * per_side, q = sv_div(x, inv_words), w = x - q * words;
+    const int row = (dir ? r1 : r0 - A.depth) + (q >> 2), py = (q >> 1) & 1;  // the neighbours' rows next to ours
+    const bool on = updates && e < 2 * per_side && (dir ? band + 1 < A.bands : band > 0) && row >= (py ? 0 : 1) &&
+                    row <= (n - 1 - py) / 2;
+    recv_from[i] = on ? slot(dir ? band + 1 : band - 1, 1 - dir) + x : -1;
+    recv_to[i] = (q & 3) * cs + (row - w0) * P + 1 + w;
+  }
+  auto send = [&](uint32_t per, int at, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(A.xbuf + (per & 1) * xparity + at),
+                 "l"(((uint64_t)(per + 1) << 32) | v)
+                 : "memory");
+  };
+  auto receive = [&](uint32_t per) {
+    const uint64_t* const buf = A.xbuf + (per & 1) * xparity;
+    uint64_t v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (recv_from[i] >= 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[i]) : "l"(buf + recv_from[i]) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (recv_from[i] < 0) continue;
+      for (long it = 0; !dead && (uint32_t)(v[i] >> 32) != per + 1; ++it) {
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[i]) : "l"(buf + recv_from[i]) : "memory");
+        if (it >= A.max_spin) {
+          dead = true;
+          atomicExch(A.error, 1);
+        } else if ((it & 1023) == 1023 && *static_cast<volatile int*>(A.error)) {
+          dead = true;
+        }
+      }
+      if (!dead) S[recv_to[i]] = (uint32_t)v[i];
+    }
+    group_sync(A.group);
+  };
+
+  if (!updates) draw_batch(0);
+  __syncthreads();
+  // Held in registers: a parameter read again in each phase is a constant load on its critical path.
+  int depth = A.depth, sweeps = A.sweeps, items = A.items, group = A.group, row_words = P, class_words = cs;
+  asm volatile("" : "+r"(depth), "+r"(sweeps), "+r"(items), "+r"(group), "+r"(row_words), "+r"(class_words));
+  int in_period = 0;  // sweeps since the last exchange
+  uint32_t period = 0;
+  int2 ph = phase_tab[2 * min(A.depth, A.sweeps)];  // the phase's first row and its words
+  for (int b = 0; b < batches; ++b) {
+    if (updates) {
+      const uint32_t* bits = drawn + (b & 1) * set_words;
+      const int last = min(phases - b * A.batch, A.batch);
+      for (int q = 0; q < last; ++q) {
+        const int f = b * A.batch + q, py = f & 1;
+        const int left = min(depth - in_period, sweeps - (f >> 1));
+        // Classes: a, b = (0, py), (1, py), which move; c, d = (0, 1 - py), (1, 1 - py), which do not.  Sub-sweep
+        // px = 0 reads points k - 1, k of b and d and k of c; px = 1 points k, k + 1 of a and c and k of d:
+        // one set of loads serves both, but for the word of a to the right.
+        const bool mine = ut < ph.y;
+        const int flip_side = py ? 0 : ~0;  // sigma of h' + 1 is h at odd x + y, ~h at even
+        const int at = mine ? (ph.x - w0 + my_row) * row_words + 1 + my_word : row_words + 1;
+        uint32_t* const pa = S + 2 * py * class_words + at;
+        const uint32_t* const pc = S + 2 * (1 - py) * class_words + at - (py ? 0 : row_words);
+        const uint32_t va = pa[0], vb = pa[class_words], vb_w = pa[class_words - 1];
+        const uint32_t c_n = pc[0], c_s = pc[row_words], c_ne = pc[1], c_se = pc[row_words + 1];
+        const uint32_t d_n = pc[class_words], d_s = pc[class_words + row_words], d_nw = pc[class_words - 1], d_sw = pc[class_words + row_words - 1];
+        uint32_t drawn0[M], drawn1[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) drawn0[m] = bits[m * items + ut], drawn1[m] = bits[sub_words + m * items + ut];
+        bits += 2 * sub_words;
+        uint32_t now;
+        {
+          const uint32_t hw = __funnelshift_l(vb_w, vb, 1);
+          const uint32_t flip = ~(vb ^ hw) & ~(vb ^ c_n) & ~(vb ^ c_s) & (mine ? my_mask[0] : 0u);
+          const uint32_t sup = vb ^ flip_side;
+          const uint32_t lt = sv_pick<kSum>(drawn0, ~(__funnelshift_l(d_nw, d_n, 1) ^ sup), ~(d_s ^ sup), ~(d_n ^ sup),
+                                            ~(__funnelshift_l(d_sw, d_s, 1) ^ sup));
+          now = (va & ~flip) | (flip & ~(lt ^ sup));
+          if (mine) pa[0] = now;
+        }
+        const int next_left = py ? (left > 1 ? left - 1 : min(depth, sweeps - (f >> 1) - 1)) : left;
+        ph = phase_tab[2 * next_left + 1 - py];
+        group_sync(group);
+        {
+          const uint32_t sup = now ^ ~flip_side;
+          const uint32_t lt = sv_pick<kSum>(drawn1, ~(c_n ^ sup), ~(__funnelshift_r(c_s, c_se, 1) ^ sup),
+                                            ~(__funnelshift_r(c_n, c_ne, 1) ^ sup), ~(c_s ^ sup));
+          const uint32_t he = __funnelshift_r(now, pa[1], 1);
+          const uint32_t flip = ~(now ^ he) & ~(now ^ d_n) & ~(now ^ d_s) & (mine ? my_mask[1] : 0u);
+          const uint32_t moved = (vb & ~flip) | (flip & ~(lt ^ sup));
+          if (mine) pa[class_words] = moved;
+          // The last sweep before an exchange leaves the boundary rows as the neighbours need them.
+          if (left == 1 && A.bands > 1) {
+            const int up = py ? send_up[1] : send_up[0], dn = py ? send_dn[1] : send_dn[0];
+            if (up >= 0) {
+              send(period, up, now);
+              send(period, up + words, moved);
+            }
+            if (dn >= 0) {
+              send(period, dn, now);
+              send(period, dn + words, moved);
+            }
+          }
+        }
+        group_sync(group);
+        if (py && ++in_period == depth) {
+          in_period = 0;
+          if (A.bands > 1 && (f >> 1) + 1 < sweeps) receive(period++);
+        }
+      }
+    } else if (b + 1 < batches) {
+      draw_batch(b + 1);
+    }
+    __syncthreads();
+  }
+  const int own = (band + 1 == A.bands ? A.R : r1) - r0;  // the last row may be fixed: the last band's
   for (int i = tid; i < NCH * 4 * own * P; i += nt) {
     const int p = i % P, lr = (i / P) % own, cc = i / (P * own);
-    A.base[(size_t)(cc >> 2) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(r0 + lr) * P + p] =
-        sm[((size_t)cc * A.rpc + lr) * P + p];
+    A.dst[(size_t)(cc >> 2) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(r0 + lr) * P + p] =
+        sm[cc * cs + (r0 - w0 + lr) * P + p];
   }
 }
 
@@ -358,11 +577,13 @@ void sv_unpack(const uint32_t* bits, const SvGeom& G, const int32_t* start, int3
 namespace {
 
 struct SvDevice {
-  uint32_t* chains = nullptr;
-  uint32_t* flag = nullptr;
+  uint32_t* chains = nullptr;  // the state of the per-sub-sweep kernels; the resident engine's start
+  uint32_t* other = nullptr;   // resident engine: two more states, written in turn
+  uint64_t* xbuf = nullptr;
+  int* flag = nullptr;  // {chains differ, a wait gave up}
+  cudaStream_t stream = nullptr;
   ~SvDevice() {
-    if (chains) cudaFree(chains);
-    if (flag) cudaFree(flag);
+    for (void* p : {(void*)chains, (void*)other, (void*)xbuf, (void*)flag}) dev_free(p, stream);
   }
 };
 
@@ -385,125 +606,174 @@ rt_status sv_check_device() {
   return RT_OK;
 }
 
-struct SvClusterPlan {
+struct SvBandPlan {
   bool ok = false;
-  int C = 0, rpc = 0, threads = 0;
-  size_t smem = 0;
+  bool sum = false;  // thresholds depend on k1 + k2 only
+  int bands = 0, depth = 0, group = 0, batch = 0, items = 0, rows = 0, threads = 0;
+  size_t smem = 0, xbuf_words = 0;
+  void* kernel = nullptr;
 };
 
-template <int NCH>
-SvClusterPlan sv_cluster_plan_for(const SvGeom& G) {
-  SvClusterPlan best;
-  const int words = (G.n / 2) / 32 + 1;
-  for (int cmax : {16, 8}) {
-    SvClusterPlan p;
-    p.rpc = (G.R + cmax - 1) / cmax;
-    p.C = (G.R + p.rpc - 1) / p.rpc;
-    p.smem = (size_t)NCH * 4 * p.rpc * G.P * sizeof(uint32_t);
-    if (p.smem > 200 * 1024) continue;
-    p.threads = std::min(sv_cluster_max_threads<NCH>(), std::max(64, (p.rpc * words + 31) / 32 * 32));
-    auto kern = k_sv_cluster<NCH>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess) {
-      cudaGetLastError();
-      continue;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.C);
-    cfg.blockDim = dim3(p.threads);
-    cfg.dynamicSmemBytes = p.smem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = p.C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
-      cudaGetLastError();
-      continue;
-    }
-    p.ok = true;
+bool sv_sum_thresholds(const std::vector<uint32_t>& T) {
+  return T[1] == T[3] && T[2] == T[4] && T[4] == T[6] && T[5] == T[7];
+}
+
+SvBandPlan sv_band_plan(const SvGeom& G, int chains, const std::vector<uint32_t>& T) {
+  SvBandPlan p;
+  const int n = G.n, movable = (n - 1) / 2 + 1, words = (n - 1) / 2 / 32 + 1;
+  int dev = 0, sms = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
+    cudaGetLastError();
     return p;
   }
-  return best;
+  p.sum = sv_sum_thresholds(T);
+  const int M = p.sum ? 5 : 9;
+  // One band where half a warp holds a sub-sweep (n = 30: 0.84 us a sweep, two bands 0.95-1.0; n = 40: 1.08 and
+  // 0.88).  Else bands of `depth` rows, so that a band's words with its 2 depth - 1 spare rows fill one or two
+  // warps: depth 4, 3, 2 at 2, 3, 4 or more words a row (n = 101: depth 3 and 4 0.86-0.88 us, 2 0.96; n = 190: 3
+  // 1.16, 4 1.23; n = 256: 2 1.10, 3 1.23; n = 512: 2 1.10, 1 1.50); depth 1 once every band has more than two
+  // rows (n = 600: depth 2 1.23, 1 1.83; n = 700: 2.03 and 1.96; n = 1024: 2.5 and 1.9).
+  p.depth = words <= 2 ? 4 : words == 3 ? 3 : movable <= 2 * sms ? 2 : 1;
+  p.bands = std::min(sms, movable / p.depth);
+  if (movable * words <= 16 || p.bands < 2) p.bands = 1, p.depth = 1;
+  int most = 0;
+  for (int b = 0; b < p.bands; ++b) {
+    const int r0 = sv_band_row(b, p.bands, movable), r1 = sv_band_row(b + 1, p.bands, movable);
+    if (p.bands > 1 && r1 - r0 < p.depth) return p;
+    int lo, hi;
+    for (int py = 0; py < 2; ++py) {
+      sv_phase_rows(n, r0, r1, py, p.depth, &lo, &hi);
+      most = std::max(most, hi - lo);
+    }
+    p.rows = std::max(p.rows, std::min(r1 + p.depth, G.R) - std::max(r0 - p.depth, 0));
+  }
+  p.items = std::max(4, (most * words + 3) / 4 * 4);
+  // a word of a phase each; in an exchange up to four words of the neighbours' rows
+  p.group = (std::max(p.items, p.bands > 1 ? 2 * p.depth * words : 0) + 31) / 32 * 32;
+  // Draw warps share the schedulers with the update warps, which they slow: no more of them than keep ahead
+  // (n = 512, 40 words: 4, 6, 8, 12 draw warps 1.14, 1.10, 1.17, 1.25 us; n = 1024, 80 words: 8, 12, 16 1.93,
+  // 1.84, 1.88 us).  Batches long enough that the barrier at their end does not count (n = 512: 4 and 8
+  // phases 1.14 and 1.10 us).
+  const int draw_warps = p.items <= 20 ? 4 : p.items <= 56 ? 6 : 12;
+  p.batch = p.items <= 56 ? 8 : p.items <= 96 ? 4 : p.items <= 256 ? 2 : 1;
+  auto bytes = [&]() {
+    return (((size_t)chains * 4 * p.rows * G.P + 3) / 4 * 4 + (size_t)2 * p.batch * 2 * M * p.items +
+            4 * (size_t)(p.depth + 1) + p.group) * sizeof(uint32_t);  // idle lanes read past the drawn bits
+  };
+  p.smem = bytes();
+  if (chains * p.group > 512 || p.smem > 220 * 1024 || (p.bands > 1 && !coop) || p.bands > sms) return p;
+  p.threads = chains * p.group + 32 * std::min(draw_warps, (kSvBandThreads - chains * p.group) / 32);
+  p.xbuf_words = (size_t)2 * p.bands * 2 * chains * p.depth * 4 * words;
+  p.kernel = chains == 1 ? (p.sum ? (void*)k_sv_bands<1, true> : (void*)k_sv_bands<1, false>)
+                         : (p.sum ? (void*)k_sv_bands<2, true> : (void*)k_sv_bands<2, false>);
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.threads, p.smem) != cudaSuccess) {
+    cudaGetLastError();
+    return p;
+  }
+  p.ok = per_sm >= 1;
+  return p;
 }
 
-SvClusterPlan sv_cluster_plan(const SvGeom& G, int chains) {
-  return chains == 1 ? sv_cluster_plan_for<1>(G) : sv_cluster_plan_for<2>(G);
-}
+// Allocates and runs: `chains` (1 or 2) chains start back to back in dev.chains.
+struct SvRun {
+  SvGeom G;
+  int chains;
+  std::vector<uint32_t> T;
+  SvBandPlan plan;
+  SvDevice dev;
+  cudaStream_t st;
+  bool bands = false;
 
-// Per-CTA work above which the whole-GPU per-sub-sweep kernels are faster than one cluster.
-constexpr int kSvClusterMaxItems = 256;
+  // keep: run() is called again, from the same start.
+  rt_status prepare(int engine, bool keep) {
+    dev.stream = st;
+    // Engine 2 is refused where 16 CTAs cannot hold the chains.
+    if (engine == 2 && (size_t)chains * 4 * ((G.R + 15) / 16) * G.P * sizeof(uint32_t) > 200 * 1024)
+      return fail(RT_ERR_INVALID_ARGUMENT, "six-vertex: no thread-block cluster holds this size (engine 2)");
+    if (engine != 1) plan = sv_band_plan(G, chains, T);
+    // 256 words a band (n = 2048): 5.4 us a sweep, per-sub-sweep kernels 8.9; 484 (n = 2800): 13-15 and 11.
+    bands = plan.ok && (engine == 2 || plan.items <= 320);
+    const size_t bytes = chains * G.chain_words * sizeof(uint32_t);
+    if (rt_status e = dev_alloc(&dev.chains, bytes, st)) return e;
+    if (bands || keep)
+      if (rt_status e = dev_alloc(&dev.other, (bands ? 2 : 1) * bytes, st)) return e;
+    if (rt_status e = dev_alloc(&dev.flag, 2 * sizeof(int), st)) return e;
+    if (bands && plan.bands > 1)
+      if (rt_status e = dev_alloc(&dev.xbuf, plan.xbuf_words * sizeof(uint64_t), st)) return e;
+    cudaMemsetAsync(dev.flag, 0, 2 * sizeof(int), st);
+    return RT_OK;
+  }
 
-bool sv_use_cluster(const SvGeom& G, const SvClusterPlan& p, int engine) {
-  if (engine == 1 || !p.ok) return false;
-  if (engine == 2) return true;
-  return (int64_t)p.rpc * ((G.n / 2) / 32 + 1) <= kSvClusterMaxItems;
-}
-
-// Sub-sweeps [s0, s0 + count) on `chains` (1 or 2) chains stored back to back at dev;
-// returns the kernel launches, or -1 when engine 2 was asked for and no cluster fits.
-int64_t sv_run(uint32_t* dev, int chains, const SvGeom& G, const std::vector<uint32_t>& T, uint64_t seed,
-               uint32_t stream, int64_t s0, int64_t count, cudaStream_t st, int engine) {
-  const SvClusterPlan plan = engine == 1 ? SvClusterPlan{} : sv_cluster_plan(G, chains);
-  if (engine == 2 && !plan.ok) return -1;
-  int64_t launches = 0;
-  if (sv_use_cluster(G, plan, engine)) {
-    SvClusterArgs A{};
-    A.base = dev;
+  // Sub-sweeps [s0, s0 + count), whole sweeps, from the start states; returns where the states are.
+  uint32_t* run(uint64_t seed, uint32_t stream, int64_t s0, int64_t count) {
+    const size_t words = chains * G.chain_words;
+    if (count == 0) return dev.chains;
+    if (!bands) {
+      SvLaunch L{};
+      L.base = dev.chains;
+      if (dev.other) {
+        L.base = dev.other;
+        cudaMemcpyAsync(dev.other, dev.chains, words * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+      }
+      L.chain_words = G.chain_words;
+      L.class_words = G.class_words;
+      L.P = G.P;
+      L.n = G.n;
+      sv_leaves(T.data(), L.leaf);
+      L.seed = seed;
+      L.stream = stream;
+      for (int64_t s = s0; s < s0 + count; ++s) {
+        fill_launch(L, G, s);
+        const int threads = L.words * L.rows;
+        if (threads <= 0) continue;
+        pdl_launch(k_sv_sub, dim3((threads + 127) / 128, chains), dim3(128), st, L);
+      }
+      return L.base;
+    }
+    SvBandArgs A{};
     A.chain_words = G.chain_words;
     A.class_words = G.class_words;
     A.P = G.P;
     A.n = G.n;
     A.R = G.R;
-    A.rpc = plan.rpc;
-    sv_leaves(T.data(), A.leaf);
+    A.words = (G.n - 1) / 2 / 32 + 1;
+    A.bands = plan.bands;
+    A.depth = plan.depth;
+    A.group = plan.group;
+    A.batch = plan.batch;
+    A.items = plan.items;
+    A.rows = plan.rows;
+    uint32_t order[9];
+    const int by_sum[9] = {0, 1, 2, 5, 8, 0, 0, 0, 0};  // a threshold of each k1 + k2
+    for (int m = 0; m < 9; ++m) order[m] = T[plan.sum ? by_sum[m] : m];
+    sv_leaves(order, A.leaf);
     A.seed = seed;
     A.stream = stream;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.C);
-    cfg.blockDim = dim3(plan.threads);
-    cfg.dynamicSmemBytes = plan.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = plan.C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    constexpr int64_t kChunk = 8192;  // sub-sweeps per launch
-    for (int64_t done = 0; done < count; done += kChunk) {
-      A.s0 = s0 + done;
-      A.count = std::min(kChunk, count - done);
-      if (chains == 1)
-        cudaLaunchKernelEx(&cfg, k_sv_cluster<1>, A);
-      else
-        cudaLaunchKernelEx(&cfg, k_sv_cluster<2>, A);
-      ++launches;
+    A.xbuf = dev.xbuf;
+    A.error = dev.flag + 1;
+    A.max_spin = 1L << 22;
+    A.src = dev.chains;
+    constexpr int64_t kChunk = 1 << 14;  // sweeps per launch: bounds one launch to a fraction of a second
+    for (int64_t done = 0; done < count / 4; done += kChunk) {
+      A.dst = A.src == dev.other ? dev.other + words : dev.other;
+      A.s0 = s0 + 4 * done;
+      A.sweeps = (int)std::min(kChunk, count / 4 - done);
+      void* args[] = {&A};
+      if (plan.bands > 1) {
+        cudaMemsetAsync(dev.xbuf, 0, plan.xbuf_words * sizeof(uint64_t), st);  // no stale tags
+        cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.bands), dim3(plan.threads), args, plan.smem, st);
+      } else {
+        cudaLaunchKernel(plan.kernel, dim3(1), dim3(plan.threads), args, plan.smem, st);
+      }
+      A.src = A.dst;
     }
-    return launches;
+    return const_cast<uint32_t*>(A.src);
   }
-  SvLaunch L{};
-  L.base = dev;
-  L.chain_words = G.chain_words;
-  L.class_words = G.class_words;
-  L.P = G.P;
-  L.n = G.n;
-  sv_leaves(T.data(), L.leaf);
-  L.seed = seed;
-  L.stream = stream;
-  for (int64_t s = s0; s < s0 + count; ++s) {
-    fill_launch(L, G, s);
-    const int threads = L.words * L.rows;
-    if (threads <= 0) continue;
-    pdl_launch(k_sv_sub, dim3((threads + 127) / 128, chains), dim3(128), st, L);
-    ++launches;
-  }
-  return launches;
-}
+};
 
 int64_t sv_interior_points(int n) { return (int64_t)(n - 1) * (n - 1); }
 
@@ -584,32 +854,30 @@ RT_API rt_status rt_sv_walk(int32_t* h, int32_t n, int64_t sweeps, int64_t seed,
   const SvGeom G = sv_geom(n);
   const std::vector<uint32_t> T = sv_thresholds_host(a, b, c);
   cudaStream_t st = (cudaStream_t)o.cuda_stream;
-  SvDevice dev;
-  if (cudaMalloc(&dev.chains, G.chain_words * sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(RT_ERR_OUT_OF_MEMORY, "six-vertex walk: device allocation failed");
-  }
+  SvRun R{G, 1, T};
+  R.st = st;
+  if (rt_status e = R.prepare(o.engine, false)) return e;
   std::vector<uint32_t> bits(G.chain_words);
   sv_pack(h, G, bits.data());
-  cudaMemcpyAsync(dev.chains, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(R.dev.chains, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, st);
-  const int64_t launches = sv_run(dev.chains, 1, G, T, (uint64_t)seed, o.fast_stream, 0, 4 * sweeps, st, o.engine);
-  if (launches < 0) {
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return fail(RT_ERR_INVALID_ARGUMENT, "six-vertex walk: no thread-block cluster holds this size (engine 2)");
-  }
+  const uint32_t* at = R.run((uint64_t)seed, o.fast_stream, 0, 4 * sweeps);
+  cudaError_t err = cudaGetLastError();
   cudaEventRecord(e1, st);
-  cudaMemcpyAsync(bits.data(), dev.chains, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-  const cudaError_t err = cudaStreamSynchronize(st);
+  int flag[2] = {0, 0};
+  cudaMemcpyAsync(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(flag, R.dev.flag, sizeof flag, cudaMemcpyDeviceToHost, st);
+  const cudaError_t waited = cudaStreamSynchronize(st);
+  if (err == cudaSuccess) err = waited;
   float ms = 0.f;
   if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (err != cudaSuccess) return fail(RT_ERR_CUDA, std::string("six-vertex walk: ") + cudaGetErrorString(err));
+  if (flag[1]) return fail(RT_ERR_TIMEOUT, "six-vertex walk: a band gave up waiting for a neighbour's rows");
   std::vector<int32_t> start(h, h + (size_t)(n + 1) * (n + 1));
   sv_unpack(bits.data(), G, start.data(), h);
   if (stats) {
@@ -654,41 +922,38 @@ RT_API rt_status rt_sv_cftp(const int32_t* hmax, const int32_t* hmin, int32_t n,
   const SvGeom G = sv_geom(n);
   const std::vector<uint32_t> T = sv_thresholds_host(a, b, c);
   cudaStream_t st = (cudaStream_t)o.cuda_stream;
-  SvDevice dev;
-  if (cudaMalloc(&dev.chains, 2 * G.chain_words * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&dev.flag, sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(RT_ERR_OUT_OF_MEMORY, "six-vertex cftp: device allocation failed");
-  }
+  SvRun R{G, 2, T};
+  R.st = st;
+  if (rt_status e = R.prepare(o.engine, true)) return e;
   std::vector<uint32_t> start(2 * G.chain_words);
   sv_pack(hmax, G, start.data());
   sv_pack(hmin, G, start.data() + G.chain_words);
+  cudaMemcpyAsync(R.dev.chains, start.data(), start.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
   if (stats) std::memset(stats, 0, sizeof *stats);
+  const uint32_t* at = R.dev.chains;
   float total_ms = 0.f;
   int64_t Tsw = first_sweeps, total_sub = 0;
   for (int attempt = 1; attempt <= max_attempts; ++attempt, Tsw *= 2) {
     if (Tsw > ((int64_t)1 << 44)) break;
-    cudaMemcpyAsync(dev.chains, start.data(), start.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(dev.flag, 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(R.dev.flag, 0, 2 * sizeof(int), st);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
-    if (sv_run(dev.chains, 2, G, T, (uint64_t)seed, o.fast_stream, -4 * Tsw, 4 * Tsw, st, o.engine) < 0) {
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      return fail(RT_ERR_INVALID_ARGUMENT, "six-vertex cftp: no thread-block cluster holds this size (engine 2)");
-    }
+    at = R.run((uint64_t)seed, o.fast_stream, -4 * Tsw, 4 * Tsw);
     cudaEventRecord(e1, st);
-    k_sv_diff<<<64, 256, 0, st>>>(dev.chains, dev.chains + G.chain_words, G.chain_words, dev.flag);
-    uint32_t differ = 1;
-    cudaMemcpyAsync(&differ, dev.flag, sizeof differ, cudaMemcpyDeviceToHost, st);
-    const cudaError_t err = cudaStreamSynchronize(st);
+    k_sv_diff<<<64, 256, 0, st>>>(at, at + G.chain_words, G.chain_words, (uint32_t*)R.dev.flag);
+    cudaError_t err = cudaGetLastError();
+    int flag[2] = {1, 0};
+    cudaMemcpyAsync(flag, R.dev.flag, sizeof flag, cudaMemcpyDeviceToHost, st);
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    if (err == cudaSuccess) err = waited;
     float ms = 0.f;
     if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (err != cudaSuccess) return fail(RT_ERR_CUDA, std::string("six-vertex cftp: ") + cudaGetErrorString(err));
+    if (flag[1]) return fail(RT_ERR_TIMEOUT, "six-vertex cftp: a band gave up waiting for a neighbour's rows");
     total_ms += ms;
     total_sub += 4 * Tsw;
     if (stats) {
@@ -697,9 +962,9 @@ RT_API rt_status rt_sv_cftp(const int32_t* hmax, const int32_t* hmin, int32_t n,
       stats->flip_attempts += 2 * sv_interior_points(n) * Tsw;
       stats->seconds = total_ms * 1e-3;
     }
-    if (!differ) {
+    if (!flag[0]) {
       std::vector<uint32_t> bits(G.chain_words);
-      cudaMemcpy(bits.data(), dev.chains, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost);
+      cudaMemcpy(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost);
       sv_unpack(bits.data(), G, hmax, out);
       if (stats) stats->final_steps = 4 * Tsw;
       return RT_OK;
@@ -707,7 +972,7 @@ RT_API rt_status rt_sv_cftp(const int32_t* hmax, const int32_t* hmin, int32_t n,
   }
   // not coalesced: out holds the top chain of the last attempt
   std::vector<uint32_t> bits(G.chain_words);
-  if (cudaMemcpy(bits.data(), dev.chains, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost) == cudaSuccess)
+  if (cudaMemcpy(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost) == cudaSuccess)
     sv_unpack(bits.data(), G, hmax, out);
   return fail(RT_ERR_NOT_COALESCED, "six-vertex cftp: chains did not coalesce within max_attempts");
 }
