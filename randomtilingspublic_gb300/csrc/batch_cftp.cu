@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "batch_cftp.cuh"
+#include "batch_planes.cuh"
 #include "domino_rules.h"
 #include "rng.cuh"
 #include "rt_internal.h"
@@ -31,7 +32,9 @@
 namespace rt {
 namespace {
 
-constexpr int kBatchThreads = 256;
+// 512 threads, two CTAs an SM: 512 mixed instances 61 ms; 384 threads and three CTAs 69, 512 and three (40
+// registers) 98, 256 and four 86; one hexagon of side 32 30 ms, with 256 threads 37.
+constexpr int kBatchThreads = 512;
 
 #define BT_CUDA(expr)                                                                   \
   do {                                                                                  \
@@ -61,6 +64,7 @@ struct BatchArgs {
   unsigned* finished;  // instances whose result is final
   int* error;          // set when a bounded wait for an instance's lock gave up
   long max_spin;       // bound of that wait, and of a helper's rounds without work
+  size_t smem;         // dynamic shared memory of a CTA
 };
 
 // One domino half-sweep of colour t on both chains of an instance held whole in shared
@@ -84,81 +88,79 @@ __device__ void lozenge_step(uint8_t* sm, const DevInstance& in, int r, int64_t 
   __syncthreads();
 }
 
-// Runs one instance's CFTP in shared memory: tmax / tmin / out are its colour arrays in
-// global or mapped host memory (loaded with volatile reads, since a serving slot is reused).
-// Returns the attempts run (negative when it did not coalesce) and the last look-back.
-__device__ void run_instance(uint8_t* sm, const DevInstance& in, const uint8_t* tmax, const uint8_t* tmin, uint8_t* out,
-                             uint32_t lz_c4, uint32_t lz_c8, uint32_t* red, int* attempts_out, int64_t* look_out) {
-  const int ncol = in.model == 0 ? 2 : 3;
-  const size_t chain = (size_t)ncol * in.N * in.P;
-  const uint32_t* gmax = reinterpret_cast<const uint32_t*>(tmax);
-  const uint32_t* gmin = reinterpret_cast<const uint32_t*>(tmin);
-  uint32_t* s32 = reinterpret_cast<uint32_t*>(sm);
-  const int words = (int)(chain / 4);
-  int attempts = 0;
-  int64_t look = 0;
-  bool done = false;
-  for (int att = 0; att < in.max_attempts && !done; ++att) {
-    // chain 0 starts at the min tiling, chain 1 at the max tiling
-    for (int w = threadIdx.x; w < words; w += kBatchThreads) {
-      s32[w] = __ldcv(gmin + w);
-      s32[words + w] = __ldcv(gmax + w);
-    }
-    __syncthreads();
-    const int64_t T = in.first_sweeps << att;
-    look = ncol * T;
-    for (int64_t h = -look; h < 0; ++h) {
-      if (in.model == 0) domino_half_sweep(sm, in, (h & 1) ? 0 : 1, h);
-      else lozenge_step(sm, in, (int)(((h % 3) + 3) % 3), h, lz_c4, lz_c8);
-    }
-    uint32_t differ = 0;
-    for (int w = threadIdx.x; w < words; w += kBatchThreads) differ += s32[w] != s32[words + w];
-    differ = block_sum<kBatchThreads>(differ, red);
-    attempts = att + 1;
-    done = differ == 0;
-  }
-  uint32_t* gout = reinterpret_cast<uint32_t*>(out);
-  for (int w = threadIdx.x; w < words; w += kBatchThreads) __stcg(gout + w, s32[words + w]);
-  *attempts_out = done ? attempts : -attempts;
-  *look_out = look;
-}
-
 __device__ __forceinline__ int ld_volatile_i(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p) {
   return *reinterpret_cast<const volatile unsigned long long*>(p);
 }
 
 // Attempt att of an instance in shared memory (chain 0 from the min tiling, chain 1 from the
-// max tiling, half-sweeps [-look, 0)): 1 coalesced, 0 not, -1 abandoned because a smaller
-// attempt of the instance coalesced meanwhile (checked every 256 steps).
-__device__ int run_attempt(uint8_t* sm, const DevInstance& in, const InstState* st, int att, const uint8_t* tilings,
-                           uint32_t lz_c4, uint32_t lz_c8, uint32_t* red, int* s_flag) {
+// max tiling, half-sweeps [-look, 0)): 1 coalesced, 0 not, -1 abandoned because stop() said so
+// (asked every 256 steps).  As bit planes where they hold the instance (*planes), else as bytes.
+template <class Stop>
+__device__ int run_attempt(uint8_t* sm, size_t smem, const DevInstance& in, int att, const uint8_t* tmax,
+                           const uint8_t* tmin, uint32_t lz_c4, uint32_t lz_c8, uint32_t* red, bool* planes, Stop stop) {
+  __shared__ int s_cnt[3];
   const int ncol = in.model == 0 ? 2 : 3;
   const int words = (int)((size_t)ncol * in.N * in.P / 4);
-  const uint32_t* gmax = reinterpret_cast<const uint32_t*>(tilings + in.off_max);
-  const uint32_t* gmin = reinterpret_cast<const uint32_t*>(tilings + in.off_min);
+  const uint32_t* gmax = reinterpret_cast<const uint32_t*>(tmax);
+  const uint32_t* gmin = reinterpret_cast<const uint32_t*>(tmin);
   uint32_t* s32 = reinterpret_cast<uint32_t*>(sm);
-  for (int w = threadIdx.x; w < words; w += kBatchThreads) {
-    s32[w] = __ldcv(gmin + w);
-    s32[words + w] = __ldcv(gmax + w);
-  }
-  __syncthreads();
   const int64_t look = ncol * (in.first_sweeps << att);
-  for (int64_t h = -look; h < 0; ++h) {
-    if (in.model == 0) domino_half_sweep(sm, in, (h & 1) ? 0 : 1, h);
-    else lozenge_step(sm, in, (int)(((h % 3) + 3) % 3), h, lz_c4, lz_c8);
-    if (((h + look) & 255) == 255) {  // uniform over the CTA
-      if (threadIdx.x == 0) *s_flag = ld_volatile_i(&st->best) < att;
-      __syncthreads();
-      const int stop = *s_flag;
-      __syncthreads();
-      if (stop) return -1;
-    }
-  }
+  const BpLayout L = bp_layout(in.model, in.N, in.P);
+  // the plane kernels' first interval is [0, width up)
+  *planes = (size_t)L.words * 4 <= smem &&
+            (in.model != 0 || (in.lo_up[0] | in.lo_up[1] | in.lo_up[2] | in.lo_up[3]) == 0) &&
+            bp_load<kBatchThreads>(s32, L, in, gmax, gmin, s_cnt);
   uint32_t differ = 0;
-  for (int w = threadIdx.x; w < words; w += kBatchThreads) differ += s32[w] != s32[words + w];
+  if (*planes) {
+    const int items = s_cnt[0], units = s_cnt[1];
+    const bool ran = in.model == 0 ? bp_domino<kBatchThreads>(s32, L, in, look, items, units, stop)
+                                   : bp_lozenge<kBatchThreads>(s32, L, in, look, lz_c4, lz_c8, items, units, stop);
+    if (!ran) return -1;
+    differ = bp_differ<kBatchThreads>(s32, L, in);
+  } else {
+    __syncthreads();  // bp_load's reads
+    for (int w = threadIdx.x; w < words; w += kBatchThreads) {
+      s32[w] = __ldcv(gmin + w);
+      s32[words + w] = __ldcv(gmax + w);
+    }
+    __syncthreads();
+    for (int64_t h = -look; h < 0; ++h) {
+      if (in.model == 0) domino_half_sweep(sm, in, (h & 1) ? 0 : 1, h);
+      else lozenge_step(sm, in, (int)(((h % 3) + 3) % 3), h, lz_c4, lz_c8);
+      if (((h + look) & 255) == 255 && stop()) return -1;
+    }
+    for (int w = threadIdx.x; w < words; w += kBatchThreads) differ += s32[w] != s32[words + w];
+  }
   differ = block_sum<kBatchThreads>(differ, red);
   return differ == 0 ? 1 : 0;
+}
+
+// Writes the top chain of an attempt, in shared memory as run_attempt left it.
+__device__ void write_top(const uint8_t* sm, const DevInstance& in, bool planes, uint8_t* out) {
+  const uint32_t* s32 = reinterpret_cast<const uint32_t*>(sm);
+  const BpLayout L = bp_layout(in.model, in.N, in.P);
+  const int words = (int)((size_t)(in.model == 0 ? 2 : 3) * in.N * in.P / 4);
+  uint32_t* gout = reinterpret_cast<uint32_t*>(out);
+  for (int w = threadIdx.x; w < words; w += kBatchThreads)
+    __stcg(gout + w, planes ? bp_bytes_of(s32, L, in, 1, w) : s32[words + w]);
+}
+
+// Runs one instance's CFTP in shared memory: tmax / tmin / out are its colour arrays in
+// global or mapped host memory (loaded with volatile reads, since a serving slot is reused).
+// Returns the attempts run (negative when it did not coalesce) and the last look-back.
+__device__ void run_instance(uint8_t* sm, size_t smem, const DevInstance& in, const uint8_t* tmax, const uint8_t* tmin,
+                             uint8_t* out, uint32_t lz_c4, uint32_t lz_c8, uint32_t* red, int* attempts_out,
+                             int64_t* look_out) {
+  int attempts = 0;
+  bool done = false, planes = false;
+  for (int att = 0; att < in.max_attempts && !done; ++att) {
+    done = run_attempt(sm, smem, in, att, tmax, tmin, lz_c4, lz_c8, red, &planes, [] { return false; }) == 1;
+    attempts = att + 1;
+  }
+  write_top(sm, in, planes, out);
+  *attempts_out = done ? attempts : -attempts;
+  *look_out = (in.model == 0 ? 2 : 3) * (in.first_sweeps << (attempts - 1));
 }
 
 // Records attempt att (outcome of run_attempt).  A coalesced attempt smaller than any
@@ -166,10 +168,9 @@ __device__ int run_attempt(uint8_t* sm, const DevInstance& in, const InstState* 
 // instance's output under the instance's lock.  The CTA whose record completes the instance
 // (a coalesced attempt and every smaller one finished, or every attempt finished) writes the
 // attempt count and the look-back: the result is that of running the attempts in order.
-__device__ void record_attempt(uint8_t* sm, DevInstance* g, const DevInstance& in, InstState* st, int att, int outcome,
-                               uint8_t* tilings, const BatchArgs& a, int* s_flag) {
+__device__ void record_attempt(const uint8_t* sm, bool planes, DevInstance* g, const DevInstance& in, InstState* st,
+                               int att, int outcome, uint8_t* tilings, const BatchArgs& a, int* s_flag) {
   const int ncol = in.model == 0 ? 2 : 3;
-  const int words = (int)((size_t)ncol * in.N * in.P / 4);
   if (outcome == 1 || (outcome == 0 && att == in.max_attempts - 1)) {
     if (threadIdx.x == 0) {
       int write = 0;
@@ -192,9 +193,7 @@ __device__ void record_attempt(uint8_t* sm, DevInstance* g, const DevInstance& i
     }
     __syncthreads();
     if (*s_flag) {
-      const uint32_t* s32 = reinterpret_cast<const uint32_t*>(sm);
-      uint32_t* gout = reinterpret_cast<uint32_t*>(tilings + in.off_out);
-      for (int w = threadIdx.x; w < words; w += kBatchThreads) __stcg(gout + w, s32[words + w]);
+      write_top(sm, in, planes, tilings + in.off_out);
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -253,7 +252,7 @@ __device__ int helper_limit(const DevInstance& in, const InstState* st) {
   return min(owner_limit(in, st), lowest_unfinished + 1 + kSpeculate);
 }
 
-__global__ void __launch_bounds__(kBatchThreads, 4) k_batch_cftp(BatchArgs a, uint32_t lz_c4, uint32_t lz_c8) {
+__global__ void __launch_bounds__(kBatchThreads, 2) k_batch_cftp(BatchArgs a, uint32_t lz_c4, uint32_t lz_c8) {
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ DevInstance s_in;
   __shared__ int s_idx, s_att, s_flag, s_pick;
@@ -323,8 +322,18 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch_cftp(BatchArgs a, ui
     if (threadIdx.x == 0) s_in = *g;  // read by every thread from shared memory
     __syncthreads();
     const DevInstance& in = s_in;
-    const int outcome = run_attempt(sm, in, &a.state[idx], att, a.tilings, lz_c4, lz_c8, red, &s_flag);
-    record_attempt(sm, g, in, &a.state[idx], att, outcome, a.tilings, a, &s_flag);
+    // Abandoned once a smaller attempt of the instance has coalesced.
+    auto stop = [&]() -> bool {
+      if (threadIdx.x == 0) s_flag = ld_volatile_i(&a.state[idx].best) < att;
+      __syncthreads();
+      const bool now = s_flag;
+      __syncthreads();
+      return now;
+    };
+    bool planes;
+    const int outcome = run_attempt(sm, a.smem, in, att, a.tilings + in.off_max, a.tilings + in.off_min, lz_c4, lz_c8, red,
+                                    &planes, stop);
+    record_attempt(sm, planes, g, in, &a.state[idx], att, outcome, a.tilings, a, &s_flag);
   }
 }
 
@@ -345,6 +354,7 @@ struct ServeArgs {
   int slots;
   size_t slot_bytes;
   long idle_polls;             // polls without work before a CTA leaves
+  size_t smem;                 // dynamic shared memory of a CTA
 };
 
 __device__ __forceinline__ uint64_t ld_acquire_sys(const uint64_t* p) {
@@ -361,7 +371,7 @@ __device__ __forceinline__ void st_release_sys(uint64_t* p, uint64_t v) {
 // request's CFTP and releases its done word.  A CTA leaves after idle_polls polls without
 // work or when the host sets shutdown; the host relaunches the kernel when it finds
 // published work and no kernel running.
-__global__ void __launch_bounds__(kBatchThreads) k_serve(ServeArgs a, uint32_t lz_c4, uint32_t lz_c8) {
+__global__ void __launch_bounds__(kBatchThreads, 2) k_serve(ServeArgs a, uint32_t lz_c4, uint32_t lz_c8) {
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ long long s_ticket;
   __shared__ uint32_t red[kBatchThreads / 32];
@@ -399,7 +409,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_serve(ServeArgs a, uint32_t l
     uint8_t* base = a.data + (size_t)slot * a.slot_bytes;
     int att;
     int64_t look;
-    run_instance(sm, in, base + in.off_max, base + in.off_min, base + in.off_out, lz_c4, lz_c8, red, &att, &look);
+    run_instance(sm, a.smem, in, base + in.off_max, base + in.off_min, base + in.off_out, lz_c4, lz_c8, red, &att, &look);
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -492,6 +502,12 @@ bool split_ok(const int32_t* t, const DevInstance& d, uint8_t* dst) {
   return true;
 }
 
+// Shared memory of a CTA that runs an instance: both chains as bytes, and as planes where they fit.
+size_t smem_of(const DevInstance& d, size_t limit) {
+  const size_t bytes = (size_t)2 * (d.model == RT_MODEL_DOMINO ? 2 : 3) * d.N * d.P, planes = bp_bytes(d.model, d.N, d.P);
+  return planes <= limit ? std::max(bytes, planes) : bytes;
+}
+
 size_t chain_bytes_of(const DevInstance& d) { return (size_t)(d.model == RT_MODEL_DOMINO ? 2 : 3) * d.N * d.P; }
 
 // Runs `work` (which takes items off a shared counter) on up to 32 host threads, fewer for
@@ -552,7 +568,7 @@ RT_API rt_status rt_cftp_batch(rt_cftp_instance* inst, int32_t count, void* cuda
     size_t chain = 0;
     if (rt_status st = pack_instance(x, &all[(size_t)k], &chain)) return st;
     if (2 * chain <= smem_limit) {
-      smem_max = std::max(smem_max, 2 * chain);
+      smem_max = std::max(smem_max, smem_of(all[(size_t)k], smem_limit));
       packed_idx.push_back(k);
       ++n_small;
     } else {
@@ -560,6 +576,8 @@ RT_API rt_status rt_cftp_batch(rt_cftp_instance* inst, int32_t count, void* cuda
       if (csize[(size_t)k] == 0) large_idx.push_back(k);
     }
   }
+  // The largest first: they take longest, and the CTAs that run out of instances help with their attempts.
+  std::stable_sort(packed_idx.begin(), packed_idx.end(), [&](int x, int y) { return inst[x].n_side > inst[y].n_side; });
   std::vector<ClusterGroup> groups;
   for (int C = 2; C <= 16; ++C) {
     ClusterGroup g;
@@ -651,9 +669,11 @@ RT_API rt_status rt_cftp_batch(rt_cftp_instance* inst, int32_t count, void* cuda
       cudaFuncSetAttribute(k_batch_cftp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
       int per_sm = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_cftp, kBatchThreads, smem_max);
-      grid = std::max(1, std::min(n_small, std::max(1, per_sm) * sms));
+      // Few instances: the SMs left over run attempts ahead of the instances' own CTAs (one hexagon of side 32:
+      // 55 -> 30 ms; 64 mixed instances 49 -> 37 ms).
+      grid = std::max(1, std::min(std::max(n_small, std::min(sms, 4 * n_small)), std::max(1, per_sm) * sms));
       BatchArgs ba{d_inst, d_state, n_small, d_tilings, d_queue, d_queue + 1, reinterpret_cast<int*>(d_queue + 2),
-                   1L << 24};
+                   1L << 24, smem_max};
       k_batch_cftp<<<grid, kBatchThreads, smem_max, stream>>>(ba, c4, c8);
       cudaError_t le = cudaGetLastError();
       if (le != cudaSuccess) {
@@ -784,7 +804,7 @@ struct rt_server {
 };
 
 static rt_status server_launch(rt_server* s) {
-  ServeArgs a{s->d_ring, s->d_desc, s->d_data, s->d_done, s->d_head, s->slots, s->slot_bytes, s->idle_polls};
+  ServeArgs a{s->d_ring, s->d_desc, s->d_data, s->d_done, s->d_head, s->slots, s->slot_bytes, s->idle_polls, s->smem};
   k_serve<<<s->grid, kBatchThreads, s->smem, s->stream>>>(a, lz_cut(0.4), lz_cut(0.8));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("server launch: ") + cudaGetErrorString(e));
@@ -825,6 +845,10 @@ RT_API rt_status rt_server_create(const rt_server_opts* o, rt_server** out) {
   const size_t chain = std::max((size_t)2 * o->max_side * pd, (size_t)3 * o->max_side * pl);
   s->slot_bytes = (3 * chain + 255) / 256 * 256;
   s->smem = 2 * chain;
+  for (int model : {RT_MODEL_DOMINO, RT_MODEL_LOZENGE}) {
+    const size_t planes = bp_bytes(model, o->max_side, (int)(model == RT_MODEL_DOMINO ? pd : pl));
+    if (planes <= (size_t)optin - 1024) s->smem = std::max(s->smem, planes);
+  }
   if (s->smem > (size_t)optin - 1024) return fail(RT_ERR_INVALID_ARGUMENT, "server_create: max_side too large for one CTA");
   s->budget = o->memory_budget_bytes;
   s->idle_polls = (long)std::max(1.0, (o->idle_seconds > 0 ? o->idle_seconds : 0.25) * 2.0e6);
