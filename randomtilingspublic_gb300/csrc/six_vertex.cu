@@ -502,6 +502,49 @@ __global__ void k_sv_diff(const uint32_t* a, const uint32_t* b, size_t words, ui
   if ((threadIdx.x & 31) == 0 && acc) atomicOr(flag, 1u);
 }
 
+// Heights (n + 1) x (n + 1) to one chain's class words, a warp per row and 64 columns; *bad is set where
+// two neighbours do not differ by one.
+__global__ void __launch_bounds__(256) k_sv_pack(const int32_t* h, uint32_t* chain, SvGeom G, int* bad) {
+  const int lane = threadIdx.x & 31, n = G.n, L = n + 1, words = G.P - 2;
+  const int it = blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+  if (it >= L * words) return;
+  const int y = it / words, w = it - y * words, o = __ldg(h) & 1;
+  bool wrong = false;
+#pragma unroll
+  for (int px = 0; px < 2; ++px) {
+    const int x = 2 * (32 * w + lane) + px;
+    uint32_t sigma = 0;
+    if (x <= n) {
+      const int v = h[(size_t)y * L + x];
+      wrong = wrong || (x < n && abs(h[(size_t)y * L + x + 1] - v) != 1) || (y < n && abs(h[(size_t)(y + 1) * L + x] - v) != 1);
+      sigma = (uint32_t)((v - o - ((x + y) & 1)) >> 1) & 1u;
+    }
+    const uint32_t bits = __ballot_sync(~0u, sigma);
+    if (lane == 0) chain[(size_t)(px | ((y & 1) << 1)) * G.class_words + (size_t)(y >> 1) * G.P + 1 + w] = bits;
+  }
+  if (__any_sync(~0u, wrong) && lane == 0) *bad = 1;
+}
+
+// The heights of a chain's class words, a warp per row: along a row the height moves by the step of
+// +-1 between two residues mod 4, from the left column, which never moves (h holds the start heights).
+__global__ void __launch_bounds__(256) k_sv_unpack(const uint32_t* chain, SvGeom G, int32_t* h) {
+  const int lane = threadIdx.x & 31, n = G.n, L = n + 1, y = blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+  if (y > n) return;
+  const uint32_t* const even = chain + (size_t)((y & 1) << 1) * G.class_words + (size_t)(y >> 1) * G.P + 1;
+  const uint32_t* const odd = even + G.class_words;
+  auto residue = [&](int x) -> int {  // without the start's parity, which both ends of a step share
+    const int k = x >> 1;
+    return ((x + y) & 1) + 2 * (int)(((x & 1 ? odd : even)[k >> 5] >> (k & 31)) & 1u);
+  };
+  int base = h[(size_t)y * L];
+  for (int x0 = 1; x0 <= n; x0 += 32) {
+    const int x = x0 + lane;
+    const uint32_t ups = __ballot_sync(~0u, x <= n && ((residue(min(x, n)) - residue(min(x, n) - 1)) & 3) == 1);
+    if (x <= n) h[(size_t)y * L + x] = base + 2 * __popc(ups & (0xffffffffu >> (31 - lane))) - (lane + 1);
+    base += 2 * __popc(ups) - 32;
+  }
+}
+
 void fill_launch(SvLaunch& L, const SvGeom& G, int64_t s) {
   L.px = (int)(s & 1);
   L.py = (int)((s >> 1) & 1);
@@ -580,10 +623,11 @@ struct SvDevice {
   uint32_t* chains = nullptr;  // the state of the per-sub-sweep kernels; the resident engine's start
   uint32_t* other = nullptr;   // resident engine: two more states, written in turn
   uint64_t* xbuf = nullptr;
-  int* flag = nullptr;  // {chains differ, a wait gave up}
+  int32_t* heights = nullptr;
+  int* flag = nullptr;  // {chains differ or heights not valid, a wait gave up}
   cudaStream_t stream = nullptr;
   ~SvDevice() {
-    for (void* p : {(void*)chains, (void*)other, (void*)xbuf, (void*)flag}) dev_free(p, stream);
+    for (void* p : {(void*)chains, (void*)other, (void*)xbuf, (void*)heights, (void*)flag}) dev_free(p, stream);
   }
 };
 
@@ -849,17 +893,41 @@ RT_API rt_status rt_sv_walk(int32_t* h, int32_t n, int64_t sweeps, int64_t seed,
   if (o.fast_stream >= 65536u) return fail(RT_ERR_INVALID_ARGUMENT, "fast_stream must be < 65536");
   double a, b, c;
   if (rt_status st = sv_check_common(n, abc, &a, &b, &c)) return st;
-  if (!sv_valid_heights(h, n)) return fail(RT_ERR_INVALID_ARGUMENT, "six-vertex: not a height function (|dh| != 1)");
-  if (rt_status st = sv_check_device()) return st;
   const SvGeom G = sv_geom(n);
+  const size_t points = (size_t)(n + 1) * (n + 1);
+  // Packed, checked and unpacked on the device from n = 96 up, where the host's 5 ns a point pass the device's two
+  // launches and one wait (walk of 4 sweeps without them: n = 95 on the host 81 us, n = 96 on the device 67, n = 512
+  // 1.4 ms and 92 us); the heights on the device take four bytes a point, 1 GB at most.
+  bool on_device = n >= 96 && n <= 16384;
+  const rt_status no_device = sv_check_device();
+  if (no_device) on_device = false;
+  const char* const invalid = "six-vertex: not a height function (|dh| != 1)";
+  if (!on_device && !sv_valid_heights(h, n)) return fail(RT_ERR_INVALID_ARGUMENT, invalid);
+  if (no_device) return sv_check_device();
   const std::vector<uint32_t> T = sv_thresholds_host(a, b, c);
   cudaStream_t st = (cudaStream_t)o.cuda_stream;
   SvRun R{G, 1, T};
   R.st = st;
-  if (rt_status e = R.prepare(o.engine, false)) return e;
-  std::vector<uint32_t> bits(G.chain_words);
-  sv_pack(h, G, bits.data());
-  cudaMemcpyAsync(R.dev.chains, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+  if (rt_status e = R.prepare(o.engine, false)) {
+    if (on_device && !sv_valid_heights(h, n)) return fail(RT_ERR_INVALID_ARGUMENT, invalid);
+    return e;
+  }
+  std::vector<uint32_t> bits;
+  if (on_device) {
+    if (rt_status e = dev_alloc(&R.dev.heights, points * sizeof(int32_t), st)) return e;
+    int bad = 0;
+    cudaMemcpyAsync(R.dev.heights, h, points * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(R.dev.chains, 0, G.chain_words * sizeof(uint32_t), st);  // the guard words
+    k_sv_pack<<<((n + 1) * (G.P - 2) + 7) / 8, 256, 0, st>>>(R.dev.heights, R.dev.chains, G, R.dev.flag);
+    cudaMemcpyAsync(&bad, R.dev.flag, sizeof bad, cudaMemcpyDeviceToHost, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("six-vertex walk: ") + cudaGetErrorString(e));
+    if (bad) return fail(RT_ERR_INVALID_ARGUMENT, invalid);
+  } else {
+    bits.resize(G.chain_words);
+    sv_pack(h, G, bits.data());
+    cudaMemcpyAsync(R.dev.chains, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+  }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -868,9 +936,12 @@ RT_API rt_status rt_sv_walk(int32_t* h, int32_t n, int64_t sweeps, int64_t seed,
   cudaError_t err = cudaGetLastError();
   cudaEventRecord(e1, st);
   int flag[2] = {0, 0};
-  cudaMemcpyAsync(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(flag, R.dev.flag, sizeof flag, cudaMemcpyDeviceToHost, st);
-  const cudaError_t waited = cudaStreamSynchronize(st);
+  if (on_device)
+    k_sv_unpack<<<(n + 1 + 7) / 8, 256, 0, st>>>(at, G, R.dev.heights);
+  else
+    cudaMemcpyAsync(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  cudaError_t waited = cudaStreamSynchronize(st);
   if (err == cudaSuccess) err = waited;
   float ms = 0.f;
   if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -878,8 +949,16 @@ RT_API rt_status rt_sv_walk(int32_t* h, int32_t n, int64_t sweeps, int64_t seed,
   cudaEventDestroy(e1);
   if (err != cudaSuccess) return fail(RT_ERR_CUDA, std::string("six-vertex walk: ") + cudaGetErrorString(err));
   if (flag[1]) return fail(RT_ERR_TIMEOUT, "six-vertex walk: a band gave up waiting for a neighbour's rows");
-  std::vector<int32_t> start(h, h + (size_t)(n + 1) * (n + 1));
-  sv_unpack(bits.data(), G, start.data(), h);
+  if (on_device) {
+    if (cudaMemcpyAsync(h, R.dev.heights, points * sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        (waited = cudaStreamSynchronize(st)) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(RT_ERR_CUDA, "six-vertex walk: copying the heights back failed");
+    }
+  } else {
+    std::vector<int32_t> start(h, h + points);
+    sv_unpack(bits.data(), G, start.data(), h);
+  }
   if (stats) {
     std::memset(stats, 0, sizeof *stats);
     stats->attempts = 1;

@@ -65,3 +65,23 @@ def test_engine_two_serves_and_refuses_what_it_did(rt):
     h = S.MinHeight(6000)
     with pytest.raises(rt.RTError):
         S(engine=2).Walk(h, 1, 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [95, 96, 97, 127, 128, 160])
+def test_heights_packed_on_the_device(rt, orc, n):
+    # sizes around the rule and around words of 32 points; heights of any parity and offset
+    S = rt.SixVertexTiler
+    for off in (0, 1, -6):
+        a = S.MaxHeight(n) + np.int32(off)
+        b = a.copy()
+        S(0.9, 1.0, 1.3, fast_stream=2).Walk(a, 9, 31)
+        orc.sv_walk(b, n, 0, 36, 31, 2, 0.9, 1.0, 1.3)
+        assert np.array_equal(a, b)
+    for y, x in ((0, 0), (n, n), (n // 2, n), (3, 64)):
+        bad = S.MinHeight(n)
+        bad[y * (n + 1) + x] += 1
+        kept = bad.copy()
+        with pytest.raises(rt.RTError, match="not a height function"):
+            S().Walk(bad, 3, 1)
+        assert np.array_equal(bad, kept)
