@@ -40,8 +40,9 @@ struct ClArgs {
   const uint8_t* start_base;
   const int4* attempt_desc;
   const uint32_t* epoch_seeds;
-  int* result;
-  int* error;      // set when a bounded wait gave up
+  size_t team_stride;  // bytes between the chains of two teams (clusters that run attempts side by side)
+  int* best;           // smallest attempt that coalesced
+  int* error;          // [team], set when a bounded wait gave up
   long max_spin;
   int silent_cta_plus1;
 };
@@ -65,6 +66,8 @@ struct ClPlan {
 // Words per half-sweep up to which the automatic choice is the cluster.
 int64_t cl_auto_words(bool fast);
 
+constexpr int kClTeams = 4;  // attempts of a coupling from the past side by side
+
 struct ClusterEngine {
   ClPlan plan;
   bool ready = false;
@@ -75,7 +78,8 @@ struct ClusterEngine {
   int64_t runs_cap = 0;
   uint32_t* d_epoch = nullptr;  // epoch seeds then attempt descriptors
   size_t epoch_cap = 0;
-  int* d_result = nullptr;  // {attempts run, coalesced, error}
+  int* d_result = nullptr;     // {smallest attempt that coalesced, error of each team}
+  uint8_t* d_teams = nullptr;  // two chains per team
   bool pending_error_check = false;
 
   ~ClusterEngine();

@@ -1007,6 +1007,9 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   // kLaunchHalfSweeps (a launch of well under a second at order 1024); an attempt longer than
   // that, or a sampler the run kernel does not take, runs attempt by attempt from the host.
   const int64_t kLaunchHalfSweeps = (int64_t)1 << 21;
+  // TinyMT colours are drawn on the host for every attempt of a group, needed or not (5 ns a half-sweep): the
+  // first groups are short (order 15, first look-back 372: 1.6 ms, with one group 11.4).
+  int64_t group_half_sweeps = fast ? kLaunchHalfSweeps : (int64_t)1 << 14;
   bool pers = false;
   if (rt_status st = s->use_persistent(&pers)) return st;
   const bool one_launch = pers && !s->on_grid && (s->resident == 2 || s->resident == 4) && o.rng_mode != RT_RNG_MTGP;
@@ -1015,8 +1018,10 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   while (att < max_attempts && !coalesced) {
     int n = 0;
     int64_t tot = 0;
-    while (one_launch && att + n < max_attempts && tot + look_back(att + n) <= kLaunchHalfSweeps)
+    while (one_launch && att + n < max_attempts &&
+           tot + look_back(att + n) <= (n ? group_half_sweeps : kLaunchHalfSweeps))
       tot += look_back(att + n++);
+    group_half_sweeps = std::min(8 * group_half_sweeps, kLaunchHalfSweeps);
     if (n > 0) {
       std::vector<std::vector<RunEngine::Epoch>> epochs((size_t)n);
       for (int q = 0; !fast && q < n; ++q)

@@ -21,6 +21,9 @@
 // Draws do not depend on the state: warps of their own make them, a run ahead, and compose a run's
 // steps into one pair of move words per 32 slots (as domino_cluster.cu).
 //
+// Coupling from the past where one CTA holds the chains: four CTAs run attempts side by side, as in
+// domino_cluster.cu (exact sample of the hexagon of side 20 in fast mode: 7.3 -> 5.9 ms).
+//
 // What bounds it: the exchange of each run, 0.5 us in a cluster and 0.85 us through L2.  The byte kernel
 // (lozenge_resident.cu) spent its step on the rotation and rebuild of bytes: hexagon 512 0.73 us a step
 // (TinyMT; before 2.20) and 0.91 us (fast mode; 2.14), hexagon 20 0.36 (1.39) and 0.35 (1.36).  It stays for inputs whose edges disagree or whose candidates
@@ -53,7 +56,7 @@ struct LbArgs {
   uint32_t lo_up, w_up, lo_dn, w_dn;  // TinyMT: times 2^9, tested on the tempered word
   uint4* tmt;
   const uint4* tmt_params;
-  const uint32_t* runs;  // TinyMT: (colour << 30) | length
+  const uint32_t* runs;  // TinyMT: (colour << 30) | (epoch start << 29) | length
   int nruns;             // fast mode: steps
   uint64_t seed;
   uint32_t stream;
@@ -61,6 +64,15 @@ struct LbArgs {
   uint64_t* xbuf;  // [2 parities][band][to above, to below][word][chain]
   int* error;
   long max_spin;
+  // Coupling from the past (attempts > 0, two chains, kLbOne): CTA `team` runs attempts team, team + teams, ...
+  // from the chains at start, into chains of its own at base + team * team_stride.
+  int attempts;
+  int64_t first_sweeps;  // fast mode: attempt k runs 3 first_sweeps << k steps up to step 0
+  const uint8_t* start;
+  size_t team_stride;
+  int* best;                    // smallest attempt that coalesced
+  const int4* attempt_desc;     // TinyMT: {first run, runs, first epoch seed, 0}
+  const uint32_t* epoch_seeds;  // a run that starts an epoch (bit 29) seeds the generators from the next
 };
 
 __device__ __forceinline__ uint32_t lb_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -124,9 +136,12 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   __shared__ __align__(8) uint64_t s_bar[2][2];  // [from above, from below][run parity]
   __shared__ uint32_t s_colour[2];
   __shared__ int s_failed;
+  __shared__ int s_stop;  // a smaller attempt coalesced
   constexpr bool kFast = kMode == kLbFast, kParams = kMode == kLbTmtParams;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)(blockDim.x >> 5);
-  const int ndraw = a.draw_warps, nslots = ndraw * KS, band = blockIdx.x;
+  const int ndraw = a.draw_warps, nslots = ndraw * KS, band = kForm == kLbOne ? 0 : (int)blockIdx.x;
+  const bool cftp = kForm == kLbOne && NCH == 2 && a.attempts > 0;
+  uint8_t* const base = a.base + (cftp ? blockIdx.x * a.team_stride : 0);
   const int r0 = a.row_start[band], r1 = a.row_start[band + 1], R = r1 - r0, wn = a.wn, wlo = a.wlo, W = a.words;
   const bool has_up = band > 0, has_dn = band + 1 < a.bands;
   // Shared memory: planes [rows r0 .. r1][wn][NCH][12]; a scratch word; received toggles [from above,
@@ -156,27 +171,30 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
     for (int k = 0; k < n; ++k) sslot[at + k] = (uint32_t)y << 16 | (uint32_t)(f + k);
   }
   // planes of rows r0 .. r1: a warp per row and word, lane l reads slot 32 w + l of the three residues
-  for (int it = warp; it < (R + 1) * wn; it += nwarps) {
-    const int y = it / wn, x = it - y * wn, i = r0 + y, m = 32 * (wlo + x) + lane;
-    const bool in = i < a.N && m >= 0 && m < a.P;
+  auto load_planes = [&](const uint8_t* src) {
+    for (int it = warp; it < (R + 1) * wn; it += nwarps) {
+      const int y = it / wn, x = it - y * wn, i = r0 + y, m = 32 * (wlo + x) + lane;
+      const bool in = i < a.N && m >= 0 && m < a.P;
 #pragma unroll
-    for (int c = 0; c < NCH; ++c) {
-      uint32_t bits[9];
+      for (int c = 0; c < NCH; ++c) {
+        uint32_t bits[9];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const int col = (q + 3 - i % 3) % 3;  // colour of residue q in row i
-        const uint32_t v =
-            in ? a.base[(size_t)c * a.chain_stride + (size_t)col * a.colour_stride + (size_t)i * a.P + m] : 0u;
-        bits[q] = __ballot_sync(~0u, v & 8u);
-        bits[3 + q] = __ballot_sync(~0u, v & 2u);
-        bits[6 + q] = __ballot_sync(~0u, v & 1u);
+        for (int q = 0; q < 3; ++q) {
+          const int col = (q + 3 - i % 3) % 3;  // colour of residue q in row i
+          const uint32_t v =
+              in ? src[(size_t)c * a.chain_stride + (size_t)col * a.colour_stride + (size_t)i * a.P + m] : 0u;
+          bits[q] = __ballot_sync(~0u, v & 8u);
+          bits[3 + q] = __ballot_sync(~0u, v & 2u);
+          bits[6 + q] = __ballot_sync(~0u, v & 1u);
+        }
+        uint32_t mine = 0u;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) mine = lane == k ? bits[k] : mine;
+        if (lane < kLbWord) PL(y, x, c)[lane] = mine;
       }
-      uint32_t mine = 0u;
-#pragma unroll
-      for (int k = 0; k < 9; ++k) mine = lane == k ? bits[k] : mine;
-      if (lane < kLbWord) PL(y, x, c)[lane] = mine;
     }
-  }
+  };
+  if (!cftp) load_planes(base);
   __syncthreads();
 
   // Update warps: the first holds the last row, the second the first row (all W words, so that the
@@ -259,7 +277,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       if (sslot[warp * KS + s] != ~0u) n_mine = s + 1;
       bool v;
       const int64_t g = gen_index(s, &v);
-      if (v) gen[s] = a.tmt[g];
+      if (v && !cftp) gen[s] = a.tmt[g];
     }
   } else {
 #pragma unroll
@@ -270,9 +288,22 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       if (__any_sync(~0u, e != ~0u)) n_mine = g + 1;
     }
   }
-  auto draw_run = [&](uint32_t run, int64_t h, uint2* out) {
+  auto draw_run = [&](uint32_t run, int64_t h, uint32_t reseed_to, uint2* out) {
     if constexpr (!kFast) {
-      const int L = (int)(run & 0x3fffffffu);
+      const int L = (int)(run & 0x1fffffffu);
+      if ((run >> 29) & 1u) {  // an epoch's generators (as k_lz_seed)
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+          bool v;
+          const int64_t g = gen_index(s, &v);
+          uint32_t m1 = kTmtMat1, m2 = kTmtMat2, tm = kTmtTmat;
+          if (kParams) {
+            const uint4 p = __ldg(&a.tmt_params[v ? g : 0]);
+            m1 = p.x, m2 = p.y, tm = p.z;
+          }
+          if (v) gen[s] = tmt_seed(reseed_to + (uint32_t)g, m1, m2, tm);
+        }
+      }
       // Every lane composes the moves of all its warp's words where registers allow it, else lane s
       // those of slot s.
       constexpr bool kAll = KS <= 4;
@@ -332,18 +363,45 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       }
     }
   };
-  const int nruns = a.nruns;
-  const int c0 = kFast ? (int)(((a.h0 % 3) + 3) % 3) : 0;
+  const int n_att = cftp ? a.attempts : 1, teams = (int)gridDim.x;
+  bool stopped = false;
+  for (int att = cftp ? (int)blockIdx.x : 0; att < n_att; att += teams) {
+  int nruns = a.nruns, epoch = 0;
+  const uint32_t* runs = a.runs;
+  int64_t h0 = a.h0;
+  if (cftp) {
+    if (kFast) {
+      nruns = (int)(3 * (a.first_sweeps << att));
+      h0 = -(int64_t)nruns;
+    } else {
+      const int4 d = a.attempt_desc[att];
+      runs += d.x;
+      nruns = d.y;
+      epoch = d.z;
+    }
+    load_planes(a.start);
+  }
+  const int c0 = kFast ? (int)(((h0 % 3) + 3) % 3) : 0;
   auto run_at = [&](int j) -> uint32_t {
     if (kFast) return (uint32_t)((c0 + j) % 3) << 30 | 1u;
-    return j < nruns ? __ldg(&a.runs[j]) : 0u;
+    return j < nruns ? __ldg(&runs[j]) : 0u;
+  };
+  auto seed_of = [&](uint32_t run) -> uint32_t {
+    return !kFast && ((run >> 29) & 1u) ? __ldg(&a.epoch_seeds[epoch++]) : 0u;
   };
   uint32_t next = run_at(1);
   if (!updates && nruns > 0) {
     const uint32_t run = run_at(0);
-    draw_run(run, a.h0, smove);
+    draw_run(run, h0, seed_of(run), smove);
     if (tid == 0) s_colour[0] = run >> 30;
   }
+  // Every 256 runs: has a smaller attempt coalesced?
+  auto told_stop = [&](int j) {
+    if (!cftp || (j & 255) != 255) return false;
+    if (tid == 0) s_stop = *static_cast<volatile int*>(a.best) < att;
+    __syncthreads();
+    return *static_cast<volatile int*>(&s_stop) != 0;
+  };
   if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
   else __syncthreads();
 
@@ -454,6 +512,10 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       r_last = r;
       if (kForm == kLbOne || (j & 63) != 63) {
         lb_cta_sync();
+        if (told_stop(j)) {
+          stopped = true;
+          break;
+        }
       } else if (__syncthreads_or(failed ? 1 : 0)) {  // a band that gave up leaves within 64 runs
         failed = true;
         break;
@@ -464,11 +526,15 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       const uint32_t after = run_at(j + 2);
       if (j + 1 < nruns) {
         if (tid == 0) s_colour[(j + 1) & 1] = next >> 30;
-        draw_run(next, a.h0 + j + 1, smove + ((j + 1) & 1) * nslots);
+        draw_run(next, h0 + j + 1, seed_of(next), smove + ((j + 1) & 1) * nslots);
       }
       next = after;
       if (kForm == kLbOne || (j & 63) != 63) {
         lb_cta_sync();
+        if (told_stop(j)) {
+          stopped = true;
+          break;
+        }
       } else if (__syncthreads_or(0)) {
         failed = true;
         break;
@@ -490,6 +556,20 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
     if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
   }
   __syncthreads();
+  if (!cftp) break;
+  if (stopped) return;
+  uint32_t differ = 0u;
+  if (NCH == 2)
+    for (int k = tid; k < (R + 1) * wn * kLbWord; k += (int)blockDim.x) {
+      const uint32_t* p = lsm + (size_t)(k / kLbWord) * 2 * kLbWord + k % kLbWord;
+      differ |= p[0] ^ p[kLbWord];
+    }
+  if (!__syncthreads_or(differ != 0u)) {
+    if (tid == 0) atomicMin(a.best, att);
+    break;
+  }
+  }
+  __syncthreads();
   // Rows r0 .. r1 - 1 back to the chains: slots [1, M - 2] of the window's inner words.
   for (int it = warp; it < R * (wn - 2); it += nwarps) {
     const int y = it / (wn - 2), x = 1 + it - y * (wn - 2), i = r0 + y, m = 32 * (wlo + x) + lane;
@@ -505,11 +585,12 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
         const uint32_t sw = q == 0 ? __funnelshift_l(dl[3 + qw], d[3 + qw], 1) : d[3 + qw];
         const uint32_t v = bit(p[q]) * 8u + bit(p[3 + q]) * 2u + bit(p[6 + q]) + bit(w) * 4u + bit(sw) * 16u + bit(d[6 + q]) * 32u;
         const int col = (q + 3 - i % 3) % 3;
-        a.base[(size_t)c * a.chain_stride + (size_t)col * a.colour_stride + (size_t)i * a.P + m] = (uint8_t)v;
+        base[(size_t)c * a.chain_stride + (size_t)col * a.colour_stride + (size_t)i * a.P + m] = (uint8_t)v;
       }
     }
   }
   if constexpr (!kFast) {
+    if (cftp) return;  // every epoch seeds its generators
 #pragma unroll
     for (int s = 0; s < KS; ++s) {
       if (updates) continue;
@@ -690,7 +771,7 @@ LbPlan lb_plan(const LzResidentGeom& g, const LzResidentRule& rule, const std::v
 }
 
 LbState::~LbState() {
-  for (void* p : {(void*)d_rows, (void*)d_runs, (void*)d_xbuf, (void*)d_error}) dev_free(p, stream);
+  for (void* p : {(void*)d_rows, (void*)d_runs, (void*)d_xbuf, (void*)d_error, (void*)d_epoch, (void*)d_teams}) dev_free(p, stream);
 }
 
 #define LB_CUDA(expr)                                                                   \
@@ -700,71 +781,158 @@ LbState::~LbState() {
       return fail(RT_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(_e));     \
   } while (0)
 
-rt_status lb_run(LbState& st, const LzResidentGeom& g, uint8_t* base, const LzResidentRule& rule, bool tinymt, uint4* tmt,
-                 const uint4* params, const int* d_cand, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed,
-                 uint32_t fast_stream, int64_t h0, cudaStream_t s) {
+namespace {
+
+rt_status lb_prepare(LbState& st, const LzResidentGeom& g, cudaStream_t s) {
   const LbPlan& p = st.plan;
   st.stream = s;
   if (!st.d_rows) {
     if (rt_status e = dev_alloc(&st.d_rows, sizeof p.row_start, s)) return e;
-    if (rt_status e = dev_alloc(&st.d_error, sizeof(int), s)) return e;
+    if (rt_status e = dev_alloc(&st.d_error, 2 * sizeof(int), s)) return e;
     LB_CUDA(cudaMemcpyAsync(st.d_rows, p.row_start, sizeof p.row_start, cudaMemcpyHostToDevice, s));
     if (p.form == kLbGrid) {
       st.xbuf_bytes = (size_t)2 * p.bands * 2 * p.words * g.nch * sizeof(uint64_t);
       if (rt_status e = dev_alloc(&st.d_xbuf, st.xbuf_bytes, s)) return e;
     }
   }
+  return RT_OK;
+}
+
+LbArgs lb_args(const LbState& st, const LzResidentGeom& g, uint8_t* base, const LzResidentRule& rule, bool tinymt,
+               uint4* tmt, const uint4* params, const int* d_cand, uint64_t fast_seed, uint32_t fast_stream) {
+  const LbPlan& p = st.plan;
+  LbArgs a{};
+  a.base = base;
+  a.colour_stride = g.colour_stride;
+  a.chain_stride = g.chain_stride;
+  a.N = g.N;
+  a.M = g.M;
+  a.P = g.P;
+  a.bands = p.bands;
+  a.draw_warps = p.draw_warps;
+  a.row_start = st.d_rows;
+  a.cand = d_cand;
+  a.wlo = p.wlo;
+  a.wn = p.wn;
+  a.w0 = p.w0;
+  a.words = p.words;
+  const int sh = tinymt ? 9 : 0;
+  a.lo_up = rule.lo_up << sh;
+  a.w_up = rule.w_up << sh;
+  a.lo_dn = rule.lo_dn << sh;
+  a.w_dn = rule.w_dn << sh;
+  a.tmt = tmt;
+  a.tmt_params = params;
+  a.seed = fast_seed;
+  a.stream = fast_stream;
+  a.xbuf = st.d_xbuf;
+  a.error = st.d_error;
+  a.max_spin = 1L << 22;
+  return a;
+}
+
+// Appends the runs of equal colour of a sequence of steps.
+void lb_runs(const uint8_t* colours, int64_t n, bool epoch, std::vector<uint32_t>* runs) {
+  const size_t from = runs->size();
+  for (int64_t k = 0; k < n; ++k) {
+    const uint32_t c = colours[k];
+    if (runs->size() > from && (runs->back() >> 30) == c) ++runs->back();
+    else runs->push_back(c << 30 | (epoch && k == 0 ? 1u << 29 : 0u) | 1u);
+  }
+}
+
+rt_status lb_upload_runs(LbState& st, const std::vector<uint32_t>& runs, cudaStream_t s) {
+  if (st.runs_cap < (int64_t)runs.size()) {
+    dev_free(st.d_runs, s);
+    st.d_runs = nullptr;
+    st.runs_cap = 0;
+    if (rt_status e = dev_alloc(&st.d_runs, runs.size() * sizeof(uint32_t), s)) return e;
+    st.runs_cap = (int64_t)runs.size();
+  }
+  LB_CUDA(cudaMemcpyAsync(st.d_runs, runs.data(), runs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  return RT_OK;
+}
+
+}  // namespace
+
+rt_status lb_cftp(LbState& st, const LzResidentGeom& g, uint8_t* base, const uint8_t* start, const LzResidentRule& rule,
+                  bool tinymt, const uint4* params, const int* d_cand, int n,
+                  const std::vector<std::vector<LbEpoch>>& epochs, int64_t first_sweeps, uint64_t fast_seed,
+                  uint32_t fast_stream, int* attempts_run, bool* coalesced, cudaStream_t s) {
+  const LbPlan& p = st.plan;
+  if (p.form != kLbOne || g.nch != 2 || n < 1) return fail(RT_ERR_INVALID_ARGUMENT, "lozenge cftp: one CTA, two chains");
+  if (rt_status e = lb_prepare(st, g, s)) return e;
+  LbArgs a = lb_args(st, g, base, rule, tinymt, nullptr, params, d_cand, fast_seed, fast_stream);
+  std::vector<uint32_t> runs, seeds;
+  std::vector<int4> desc;
+  if (tinymt) {
+    for (int k = 0; k < n; ++k) {
+      int4 d = make_int4((int)runs.size(), 0, (int)seeds.size(), 0);
+      for (const LbEpoch& e : epochs[(size_t)k]) {
+        seeds.push_back(e.seed);
+        lb_runs(e.colours->data(), (int64_t)e.colours->size(), true, &runs);
+      }
+      d.y = (int)runs.size() - d.x;
+      desc.push_back(d);
+    }
+    if (rt_status e = lb_upload_runs(st, runs, s)) return e;
+    const size_t desc_off = (seeds.size() * sizeof(uint32_t) + 15) / 16 * 16, bytes = desc_off + desc.size() * sizeof(int4);
+    if (st.epoch_cap < bytes) {
+      dev_free(st.d_epoch, s);
+      st.d_epoch = nullptr;
+      st.epoch_cap = 0;
+      if (rt_status e = dev_alloc(&st.d_epoch, bytes, s)) return e;
+      st.epoch_cap = bytes;
+    }
+    LB_CUDA(cudaMemcpyAsync(st.d_epoch, seeds.data(), seeds.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    LB_CUDA(cudaMemcpyAsync(st.d_epoch + desc_off, desc.data(), desc.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+    a.runs = st.d_runs;
+    a.epoch_seeds = reinterpret_cast<const uint32_t*>(st.d_epoch);
+    a.attempt_desc = reinterpret_cast<const int4*>(st.d_epoch + desc_off);
+  }
+  const int teams = std::min(n, kLbTeams);
+  a.attempts = n;
+  a.first_sweeps = first_sweeps;
+  a.start = start;
+  a.team_stride = 2 * g.chain_stride;
+  if (!st.d_teams)
+    if (rt_status e = dev_alloc(&st.d_teams, kLbTeams * a.team_stride, s)) return e;
+  a.base = st.d_teams;
+  for (int k = 0; k < teams; ++k)  // the cells that no attempt writes
+    LB_CUDA(cudaMemcpyAsync(st.d_teams + k * a.team_stride, start, a.team_stride, cudaMemcpyDeviceToDevice, s));
+  a.best = st.d_error + 1;
+  LB_CUDA(cudaMemsetAsync(a.best, 0x7f, sizeof(int), s));  // no attempt yet
+  void* args[] = {&a};
+  LB_CUDA(cudaLaunchKernel(p.kernel, dim3((unsigned)teams), dim3((unsigned)p.threads()), args, p.smem, s));
+  int best = 0;
+  LB_CUDA(cudaMemcpyAsync(&best, a.best, sizeof best, cudaMemcpyDeviceToHost, s));
+  LB_CUDA(cudaStreamSynchronize(s));
+  *coalesced = best < n;
+  *attempts_run = *coalesced ? best + 1 : n;
+  LB_CUDA(cudaMemcpyAsync(base, st.d_teams + (*attempts_run - 1) % teams * a.team_stride, a.team_stride,
+                          cudaMemcpyDeviceToDevice, s));
+  return RT_OK;
+}
+
+rt_status lb_run(LbState& st, const LzResidentGeom& g, uint8_t* base, const LzResidentRule& rule, bool tinymt, uint4* tmt,
+                 const uint4* params, const int* d_cand, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed,
+                 uint32_t fast_stream, int64_t h0, cudaStream_t s) {
+  const LbPlan& p = st.plan;
+  if (rt_status e = lb_prepare(st, g, s)) return e;
   constexpr int64_t kChunk = 1 << 16;  // steps per launch
   std::vector<uint32_t> runs;
   for (int64_t done = 0; done < steps; done += kChunk) {
     const int64_t n = std::min(kChunk, steps - done);
-    LbArgs a{};
-    a.base = base;
-    a.colour_stride = g.colour_stride;
-    a.chain_stride = g.chain_stride;
-    a.N = g.N;
-    a.M = g.M;
-    a.P = g.P;
-    a.bands = p.bands;
-    a.draw_warps = p.draw_warps;
-    a.row_start = st.d_rows;
-    a.cand = d_cand;
-    a.wlo = p.wlo;
-    a.wn = p.wn;
-    a.w0 = p.w0;
-    a.words = p.words;
-    const int sh = tinymt ? 9 : 0;
-    a.lo_up = rule.lo_up << sh;
-    a.w_up = rule.w_up << sh;
-    a.lo_dn = rule.lo_dn << sh;
-    a.w_dn = rule.w_dn << sh;
-    a.tmt = tmt;
-    a.tmt_params = params;
-    a.seed = fast_seed;
-    a.stream = fast_stream;
+    LbArgs a = lb_args(st, g, base, rule, tinymt, tmt, params, d_cand, fast_seed, fast_stream);
     a.h0 = h0 + done;
     a.nruns = (int)n;
     if (tinymt) {
       runs.clear();
-      for (int64_t k = 0; k < n; ++k) {
-        const uint32_t c = colours_host[done + k];
-        if (!runs.empty() && (runs.back() >> 30) == c) ++runs.back();
-        else runs.push_back(c << 30 | 1u);
-      }
-      if (st.runs_cap < (int64_t)runs.size()) {
-        dev_free(st.d_runs, s);
-        st.d_runs = nullptr;
-        st.runs_cap = 0;
-        if (rt_status e = dev_alloc(&st.d_runs, runs.size() * sizeof(uint32_t), s)) return e;
-        st.runs_cap = (int64_t)runs.size();
-      }
-      LB_CUDA(cudaMemcpyAsync(st.d_runs, runs.data(), runs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+      lb_runs(colours_host + done, n, false, &runs);
+      if (rt_status e = lb_upload_runs(st, runs, s)) return e;
       a.runs = st.d_runs;
       a.nruns = (int)runs.size();
     }
-    a.xbuf = st.d_xbuf;
-    a.error = st.d_error;
-    a.max_spin = 1L << 22;
     if (!st.pending) LB_CUDA(cudaMemsetAsync(st.d_error, 0, sizeof(int), s));
     if (st.d_xbuf) LB_CUDA(cudaMemsetAsync(st.d_xbuf, 0, st.xbuf_bytes, s));  // no stale tags
     void* args[] = {&a};

@@ -314,7 +314,6 @@ struct LzSampler {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int64_t interior[3] = {0, 0, 0};
-  int64_t steps_by_colour[3] = {0, 0, 0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::unique_ptr<LzResidentState> res;  // the resident engine for `res_nch` swept chains
   int res_nch = 0;
@@ -518,8 +517,7 @@ struct LzSampler {
         pdl_launch(k_lz_rotate_mtgp, dim3(g.gx, g.gy), dim3(kMtgpBlock, kMtgpBlock), stream, v, r, rule,
                    static_cast<curandStateMtgp32*>(mtgp));
         pdl_launch(k_lz_update_w, gu, dim3(32, 8), stream, v, r);
-        steps_by_colour[r]++;
-      }
+        }
       return check();
     }
     LbState* lb = nullptr;
@@ -528,7 +526,6 @@ struct LzSampler {
       const LzResidentRule rr{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn};
       if (rt_status st = lb_run(*lb, geom(), base, rr, true, tmt, tmt_params, d_cand, colours, steps, 0, 0, 0, stream))
         return st;
-      for (int64_t s = 0; s < steps; ++s) steps_by_colour[colours[s]]++;
       return RT_OK;
     }
     LzResidentState* rs = nullptr;
@@ -537,7 +534,6 @@ struct LzSampler {
       const LzResidentRule rr{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn};
       if (rt_status st = lz_resident_run(*rs, geom(), base, rr, true, tmt, tmt_params, colours, steps, 0, 0, 0, stream))
         return st;
-      for (int64_t s = 0; s < steps; ++s) steps_by_colour[colours[s]]++;
       return RT_OK;
     }
     const dim3 gr((M + 127) / 128, N), gu((P / 4 + 31) / 32, (N - 2 + 7) / 8);
@@ -545,7 +541,6 @@ struct LzSampler {
       const int r = colours[s];
       pdl_launch(k_lz_rotate_tmt, gr, dim3(128), stream, v, r, rule);
       pdl_launch(k_lz_update_w, gu, dim3(32, 8), stream, v, r);
-      steps_by_colour[r]++;
     }
     return check();
   }
@@ -557,7 +552,6 @@ struct LzSampler {
       if (rt_status st = lb_run(*lb, geom(), base, rr, false, nullptr, nullptr, d_cand, nullptr, steps, seed_value,
                                 opts.fast_stream, h0, stream))
         return st;
-      for (int64_t s = 0; s < steps; ++s) steps_by_colour[(((h0 + s) % 3) + 3) % 3]++;
       return RT_OK;
     }
     LzResidentState* rs = nullptr;
@@ -567,7 +561,6 @@ struct LzSampler {
       if (rt_status st = lz_resident_run(*rs, geom(), base, rr, false, nullptr, nullptr, nullptr, steps, seed_value,
                                          opts.fast_stream, h0, stream))
         return st;
-      for (int64_t s = 0; s < steps; ++s) steps_by_colour[(((h0 + s) % 3) + 3) % 3]++;
       return RT_OK;
     }
     const LzView v = view();
@@ -578,7 +571,6 @@ struct LzSampler {
       const int r = (int)(((h % 3) + 3) % 3);
       pdl_launch(k_lz_rotate_fast, gr, dim3(32, 8), stream, v, r, rule, seed_value, opts.fast_stream, h);
       pdl_launch(k_lz_update_w, gu, dim3(32, 8), stream, v, r);
-      steps_by_colour[r]++;
     }
     return check();
   }
@@ -662,50 +654,97 @@ RT_API rt_status rt_lozenge_cftp(const int32_t* tmax, const int32_t* tmin, int32
   if (rt_status st = s->copy_chain(2, 0)) return st;
   if (rt_status st = s->load(3, tmax)) return st;
   s->active = 2;
+  const bool fast = o.rng_mode == RT_RNG_FAST;
+  // Epoch k is created by attempt k with the driver's k-th draw as its seed; attempt a runs epochs a, a-1, ..., 0,
+  // each one reference Walk(t, steps_k, seed_k) on both chains.
   std::mt19937 drv((uint32_t)driver_seed);
-  std::vector<int64_t> steps{first_steps};
-  std::vector<uint32_t> seeds{(uint32_t)drv()};
+  std::vector<int64_t> ep_steps;
+  std::vector<uint32_t> ep_seed;
+  std::vector<std::vector<uint8_t>> ep_colours((size_t)max_attempts);
+  for (int k = 0; !fast && k < max_attempts; ++k) {
+    ep_seed.push_back((uint32_t)drv());
+    ep_steps.push_back(k == 0 ? first_steps : (schedule == 0 ? 2 * ep_steps[0] : 2 * ep_steps[(size_t)k - 1]));
+  }
+  auto colours_of = [&](int k) -> const std::vector<uint8_t>& {
+    if (ep_colours[(size_t)k].empty()) ep_colours[(size_t)k] = lz_colours(ep_seed[(size_t)k], ep_steps[(size_t)k]);
+    return ep_colours[(size_t)k];
+  };
+  auto look_back = [&](int att) -> int64_t {
+    if (fast) return 3 * (first_steps << att);
+    int64_t t = 0;
+    for (int k = 0; k <= att; ++k) t += ep_steps[(size_t)k];
+    return t;
+  };
   rt_cftp_stats st_out{};
   float ms_total = 0.f;
-  for (int attempt = 1; attempt <= max_attempts; ++attempt) {
-    if (rt_status st = s->copy_chain(0, 2)) return st;
-    if (rt_status st = s->copy_chain(1, 3)) return st;
-    int64_t before[3] = {s->steps_by_colour[0], s->steps_by_colour[1], s->steps_by_colour[2]};
-    cudaEventRecord(s->ev0, s->stream);
-    int64_t look_back = 0;
-    if (o.rng_mode != RT_RNG_FAST) {
-      // Each epoch is one reference Walk(t, steps_k, seed_k) on both chains.
-      for (size_t k = 0; k < steps.size(); ++k) {
-        if (rt_status st = s->seed(seeds[k])) return st;
-        std::vector<uint8_t> col = lz_colours(seeds[k], steps[k]);
-        if (rt_status st = s->run(col.data(), steps[k])) return st;
-        look_back += steps[k];
-      }
+  auto account = [&](int att) {
+    st_out.attempts = att + 1;
+    st_out.total_steps += look_back(att);
+    st_out.final_steps = look_back(att);
+    int64_t by[3] = {0, 0, 0};
+    if (fast) {
+      by[0] = by[1] = by[2] = first_steps << att;
     } else {
-      const int64_t T = first_steps << (attempt - 1);
-      if (rt_status st = s->run_fast((uint64_t)driver_seed, -3 * T, 3 * T)) return st;
-      look_back = 3 * T;
+      for (int k = 0; k <= att; ++k)
+        for (uint8_t c : colours_of(k)) by[c]++;
     }
-    cudaEventRecord(s->ev1, s->stream);
-    int64_t nd = -1;
-    if (rt_status st = s->diff(0, 1, &nd)) return st;
+    for (int c = 0; c < 3; ++c) st_out.flip_attempts += 2 * by[c] * s->interior[c];
+  };
+  // Where one CTA holds the chains, attempts go to it in groups, side by side; the first groups are short where
+  // their colours are drawn on the host, needed or not.  Longer attempts and other engines run one by one.
+  const int64_t kLaunchSteps = (int64_t)1 << 21;
+  int64_t group_steps = fast ? kLaunchSteps : (int64_t)1 << 14;
+  LbState* lb = nullptr;
+  if (rt_status st = s->bit_engine(&lb)) return st;
+  const bool one_launch = lb && lb->plan.form == kLbOne;
+  int att = 0;
+  bool coalesced = false;
+  while (att < max_attempts && !coalesced) {
+    int n = 0;
+    int64_t total = 0;
+    while (one_launch && att + n < max_attempts && total + look_back(att + n) <= (n ? group_steps : kLaunchSteps))
+      total += look_back(att + n++);
+    group_steps = std::min(8 * group_steps, kLaunchSteps);
+    cudaEventRecord(s->ev0, s->stream);
+    int ran = 1;
+    if (n > 0) {
+      std::vector<std::vector<LbEpoch>> epochs((size_t)n);
+      for (int q = 0; !fast && q < n; ++q)
+        for (int k = att + q; k >= 0; --k) epochs[(size_t)q].push_back({ep_seed[(size_t)k], &colours_of(k)});
+      const LzResidentRule rr{s->rule.lo_up, s->rule.w_up, s->rule.lo_dn, s->rule.w_dn};
+      if (rt_status st = lb_cftp(*lb, s->geom(), s->base, s->base + 2 * s->chain_stride, rr, !fast, s->tmt_params, s->d_cand,
+                                 n, epochs, fast ? first_steps << att : 0, (uint64_t)driver_seed, o.fast_stream, &ran,
+                                 &coalesced, s->stream))
+        return st;
+      cudaEventRecord(s->ev1, s->stream);
+      cudaEventSynchronize(s->ev1);
+    } else {
+      if (rt_status st = s->copy_chain(0, 2)) return st;
+      if (rt_status st = s->copy_chain(1, 3)) return st;
+      if (!fast) {
+        for (int k = att; k >= 0; --k) {
+          if (rt_status st = s->seed(ep_seed[(size_t)k])) return st;
+          if (rt_status st = s->run(colours_of(k).data(), ep_steps[(size_t)k])) return st;
+        }
+      } else {
+        const int64_t T = first_steps << att;
+        if (rt_status st = s->run_fast((uint64_t)driver_seed, -3 * T, 3 * T)) return st;
+      }
+      cudaEventRecord(s->ev1, s->stream);
+      int64_t nd = -1;
+      if (rt_status st = s->diff(0, 1, &nd)) return st;
+      coalesced = nd == 0;
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, s->ev0, s->ev1);
     ms_total += ms;
-    st_out.attempts = attempt;
-    st_out.total_steps += look_back;
-    st_out.final_steps = look_back;
-    for (int c = 0; c < 3; ++c) st_out.flip_attempts += 2 * (s->steps_by_colour[c] - before[c]) * s->interior[c];
-    st_out.seconds = ms_total * 1e-3;
-    if (nd == 0) {
-      if (stats) *stats = st_out;
-      return s->store(1, out);
-    }
-    if (o.rng_mode != RT_RNG_FAST) {
-      const int64_t next = schedule == 0 ? steps.back() * 2 : steps.front() * 2;
-      steps.insert(steps.begin(), next);
-      seeds.insert(seeds.begin(), (uint32_t)drv());
-    }
+    for (int q = 0; q < ran; ++q) account(att + q);
+    att += ran;
+  }
+  st_out.seconds = ms_total * 1e-3;
+  if (coalesced) {
+    if (stats) *stats = st_out;
+    return s->store(1, out);
   }
   if (stats) *stats = st_out;
   if (rt_status st = s->store(1, out)) return st;

@@ -129,3 +129,28 @@ def test_cluster_wait_gives_up_and_the_sampler_stays_usable(rt, rng):
     want = [ref.store(0), ref.store(1)]
     ref.close()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rng,schedule", [("fast", 1), ("tinymt", 0), ("tinymt", 1)])
+def test_attempts_side_by_side_return_the_smallest(rt, rng, schedule):
+    # The first look-back decides which of the four clusters runs the attempt that coalesces; several coalesce at once
+    # where the first is already long enough, and the chain must then be the first one's.
+    D = rt.DominoTiler
+    sizes = ((3, (1, 2, 4, 8, 256)), (12, (4, 16, 64, 256, 4096)))
+    if schedule == 0:  # look-backs grow by 2 first only
+        sizes = ((3, (2, 4, 8, 256)), (12, (128, 256, 512, 4096)))
+    for order, firsts in sizes:
+        d = D.AztecDiamond(order)
+        tmax, tmin = D.MaxTiling(d), D.MinTiling(d)
+        seen = set()
+        for first in firsts:
+            runs = [D(rule="cftp", rng=rng, engine=engine).cftp(tmax, tmin, 77 + first, first_steps=first,
+                                                                schedule=schedule, max_attempts=36)
+                    for engine in (0, 1)]
+            (a, sa), (b, sb) = runs
+            assert np.array_equal(a, b)
+            assert {k: sa[k] for k in ("attempts", "total_steps", "final_steps", "flip_attempts")} == {
+                k: sb[k] for k in ("attempts", "total_steps", "final_steps", "flip_attempts")}
+            seen.add(sa["attempts"])
+        assert len(seen) >= 3

@@ -84,3 +84,27 @@ def test_states_that_are_no_tilings(rt, mode):
     first = int(np.nonzero(t.reshape(n, n).any(1))[0][0])
     up = np.roll(t.reshape(n, n), -(first - 1), axis=0).ravel().copy()
     assert np.array_equal(_walk(rt, up, 200, 3, mode, 0), _walk(rt, up, 200, 3, mode, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rng,schedule", [("fast", 1), ("tinymt", 0), ("tinymt", 1)])
+def test_attempts_side_by_side_return_the_smallest(rt, rng, schedule):
+    # The first look-back decides which of the four CTAs runs the attempt that coalesces; several coalesce at once
+    # where the first is already long enough, and the chain must then be the first one's.
+    L = rt.LozengeTiler
+    sizes = ((2, (1, 4, 16, 512)), (9, (8, 32, 128, 8192)))
+    if schedule == 0:  # look-backs grow by 2 first only
+        sizes = ((2, (4, 16, 512)), (9, (512, 1024, 8192)))
+    for side, firsts in sizes:
+        d = L.Hexagon(side)
+        tmax, tmin = L.MaxTiling(d), L.MinTiling(d)
+        seen = set()
+        for first in firsts:
+            runs = [L(rng=rng, engine=engine).cftp(tmax, tmin, 77 + first, first_steps=first, schedule=schedule,
+                                                   max_attempts=36) for engine in (0, 1)]
+            (a, sa), (b, sb) = runs
+            assert np.array_equal(a, b)
+            keys = ("attempts", "total_steps", "final_steps", "flip_attempts")
+            assert [sa[k] for k in keys] == [sb[k] for k in keys]
+            seen.add(sa["attempts"])
+        assert len(seen) >= 2
