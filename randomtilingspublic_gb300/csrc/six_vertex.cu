@@ -185,8 +185,16 @@ struct SvBandArgs {
   uint64_t* xbuf;       // [period parity][band][to above, to below][chain][row][class][word], tags cleared
   int* error;
   long max_spin;
+  // Coupling from the past (couple, two chains): blockIdx.y = k runs attempt attempt0 + k, sub-sweeps
+  // [-4 first << attempt, 0), into the k-th pair of chains at dst, and leaves once a smaller one has coalesced.
+  int couple, attempt0;
+  int64_t first;
+  size_t xteam;         // words of xbuf a team
+  int* best;            // smallest attempt that coalesced
+  int2* team;           // [k] {bands whose chains differ, bands done}
 };
 
+constexpr int kSvTeams = 4;  // attempts side by side
 constexpr int kSvDrawPlanes = 16;
 constexpr int kSvBandThreads = 640;
 
@@ -292,6 +300,12 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int n = A.n, P = A.P, words = A.words, band = blockIdx.x;
   const int movable = (n - 1) / 2 + 1;  // rows that can change
+  __shared__ int s_stop[2];  // a smaller attempt coalesced, by parity of the batch
+  const bool couple = NCH == 2 && A.couple;
+  const int team = couple ? (int)blockIdx.y : 0, attempt = A.attempt0 + team;
+  const int all_sweeps = couple ? (int)(A.first << attempt) : A.sweeps;
+  const int64_t s0 = couple ? -4 * (int64_t)all_sweeps : A.s0;
+  uint64_t* const xbuf = A.xbuf + team * A.xteam;
   const int r0 = sv_band_row(band, A.bands, movable), r1 = sv_band_row(band + 1, A.bands, movable);
   const int w0 = max(r0 - A.depth, 0), w1 = min(r1 + A.depth, A.R);  // the window's rows
   const int cs = A.rows * P;
@@ -315,9 +329,9 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
 
   const int updaters = NCH * A.group;
   const bool updates = tid < updaters;
-  const int phases = 2 * A.sweeps, batches = (phases + A.batch - 1) / A.batch;
+  const int phases = 2 * all_sweeps, batches = (phases + A.batch - 1) / A.batch;
   // Draws of batch b: tasks of 32 words in turn over the draw warps.
-  int ahead = 0, drawn_left = min(A.depth, A.sweeps);  // the sweep reached, and sweeps left before the exchange after it
+  int ahead = 0, drawn_left = min(A.depth, all_sweeps);  // the sweep reached, and sweeps left before the exchange after it
   int2 rows_of[2] = {phase_tab[2 * drawn_left], phase_tab[2 * drawn_left + 1]};
   auto draw_batch = [&](int b) {
     const int dw = warp - (updaters >> 5), ndw = (nt - updaters) >> 5;
@@ -330,7 +344,7 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
       const int lo = py ? rows_of[1].x : rows_of[0].x, items = py ? rows_of[1].y : rows_of[0].y;
       if (py && A.depth > 1) {
         ++ahead;
-        drawn_left = drawn_left > 1 ? drawn_left - 1 : min(A.depth, A.sweeps - ahead);
+        drawn_left = drawn_left > 1 ? drawn_left - 1 : min(A.depth, all_sweeps - ahead);
         rows_of[0] = phase_tab[2 * drawn_left], rows_of[1] = phase_tab[2 * drawn_left + 1];
       }
       for (int e0 = 0; e0 < 2 * items; e0 += 32, turn = turn + 1 == ndw ? 0 : turn + 1) {
@@ -338,7 +352,7 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
         const int e = e0 + lane;
         if (e >= 2 * items) continue;
         const int px = e >= items ? 1 : 0, it = e - px * items, rr = sv_div(it, inv_words), w = it - rr * words;
-        const uint64_t s = (uint64_t)(A.s0 + 2 * (int64_t)f + px);
+        const uint64_t s = (uint64_t)(s0 + 2 * (int64_t)f + px);
         const uint32_t imask = interior_mask(w, px ? 0 : 1, (n - 1 - px) / 2);
         sv_draw_word<M>(set + (2 * q + px) * sub_words, it, A.items, A.leaf, imask, (uint32_t)w, (uint32_t)(lo + rr),
                         (uint32_t)s, ((uint32_t)(s >> 32) & 0xffffu) | (A.stream << 16), A.seed);
@@ -383,12 +397,12 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
     recv_to[i] = (q & 3) * cs + (row - w0) * P + 1 + w;
   }
   auto send = [&](uint32_t per, int at, uint32_t v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(A.xbuf + (per & 1) * xparity + at),
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xbuf + (per & 1) * xparity + at),
                  "l"(((uint64_t)(per + 1) << 32) | v)
                  : "memory");
   };
   auto receive = [&](uint32_t per) {
-    const uint64_t* const buf = A.xbuf + (per & 1) * xparity;
+    const uint64_t* const buf = xbuf + (per & 1) * xparity;
     uint64_t v[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -401,7 +415,8 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
         if (it >= A.max_spin) {
           dead = true;
           atomicExch(A.error, 1);
-        } else if ((it & 1023) == 1023 && *static_cast<volatile int*>(A.error)) {
+        } else if ((it & 255) == 255 && (*static_cast<volatile int*>(A.error) ||
+                                         (couple && *static_cast<volatile int*>(A.best) < attempt))) {
           dead = true;
         }
       }
@@ -413,11 +428,11 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
   if (!updates) draw_batch(0);
   __syncthreads();
   // Held in registers: a parameter read again in each phase is a constant load on its critical path.
-  int depth = A.depth, sweeps = A.sweeps, items = A.items, group = A.group, row_words = P, class_words = cs;
+  int depth = A.depth, sweeps = all_sweeps, items = A.items, group = A.group, row_words = P, class_words = cs;
   asm volatile("" : "+r"(depth), "+r"(sweeps), "+r"(items), "+r"(group), "+r"(row_words), "+r"(class_words));
   int in_period = 0;  // sweeps since the last exchange
   uint32_t period = 0;
-  int2 ph = phase_tab[2 * min(A.depth, A.sweeps)];  // the phase's first row and its words
+  int2 ph = phase_tab[2 * min(A.depth, all_sweeps)];  // the phase's first row and its words
   for (int b = 0; b < batches; ++b) {
     if (updates) {
       const uint32_t* bits = drawn + (b & 1) * set_words;
@@ -480,15 +495,31 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
           if (A.bands > 1 && (f >> 1) + 1 < sweeps) receive(period++);
         }
       }
-    } else if (b + 1 < batches) {
-      draw_batch(b + 1);
+    } else {
+      if (couple && tid == updaters) s_stop[b & 1] = *static_cast<volatile int*>(A.best) < attempt;
+      if (b + 1 < batches) draw_batch(b + 1);
     }
     __syncthreads();
+    if (couple && *static_cast<volatile int*>(&s_stop[b & 1])) return;
+  }
+  if (couple) {  // the last band to finish knows whether any differs
+    const int mine = (band + 1 == A.bands ? A.R : r1) - r0;
+    bool differ = false;
+    for (int i = tid; i < 4 * mine * P; i += nt) {
+      const int at = (i / (mine * P)) * cs + (r0 - w0) * P + i % (mine * P);
+      differ = differ || sm[at] != sm[4 * cs + at];
+    }
+    const int any = __syncthreads_or(differ || dead ? 1 : 0);
+    if (tid == 0) {
+      if (any) atomicAdd(&A.team[team].x, 1);
+      __threadfence();
+      if (atomicAdd(&A.team[team].y, 1) == A.bands - 1 && atomicAdd(&A.team[team].x, 0) == 0) atomicMin(A.best, attempt);
+    }
   }
   const int own = (band + 1 == A.bands ? A.R : r1) - r0;  // the last row may be fixed: the last band's
   for (int i = tid; i < NCH * 4 * own * P; i += nt) {
     const int p = i % P, lr = (i / P) % own, cc = i / (P * own);
-    A.dst[(size_t)(cc >> 2) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(r0 + lr) * P + p] =
+    A.dst[(size_t)(2 * team + (cc >> 2)) * A.chain_words + (size_t)(cc & 3) * A.class_words + (size_t)(r0 + lr) * P + p] =
         sm[cc * cs + (r0 - w0 + lr) * P + p];
   }
 }
@@ -621,10 +652,10 @@ namespace {
 
 struct SvDevice {
   uint32_t* chains = nullptr;  // the state of the per-sub-sweep kernels; the resident engine's start
-  uint32_t* other = nullptr;   // resident engine: two more states, written in turn
+  uint32_t* other = nullptr;   // resident engine: two more states, written in turn, or one of each attempt side by side
   uint64_t* xbuf = nullptr;
   int32_t* heights = nullptr;
-  int* flag = nullptr;  // {chains differ or heights not valid, a wait gave up}
+  int* flag = nullptr;  // {chains differ or heights not valid, a wait gave up, SvBandArgs::best, unused, SvBandArgs::team}
   cudaStream_t stream = nullptr;
   ~SvDevice() {
     for (void* p : {(void*)chains, (void*)other, (void*)xbuf, (void*)heights, (void*)flag}) dev_free(p, stream);
@@ -653,7 +684,7 @@ rt_status sv_check_device() {
 struct SvBandPlan {
   bool ok = false;
   bool sum = false;  // thresholds depend on k1 + k2 only
-  int bands = 0, depth = 0, group = 0, batch = 0, items = 0, rows = 0, threads = 0;
+  int bands = 0, depth = 0, group = 0, batch = 0, items = 0, rows = 0, threads = 0, sms = 0;
   size_t smem = 0, xbuf_words = 0;
   void* kernel = nullptr;
 };
@@ -672,6 +703,7 @@ SvBandPlan sv_band_plan(const SvGeom& G, int chains, const std::vector<uint32_t>
     cudaGetLastError();
     return p;
   }
+  p.sms = sms;
   p.sum = sv_sum_thresholds(T);
   const int M = p.sum ? 5 : 9;
   // One band where half a warp holds a sub-sweep (n = 30: 0.84 us a sweep, two bands 0.95-1.0; n = 40: 1.08 and
@@ -731,6 +763,7 @@ struct SvRun {
   SvDevice dev;
   cudaStream_t st;
   bool bands = false;
+  int teams = 1;  // attempts side by side
 
   // keep: run() is called again, from the same start.
   rt_status prepare(int engine, bool keep) {
@@ -741,15 +774,67 @@ struct SvRun {
     if (engine != 1) plan = sv_band_plan(G, chains, T);
     // 256 words a band (n = 2048): 5.4 us a sweep, per-sub-sweep kernels 8.9; 484 (n = 2800): 13-15 and 11.
     bands = plan.ok && (engine == 2 || plan.items <= 320);
+    if (bands && keep) teams = std::max(1, std::min(kSvTeams, plan.sms / plan.bands));
     const size_t bytes = chains * G.chain_words * sizeof(uint32_t);
     if (rt_status e = dev_alloc(&dev.chains, bytes, st)) return e;
     if (bands || keep)
-      if (rt_status e = dev_alloc(&dev.other, (bands ? 2 : 1) * bytes, st)) return e;
-    if (rt_status e = dev_alloc(&dev.flag, 2 * sizeof(int), st)) return e;
+      if (rt_status e = dev_alloc(&dev.other, (bands ? std::max(2, teams) : 1) * bytes, st)) return e;
+    if (rt_status e = dev_alloc(&dev.flag, kFlagBytes, st)) return e;
     if (bands && plan.bands > 1)
-      if (rt_status e = dev_alloc(&dev.xbuf, plan.xbuf_words * sizeof(uint64_t), st)) return e;
-    cudaMemsetAsync(dev.flag, 0, 2 * sizeof(int), st);
+      if (rt_status e = dev_alloc(&dev.xbuf, teams * plan.xbuf_words * sizeof(uint64_t), st)) return e;
+    cudaMemsetAsync(dev.flag, 0, kFlagBytes, st);
     return RT_OK;
+  }
+
+  static constexpr size_t kFlagBytes = (4 + 2 * kSvTeams) * sizeof(int);
+
+  SvBandArgs band_args(uint64_t seed, uint32_t stream) const {
+    SvBandArgs A{};
+    A.chain_words = G.chain_words;
+    A.class_words = G.class_words;
+    A.P = G.P;
+    A.n = G.n;
+    A.R = G.R;
+    A.words = (G.n - 1) / 2 / 32 + 1;
+    A.bands = plan.bands;
+    A.depth = plan.depth;
+    A.group = plan.group;
+    A.batch = plan.batch;
+    A.items = plan.items;
+    A.rows = plan.rows;
+    uint32_t order[9];
+    const int by_sum[9] = {0, 1, 2, 5, 8, 0, 0, 0, 0};  // a threshold of each k1 + k2
+    for (int m = 0; m < 9; ++m) order[m] = T[plan.sum ? by_sum[m] : m];
+    sv_leaves(order, A.leaf);
+    A.seed = seed;
+    A.stream = stream;
+    A.xbuf = dev.xbuf;
+    A.error = dev.flag + 1;
+    A.max_spin = 1L << 22;
+    return A;
+  }
+
+  // Attempts [attempt0, attempt0 + n) of a coupling from the past side by side (n <= teams), attempt k from sweep
+  // -(first << k); dev.flag's best tells the smallest that coalesced.
+  void couple(uint64_t seed, uint32_t stream, int64_t first, int attempt0, int n) {
+    SvBandArgs A = band_args(seed, stream);
+    A.src = dev.chains;
+    A.dst = dev.other;
+    A.couple = 1;
+    A.attempt0 = attempt0;
+    A.first = first;
+    A.xteam = plan.xbuf_words;
+    A.best = dev.flag + 2;
+    A.team = reinterpret_cast<int2*>(dev.flag + 4);
+    cudaMemsetAsync(dev.flag, 0, kFlagBytes, st);
+    cudaMemsetAsync(A.best, 0x7f, sizeof(int), st);
+    void* args[] = {&A};
+    if (plan.bands > 1) {
+      cudaMemsetAsync(dev.xbuf, 0, n * plan.xbuf_words * sizeof(uint64_t), st);  // no stale tags
+      cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.bands, n), dim3(plan.threads), args, plan.smem, st);
+    } else {
+      cudaLaunchKernel(plan.kernel, dim3(1, n), dim3(plan.threads), args, plan.smem, st);
+    }
   }
 
   // Sub-sweeps [s0, s0 + count), whole sweeps, from the start states; returns where the states are.
@@ -778,28 +863,7 @@ struct SvRun {
       }
       return L.base;
     }
-    SvBandArgs A{};
-    A.chain_words = G.chain_words;
-    A.class_words = G.class_words;
-    A.P = G.P;
-    A.n = G.n;
-    A.R = G.R;
-    A.words = (G.n - 1) / 2 / 32 + 1;
-    A.bands = plan.bands;
-    A.depth = plan.depth;
-    A.group = plan.group;
-    A.batch = plan.batch;
-    A.items = plan.items;
-    A.rows = plan.rows;
-    uint32_t order[9];
-    const int by_sum[9] = {0, 1, 2, 5, 8, 0, 0, 0, 0};  // a threshold of each k1 + k2
-    for (int m = 0; m < 9; ++m) order[m] = T[plan.sum ? by_sum[m] : m];
-    sv_leaves(order, A.leaf);
-    A.seed = seed;
-    A.stream = stream;
-    A.xbuf = dev.xbuf;
-    A.error = dev.flag + 1;
-    A.max_spin = 1L << 22;
+    SvBandArgs A = band_args(seed, stream);
     A.src = dev.chains;
     constexpr int64_t kChunk = 1 << 14;  // sweeps per launch: bounds one launch to a fraction of a second
     for (int64_t done = 0; done < count / 4; done += kChunk) {
@@ -1011,19 +1075,31 @@ RT_API rt_status rt_sv_cftp(const int32_t* hmax, const int32_t* hmin, int32_t n,
   if (stats) std::memset(stats, 0, sizeof *stats);
   const uint32_t* at = R.dev.chains;
   float total_ms = 0.f;
-  int64_t Tsw = first_sweeps, total_sub = 0;
-  for (int attempt = 1; attempt <= max_attempts; ++attempt, Tsw *= 2) {
-    if (Tsw > ((int64_t)1 << 44)) break;
-    cudaMemsetAsync(R.dev.flag, 0, 2 * sizeof(int), st);
+  int64_t total_sub = 0;
+  // Attempts in groups of up to four, side by side (n = 48, first 64 sweeps: 3.9 -> 2.4 ms), up to 2^17 sweeps each
+  // (about 0.1 s); longer ones alone, in several launches.
+  for (int attempt = 0; attempt < max_attempts;) {
+    if (attempt > 44 || first_sweeps > ((int64_t)1 << 44) >> attempt) break;
+    int n = 0;
+    while (R.bands && n < R.teams && attempt + n < max_attempts && attempt + n < 44 &&
+           first_sweeps <= ((int64_t)1 << 17) >> (attempt + n))
+      ++n;
+    const int64_t Tsw = first_sweeps << attempt;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
-    at = R.run((uint64_t)seed, o.fast_stream, -4 * Tsw, 4 * Tsw);
-    cudaEventRecord(e1, st);
-    k_sv_diff<<<64, 256, 0, st>>>(at, at + G.chain_words, G.chain_words, (uint32_t*)R.dev.flag);
+    if (n > 0) {
+      R.couple((uint64_t)seed, o.fast_stream, first_sweeps, attempt, n);
+      cudaEventRecord(e1, st);
+    } else {
+      cudaMemsetAsync(R.dev.flag, 0, 2 * sizeof(int), st);
+      at = R.run((uint64_t)seed, o.fast_stream, -4 * Tsw, 4 * Tsw);
+      cudaEventRecord(e1, st);
+      k_sv_diff<<<64, 256, 0, st>>>(at, at + G.chain_words, G.chain_words, (uint32_t*)R.dev.flag);
+    }
     cudaError_t err = cudaGetLastError();
-    int flag[2] = {1, 0};
+    int flag[3] = {1, 0, 0};
     cudaMemcpyAsync(flag, R.dev.flag, sizeof flag, cudaMemcpyDeviceToHost, st);
     const cudaError_t waited = cudaStreamSynchronize(st);
     if (err == cudaSuccess) err = waited;
@@ -1034,18 +1110,27 @@ RT_API rt_status rt_sv_cftp(const int32_t* hmax, const int32_t* hmin, int32_t n,
     if (err != cudaSuccess) return fail(RT_ERR_CUDA, std::string("six-vertex cftp: ") + cudaGetErrorString(err));
     if (flag[1]) return fail(RT_ERR_TIMEOUT, "six-vertex cftp: a band gave up waiting for a neighbour's rows");
     total_ms += ms;
-    total_sub += 4 * Tsw;
-    if (stats) {
-      stats->attempts = attempt;
-      stats->total_steps = total_sub;
-      stats->flip_attempts += 2 * sv_interior_points(n) * Tsw;
-      stats->seconds = total_ms * 1e-3;
+    int ran = 1;
+    bool differ = flag[0] != 0;
+    if (n > 0) {
+      differ = flag[2] >= attempt + n;
+      ran = differ ? n : flag[2] - attempt + 1;
+      at = R.dev.other + (size_t)(ran - 1) * 2 * G.chain_words;
     }
-    if (!flag[0]) {
+    for (int k = 0; k < ran; ++k, ++attempt) {
+      total_sub += 4 * (first_sweeps << attempt);
+      if (stats) {
+        stats->attempts = attempt + 1;
+        stats->total_steps = total_sub;
+        stats->flip_attempts += 2 * sv_interior_points(G.n) * (first_sweeps << attempt);
+        stats->seconds = total_ms * 1e-3;
+      }
+    }
+    if (!differ) {
       std::vector<uint32_t> bits(G.chain_words);
       cudaMemcpy(bits.data(), at, bits.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost);
       sv_unpack(bits.data(), G, hmax, out);
-      if (stats) stats->final_steps = 4 * Tsw;
+      if (stats) stats->final_steps = 4 * (first_sweeps << (attempt - 1));
       return RT_OK;
     }
   }

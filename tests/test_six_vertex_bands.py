@@ -43,15 +43,19 @@ def test_walk_in_several_launches(rt):
         assert np.array_equal(a, b)
 
 
+# Attempts run side by side in groups: the first look-back decides which of a group coalesces first.
 @pytest.mark.gpu
 @pytest.mark.parametrize("abc", [(1.0, 1.0, 1.5), (0.9, 0.7, 1.1)])
 @pytest.mark.parametrize("n", [3, 16, 32, 33, 40, 66])
 def test_cftp_matches_sub_sweep_kernels(rt, n, abc):
     S = rt.SixVertexTiler
-    out, st = S(*abc, fast_stream=1).cftp(S.MaxHeight(n), S.MinHeight(n), 21, first_sweeps=16, max_attempts=16)
-    ref, sr = S(*abc, fast_stream=1, engine=1).cftp(S.MaxHeight(n), S.MinHeight(n), 21, first_sweeps=16, max_attempts=16)
-    assert np.array_equal(out, ref)
-    assert st["attempts"] == sr["attempts"] and st["total_steps"] == sr["total_steps"]
+    for first in (1, 3, 16, 600) if n < 40 else (16, 600):
+        out, st = S(*abc, fast_stream=1).cftp(S.MaxHeight(n), S.MinHeight(n), 21, first_sweeps=first, max_attempts=16)
+        ref, sr = S(*abc, fast_stream=1, engine=1).cftp(S.MaxHeight(n), S.MinHeight(n), 21, first_sweeps=first,
+                                                        max_attempts=16)
+        assert np.array_equal(out, ref)
+        for key in ("attempts", "total_steps", "final_steps", "flip_attempts"):
+            assert st[key] == sr[key], (first, key)
 
 
 @pytest.mark.gpu
