@@ -17,6 +17,8 @@
 // access; tagged words polled in shared memory: 0.57 us).  The draws do not depend on the state,
 // so warps of their own make them, a run ahead: they compose a run's half-sweeps into one pair of
 // move words per 32 cells, and the update warps apply those in a dozen logic operations.
+// It serves couplings from the past and launches that ask for 1..16 bands; a walk's exchange every few runs
+// (k_deep in domino_grid.cu) is faster, but takes every SM.
 // Measured (us per half-sweep, before: the best band shape): order 16 0.22 (before 0.66), order 100
 // 0.36 (0.82), order 200 0.88 (1.07) in TinyMT mode; order 16 0.35 (1.27), order 100 0.53 (1.58),
 // order 250 1.03 (1.48) in fast mode, where the draws of 16 SMs take over from the exchange.

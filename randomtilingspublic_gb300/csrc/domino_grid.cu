@@ -13,10 +13,11 @@
 // launch alternate in colour, so the two parities' slots hold the last changes of both planes when
 // the launch ends.  Every wait is bounded.
 //
-// Bound: small and mid-size domains by the exchange, 0.85 us a run through L2; from order 700 up by the
-// issue of the draws (order 1024: 237 words a band, about 24 instructions a word and half-sweep).  The
-// band kernel with polled deltas it replaces (domino_bits.cu) draws, exchanges and writes back in
-// turn.
+// Bound: mid-size domains by the exchange, 0.85 us a run through L2 (k_deep below makes one exchange serve
+// several runs); from order 700 up by the issue of the draws (order 1024: 237 words a band, about 24
+// instructions a word and half-sweep).  Measured (us per half-sweep, before: the band kernel with polled
+// deltas, domino_bits.cu, which draws, exchanges and writes back in turn): TinyMT order 400 0.62 (1.05), 512
+// 0.71 (1.2), 1024 with two chains 1.36 (1.95); fast mode order 1024 1.35 (3.2).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,6 +61,7 @@ struct GrArgs {
   int* error;
   long max_spin;
   int silent_band_plus1;
+  int depth, first, last;  // k_deep: runs between exchanges; the first and last row of any band
 };
 
 // Bounded wait for the element's tag; false (and the error word set) when it gave up, or another band did.
@@ -363,6 +365,272 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_gri
   cl_store_window<NCH>(sm, a.base, a.chain_stride, a.colour_stride, a.P, a.cols, r0 - 1, R, wlo, wn);
 }
 
+// The same sweep with an exchange every `depth` runs: a band also updates rows beyond its own, whose draws it
+// repeats, one row fewer on each side with every run, and takes the rows around its own anew (all four planes,
+// from the bands that own them) before the next `depth` runs.  One word or chain per update lane.  The draw
+// warps are a period of `depth` runs ahead, and only the update warps meet after every run.
+// Bound: a run's dependent instructions, 0.13 us, the exchange of a period, 0.7 us, and the issue of the draws,
+// the spare rows' included.  Measured (us per half-sweep, before: one cluster, domino_cluster.cu): TinyMT order
+// 16 0.17 (0.22), 40 0.23 (0.30), 100 0.30 (0.37), 200 0.38 (0.50 in k_grid); fast mode order 16 0.22 (0.31),
+// 40 0.27 (0.51), 100 0.34 (0.54), 300 0.56 (1.08 in k_grid).
+constexpr int kGrMove = 4;  // words of an exchange a lane sends, and takes
+constexpr int kGrMaxDepth = 12;
+
+template <int NCH, int kMode, int KS>
+__global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_deep(const __grid_constant__ GrArgs a) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  __shared__ uint4 srule[4];
+  __shared__ int s_cnt[2];
+  __shared__ uint32_t s_colour[2][kGrMaxDepth];
+  constexpr bool kFast = kMode == kClFast, kParams = kMode == kClTmtParams;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)(blockDim.x >> 5);
+  const int ndraw = a.draw_warps, nslots = ndraw * KS, band = blockIdx.x, depth = a.depth;
+  const int r0 = a.row_start[band], r1 = a.row_start[band + 1];
+  const int u0 = max(r0 - (depth - 1), a.first), u1 = min(r1 + depth, a.last + 1);  // rows updated in some run
+  const int i0 = u0 - 1, R = u1 - i0;                                              // window rows
+  const int wlo = a.windows[2 * band], wn = a.windows[2 * band + 1];
+  if (tid < 4)
+    srule[tid] = kFast ? make_uint4(a.rule.w_up[tid], a.rule.lo_dn[tid], a.rule.w_dn[tid], 0u)
+                       : make_uint4(a.rule.w_up[tid] << 9, a.rule.lo_dn[tid] << 9, a.rule.w_dn[tid] << 9, 0u);
+  // Shared memory as in k_grid: planes, a scratch word, slots, moves [period parity][run of the period][slot], the
+  // slot of each item.
+  uint32_t* const pad = sm + R * 4 * wn * NCH;
+  uint2* const sslot = reinterpret_cast<uint2*>(pad + kClPad);
+  uint2* const smove = sslot + nslots;
+  uint16_t* const sitem = reinterpret_cast<uint16_t*>(smove + 2 * depth * nslots);
+  for (int k = tid; k < nslots; k += (int)blockDim.x) sslot[k] = make_uint2(0u, 0u);
+  if (tid < 2) s_cnt[tid] = 0;
+  __syncthreads();
+  auto row_words = [&](int i, int* w0) -> int {
+    const int lo = i >= 1 && i <= a.N - 2 ? a.cand[i] : INT_MAX, hi = i >= 1 && i <= a.N - 2 ? a.cand[a.N + i] : 0;
+    if (lo == INT_MAX) return 0;
+    *w0 = lo >> 5;
+    return (hi >> 5) - (lo >> 5) + 1;
+  };
+  for (int i = u0 + tid; i < u1; i += (int)blockDim.x) {
+    int w0 = 0;
+    const int c = row_words(i, &w0);
+    if (c) atomicAdd(&s_cnt[i & 1], c);
+  }
+  __syncthreads();
+  const int c0 = s_cnt[0], c1 = s_cnt[1], nwords = c0 + c1;
+  const int need0 = (c0 + KS - 1) / KS, need1 = (c1 + KS - 1) / KS;
+  int cw0 = nwords > 0 ? (ndraw * c0 + nwords / 2) / nwords : ndraw;
+  cw0 = min(max(cw0, need0), ndraw - need1);
+  const int cw1 = ndraw - cw0;
+  const int per0 = cw0 ? (c0 + cw0 - 1) / cw0 : 1, per1 = cw1 ? (c1 + cw1 - 1) / cw1 : 1;
+  for (int i = u0 + tid; i < u1; i += (int)blockDim.x) {
+    int w0 = 0, before = 0, item = 0;
+    const int c = row_words(i, &w0);
+    for (int q = u0; q < i; ++q) {
+      int x;
+      const int n = row_words(q, &x);
+      if (((q ^ i) & 1) == 0) before += n;
+      item += n;
+    }
+    const int per = (i & 1) ? per1 : per0, first = (i & 1) ? cw0 : 0;
+    for (int k = 0; k < c; ++k) {
+      const int w = w0 + k, at = before + k, slot = (first + at / per) * KS + at % per;
+      const int blo = max(a.cand[i] - 32 * w, 0), bhi = min(a.cand[a.N + i] - 32 * w, 31);
+      sslot[slot] = make_uint2(((uint32_t)i << 16) | (uint32_t)w, (0xffffffffu << blo) & (0xffffffffu >> (31 - bhi)));
+      sitem[item + k] = (uint16_t)slot;
+    }
+  }
+  cl_load_window<NCH>(sm, a.base, a.chain_stride, a.colour_stride, a.P, i0, R, wlo, wn);
+  __syncthreads();
+  auto run_at = [&](int j) -> uint32_t {
+    if (kFast) return ((a.h0 + j) & 1) ? 1u : 0x80000001u;  // even half-sweeps black (colour 1)
+    return j < a.nruns ? __ldg(&a.runs[j]) : 0u;
+  };
+  // Runs left before the next exchange at which row i is first needed.
+  auto needed = [&](int i) { return i < r0 ? r0 - i + 1 : (i >= r1 ? i - r1 + 1 : 1); };
+  const int nruns = a.nruns, periods = (nruns + depth - 1) / depth;
+  bool dead = false;  // a wait gave up: no more waits, the launch runs to its end
+  if (warp >= ndraw) {
+    // ---- update warps
+    const int ut = tid - 32 * ndraw, nupd = 32 * (nwarps - ndraw);
+    const uint32_t pitch = (uint32_t)(wn * NCH * 16), move_bytes = (uint32_t)(nslots * sizeof(uint2));
+    const int k = ut / NCH, c = ut % NCH, slot = k < nwords ? (int)sitem[k] : 0;
+    const uint2 e = k < nwords ? sslot[slot] : make_uint2(0u, 0u);
+    const uint32_t valid = e.y;
+    const int i = (int)(e.x >> 16), w = (int)(e.x & 0xffffu), need = valid ? needed(i) : INT_MAX;
+    const bool odd = i & 1;
+    const uint32_t move_at = (uint32_t)__cvta_generic_to_shared(smove + slot);
+    const uint32_t above = (uint32_t)__cvta_generic_to_shared(valid ? sm + (((i - 1 - i0) * wn + w - wlo) * NCH + c) * 4 : pad + 8);
+    const uint32_t here = valid ? above + pitch : above;
+    // Exchange words: of row i those that its own, the row above's or the row below's candidates change, and the
+    // word to the left (its last HO bit).  Per lane, the same every time; ~0: none.
+    const bool silent = band + 1 == a.silent_band_plus1;  // test hook: publishes nothing
+    const uint32_t parity = (uint32_t)((a.last - a.first + 1) * a.xn * NCH * 4);
+    uint32_t send_at[kGrMove], send_to[kGrMove], take_at[kGrMove], take_to[kGrMove];
+    auto element = [&](int row, int q, uint32_t* local, uint32_t* global) {
+      const int p = q & 3, cc = (q >> 2) % NCH, ww = a.xlo + (q >> 2) / NCH;
+      int lo = INT_MAX, hi = -1;
+      for (int r = row - 1; r <= row + 1; ++r) {
+        int first = 0;
+        const int n = row_words(r, &first);
+        if (n) lo = min(lo, first - 1), hi = max(hi, first + n - 1);
+      }
+      if (row < a.first || row > a.last || row < i0 || row >= u1 || ww < lo || ww > hi || ww < wlo || ww >= wlo + wn) return;
+      *local = (uint32_t)__cvta_generic_to_shared(sm + (((row - i0) * wn + ww - wlo) * NCH + cc) * 4 + p);
+      *global = (uint32_t)((row - a.first) * a.xn * NCH * 4 + q);
+    };
+    const int per_row = a.xn * NCH * 4, own = r1 - r0, edge_rows = min(own, 2 * depth);
+#pragma unroll
+    for (int m = 0; m < kGrMove; ++m) {
+      send_at[m] = take_at[m] = ~0u;
+      send_to[m] = take_to[m] = 0u;
+      const int x = ut + m * nupd, y = x / per_row, q = x - y * per_row;
+      if (y < edge_rows && !silent) element(own <= 2 * depth || y < depth ? r0 + y : r1 - 2 * depth + y, q, &send_at[m], &send_to[m]);
+      if (y < 2 * depth) element(y < depth ? r0 - depth + y : r1 + y - depth, q, &take_at[m], &take_to[m]);
+    }
+    auto exchange = [&](uint32_t period) {
+      uint64_t* const buf = a.xbuf + (period & 1u) * parity;
+      uint64_t v[kGrMove];
+#pragma unroll
+      for (int m = 0; m < kGrMove; ++m)
+        if (send_at[m] != ~0u) gr_send(buf + send_to[m], period + 1u, cl_lds(send_at[m]));
+#pragma unroll
+      for (int m = 0; m < kGrMove; ++m)
+        if (take_at[m] != ~0u) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[m]) : "l"(buf + take_to[m]) : "memory");
+#pragma unroll
+      for (int m = 0; m < kGrMove; ++m) {
+        if (take_at[m] == ~0u) continue;
+        uint32_t got = (uint32_t)v[m];
+        if ((uint32_t)(v[m] >> 32) != period + 1u && !dead && !gr_recv(buf + take_to[m], period + 1u, got, a.max_spin, a.error))
+          dead = true;
+        if (!dead) cl_sts(take_at[m], got);
+      }
+      asm volatile("bar.sync 1, %0;" ::"r"(nupd) : "memory");
+    };
+    __syncthreads();  // the first period's moves are drawn
+    for (int q = 0; q < periods; ++q) {
+      if (q > 0) exchange((uint32_t)q - 1u);
+      const int len = min(depth, nruns - q * depth);
+      uint32_t at = move_at + (uint32_t)((q & 1) * depth) * move_bytes;
+      for (int r = 0; r < len; ++r, at += move_bytes) {
+        const uint32_t t = s_colour[q & 1][r];
+        if (need <= len - r) {
+          const uint32_t off_u = t ? 0u : 4u, off_d = 4u - off_u;
+          const uint2 move = cl_lds2(at);
+          const uint2 ab = cl_lds2(above);
+          const uint4 me = cl_lds4(here);
+          const uint32_t west = cl_lds(here - 16u * NCH + 12u);
+          const bool aligned = odd == (t != 0u);  // left HE, right HO of the same word
+          const uint32_t U = t ? ab.x : ab.y, D = t ? me.y : me.x;
+          const uint32_t lft = aligned ? me.z : __funnelshift_l(west, me.w, 1), rgt = aligned ? me.w : me.z;
+          const uint32_t flip = ~(U ^ D) & ~(lft ^ rgt) & (U ^ lft) & valid;
+          const uint32_t T = flip & ((U & ~move.x) | (~U & move.y));
+          cl_sts(above + off_u, U ^ T);
+          cl_sts(here + off_d, D ^ T);
+          cl_sts(here + 8u, me.z ^ T);
+          cl_xor(here + 12u, aligned ? T : T >> 1);
+          cl_xor_if(here - 16u * NCH + 12u, aligned ? 0u : T << 31);
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(nupd) : "memory");
+      }
+      cl_cta_sync();
+    }
+    // The rows around its own as the other bands leave them; and no band writes back before the bands around it
+    // have loaded.
+    if (periods > 0) exchange((uint32_t)periods - 1u);
+  } else {
+    // ---- draw warps
+    const int par = (int)((sslot[warp * KS].x >> 16) & 1u);
+    auto gen_index = [&](int s, bool* v) -> int64_t {
+      const uint2 e = sslot[warp * KS + s];
+      *v = (e.y >> lane) & 1u;
+      return (int64_t)((int)(e.x >> 16) - 1) * a.cols + (32 * (int)(e.x & 0xffffu) + lane - 1);
+    };
+    auto params_of = [&](int s, uint32_t& m1, uint32_t& m2, uint32_t& tm) {
+      m1 = kTmtMat1;
+      m2 = kTmtMat2;
+      tm = kTmtTmat;
+      if (kParams) {
+        bool v;
+        const int64_t g = gen_index(s, &v);
+        const uint4 p = __ldg(&a.tmt_params[v ? g : 0]);
+        m1 = p.x;
+        m2 = p.y;
+        tm = p.z;
+      }
+    };
+    uint4 gen[kFast ? 1 : KS];
+    uint32_t f_row[kFast ? KS / 4 : 1], f_quad[kFast ? KS / 4 : 1];
+    int f_need[kFast ? KS / 4 : 1];  // runs left at which the group is first needed
+    if constexpr (!kFast) {
+#pragma unroll
+      for (int s = 0; s < KS; ++s) {
+        bool v;
+        const int64_t g = gen_index(s, &v);
+        gen[s] = make_uint4(0u, 0u, 0u, 0u);
+        if (v) gen[s] = a.tmt[g];
+      }
+    } else {
+#pragma unroll
+      for (int g = 0; g < KS / 4; ++g) {
+        const uint2 e = sslot[warp * KS + 4 * g + (lane >> 3)];
+        f_row[g] = e.x >> 16;
+        f_quad[g] = (e.x & 0xffffu) * 8u + (uint32_t)(lane & 7);
+        f_need[g] = __reduce_min_sync(~0u, e.y ? needed((int)f_row[g]) : INT_MAX);
+      }
+    }
+    // A period's runs, from run j0 on.
+    auto draw_period = [&](int q) {
+      const int j0 = q * depth, len = min(depth, nruns - j0);
+      uint2* const out = smove + (q & 1) * depth * nslots;
+      if constexpr (!kFast) {
+        for (int r = 0; r < len; ++r) {
+          const uint32_t run = run_at(j0 + r);
+          if (tid == 0) s_colour[q & 1][r] = run >> 31;
+          cl_moves_tmt<KS>(gen, srule[par | ((int)(run >> 31) << 1)], (int)(run & 0x3fffffffu),
+                           out + r * nslots + warp * KS, params_of);
+        }
+      } else {
+        // two runs at a time: a Philox block is a chain of its own
+        for (int r = 0; r < len; r += 2) {
+          const uint32_t c0 = run_at(j0 + r) >> 31, c1 = c0 ^ 1u;
+          if (tid == 0) {
+            s_colour[q & 1][r] = c0;
+            if (r + 1 < len) s_colour[q & 1][r + 1] = c1;
+          }
+          const uint4 rl0 = srule[par | (int)(c0 << 1)], rl1 = srule[par | (int)(c1 << 1)];
+#pragma unroll
+          for (int g = 0; g < KS / 4; ++g) {
+            if (f_need[g] > len - r) continue;
+            uint2* const to = out + r * nslots + warp * KS + 4 * g;
+            if (f_need[g] <= len - r - 1) {
+              cl_moves_fast2(a.seed, a.stream, a.h0 + j0 + r, f_row[g], f_quad[g], rl0, rl1, to, to + nslots);
+            } else {
+              cl_moves_fast(a.seed, a.stream, a.h0 + j0 + r, f_row[g], f_quad[g], rl0, to);
+            }
+          }
+        }
+      }
+    };
+    if (periods > 0) draw_period(0);
+    __syncthreads();
+    for (int q = 0; q < periods; ++q) {
+      if (q + 1 < periods) draw_period(q + 1);
+      cl_cta_sync();
+    }
+    __syncthreads();  // the bands around have loaded (the last exchange)
+    if constexpr (!kFast) {
+#pragma unroll
+      for (int s = 0; s < KS; ++s) {
+        bool v;
+        const int64_t g = gen_index(s, &v);
+        const int i = (int)(sslot[warp * KS + s].x >> 16);
+        if (v && i >= r0 && i < r1) a.tmt[g] = gen[s];
+      }
+    }
+  }
+  if (warp >= ndraw) __syncthreads();
+  if (__syncthreads_or(dead ? 1 : 0) && tid == 0) atomicExch(a.error, 1);
+  cl_store_window<NCH>(sm + (r0 - 1 - i0) * 4 * wn * NCH, a.base, a.chain_stride, a.colour_stride, a.P, a.cols, r0 - 1, r1 - r0 + 1,
+                       wlo, wn);
+}
+
 template <int NCH, int kMode, int UI>
 void* gr_kernel_ks(int ks) {
   if constexpr (kMode == kClFast) {
@@ -390,6 +658,15 @@ void* gr_kernel_mode(int mode, int ks) {
 void* gr_kernel(int nch, int mode, int ks, int ui) {
   if (nch == 1) return ui == 1 ? gr_kernel_mode<1, 1>(mode, ks) : gr_kernel_mode<1, 4>(mode, ks);
   return ui == 1 ? gr_kernel_mode<2, 1>(mode, ks) : gr_kernel_mode<2, 4>(mode, ks);
+}
+
+template <int NCH>
+void* gr_deep_kernel(int mode, int ks) {
+  if (mode == kClFast) return ks == 4 ? (void*)k_deep<NCH, kClFast, 4> : (void*)k_deep<NCH, kClFast, 8>;
+  if (mode == kClTmt)
+    return ks == 1 ? (void*)k_deep<NCH, kClTmt, 1> : (ks == 2 ? (void*)k_deep<NCH, kClTmt, 2> : (void*)k_deep<NCH, kClTmt, 4>);
+  return ks == 1 ? (void*)k_deep<NCH, kClTmtParams, 1>
+                 : (ks == 2 ? (void*)k_deep<NCH, kClTmtParams, 2> : (void*)k_deep<NCH, kClTmtParams, 4>);
 }
 
 #define RT_CUDA_G(expr)                                                                 \
@@ -512,8 +789,91 @@ void GrPlan::build(const std::vector<int>& lo, const std::vector<int>& hi, int N
   ok = true;
 }
 
+// The same domain with an exchange every `runs` runs; false where no form of k_deep holds it.
+bool GrPlan::build_deep(const std::vector<int>& lo, const std::vector<int>& hi, int N, int nch, bool fast, int bands_max, int runs) {
+  const int rows = N - 2;
+  std::vector<int> cnt(N + 1, 0);
+  int w0 = INT_MAX, w1 = -1;
+  first = last = -1;
+  for (int i = 1; i <= rows; ++i) {
+    if (lo[i] < 0) continue;
+    cnt[i] = hi[i] / 32 - lo[i] / 32 + 1;
+    w0 = std::min(w0, lo[i] / 32);
+    w1 = std::max(w1, hi[i] / 32);
+    if (first < 0) first = i;
+    last = i;
+  }
+  first = std::max(1, first - 1);
+  last = std::min(rows, last + 1);
+  xlo = w0 - 1;
+  xn = w1 - w0 + 2;
+  const int total = last - first + 1;
+  bands = std::min(std::min(bands_max, kGrMaxBands), total);
+  for (int k = 0; k <= bands; ++k) row_start[k] = first + (int)((int64_t)total * k / bands);
+  size_t window_max = 0;
+  int64_t words_max = 0, send_max = 0;
+  std::vector<int64_t> par((size_t)bands * 2, 0);
+  for (int k = 0; k < bands; ++k) {
+    const int r0 = row_start[k], r1 = row_start[k + 1], u0 = std::max(r0 - (runs - 1), first), u1 = std::min(r1 + runs, last + 1);
+    int a0 = INT_MAX, a1 = -1;
+    for (int i = u0 - 1; i <= u1; ++i)
+      if (i >= 1 && i <= rows && lo[i] >= 0) {
+        a0 = std::min(a0, lo[i] / 32);
+        a1 = std::max(a1, hi[i] / 32);
+      }
+    if (a1 < 0) a0 = a1 = w0;
+    windows[2 * k] = a0 - 2;
+    windows[2 * k + 1] = a1 - a0 + 5;
+    window_max = std::max(window_max, (size_t)(u1 - u0 + 1) * windows[2 * k + 1]);
+    for (int i = u0; i < u1; ++i) par[2 * k + (i & 1)] += cnt[i];
+    words_max = std::max(words_max, par[2 * k] + par[2 * k + 1]);
+    send_max = std::max<int64_t>(send_max, std::max(std::min(r1 - r0, 2 * runs), 2 * runs) * (int64_t)xn * nch * 4);
+  }
+  if (words_max * nch > 320) return false;
+  update_warps = (int)std::max<int64_t>(1, (std::max(words_max * nch, (send_max + kGrMove - 1) / kGrMove) + 31) / 32);
+  per_lane = 1;
+  slots = 0;
+  for (int ks : {1, 2, 4, 8}) {
+    if (fast ? ks < 4 : ks > 4) continue;
+    int64_t draw = 1;
+    for (int k = 0; k < bands; ++k) draw = std::max<int64_t>(draw, (par[2 * k] + ks - 1) / ks + (par[2 * k + 1] + ks - 1) / ks);
+    if (draw + update_warps > gr_max_threads(fast, ks) / 32) continue;
+    slots = ks;
+    draw_warps = (int)draw;
+    break;
+  }
+  if (!slots) return false;
+  smem_bytes = (window_max * 4 * nch + kClPad) * sizeof(uint32_t) +
+               (1 + 2 * (size_t)runs) * (size_t)draw_warps * slots * sizeof(uint2) + (size_t)words_max * sizeof(uint16_t) + 16;
+  if (smem_bytes > 200 * 1024) return false;
+  depth = runs;
+  return true;
+}
+
 GridEngine::~GridEngine() {
   for (void* p : {(void*)d_rows, (void*)d_xbuf, (void*)d_runs}) dev_free(p, stream);
+}
+
+// Runs between exchanges: more of them share one exchange, but a band of rho rows draws for rho + 2 d - 1.
+// Measured (us per half-sweep, diamonds, one chain; d = 1 is k_grid):
+//   TinyMT  order 16: d = 4 0.19, 6 0.17, 8 0.19    40: 4 0.22, 6 0.23, 8 0.25    64: 4 0.25, 6 0.24, 8 0.28
+//           100: 1 0.51, 2 0.41, 3 0.35, 4 0.30, 6 0.37    200: 1 0.50, 2 0.38, 3 0.41    250: 1 0.54, 2 0.47, 3 0.57
+//           300: 1 0.57, 2 0.60
+//   fast    order 24: d = 4 0.35, 8 0.29, 12 0.22    64: 4 0.45, 8 0.31, 12 0.29    100: 1 0.99, 4 0.42, 8 0.35
+//           150: 4 0.45, 6 0.37, 8 0.37, 12 0.48    200: 1 1.06, 3 0.52, 4 0.45, 6 0.44, 8 0.50
+//           300: 1 1.08, 3 0.57, 4 0.56, 6 0.60    400: 2 0.72, 3 0.76    512: 2 0.95, 3 1.23
+// (rows of 1, 2, 3, 4, 5, 7, 8, 10, 13 and 17 words).  Wider rows than the last ones: d = 1.
+static int gr_depth(const GrPlan& p, bool fast) {
+  const int rho = (p.row_start[p.bands] - p.row_start[0] + p.bands - 1) / p.bands;
+  const auto words = [&](int d) { return (rho + 2 * d - 1) * p.xn; };
+  if (fast) {
+    for (int d = 12; d > 2; --d)
+      if (words(d) <= (d > 8 ? 75 : 110)) return d;
+    return words(2) <= 175 ? 2 : 1;
+  }
+  for (int d = 6; d > 2; --d)
+    if (words(d) <= 36) return d;
+  return words(2) <= 56 ? 2 : 1;
 }
 
 rt_status GridEngine::prepare(DmSampler& s) {
@@ -547,9 +907,17 @@ rt_status GridEngine::prepare(DmSampler& s) {
     plan.why = "device lacks cooperative launch";
     return RT_OK;
   }
-  plan.build(s.cand_lo, s.cand_hi, s.N, nch, fast, s.eff_bands > 0 ? std::min(s.eff_bands, sms) : sms);
+  const int bands_max = s.eff_bands > 0 ? std::min(s.eff_bands, sms) : sms;
+  plan.depth = 1;
+  plan.build(s.cand_lo, s.cand_hi, s.N, nch, fast, bands_max);
   if (!plan.ok) return RT_OK;
-  kernel = gr_kernel(nch, fast ? kClFast : (s.tmt_params ? kClTmtParams : kClTmt), plan.slots, plan.per_lane);
+  const int mode = fast ? kClFast : (s.tmt_params ? kClTmtParams : kClTmt);
+  if (const int runs = gr_depth(plan, fast); runs > 1) {
+    GrPlan deep = plan;
+    if (deep.build_deep(s.cand_lo, s.cand_hi, s.N, nch, fast, bands_max, runs)) plan = deep;
+  }
+  kernel = plan.depth > 1 ? (nch == 1 ? gr_deep_kernel<1>(mode, plan.slots) : gr_deep_kernel<2>(mode, plan.slots))
+                          : gr_kernel(nch, mode, plan.slots, plan.per_lane);
   RT_CUDA_G(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_G(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, plan.threads(), plan.smem_bytes));
@@ -560,7 +928,8 @@ rt_status GridEngine::prepare(DmSampler& s) {
   }
   if (!d_rows) {
     if (rt_status st = dev_alloc(&d_rows, (3 * kGrMaxBands + 2) * sizeof(int), stream)) return st;
-    xbuf_bytes = (size_t)2 * plan.bands * 2 * plan.xn * nch * sizeof(uint64_t);
+    xbuf_bytes = plan.depth > 1 ? (size_t)2 * (plan.last - plan.first + 1) * plan.xn * nch * 4 * sizeof(uint64_t)
+                                : (size_t)2 * plan.bands * 2 * plan.xn * nch * sizeof(uint64_t);
     if (rt_status st = dev_alloc(&d_xbuf, xbuf_bytes, stream)) return st;
   }
   RT_CUDA_G(cudaMemcpyAsync(d_rows, plan.row_start, sizeof plan.row_start, cudaMemcpyHostToDevice, stream));
@@ -590,6 +959,9 @@ rt_status GridEngine::launch(DmSampler& s, const uint8_t* colours_host, int64_t 
     a.windows = d_rows + kGrMaxBands + 1;
     a.xlo = plan.xlo;
     a.xn = plan.xn;
+    a.depth = plan.depth;
+    a.first = plan.first;
+    a.last = plan.last;
     a.rule = s.rule;
     a.stream = s.opts.fast_stream;
     a.xbuf = d_xbuf;

@@ -24,9 +24,12 @@ struct GrPlan {
   int xlo = 0, xn = 0;                // first word and words of an exchange row
   int64_t words = 0, draw_cells = 0;
   size_t smem_bytes = 0;
+  int depth = 1;            // runs between exchanges (1: k_grid, more: k_deep)
+  int first = 0, last = 0;  // k_deep: first and last row of any band
   int threads() const { return 32 * (draw_warps + update_warps); }
   // From each colour-array row's first and last flip-candidate column (-1: none).
   void build(const std::vector<int>& lo, const std::vector<int>& hi, int N, int nch, bool fast, int bands_max);
+  bool build_deep(const std::vector<int>& lo, const std::vector<int>& hi, int N, int nch, bool fast, int bands_max, int runs);
 };
 
 struct GridEngine {

@@ -149,10 +149,8 @@ __device__ __forceinline__ void cl_moves_tmt(uint4 (&gen)[KS], uint4 rl, int L, 
 
 // Fast mode: one half-sweep of four words, lane l quad l % 8 of word l / 8 (row, quad: its Philox
 // counter); four tests each way as one nibble, two lanes' nibbles as one byte of the word's moves.
-__device__ __forceinline__ void cl_moves_fast(uint64_t seed, uint32_t stream, int64_t h, uint32_t row, uint32_t quad,
-                                              uint4 rl, uint2* out) {
+__device__ __forceinline__ void cl_moves_of(const uint4& d, uint4 rl, uint2* out) {
   const int lane = threadIdx.x & 31;
-  const uint4 d = fast_quad(seed, stream, h, row, quad);
   const uint32_t u = cl_nibble(d.x < rl.x, d.y < rl.x, d.z < rl.x, d.w < rl.x);
   const uint32_t v = cl_nibble(d.x - rl.y < rl.z, d.y - rl.y < rl.z, d.z - rl.y < rl.z, d.w - rl.y < rl.z);
   const uint32_t mine = (u ^ 15u) | (v << 16);
@@ -162,6 +160,17 @@ __device__ __forceinline__ void cl_moves_fast(uint64_t seed, uint32_t stream, in
     to[0] = (uint8_t)pair;
     to[4] = (uint8_t)(pair >> 16);
   }
+}
+__device__ __forceinline__ void cl_moves_fast(uint64_t seed, uint32_t stream, int64_t h, uint32_t row, uint32_t quad,
+                                              uint4 rl, uint2* out) {
+  cl_moves_of(fast_quad(seed, stream, h, row, quad), rl, out);
+}
+// Two half-sweeps, h and h + 1, whose Philox blocks are computed side by side.
+__device__ __forceinline__ void cl_moves_fast2(uint64_t seed, uint32_t stream, int64_t h, uint32_t row, uint32_t quad,
+                                               uint4 rl0, uint4 rl1, uint2* out0, uint2* out1) {
+  const uint4 d0 = fast_quad(seed, stream, h, row, quad), d1 = fast_quad(seed, stream, h + 1, row, quad);
+  cl_moves_of(d0, rl0, out0);
+  cl_moves_of(d1, rl1, out1);
 }
 
 }  // namespace rt

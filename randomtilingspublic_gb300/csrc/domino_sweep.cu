@@ -576,7 +576,8 @@ rt_status DmSampler::use_persistent(bool* yes) {
     eff_threads = tuned ? t : 0;
     return tuned;
   };
-  if (ask_table) take_entry(0);
+  // A coupling runs its attempts side by side in clusters, where one holds the domain.
+  if (ask_table && !couple) take_entry(0);
   if (engine == 1 || opts.rng_mode == RT_RNG_MTGP) return RT_OK;
   if (plan_dirty) {
     if (rt_status st = fetch_candidates()) return st;
@@ -599,6 +600,23 @@ rt_status DmSampler::use_persistent(bool* yes) {
   // exchange (cl_auto_words).  A table entry that asks for it gives way to the next where the
   // domain does not fit.
   const bool fast = opts.rng_mode == RT_RNG_FAST;
+  // With an exchange every few runs one band per SM is faster than a cluster (domino_grid.cu).
+  auto try_grid = [&](bool deep_only) -> rt_status {
+    if (grid && (grid->nch != active || grid->bands_asked != eff_bands)) grid.reset();
+    if (!grid) {
+      grid = std::make_unique<GridEngine>();
+      if (rt_status st = grid->prepare(*this)) return st;
+    }
+    if (!grid->ready || (deep_only && grid->plan.depth < 2)) return RT_OK;
+    resident = 4;
+    on_grid = true;
+    *yes = true;
+    return RT_OK;
+  };
+  if (!couple && !explicit_engine && (engine == 0 || engine == 4) && (eff_bands == 0 || eff_bands > kClMaxCtas)) {
+    if (rt_status st = try_grid(true)) return st;
+    if (on_grid) return RT_OK;
+  }
   for (int skip = 0; (engine == 0 || (engine == 4 && !(fast && explicit_engine))) && eff_bands <= kClMaxCtas &&
                      (eff_bands > 0 || engine == 0);) {
     if (cluster && (cluster->nch != active || cluster->bands_asked != eff_bands)) cluster.reset();
@@ -615,20 +633,12 @@ rt_status DmSampler::use_persistent(bool* yes) {
     if (!tuned) break;
     take_entry(++skip);
   }
+  if (ask_table && couple) take_entry(0);
   // The bit-plane kernel on every SM: where the table asks for engine 4 or bands are asked for, and
   // automatically in TinyMT mode (in fast mode without a table the run kernel stays the choice).
   if ((engine == 0 || engine == 4) && !explicit_engine && (!fast || tuned || eff_bands > 0)) {
-    if (grid && (grid->nch != active || grid->bands_asked != eff_bands)) grid.reset();
-    if (!grid) {
-      grid = std::make_unique<GridEngine>();
-      if (rt_status st = grid->prepare(*this)) return st;
-    }
-    if (grid->ready) {
-      resident = 4;
-      on_grid = true;
-      *yes = true;
-      return RT_OK;
-    }
+    if (rt_status st = try_grid(false)) return st;
+    if (on_grid) return RT_OK;
   }
   // Engine 0: the bit-plane kernel, else the run kernel, else k_persist; 4: the bit-plane
   // kernel alone; 2: the run kernel, else k_persist; 3: k_persist alone.
@@ -956,6 +966,7 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   if (rt_status st = s->load(3, tmax)) return st;
   s->active = 2;
   s->plan_dirty = true;
+  s->couple = true;
   const bool fast = o.rng_mode == RT_RNG_FAST;
   // The reference's epoch schedule (AztecDiamondCftpEx.cpp:54-77), drawn ahead for every
   // attempt: epoch k is created by attempt k with the driver's k-th draw as its seed, and

@@ -116,3 +116,23 @@ def test_grid_wait_gives_up_and_the_sampler_stays_usable(rt, rng):
     want = [ref.store(0), ref.store(1)]
     ref.close()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("rng", ["tinymt", "table", "fast"])
+@pytest.mark.parametrize("shape", [1, 2, 5, 16, 24, 61, 64, 96, 150, 200, 250, (8, 90), (300, 20), (64, 448), (301, 442)])
+def test_automatic_depth_equals_per_half_sweep_kernels(rt, rng, shape):
+    # 12, 8, .. 2 runs between exchanges (fewer in TinyMT mode): launches of fewer runs than that, of a whole number
+    # of them and of others
+    tmax, tmin = _start(rt, shape)
+    n = rt.side_of(tmax)
+    tiler = rt.DominoTiler(rule="cftp_twoperiodic", rng="fast" if rng == "fast" else "tinymt", a=1.0, b=0.7,
+                           fast_stream=5)
+    if rng == "table":
+        tiler.LoadTinyMT(np.random.RandomState(n).randint(0, 2**32, size=((n - 2) * (n // 2 - 2), 3), dtype=np.uint32))
+    steps = [(48, 11), (1, 4), (5, 5), (121, 12)]
+    for starts in ([tmin], [tmin, tmax]):
+        got, info = _chains(rt, tiler, starts, (0, 0, 0), steps)
+        assert info["engine"] == 4
+        want, _ = _chains(rt, tiler, starts, (1, 0, 0), steps)
+        for g, w in zip(got, want):
+            assert np.array_equal(g, w), (shape, rng)
