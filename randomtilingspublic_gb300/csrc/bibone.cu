@@ -11,7 +11,6 @@
 // site of the chosen class whose cycle has one half covered flips with probability 1/2.
 // Same-class cycles are edge-disjoint (the reference's colourings), and two cycles that can
 // flip together share no vertex, so byte read-modify-writes never race.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <curand_kernel.h>
 
@@ -142,7 +141,7 @@ __global__ void k_td_step_fast(uint8_t* D, int M, TdStep s, uint64_t seed, uint3
   }
 }
 
-// ---- the cluster kernel ------------------------------------------------------------------------
+// ---- the resident kernel -----------------------------------------------------------------------
 //
 // The dimers as bit planes: per vertex row three planes of 32-bit words (H, L, R), bit k of word w
 // for column 32 w + k.  A step is then a handful of logic operations per word: the cycles of 32
@@ -151,38 +150,47 @@ __global__ void k_td_step_fast(uint8_t* D, int M, TdStep s, uint64_t seed, uint3
 // words are read and toggled (shared-memory XOR) within one step without order, and one barrier
 // separates steps.
 //
-// The rows live in the shared memory of one thread-block cluster.  A CTA owns the sites of rows
-// [r0, r1) and holds rows r0 - 2 .. r1 (all that its cycles reach); a toggle of a row that a
-// neighbour holds too goes to both copies (XOR through distributed shared memory).
+// The rows live in the shared memory of every SM, a band of site rows [own0, own1) per CTA.  A step's sites of
+// row a read and change vertex rows a - 2 .. a + 1, so what a band knows shrinks by three rows on each side
+// with every step: it starts a period of `depth` steps from 3 depth rows around its own (taken from the
+// bands that own them, as 64-bit words tagged with the period, through L2; every wait bounded) and makes
+// the steps of its neighbours' sites with its own, draws included.  A small region is one CTA's.
 //
-// Draws.  Fast mode: only quads of columns with a site that can flip need their Philox block, so
-// the step first lists those (about a tenth of them), then draws for the list.  TinyMT: every
-// site's generator is in a register of the lane of its column, a ballot gives a word's acceptance
-// bits, and a step's draws are made between arrival and wait of the barrier before it.
+// Draws.  Fast mode: only quads of columns with a site that can flip need their Philox block, so a warp
+// lists those of its words (about a tenth of them), then draws for the list.  TinyMT: every site's
+// generator is in a register of the lane of its column, and a ballot gives a word's acceptance bits.
 //
-// Bound: the dependent instructions of a step's two passes and the cluster barrier between steps
-// (its release waits for the toggles across the seams): a third of the issue slots are used.
-// Rhombus 512, fast mode: 2.6 us a step; with one launch per step and a byte per vertex 5.3 us on the
-// device and 7.8 in the call, whose launches the host could not issue faster.
-constexpr int kTdClCtas = 16;
-constexpr int kTdFastThreads = 1024, kTdTmtThreads = 512;  // TinyMT: up to 128 registers a thread
-constexpr int kTdClSlots = 16;                             // TinyMT words a warp
+// Bound: the dependent instructions of a step.  Rhombus 512 with one launch per step and a byte per vertex:
+// 5.3 us a step on the device, 7.8 in the call; with the rows in one cluster and a cluster barrier per
+// step, 2.6 us (TinyMT beyond its registers: 5.1).  Now 1.67 us, TinyMT 1.90; rhombus 300 1.45 (before 2.26) and
+// 1.39 (1.94), 66 x 186 1.39 (1.88) and 1.14 (1.19), 20 x 20 0.92 (1.09) and 0.54 (0.61).
+constexpr int kTdThreads = 512;  // up to 128 registers a thread
+constexpr int kTdSlots = 16;     // TinyMT words a warp
 
 struct TdClArgs {
   uint8_t* D;  // M x M dimer bytes
-  int M, ctas, f;              // f: the first row of sites
-  int row_start[kTdClCtas + 1];
+  int M, bands;
   int w0, words;               // words that hold sites
+  int row_lo, row_hi, depth;   // site rows; steps between exchanges
   uint4* tmt;                  // generators between launches
   const uint4* tmt_params;
   uint32_t seed;
   bool first, last;
   const uint8_t* sched;        // packed TdStep per step
-  int steps, list_cap;
+  int steps, per_warp;         // per_warp: words of a pass that a warp lists (fast mode)
   uint64_t fast_seed;
   uint32_t stream;
   int64_t h0;
+  uint64_t* xbuf;  // [period parity][row from row_lo - 2][word][plane H, L, R], tags cleared
+  int* error;
+  long max_spin;
 };
+
+// First site row of band b.
+__host__ __device__ __forceinline__ int td_band_row(int b, int bands, int lo, int hi) {
+  return lo + (int)((int64_t)(hi - lo + 1) * b / bands);
+}
+constexpr int kTdMove = 4;  // words of an exchange a thread sends, and takes
 
 inline uint8_t td_pack_step(const TdStep& s) {
   return (uint8_t)(s.type | s.r1 << 2 | s.r2 << 4 | s.p1 << 5 | s.p2 << 7);
@@ -243,23 +251,18 @@ __device__ __forceinline__ uint32_t td_class_mask(const TdStep& s, int a, int a3
   return every3(s.p1 + w3 + (a3 ? 3 - a3 : 0)) & parity(s.p2);
 }
 
-__device__ __forceinline__ uint32_t td_remote(const void* p, int rank) {
-  uint32_t r;
-  const uint32_t x = (uint32_t)__cvta_generic_to_shared(p);
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(rank));
-  return r;
-}
-
 // K: TinyMT words a warp (0: fast mode).
 template <int K, bool kParams>
-__global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cluster(const __grid_constant__ TdClArgs a) {
+__global__ void __launch_bounds__(kTdThreads, 1) k_td_bands(const __grid_constant__ TdClArgs a) {
   extern __shared__ __align__(16) uint32_t tsm[];
-  __shared__ int s_count[2];
   __shared__ uint32_t s_mask[2][18];
   constexpr bool kFast = K == 0;
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
-  const int rank = (int)cooperative_groups::this_cluster().block_rank();
-  const int r0 = a.row_start[rank], r1 = a.row_start[rank + 1], rows = r1 - r0, words = a.words, Wp = words + 2;
+  const int rank = (int)blockIdx.x;
+  const int own0 = td_band_row(rank, a.bands, a.row_lo, a.row_hi), own1 = td_band_row(rank + 1, a.bands, a.row_lo, a.row_hi);
+  const int reach = a.bands > 1 ? 3 * a.depth : 3;
+  const int r0 = max(own0 - reach + 2, a.row_lo), r1 = min(own1 + reach - 1, a.row_hi + 1);  // site rows held
+  const int rows = r1 - r0, words = a.words, Wp = words + 2;
   // Window row y is vertex row r0 - 2 + y; word x is column word w0 - 1 + x; planes H, L, R, -.
   uint32_t* const planes = tsm;
   uint32_t* const list = tsm + (size_t)(rows + 3) * Wp * 4;
@@ -270,25 +273,12 @@ __global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cl
     const uint32_t h = __ballot_sync(~0u, v & kH), l = __ballot_sync(~0u, v & kL), r = __ballot_sync(~0u, v & kR);
     if (lane < 4) word(y, x, lane) = lane == 0 ? h : lane == 1 ? l : lane == 2 ? r : 0u;
   }
-  if (tid < 2) s_count[tid] = 0;
   const uint32_t self = (uint32_t)__cvta_generic_to_shared(planes);
-  const uint32_t up = rank > 0 ? td_remote(planes, rank - 1) : 0u;
-  const uint32_t dn = rank + 1 < a.ctas ? td_remote(planes, rank + 1) : 0u;
-  const int rows_up = rank > 0 ? r0 - a.row_start[rank - 1] : 0;
-  // XOR (predicated, not branched) into this CTA's copy; where the row is held twice (kSeam), into
-  // the neighbour's too: window rows 0 .. 2 are r0 - 2 and r0 - 1, owned above, and r0, held above;
-  // rows `rows` .. rows + 2 are r1 - 2 and r1 - 1, held below, and r1, owned below.
-  auto toggle_word = [&](auto seam, int y, int x, int p, uint32_t m) {
-    const uint32_t at = (uint32_t)((y * Wp + x) * 4 + p) * 4u;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q red.shared.xor.b32 [%0], %1;\n\t}" ::"r"(self + at),
+  auto toggle_word = [&](int y, int x, int p, uint32_t m) {  // (predicated, not branched)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q red.shared.xor.b32 [%0], %1;\n\t}" ::"r"(
+                     self + (uint32_t)((y * Wp + x) * 4 + p) * 4u),
                  "r"(m)
                  : "memory");
-    if constexpr (decltype(seam)::v) {
-      if (m && rank > 0 && y <= 2)
-        asm volatile("red.shared::cluster.xor.b32 [%0], %1;" ::"r"(up + at + (uint32_t)(rows_up * Wp * 16)), "r"(m) : "memory");
-      if (m && rank + 1 < a.ctas && y >= rows)
-        asm volatile("red.shared::cluster.xor.b32 [%0], %1;" ::"r"(dn + at - (uint32_t)(rows * Wp * 16)), "r"(m) : "memory");
-    }
   };
   // Sites of the word at `at` whose cycle has a half covered.
   const int pitch = Wp * 4;
@@ -304,25 +294,21 @@ __global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cl
     });
     return half[0] | half[1];
   };
-  auto toggle_in = [&](auto seam, auto c, int y, int x, uint32_t m) {
-    td_edges<decltype(c)::v>([&](auto, auto da, auto db, auto p) {
-      constexpr int d = decltype(db)::v, pl = decltype(p)::v;
-      const int yy = y + decltype(da)::v;
-      if constexpr (d == 0) {
-        toggle_word(seam, yy, x, pl, m);
-      } else if constexpr (d == 1) {
-        toggle_word(seam, yy, x, pl, m << 1);
-        toggle_word(seam, yy, x + 1, pl, m >> 31);
-      } else {
-        toggle_word(seam, yy, x, pl, m >> 1);
-        toggle_word(seam, yy, x - 1, pl, m << 31);
-      }
-    });
-  };
   // Flips the sites m of row r0 + i, word x (a cycle spans window rows i .. i + 3).
   auto toggle = [&](auto c, int i, int x, uint32_t m) {
-    if (i > 2 && i < rows - 3) toggle_in(TdI<0>{}, c, i + 2, x, m);
-    else toggle_in(TdI<1>{}, c, i + 2, x, m);
+    td_edges<decltype(c)::v>([&](auto, auto da, auto db, auto p) {
+      constexpr int d = decltype(db)::v, pl = decltype(p)::v;
+      const int yy = i + 2 + decltype(da)::v;
+      if constexpr (d == 0) {
+        toggle_word(yy, x, pl, m);
+      } else if constexpr (d == 1) {
+        toggle_word(yy, x, pl, m << 1);
+        toggle_word(yy, x + 1, pl, m >> 31);
+      } else {
+        toggle_word(yy, x, pl, m >> 1);
+        toggle_word(yy, x - 1, pl, m << 31);
+      }
+    });
   };
   auto by_cycle = [](int c, auto f) {  // c is the same for the whole grid
     switch (c) {
@@ -399,21 +385,98 @@ __global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cl
       acc = mine;
     }
   };
-  const Item first = item_at(min(kFast ? tid : warp + lane * nwarps, items - 1));  // this thread's item in every step
+  // This thread's item (fast mode: of a step that starts with the first row).
+  const int pw = a.per_warp;
+  const Item first = item_at(min(kFast ? warp * pw + lane : warp + lane * nwarps, items - 1));
+  // The rows of sites, and their items, of a step with `left` steps to go to the exchange, this one included.
+  auto row_from = [&](int left) { return max(own0 - 3 * left + 2, r0) - r0; };
+  auto row_to = [&](int left) { return min(own1 + 3 * left - 1, r1) - r0; };
+  bool dead = false;  // a wait gave up: no more waits, the launch runs to its end
+  int send_at[kTdMove], send_to[kTdMove], take_at[kTdMove], take_to[kTdMove];
+  const int row_elements = Wp * 3;
+  {
+    // a vertex row belongs to the band with its site row; the two rows above the first to the first, the row
+    // below the last to the last
+    const int v0 = rank == 0 ? own0 - 2 : own0, v1 = rank + 1 == a.bands ? own1 + 1 : own1;
+    const int mine = min(v1 - v0, 2 * reach);
+#pragma unroll
+    for (int m = 0; m < kTdMove; ++m) {
+      send_at[m] = take_at[m] = -1;
+      send_to[m] = take_to[m] = 0;
+      const int e = tid + m * T, y = e / row_elements, q = e - y * row_elements, x = q / 3, p = q - 3 * x;
+      if (y < mine) {
+        const int row = v1 - v0 <= 2 * reach || y < reach ? v0 + y : v1 - 2 * reach + y;
+        send_at[m] = ((row - r0 + 2) * Wp + x) * 4 + p;
+        send_to[m] = (row - a.row_lo + 2) * row_elements + q;
+      }
+      if (y < 2 * reach) {
+        const int row = y < reach ? v0 - reach + y : v1 + y - reach;
+        if (row >= r0 - 2 && row <= r1 && row >= a.row_lo - 2 && row <= a.row_hi + 1) {
+          take_at[m] = ((row - r0 + 2) * Wp + x) * 4 + p;
+          take_to[m] = (row - a.row_lo + 2) * row_elements + q;
+        }
+      }
+    }
+  }
+  auto exchange = [&](uint32_t period) {
+    uint64_t* const buf = a.xbuf + (period & 1u) * (uint32_t)((a.row_hi - a.row_lo + 4) * row_elements);
+    uint64_t v[kTdMove];
+#pragma unroll
+    for (int m = 0; m < kTdMove; ++m)
+      if (send_at[m] >= 0)
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(buf + send_to[m]),
+                     "l"(((uint64_t)(period + 1u) << 32) | planes[send_at[m]])
+                     : "memory");
+#pragma unroll
+    for (int m = 0; m < kTdMove; ++m)
+      if (take_at[m] >= 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[m]) : "l"(buf + take_to[m]) : "memory");
+#pragma unroll
+    for (int m = 0; m < kTdMove; ++m) {
+      if (take_at[m] < 0) continue;
+      for (long it = 0; !dead && (uint32_t)(v[m] >> 32) != period + 1u; ++it) {
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[m]) : "l"(buf + take_to[m]) : "memory");
+        if (it >= a.max_spin) {
+          dead = true;
+          atomicExch(a.error, 1);
+        } else if ((it & 1023) == 1023 && *static_cast<volatile int*>(a.error)) {
+          dead = true;
+        }
+      }
+      if (!dead) planes[take_at[m]] = (uint32_t)v[m];
+    }
+    __syncthreads();
+  };
   if (a.steps > 0) draw();
   uint32_t step = a.steps > 0 ? __ldg(&a.sched[0]) : 0u, next = a.steps > 1 ? __ldg(&a.sched[1]) : 0u;
   if (warp == nwarps - 1) make_masks(step, 0);
-  cooperative_groups::this_cluster().sync();  // the windows are loaded
+  __syncthreads();  // the window is loaded
+  int left = min(a.depth, a.steps);
+  uint32_t period = 0;
   for (int s = 0; s < a.steps; ++s) {
+    if (left == 0) {
+      exchange(period++);
+      left = min(a.depth, a.steps - s);
+    }
+    const int i_lo = row_from(left), i_hi = row_to(left), it_lo = i_lo * words, it_hi = i_hi * words;
+    --left;
     const int c = td_cycle_of(td_unpack_step(step));
     step = next;
     next = s + 2 < a.steps ? __ldg(&a.sched[s + 2]) : 0u;
     if constexpr (kFast) {
-      // the quads with a site that can flip: (row << 20) | (quad << 4) | sites
-      int* const count = &s_count[s & 1];
-      for (int it0 = warp * 32; it0 < items; it0 += T) {
-        const Item e = it0 < T ? first : item_at(min(it0 + lane, items - 1));
-        const uint32_t m = it0 + lane < items ? sites(c, s & 1, e) : 0u;
+      if (warp == nwarps - 1) make_masks(step, (s + 1) & 1);
+      // A warp's quads with a site that can flip: (row << 20) | (quad << 4) | sites.  (Sites of a class share no edge:
+      // the toggles need not wait for the other warps' lists.)
+      uint32_t* const mine = list + warp * 8 * pw;
+      for (int it0 = it_lo + warp * pw; it0 < it_hi; it0 += nwarps * pw) {
+        Item e = first;
+        if (it0 >= it_lo + nwarps * pw) {
+          e = item_at(min(it0 + lane, items - 1));
+        } else if (i_lo) {  // the first item of the whole range, i_lo rows further on
+          e.i += i_lo;
+          e.mask = ((r0 + e.i) % 6) * 3 + (a.w0 - 1 + e.x) % 3;
+          e.at += i_lo * pitch;
+        }
+        const uint32_t m = lane < pw && it0 + lane < it_hi ? sites(c, s & 1, e) : 0u;
         uint32_t quads = (m | (m >> 1) | (m >> 2) | (m >> 3)) & 0x11111111u;
         int at = __popc(quads);
 #pragma unroll
@@ -421,49 +484,40 @@ __global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cl
           const int before = __shfl_up_sync(~0u, at, o);
           if (lane >= o) at += before;
         }
-        int base = 0;
-        if (lane == 31 && at) base = atomicAdd(count, at);
-        base = __shfl_sync(~0u, base, 31);
-        uint32_t* to = list + base + at - __popc(quads);
+        const int n = __shfl_sync(~0u, at, 31);
+        uint32_t* to = mine + at - __popc(quads);
         const uint32_t tag = (uint32_t)e.i << 20 | (uint32_t)e.x << 7;
         for (; quads; quads &= quads - 1) {
           const int k = __ffs((int)quads) - 1;
           *to++ = tag | (uint32_t)k << 2 | ((m >> k) & 15u);
         }
-      }
-      __syncthreads();
-      const int n = *count;
-      if (tid == 0) s_count[(s + 1) & 1] = 0;
-      if (warp == nwarps - 1) make_masks(step, (s + 1) & 1);
-      for (int e = tid; e < n; e += T) {
-        const uint32_t v = list[e];
-        const int i = (int)(v >> 20), qx = (int)((v >> 4) & 0xffffu), x = qx >> 3, k = qx & 7;
-        const uint4 d = fast_quad(a.fast_seed, a.stream, a.h0 + s, (uint32_t)(r0 + i), (uint32_t)(8 * (a.w0 - 1) + qx));
-        const uint32_t ok = (~d.x >> 31) | ((~d.y >> 31) << 1) | ((~d.z >> 31) << 2) | ((~d.w >> 31) << 3);
-        const uint32_t m = (v & ok & 15u) << (4 * k);
-        if (m) by_cycle(c, [&](auto cc) { toggle(cc, i, x, m); });
+        __syncwarp();
+        for (int q = lane; q < n; q += 32) {
+          const uint32_t v = mine[q];
+          const int i = (int)(v >> 20), qx = (int)((v >> 4) & 0xffffu), x = qx >> 3, k = qx & 7;
+          const uint4 d = fast_quad(a.fast_seed, a.stream, a.h0 + s, (uint32_t)(r0 + i), (uint32_t)(8 * (a.w0 - 1) + qx));
+          const uint32_t ok = (~d.x >> 31) | ((~d.y >> 31) << 1) | ((~d.z >> 31) << 2) | ((~d.w >> 31) << 3);
+          const uint32_t f = (v & ok & 15u) << (4 * k);
+          if (f) by_cycle(c, [&](auto cc) { toggle(cc, i, x, f); });
+        }
+        __syncwarp();
       }
     } else {
       if (warp == nwarps - 1) make_masks(step, (s + 1) & 1);
       const int it = warp + lane * nwarps;
-      if (lane < K && it < items) {
+      if (lane < K && it >= it_lo && it < it_hi) {
         const uint32_t m = sites(c, s & 1, first) & acc;
         if (m) by_cycle(c, [&](auto cc) { toggle(cc, first.i, first.x, m); });
       }
       __syncwarp();
     }
-    const bool more = s + 1 < a.steps;
-    if (a.ctas == 1) {
-      if (more) draw();
-      __syncthreads();
-    } else {
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      if (more) draw();
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
+    if (s + 1 < a.steps) draw();
+    __syncthreads();
   }
-  for (int it = warp; it < rows * words; it += nwarps) {
-    const int i = it / words, x = 1 + it - i * words, col = 32 * (a.w0 - 1 + x) + lane;
+  // No band writes back before the bands around it have loaded.
+  if (a.bands > 1 && a.steps > 0) exchange(period);
+  for (int it = warp; it < (own1 - own0) * words; it += nwarps) {
+    const int i = own0 - r0 + it / words, x = 1 + it % words, col = 32 * (a.w0 - 1 + x) + lane;
     if (col >= a.M) continue;
     uint32_t v = 0;
 #pragma unroll
@@ -476,7 +530,8 @@ __global__ void __launch_bounds__(K ? kTdTmtThreads : kTdFastThreads, 1) k_td_cl
     for (int k = 0; k < K; ++k) {
       bool v;
       const int64_t g = gen_index(k, &v);
-      if (v) a.tmt[g] = gen[k];
+      const int row = r0 + (warp + k * nwarps) / words;
+      if (v && row >= own0 && row < own1) a.tmt[g] = gen[k];
     }
   }
 }
@@ -553,53 +608,62 @@ __global__ void k_td_unpack(const uint8_t* D, int N, int32_t* t) {
 
 struct TdClPlan {
   bool ok = false;
-  int ctas = 0, threads = 0, K = 0, w0 = 0, words = 0, list_cap = 0;
-  int row_start[kTdClCtas + 1] = {};
-  size_t smem = 0;
+  int bands = 0, threads = 0, K = 0, w0 = 0, words = 0, depth = 0, per_warp = 1;
+  size_t smem = 0, xbuf_words = 0;
   void* kernel = nullptr;
 };
 
-void* td_cluster_kernel(bool fast, bool params, int K) {
-  if (fast) return (void*)k_td_cluster<0, false>;
+void* td_kernel(bool fast, bool params, int K) {
+  if (fast) return (void*)k_td_bands<0, false>;
   switch (K) {
-    case 1: return params ? (void*)k_td_cluster<1, true> : (void*)k_td_cluster<1, false>;
-    case 2: return params ? (void*)k_td_cluster<2, true> : (void*)k_td_cluster<2, false>;
-    case 4: return params ? (void*)k_td_cluster<4, true> : (void*)k_td_cluster<4, false>;
-    case 8: return params ? (void*)k_td_cluster<8, true> : (void*)k_td_cluster<8, false>;
-    default: return params ? (void*)k_td_cluster<16, true> : (void*)k_td_cluster<16, false>;
+    case 1: return params ? (void*)k_td_bands<1, true> : (void*)k_td_bands<1, false>;
+    case 2: return params ? (void*)k_td_bands<2, true> : (void*)k_td_bands<2, false>;
+    case 4: return params ? (void*)k_td_bands<4, true> : (void*)k_td_bands<4, false>;
+    case 8: return params ? (void*)k_td_bands<8, true> : (void*)k_td_bands<8, false>;
+    default: return params ? (void*)k_td_bands<16, true> : (void*)k_td_bands<16, false>;
   }
 }
 
-// Words of sites up to which one CTA is faster than a cluster and its barrier.
-constexpr int kTdOneCta = 64;
-
-TdClPlan td_cluster_plan(const TdScan& sc, bool fast, bool params) {
+// Bands of equally many rows with an exchange every `depth` steps.
+TdClPlan td_plan_of(const TdScan& sc, bool fast, bool params, int bands, int depth) {
   TdClPlan p;
-  if (sc.row_hi < sc.row_lo || sc.flags) return p;
   const int rows = sc.row_hi - sc.row_lo + 1;
   p.w0 = sc.col_lo / 32;
   p.words = sc.col_hi / 32 - p.w0 + 1;
-  p.ctas = (int64_t)rows * p.words <= kTdOneCta ? 1 : std::max(1, std::min(kTdClCtas, rows / 3));
-  int rows_max = 0;
-  for (int k = 0; k <= p.ctas; ++k) p.row_start[k] = sc.row_lo + (int)((int64_t)rows * k / p.ctas);
-  for (int k = 0; k < p.ctas; ++k) rows_max = std::max(rows_max, p.row_start[k + 1] - p.row_start[k]);
-  const int64_t items = (int64_t)rows_max * p.words;
-  p.smem = (size_t)(rows_max + 3) * (p.words + 2) * 16;
-  if (fast) {
-    p.list_cap = (int)std::min<int64_t>(items * 8, 1 << 20);
-    p.smem += (size_t)p.list_cap * sizeof(uint32_t);
-    p.threads = items > 128 ? kTdFastThreads : 256;
-    if (rows_max > 4095 || p.words + 2 > 8191) return p;
-  } else {
-    const int64_t K = (items + kTdTmtThreads / 32 - 1) / (kTdTmtThreads / 32);
-    if (K > kTdClSlots) return p;
-    p.K = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
-    p.threads = K <= 1 ? (int)items * 32 : kTdTmtThreads;
+  p.bands = std::min(bands, rows);
+  p.depth = depth;
+  int held = 0, own = 0;
+  for (int k = 0; k < p.bands; ++k) {
+    const int o0 = td_band_row(k, p.bands, sc.row_lo, sc.row_hi), o1 = td_band_row(k + 1, p.bands, sc.row_lo, sc.row_hi);
+    held = std::max(held, std::min(o1 + 3 * depth - 1, sc.row_hi + 1) - std::max(o0 - 3 * depth + 2, sc.row_lo));
+    own = std::max(own, o1 - o0 + 2);
   }
-  p.kernel = td_cluster_kernel(fast, params, p.K);
-  if (p.smem > 200 * 1024) return p;
-  if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
-      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+  const int64_t items = (int64_t)held * p.words;
+  p.smem = (size_t)(held + 3) * (p.words + 2) * 16;
+  int64_t threads = std::min<int64_t>(kTdThreads, (items + 31) / 32 * 32);
+  if (p.bands > 1) {
+    const int64_t moves = (int64_t)6 * depth * (p.words + 2) * 3;
+    if (moves > (int64_t)kTdMove * kTdThreads) return p;
+    threads = std::max(threads, (moves + kTdMove * 32 - 1) / (kTdMove * 32) * 32);
+  }
+  if (fast) {
+    threads = std::min<int64_t>(kTdThreads, std::max<int64_t>(threads, std::min<int64_t>(items, 16) * 32));
+    p.threads = (int)threads;
+    p.per_warp = (int)std::min<int64_t>(32, (items + p.threads / 32 - 1) / (p.threads / 32));
+    p.smem += (size_t)(p.threads / 32) * 8 * p.per_warp * sizeof(uint32_t);
+    if (held > 4095 || p.words + 2 > 8191) return p;
+  } else {
+    const int64_t K = (items + kTdThreads / 32 - 1) / (kTdThreads / 32);
+    if (K > kTdSlots) return p;
+    p.K = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+    p.threads = K <= 1 ? (int)std::max(threads, items * 32) : kTdThreads;
+  }
+  p.xbuf_words = (size_t)2 * (rows + 3) * (p.words + 2) * 3;
+  p.kernel = td_kernel(fast, params, p.K);
+  int per_sm = 0;
+  if (p.smem > 200 * 1024 ||
+      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.threads, p.smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return p;
   }
@@ -607,26 +671,44 @@ TdClPlan td_cluster_plan(const TdScan& sc, bool fast, bool params) {
   return p;
 }
 
+TdClPlan td_plan(const TdScan& sc, bool fast, bool params) {
+  int dev = 0, sms = 0, coop = 0;
+  if (sc.row_hi < sc.row_lo || sc.flags || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return TdClPlan{};
+  }
+  // One CTA where that is faster than any exchange (us per step, rhombus 20 x 20: fast mode 0.92, bands 0.96 at
+  // best; TinyMT 0.54 and 0.61; 60 x 60: 1.27 and 1.26, 1.15 and 0.87).  Else a band per SM, and the deeper the fewer
+  // words a band then holds, whose draws with TinyMT are all made:
+  //   fast    66 x 186: depth 2 1.54, 3 1.42, 4 1.39    300 x 300: 1.58, 1.50, 1.45    512 x 512: 1.77, 1.70, 1.67
+  //   TinyMT  60 x 60 (40 words): 2 0.95, 3 0.87    66 x 186 (66): 1 1.45, 2 1.14, 3 1.24    300 x 300 (120): 1.56,
+  //           1.39, 1.91    512 x 512 (238 at depth 2): 1.90, 2.21
+  const int rows = sc.row_hi - sc.row_lo + 1, words = sc.col_hi / 32 - sc.col_lo / 32 + 1;
+  TdClPlan p;
+  if (!coop || rows * words <= (fast ? 128 : 32)) {
+    p = td_plan_of(sc, fast, params, 1, 1);
+    if (p.ok || !coop) return p;
+  }
+  const auto held = [&](int d) { return ((rows + sms - 1) / sms + 6 * d - 3) * words; };
+  int depth = fast ? 4 : (held(3) <= 51 ? 3 : (held(2) <= 128 ? 2 : 1));
+  for (; depth > 0 && !p.ok; --depth) p = td_plan_of(sc, fast, params, sms, depth);
+  return p;
+}
+
 struct TdClLaunch {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   TdClLaunch(const TdClPlan& p, cudaStream_t st) {
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)p.ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)p.ctas);
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3((unsigned)p.bands);
     cfg.blockDim = dim3((unsigned)p.threads);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-  }
-  bool fits(const TdClPlan& p) {
-    int clusters = 0;
-    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, p.kernel, &cfg) == cudaSuccess && clusters > 0;
-    if (!ok) cudaGetLastError();
-    return ok;
+    cfg.numAttrs = p.bands > 1 ? 1 : 0;
   }
 };
 
@@ -955,10 +1037,13 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   TdScan* d_scan = nullptr;
   uint8_t* d_sched = nullptr;
   uint4 *tmt = nullptr, *tmt_params = nullptr;
+  uint64_t* xbuf = nullptr;
+  int* d_error = nullptr;
   void* mtgp = nullptr;
   const MtgpGrid mg = mtgp_grid(M, M);
   auto cleanup = [&]() {
-    for (void* q : {(void*)d_t, (void*)dD, (void*)d_scan, (void*)d_sched, (void*)tmt, mtgp}) dev_free(q, st);
+    for (void* q : {(void*)d_t, (void*)dD, (void*)d_scan, (void*)d_sched, (void*)tmt, (void*)xbuf, (void*)d_error, mtgp})
+      dev_free(q, st);
     if (tmt_params) cudaFree(tmt_params);
   };
   auto out_of_memory = [&]() {
@@ -987,13 +1072,16 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
                                                            : "bibone walk: two dimers share a vertex");
   }
   TdClPlan plan;
-  if (o.rng_mode != RT_RNG_MTGP && steps > 0) plan = td_cluster_plan(scan, fast, o.tinymt_params != nullptr);
+  if (o.rng_mode != RT_RNG_MTGP && steps > 0) {
+    plan = td_plan(scan, fast, o.tinymt_params != nullptr);
+  }
   TdClLaunch launch(plan, st);
-  const bool in_cluster = plan.ok && launch.fits(plan);
-  constexpr int64_t chunk_max = (int64_t)1 << 20;  // steps of a cluster launch
-  if ((o.rng_mode == RT_RNG_TINYMT && (!in_cluster || steps > chunk_max) &&
+  const bool resident = plan.ok, exchanges = plan.ok && plan.bands > 1;
+  constexpr int64_t chunk_max = (int64_t)1 << 18;  // steps of a launch
+  if ((o.rng_mode == RT_RNG_TINYMT && (!resident || steps > chunk_max) &&
        dev_alloc(&tmt, (size_t)M * M * sizeof(uint4), st)) ||
-      (in_cluster && dev_alloc(&d_sched, (size_t)steps, st)) ||
+      (resident && dev_alloc(&d_sched, (size_t)steps, st)) ||
+      (exchanges && (dev_alloc(&xbuf, plan.xbuf_words * sizeof(uint64_t), st) || dev_alloc(&d_error, sizeof(int), st))) ||
       (o.rng_mode == RT_RNG_MTGP && dev_alloc(&mtgp, mtgp_state_bytes(mg.count()), st)))
     return out_of_memory();
   if (o.rng_mode == RT_RNG_TINYMT) {
@@ -1021,7 +1109,7 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  if (o.rng_mode == RT_RNG_TINYMT && !in_cluster) {
+  if (o.rng_mode == RT_RNG_TINYMT && !resident) {
     const int64_t count = (int64_t)M * M;
     k_td_seed<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(tmt, tmt_params, count, (uint32_t)seed);
   } else if (o.rng_mode == RT_RNG_MTGP) {
@@ -1034,19 +1122,18 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
     }
   }
   std::vector<uint8_t> packed;
-  if (in_cluster) {
+  if (resident) {
     packed.resize((size_t)steps);
     for (int64_t h = 0; h < steps; ++h) packed[(size_t)h] = td_pack_step(sched[(size_t)h]);
     cudaMemcpyAsync(d_sched, packed.data(), packed.size(), cudaMemcpyHostToDevice, st);
   }
   cudaError_t le = cudaSuccess;
   cudaEventRecord(e0, st);
-  for (int64_t s0 = 0; in_cluster && s0 < steps && le == cudaSuccess; s0 += chunk_max) {
+  for (int64_t s0 = 0; resident && s0 < steps && le == cudaSuccess; s0 += chunk_max) {
     TdClArgs a{};
     a.D = dD;
     a.M = M;
-    a.ctas = plan.ctas;
-    std::copy(plan.row_start, plan.row_start + kTdClCtas + 1, a.row_start);
+    a.bands = plan.bands;
     a.w0 = plan.w0;
     a.words = plan.words;
     a.tmt = tmt;
@@ -1056,14 +1143,24 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
     a.steps = (int)std::min(chunk_max, steps - s0);
     a.last = s0 + a.steps >= steps;
     a.sched = d_sched + s0;
-    a.list_cap = plan.list_cap;
+    a.per_warp = plan.per_warp;
     a.fast_seed = (uint64_t)seed;
     a.stream = o.fast_stream;
     a.h0 = s0;
+    a.depth = exchanges ? plan.depth : a.steps;
+    a.row_lo = scan.row_lo;
+    a.row_hi = scan.row_hi;
+    a.xbuf = xbuf;
+    a.error = d_error;
+    a.max_spin = 1L << 22;
+    if (exchanges) {
+      if (s0 == 0) cudaMemsetAsync(d_error, 0, sizeof(int), st);
+      cudaMemsetAsync(xbuf, 0, plan.xbuf_words * sizeof(uint64_t), st);  // no stale tags
+    }
     void* args[] = {&a};
     le = cudaLaunchKernelExC(&launch.cfg, plan.kernel, args);
   }
-  for (int64_t h = 0; !in_cluster && h < steps; ++h) {
+  for (int64_t h = 0; !resident && h < steps; ++h) {
     if (o.rng_mode == RT_RNG_TINYMT)
       pdl_launch(k_td_step_tmt, g_all, dim3(128), st, dD, tmt, (const uint4*)tmt_params, M, sched[(size_t)h]);
     else if (o.rng_mode == RT_RNG_MTGP)
@@ -1075,6 +1172,17 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   cudaEventRecord(e1, st);
   k_td_unpack<<<g_all, 128, 0, st>>>(dD, N, d_t);
   if (le == cudaSuccess) le = cudaGetLastError();
+  int gave_up = 0;
+  if (exchanges && le == cudaSuccess) {  // before the caller's tiling changes
+    cudaMemcpyAsync(&gave_up, d_error, sizeof gave_up, cudaMemcpyDeviceToHost, st);
+    le = cudaStreamSynchronize(st);
+    if (gave_up && le == cudaSuccess) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      cleanup();
+      return fail(RT_ERR_TIMEOUT, "bibone walk: a band gave up waiting for a neighbour's rows");
+    }
+  }
   if (le == cudaSuccess) cudaMemcpyAsync(tiling, d_t, cells * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
   const cudaError_t se = cudaStreamSynchronize(st);
   float ms = 0.f;

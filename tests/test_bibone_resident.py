@@ -1,6 +1,6 @@
-"""Bibone walks on the cluster kernel (dimers as bit planes): identical (whole numbers) to the oracle
-on regions from one word to many, with edges at a word's edge, from one CTA to sixteen, in every
-random mode; the statistics; and input that is refused."""
+"""Bibone walks on the resident kernel (dimers as bit planes): identical (whole numbers) to the oracle on regions
+from one word to many, with edges at a word's edge, in one CTA and in bands that exchange rows every few steps
+(steps not a multiple of the depth), in every random mode; the statistics; and input that is refused."""
 import numpy as np
 import pytest
 
@@ -40,7 +40,7 @@ def test_cone_walks_equal_the_oracle(rt, orc, n, m, mode):
 
 @pytest.mark.parametrize("mode", ["tinymt", "fast"])
 def test_largest_sizes_equal_the_oracle(rt, orc, mode):
-    # TinyMT: beyond the generators that the cluster's registers hold; fast mode: many words a row
+    # TinyMT: an exchange every step; fast mode: many words a row
     a, b, _ = _walk(rt, orc, rt.TriangleDimerTiler.RhombusBrick(420, 700), 60, 3, mode)
     assert np.array_equal(a, b)
 
