@@ -180,6 +180,12 @@ __global__ void k_scan_tiling(const int32_t* t, int N, int* cand, unsigned long 
   }
 }
 
+// No candidates yet, no flags.
+__global__ void k_scan_init(int* cand, int N) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < 2 * N) cand[k] = k < N ? INT_MAX : -1;
+}
+
 // Host-layout int32 tiling (N x N) <-> colour arrays of one chain.
 __global__ void k_split(DmView v, int ch, const int32_t* tiling) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,8 +249,7 @@ DmSampler::~DmSampler() {
   bits.reset();  // the engines free their plan buffers on the stream before the stream goes
   runs.reset();
   persist.reset();
-  for (void* p : {(void*)tmt, (void*)tmt_params, mtgp, (void*)base, (void*)scratch, (void*)counter, (void*)d_scan,
-                  (void*)d_cand})
+  for (void* p : {(void*)tmt, (void*)tmt_params, mtgp, (void*)base, (void*)scratch, (void*)counter, (void*)d_scan})
     dev_free(p, stream);
   for (void* p : {(void*)d_dom, (void*)d_hf, (void*)d_h, (void*)d_hflags})
     if (p) cudaFree(p);
@@ -299,21 +304,15 @@ rt_status DmSampler::create(int n_side, int n_chains, const rt_walk_opts& o, std
     RT_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     s->own_stream = true;
   }
-  RT_CUDA(cudaEventCreate(&s->ev0));
-  RT_CUDA(cudaEventCreate(&s->ev1));
   // Pool allocations, ordered on the sampler's stream (device_pool.cpp).
   if (rt_status st = dev_alloc(&s->base, s->chain_stride * n_chains, s->stream)) return st;
   RT_CUDA(cudaMemsetAsync(s->base, 0, s->chain_stride * n_chains, s->stream));
   if (rt_status st = dev_alloc(&s->scratch, (size_t)s->N * s->N * sizeof(int32_t), s->stream)) return st;
   if (rt_status st = dev_alloc(&s->counter, sizeof(unsigned long long), s->stream)) return st;
-  if (rt_status st = dev_alloc(&s->d_scan, 3 * sizeof(unsigned long long), s->stream)) return st;
-  if (rt_status st = dev_alloc(&s->d_cand, 2 * (size_t)s->N * sizeof(int), s->stream)) return st;
-  {
-    std::vector<int> init(2 * (size_t)s->N, -1);
-    std::fill(init.begin(), init.begin() + s->N, INT_MAX);
-    RT_CUDA(cudaMemcpyAsync(s->d_cand, init.data(), init.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
-    RT_CUDA(cudaStreamSynchronize(s->stream));
-  }
+  // flags and counts, then the candidate columns: one copy brings both to the host after a load
+  if (rt_status st = dev_alloc(&s->d_scan, kScanBytes + 2 * (size_t)s->N * sizeof(int), s->stream)) return st;
+  s->d_cand = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(s->d_scan) + kScanBytes);
+  k_scan_init<<<(2 * s->N + 255) / 256, 256, 0, s->stream>>>(s->d_cand, s->N);
   const int64_t cells = (int64_t)(s->N - 2) * (s->N / 2 - 2);
   if (o.rng_mode == RT_RNG_TINYMT) {
     if (rt_status st = dev_alloc(&s->tmt, cells * sizeof(uint4), s->stream)) return st;
@@ -353,9 +352,10 @@ rt_status DmSampler::load(int ch, const int32_t* tiling) {
   RT_CUDA(cudaMemsetAsync(d_scan, 0, 3 * sizeof(unsigned long long), stream));
   k_scan_tiling<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(scratch, N, d_cand, d_scan, ch == 0);
   launches++;
-  unsigned long long h[3] = {0, 0, 0};
-  RT_CUDA(cudaMemcpyAsync(h, d_scan, sizeof h, cudaMemcpyDeviceToHost, stream));
+  scanned.resize(kScanBytes / sizeof(unsigned long long) + (size_t)N);  // 2 N ints
+  RT_CUDA(cudaMemcpyAsync(scanned.data(), d_scan, scanned.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
   RT_CUDA(cudaStreamSynchronize(stream));
+  const unsigned long long* h = scanned.data();
   if (h[0] & 1u) return fail(RT_ERR_INVALID_ARGUMENT, "tiling values must be edge masks in [0, 15]");
   consistent = consistent && !(h[0] & 2u);
   border_candidates = border_candidates || (h[0] & 4u);
@@ -370,20 +370,18 @@ rt_status DmSampler::load(int ch, const int32_t* tiling) {
   return check_launch();
 }
 
-rt_status DmSampler::fetch_candidates() {
-  std::vector<int> both(2 * (size_t)N);
-  RT_CUDA(cudaMemcpyAsync(both.data(), d_cand, both.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
-  RT_CUDA(cudaStreamSynchronize(stream));
+void DmSampler::fetch_candidates() {
   cand_lo.assign(N, -1);
   cand_hi.assign(N, -1);
   any_candidate = false;
+  if (scanned.empty()) return;  // nothing loaded
+  const int* both = reinterpret_cast<const int*>(scanned.data() + kScanBytes / sizeof(unsigned long long));
   for (int i = 0; i < N; ++i)
     if (both[i] != INT_MAX) {
       cand_lo[i] = both[i];
       cand_hi[i] = both[N + i];
       any_candidate = true;
     }
-  return RT_OK;
 }
 
 rt_status DmSampler::store(int ch, int32_t* tiling) {
@@ -580,7 +578,7 @@ rt_status DmSampler::use_persistent(bool* yes) {
   if (ask_table && !couple) take_entry(0);
   if (engine == 1 || opts.rng_mode == RT_RNG_MTGP) return RT_OK;
   if (plan_dirty) {
-    if (rt_status st = fetch_candidates()) return st;
+    fetch_candidates();
   }
   if (!consistent || !any_candidate) {
     if (engine >= 2 && explicit_engine)
@@ -967,6 +965,8 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   s->active = 2;
   s->plan_dirty = true;
   s->couple = true;
+  RT_CUDA(cudaEventCreate(&s->ev0));
+  RT_CUDA(cudaEventCreate(&s->ev1));
   const bool fast = o.rng_mode == RT_RNG_FAST;
   // The reference's epoch schedule (AztecDiamondCftpEx.cpp:54-77), drawn ahead for every
   // attempt: epoch k is created by attempt k with the driver's k-th draw as its seed, and

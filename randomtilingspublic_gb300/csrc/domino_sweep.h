@@ -69,11 +69,12 @@ struct DmSampler {
   int64_t half_sweeps[2] = {0, 0};  // half-sweeps run per colour
   int64_t launches = 0;
   // Persistent engine state: the flip-candidate column range of each colour-array row over
-  // all loaded chains (kept on the device by the load scan, fetched when the engine is
-  // planned), whether every loaded tiling is consistent, and the engine (re)planned when
+  // all loaded chains (kept on the device by the load scan, whose last result is `scanned`), whether every loaded tiling is consistent, and the engine (re)planned when
   // either changes.
+  unsigned long long* d_scan = nullptr;  // flags, interior count of colour 0, of colour 1; then d_cand
   int* d_cand = nullptr;                 // [2][N]: lowest (INT_MAX: none) and highest column
-  unsigned long long* d_scan = nullptr;  // flags, interior count of colour 0, of colour 1
+  static constexpr size_t kScanBytes = 4 * sizeof(unsigned long long);
+  std::vector<unsigned long long> scanned;  // d_scan's block after the last load
   std::vector<int> cand_lo, cand_hi;     // host copies (-1: no candidate)
   bool any_candidate = false;
   bool consistent = true;
@@ -105,7 +106,7 @@ struct DmSampler {
   DmView view() const;
   rt_status check_launch();
   rt_status load(int ch, const int32_t* tiling);
-  rt_status fetch_candidates();
+  void fetch_candidates();
   // Device statistics: the domain the height function is taken on, then per-chain heights
   // added to running sums.
   rt_status set_domain(const int32_t* domain, int m_side);
