@@ -17,8 +17,8 @@
 // access; tagged words polled in shared memory: 0.57 us).  The draws do not depend on the state,
 // so warps of their own make them, a run ahead: they compose a run's half-sweeps into one pair of
 // move words per 32 cells, and the update warps apply those in a dozen logic operations.
-// It serves couplings from the past and launches that ask for 1..16 bands; a walk's exchange every few runs
-// (k_deep in domino_grid.cu) is faster, but takes every SM.
+// It serves launches that ask for 1..16 bands, and couplings from the past of regions that k_deep
+// (domino_grid.cu), whose exchange every few runs is faster, does not hold on a quarter of the SMs.
 // Measured (us per half-sweep, before: the best band shape): order 16 0.22 (before 0.66), order 100
 // 0.36 (0.82), order 200 0.88 (1.07) in TinyMT mode; order 16 0.35 (1.27), order 100 0.53 (1.58),
 // order 250 1.03 (1.48) in fast mode, where the draws of 16 SMs take over from the exchange.
@@ -31,8 +31,7 @@
 // Coupling from the past: attempts are independent until one coalesces, and one cluster leaves most of the
 // chip idle, so four clusters run them side by side, attempt k in cluster k mod 4; look-backs double, so
 // the time is nearly that of the attempt which coalesces.  One that has become pointless is left within
-// 1024 runs.  Measured: exact sample of order 40 in fast mode 15.9 -> 9.6 ms, of order 38 with TinyMT 20.5
-// -> 7.4 ms (there also: fewer colours drawn ahead on the host).
+// 1024 runs.  Measured: exact sample of order 40 in fast mode 15.9 -> 9.6 ms.
 //
 // TinyMT: a draw warp holds up to KS words of rows of one parity (the rule's thresholds are then
 // warp-uniform); lane l keeps the generator of cell 32 w + l of each, and two ballots turn a word's

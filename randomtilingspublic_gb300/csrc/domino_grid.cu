@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -62,16 +63,28 @@ struct GrArgs {
   long max_spin;
   int silent_band_plus1;
   int depth, first, last;  // k_deep: runs between exchanges; the first and last row of any band
+  // Coupling from the past (k_deep, couple, two chains): blockIdx.y = k runs attempt attempt0 + k from the chains
+  // at start into the k-th pair at base, and leaves once a smaller one has coalesced.
+  int couple, attempt0;
+  int64_t first_sweeps;  // fast mode: half-sweeps [-2 first_sweeps << attempt, 0)
+  const uint8_t* start;
+  size_t team_stride, xteam;
+  int* best;                    // smallest attempt that coalesced
+  int2* team;                   // [k] {bands whose chains differ, bands done}
+  const int4* attempt_desc;     // TinyMT, [k]: {first run, runs, first epoch seed, 0}
+  const uint32_t* epoch_seeds;  // a run that starts an epoch (bit 30) seeds the generators from the next
 };
 
 // Bounded wait for the element's tag; false (and the error word set) when it gave up, or another band did.
-__device__ __forceinline__ bool gr_recv(const uint64_t* g, uint32_t tag, uint32_t& v, long max_spin, int* error) {
+__device__ __forceinline__ bool gr_recv(const uint64_t* g, uint32_t tag, uint32_t& v, long max_spin, int* error,
+                                        const int* best = nullptr, int attempt = 0) {
   for (long it = 0; it <= max_spin; ++it) {
     uint64_t x;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(g) : "memory");
     v = (uint32_t)x;
     if ((uint32_t)(x >> 32) == tag) return true;
-    if ((it & 1023) == 1023 && *static_cast<volatile int*>(error)) return false;
+    if ((it & 255) == 255 && (*static_cast<volatile int*>(error) || (best && *static_cast<const volatile int*>(best) < attempt)))
+      return false;
   }
   atomicExch(error, 1);
   return false;
@@ -373,6 +386,11 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_gri
 // the spare rows' included.  Measured (us per half-sweep, before: one cluster, domino_cluster.cu): TinyMT order
 // 16 0.17 (0.22), 40 0.23 (0.30), 100 0.30 (0.37), 200 0.38 (0.50 in k_grid); fast mode order 16 0.22 (0.31),
 // 40 0.27 (0.51), 100 0.34 (0.54), 300 0.56 (1.08 in k_grid).
+//
+// Coupling from the past: four attempts side by side on a quarter of the SMs each; a band leaves an attempt once
+// a smaller one has coalesced, and the last band to finish tells whether its chains met.  Exact samples (before:
+// domino_cluster.cu, also four side by side): fast mode order 8 0.28 ms (0.57), 40 6.3 (9.6), 48 11.3 (20.0); TinyMT
+// order 15 0.74 (1.25), 32 4.0 (7.3), 48 17.9 (21.1).
 constexpr int kGrMove = 4;  // words of an exchange a lane sends, and takes
 constexpr int kGrMaxDepth = 12;
 
@@ -382,6 +400,7 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
   __shared__ uint4 srule[4];
   __shared__ int s_cnt[2];
   __shared__ uint32_t s_colour[2][kGrMaxDepth];
+  __shared__ int s_stop[2];  // a smaller attempt coalesced, by parity of the period
   constexpr bool kFast = kMode == kClFast, kParams = kMode == kClTmtParams;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)(blockDim.x >> 5);
   const int ndraw = a.draw_warps, nslots = ndraw * KS, band = blockIdx.x, depth = a.depth;
@@ -436,15 +455,32 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
       sitem[item + k] = (uint16_t)slot;
     }
   }
-  cl_load_window<NCH>(sm, a.base, a.chain_stride, a.colour_stride, a.P, i0, R, wlo, wn);
+  const bool couple = NCH == 2 && a.couple;
+  const int team = couple ? (int)blockIdx.y : 0, attempt = a.attempt0 + team;
+  cl_load_window<NCH>(sm, couple ? a.start : a.base, a.chain_stride, a.colour_stride, a.P, i0, R, wlo, wn);
   __syncthreads();
+  int nruns = a.nruns, epoch = 0;
+  const uint32_t* runs = a.runs;
+  int64_t h0 = a.h0;
+  if (couple) {
+    if (kFast) {
+      nruns = (int)(2 * (a.first_sweeps << attempt));
+      h0 = -(int64_t)nruns;
+    } else {
+      const int4 d = a.attempt_desc[team];
+      runs += d.x;
+      nruns = d.y;
+      epoch = d.z;
+    }
+  }
+  uint64_t* const xbuf = a.xbuf + team * a.xteam;
   auto run_at = [&](int j) -> uint32_t {
-    if (kFast) return ((a.h0 + j) & 1) ? 1u : 0x80000001u;  // even half-sweeps black (colour 1)
-    return j < a.nruns ? __ldg(&a.runs[j]) : 0u;
+    if (kFast) return ((h0 + j) & 1) ? 1u : 0x80000001u;  // even half-sweeps black (colour 1)
+    return j < nruns ? __ldg(&runs[j]) : 0u;
   };
   // Runs left before the next exchange at which row i is first needed.
   auto needed = [&](int i) { return i < r0 ? r0 - i + 1 : (i >= r1 ? i - r1 + 1 : 1); };
-  const int nruns = a.nruns, periods = (nruns + depth - 1) / depth;
+  const int periods = (nruns + depth - 1) / depth;
   bool dead = false;  // a wait gave up: no more waits, the launch runs to its end
   if (warp >= ndraw) {
     // ---- update warps
@@ -485,7 +521,7 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
       if (y < 2 * depth) element(y < depth ? r0 - depth + y : r1 + y - depth, q, &take_at[m], &take_to[m]);
     }
     auto exchange = [&](uint32_t period) {
-      uint64_t* const buf = a.xbuf + (period & 1u) * parity;
+      uint64_t* const buf = xbuf + (period & 1u) * parity;
       uint64_t v[kGrMove];
 #pragma unroll
       for (int m = 0; m < kGrMove; ++m)
@@ -497,7 +533,7 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
       for (int m = 0; m < kGrMove; ++m) {
         if (take_at[m] == ~0u) continue;
         uint32_t got = (uint32_t)v[m];
-        if ((uint32_t)(v[m] >> 32) != period + 1u && !dead && !gr_recv(buf + take_to[m], period + 1u, got, a.max_spin, a.error))
+        if ((uint32_t)(v[m] >> 32) != period + 1u && !dead && !gr_recv(buf + take_to[m], period + 1u, got, a.max_spin, a.error, couple ? a.best : nullptr, attempt))
           dead = true;
         if (!dead) cl_sts(take_at[m], got);
       }
@@ -530,6 +566,7 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
         asm volatile("bar.sync 1, %0;" ::"r"(nupd) : "memory");
       }
       cl_cta_sync();
+      if (couple && *static_cast<volatile int*>(&s_stop[q & 1])) return;
     }
     // The rows around its own as the other bands leave them; and no band writes back before the bands around it
     // have loaded.
@@ -564,7 +601,7 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
         bool v;
         const int64_t g = gen_index(s, &v);
         gen[s] = make_uint4(0u, 0u, 0u, 0u);
-        if (v) gen[s] = a.tmt[g];
+        if (v && !couple) gen[s] = a.tmt[g];
       }
     } else {
 #pragma unroll
@@ -583,6 +620,17 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
         for (int r = 0; r < len; ++r) {
           const uint32_t run = run_at(j0 + r);
           if (tid == 0) s_colour[q & 1][r] = run >> 31;
+          if (NCH == 2 && ((run >> 30) & 1u)) {  // InitTinyMT for an epoch (tinymt.clh:183-203, as k_tmt_seed)
+            const uint32_t seed = __ldg(&a.epoch_seeds[epoch++]);
+#pragma unroll
+            for (int s = 0; s < KS; ++s) {
+              bool v;
+              const int64_t g = gen_index(s, &v);
+              uint32_t m1, m2, tm;
+              params_of(s, m1, m2, tm);
+              if (v) gen[s] = tmt_seed(seed + (uint32_t)g, m1, m2, tm);
+            }
+          }
           cl_moves_tmt<KS>(gen, srule[par | ((int)(run >> 31) << 1)], (int)(run & 0x3fffffffu),
                            out + r * nslots + warp * KS, params_of);
         }
@@ -600,9 +648,9 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
             if (f_need[g] > len - r) continue;
             uint2* const to = out + r * nslots + warp * KS + 4 * g;
             if (f_need[g] <= len - r - 1) {
-              cl_moves_fast2(a.seed, a.stream, a.h0 + j0 + r, f_row[g], f_quad[g], rl0, rl1, to, to + nslots);
+              cl_moves_fast2(a.seed, a.stream, h0 + j0 + r, f_row[g], f_quad[g], rl0, rl1, to, to + nslots);
             } else {
-              cl_moves_fast(a.seed, a.stream, a.h0 + j0 + r, f_row[g], f_quad[g], rl0, to);
+              cl_moves_fast(a.seed, a.stream, h0 + j0 + r, f_row[g], f_quad[g], rl0, to);
             }
           }
         }
@@ -611,8 +659,10 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
     if (periods > 0) draw_period(0);
     __syncthreads();
     for (int q = 0; q < periods; ++q) {
+      if (couple && tid == 0) s_stop[q & 1] = *static_cast<volatile int*>(a.best) < attempt;
       if (q + 1 < periods) draw_period(q + 1);
       cl_cta_sync();
+      if (couple && *static_cast<volatile int*>(&s_stop[q & 1])) return;
     }
     __syncthreads();  // the bands around have loaded (the last exchange)
     if constexpr (!kFast) {
@@ -621,13 +671,28 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
         bool v;
         const int64_t g = gen_index(s, &v);
         const int i = (int)(sslot[warp * KS + s].x >> 16);
-        if (v && i >= r0 && i < r1) a.tmt[g] = gen[s];
+        if (v && !couple && i >= r0 && i < r1) a.tmt[g] = gen[s];
       }
     }
   }
   if (warp >= ndraw) __syncthreads();
-  if (__syncthreads_or(dead ? 1 : 0) && tid == 0) atomicExch(a.error, 1);
-  cl_store_window<NCH>(sm + (r0 - 1 - i0) * 4 * wn * NCH, a.base, a.chain_stride, a.colour_stride, a.P, a.cols, r0 - 1, r1 - r0 + 1,
+  const bool any_dead = __syncthreads_or(dead ? 1 : 0);
+  if (couple) {  // the last band to finish knows whether any differs (a band that left for a smaller attempt never counts)
+    uint32_t differ = 0u;
+    for (int x = tid; x < (r1 - r0) * wn; x += (int)blockDim.x) {
+      const uint4* w = reinterpret_cast<const uint4*>(sm) + ((r0 - i0) * wn + x) * 2;
+      differ |= (w[0].x ^ w[1].x) | (w[0].y ^ w[1].y) | (w[0].z ^ w[1].z) | (w[0].w ^ w[1].w);
+    }
+    const int any = __syncthreads_or(differ != 0u || any_dead ? 1 : 0);
+    if (tid == 0) {
+      if (any) atomicAdd(&a.team[team].x, 1);
+      __threadfence();
+      if (atomicAdd(&a.team[team].y, 1) == a.bands - 1 && atomicAdd(&a.team[team].x, 0) == 0) atomicMin(a.best, attempt);
+    }
+  } else if (any_dead && tid == 0) {
+    atomicExch(a.error, 1);
+  }
+  cl_store_window<NCH>(sm + (r0 - 1 - i0) * 4 * wn * NCH, a.base + team * a.team_stride, a.chain_stride, a.colour_stride, a.P, a.cols, r0 - 1, r1 - r0 + 1,
                        wlo, wn);
 }
 
@@ -851,7 +916,7 @@ bool GrPlan::build_deep(const std::vector<int>& lo, const std::vector<int>& hi, 
 }
 
 GridEngine::~GridEngine() {
-  for (void* p : {(void*)d_rows, (void*)d_xbuf, (void*)d_runs}) dev_free(p, stream);
+  for (void* p : {(void*)d_rows, (void*)d_xbuf, (void*)d_runs, (void*)d_team, (void*)d_teams, (void*)d_xteams}) dev_free(p, stream);
 }
 
 // Runs between exchanges: more of them share one exchange, but a band of rho rows draws for rho + 2 d - 1.
@@ -863,8 +928,8 @@ GridEngine::~GridEngine() {
 //           150: 4 0.45, 6 0.37, 8 0.37, 12 0.48    200: 1 1.06, 3 0.52, 4 0.45, 6 0.44, 8 0.50
 //           300: 1 1.08, 3 0.57, 4 0.56, 6 0.60    400: 2 0.72, 3 0.76    512: 2 0.95, 3 1.23
 // (rows of 1, 2, 3, 4, 5, 7, 8, 10, 13 and 17 words).  Wider rows than the last ones: d = 1.
-static int gr_depth(const GrPlan& p, bool fast) {
-  const int rho = (p.row_start[p.bands] - p.row_start[0] + p.bands - 1) / p.bands;
+static int gr_depth(const GrPlan& p, bool fast, int bands) {
+  const int rows = p.row_start[p.bands] - p.row_start[0], used = std::min(bands, rows), rho = (rows + used - 1) / used;
   const auto words = [&](int d) { return (rho + 2 * d - 1) * p.xn; };
   if (fast) {
     for (int d = 12; d > 2; --d)
@@ -908,20 +973,21 @@ rt_status GridEngine::prepare(DmSampler& s) {
     return RT_OK;
   }
   const int bands_max = s.eff_bands > 0 ? std::min(s.eff_bands, sms) : sms;
+  const int deep_bands = s.couple ? std::max(1, sms / kGrTeams) : bands_max;
   plan.depth = 1;
   plan.build(s.cand_lo, s.cand_hi, s.N, nch, fast, bands_max);
   if (!plan.ok) return RT_OK;
   const int mode = fast ? kClFast : (s.tmt_params ? kClTmtParams : kClTmt);
-  if (const int runs = gr_depth(plan, fast); runs > 1) {
+  if (const int runs = gr_depth(plan, fast, deep_bands); runs > 1) {
     GrPlan deep = plan;
-    if (deep.build_deep(s.cand_lo, s.cand_hi, s.N, nch, fast, bands_max, runs)) plan = deep;
+    if (deep.build_deep(s.cand_lo, s.cand_hi, s.N, nch, fast, deep_bands, runs)) plan = deep;
   }
   kernel = plan.depth > 1 ? (nch == 1 ? gr_deep_kernel<1>(mode, plan.slots) : gr_deep_kernel<2>(mode, plan.slots))
                           : gr_kernel(nch, mode, plan.slots, plan.per_lane);
   RT_CUDA_G(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_G(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, plan.threads(), plan.smem_bytes));
-  if ((int64_t)per_sm * sms < plan.bands) {
+  if ((int64_t)per_sm * sms < plan.bands * (s.couple && plan.depth > 1 ? kGrTeams : 1)) {
     plan.ok = false;
     plan.why = "bands cannot all be resident";
     return RT_OK;
@@ -938,36 +1004,121 @@ rt_status GridEngine::prepare(DmSampler& s) {
   return RT_OK;
 }
 
+namespace {
+
+GrArgs gr_args(const GridEngine& e, DmSampler& s) {
+  GrArgs a{};
+  a.base = s.base;
+  a.N = s.N;
+  a.P = s.P;
+  a.cols = s.N / 2 - 2;
+  a.bands = e.plan.bands;
+  a.draw_warps = e.plan.draw_warps;
+  a.chain_stride = s.chain_stride;
+  a.colour_stride = s.colour_stride;
+  a.tmt = s.tmt;
+  a.tmt_params = s.tmt_params;
+  a.cand = s.d_cand;
+  a.row_start = e.d_rows;
+  a.windows = e.d_rows + kGrMaxBands + 1;
+  a.xlo = e.plan.xlo;
+  a.xn = e.plan.xn;
+  a.depth = e.plan.depth;
+  a.first = e.plan.first;
+  a.last = e.plan.last;
+  a.rule = s.rule;
+  a.stream = s.opts.fast_stream;
+  a.xbuf = e.d_xbuf;
+  a.error = e.d_rows + 3 * kGrMaxBands + 1;
+  a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : 1L << 22;
+  a.silent_band_plus1 = s.test_silent_band + 1;
+  return a;
+}
+
+}  // namespace
+
+rt_status GridEngine::cftp(DmSampler& s, int a0, int n, const std::vector<std::vector<RunEngine::Epoch>>& epochs,
+                           int64_t first_sweeps, uint64_t fast_seed, int* attempts_run, bool* coalesced) {
+  const bool fast = s.opts.rng_mode == RT_RNG_FAST;
+  if (plan.depth < 2 || n < 1 || n > kGrTeams || nch != 2) return fail(RT_ERR_INVALID_ARGUMENT, "grid cftp: 1..4 attempts, 2 chains");
+  if (rt_status st = check_error(s)) return st;
+  GrArgs a = gr_args(*this, s);
+  a.couple = 1;
+  a.attempt0 = a0;
+  a.first_sweeps = first_sweeps;
+  a.seed = fast_seed;
+  a.start = s.base + 2 * s.chain_stride;
+  a.team_stride = 2 * s.chain_stride;
+  a.xteam = xbuf_bytes / sizeof(uint64_t);
+  constexpr size_t kWords = 4 + 2 * kGrTeams;  // {best, error, -, -, team}
+  if (!d_team) {
+    if (rt_status st = dev_alloc(&d_team, kWords * sizeof(int), stream)) return st;
+    if (rt_status st = dev_alloc(&d_teams, kGrTeams * a.team_stride, stream)) return st;
+    if (rt_status st = dev_alloc(&d_xteams, kGrTeams * xbuf_bytes, stream)) return st;
+  }
+  a.base = d_teams;
+  a.xbuf = d_xteams;
+  a.best = d_team;
+  a.error = d_team + 1;
+  a.team = reinterpret_cast<int2*>(d_team + 4);
+  std::vector<uint32_t> runs, seeds;
+  std::vector<int4> desc;
+  if (!fast) {
+    for (int k = 0; k < n; ++k) {
+      int4 d = make_int4((int)runs.size(), 0, (int)seeds.size(), 0);
+      for (const RunEngine::Epoch& e : epochs[(size_t)k]) {
+        if (!e.colours || e.colours->empty()) continue;
+        seeds.push_back(e.seed);
+        append_runs(e.colours->data(), (int64_t)e.colours->size(), true, &runs);
+      }
+      d.y = (int)runs.size() - d.x;
+      desc.push_back(d);
+    }
+    // one block: the descriptors, the epoch seeds, the runs
+    const size_t at_seeds = desc.size() * sizeof(int4), at_runs = at_seeds + seeds.size() * sizeof(uint32_t);
+    const int64_t words = (int64_t)(at_runs / sizeof(uint32_t) + runs.size());
+    if (runs_cap < words) {
+      dev_free(d_runs, s.stream);
+      d_runs = nullptr;
+      runs_cap = 0;
+      if (rt_status st = dev_alloc(&d_runs, (size_t)words * sizeof(uint32_t), s.stream)) return st;
+      runs_cap = words;
+    }
+    std::vector<uint32_t> block((size_t)words);
+    std::memcpy(block.data(), desc.data(), at_seeds);
+    std::copy(seeds.begin(), seeds.end(), block.begin() + (long)(at_seeds / sizeof(uint32_t)));
+    std::copy(runs.begin(), runs.end(), block.begin() + (long)(at_runs / sizeof(uint32_t)));
+    RT_CUDA_G(cudaMemcpyAsync(d_runs, block.data(), block.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s.stream));
+    a.attempt_desc = reinterpret_cast<const int4*>(d_runs);
+    a.epoch_seeds = d_runs + at_seeds / sizeof(uint32_t);
+    a.runs = d_runs + at_runs / sizeof(uint32_t);
+  }
+  for (int k = 0; k < n; ++k)  // the cells that no attempt writes
+    RT_CUDA_G(cudaMemcpyAsync(d_teams + k * a.team_stride, a.start, a.team_stride, cudaMemcpyDeviceToDevice, s.stream));
+  RT_CUDA_G(cudaMemsetAsync(d_team, 0, kWords * sizeof(int), s.stream));
+  RT_CUDA_G(cudaMemsetAsync(d_team, 0x7f, sizeof(int), s.stream));  // no attempt yet
+  RT_CUDA_G(cudaMemsetAsync(d_xteams, 0, n * xbuf_bytes, s.stream));  // no stale tags
+  void* args[] = {&a};
+  RT_CUDA_G(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)plan.bands, (unsigned)n), dim3((unsigned)plan.threads()), args,
+                                        plan.smem_bytes, s.stream));
+  s.launches++;
+  int res[2] = {0, 0};
+  RT_CUDA_G(cudaMemcpyAsync(res, d_team, sizeof res, cudaMemcpyDeviceToHost, s.stream));
+  RT_CUDA_G(cudaStreamSynchronize(s.stream));
+  if (res[1]) return fail(RT_ERR_TIMEOUT, "grid sweep: a band gave up waiting (a neighbour's boundary words never came)");
+  *coalesced = res[0] < a0 + n;
+  *attempts_run = *coalesced ? res[0] - a0 + 1 : n;
+  RT_CUDA_G(cudaMemcpyAsync(s.base, d_teams + (*attempts_run - 1) * a.team_stride, a.team_stride, cudaMemcpyDeviceToDevice,
+                            s.stream));
+  return RT_OK;
+}
+
 rt_status GridEngine::launch(DmSampler& s, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed, int64_t h0) {
   const int64_t chunk_max = 65536;  // bounds one launch to a fraction of a second
   std::vector<uint32_t> runs;
   for (int64_t done = 0; done < steps;) {
     const int64_t n = std::min(chunk_max, steps - done);
-    GrArgs a{};
-    a.base = s.base;
-    a.N = s.N;
-    a.P = s.P;
-    a.cols = s.N / 2 - 2;
-    a.bands = plan.bands;
-    a.draw_warps = plan.draw_warps;
-    a.chain_stride = s.chain_stride;
-    a.colour_stride = s.colour_stride;
-    a.tmt = s.tmt;
-    a.tmt_params = s.tmt_params;
-    a.cand = s.d_cand;
-    a.row_start = d_rows;
-    a.windows = d_rows + kGrMaxBands + 1;
-    a.xlo = plan.xlo;
-    a.xn = plan.xn;
-    a.depth = plan.depth;
-    a.first = plan.first;
-    a.last = plan.last;
-    a.rule = s.rule;
-    a.stream = s.opts.fast_stream;
-    a.xbuf = d_xbuf;
-    a.error = d_rows + 3 * kGrMaxBands + 1;
-    a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : 1L << 22;
-    a.silent_band_plus1 = s.test_silent_band + 1;
+    GrArgs a = gr_args(*this, s);
     a.seed = fast_seed;
     a.h0 = h0 + done;
     a.nruns = (int)n;

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "domino_rules.h"
+#include "domino_runs.h"
 #include "rt_internal.h"
 
 namespace rt {
@@ -14,6 +15,7 @@ namespace rt {
 struct DmSampler;
 
 constexpr int kGrMaxBands = 160;
+constexpr int kGrTeams = 4;  // attempts of a coupling from the past side by side
 
 struct GrPlan {
   bool ok = false;
@@ -44,10 +46,16 @@ struct GridEngine {
   uint32_t* d_runs = nullptr;
   int64_t runs_cap = 0;
   bool pending_error_check = false;
+  int* d_team = nullptr;         // couplings: {smallest attempt that coalesced, error, -, -, [k] bands that differ, done}
+  uint8_t* d_teams = nullptr;    // two chains of each attempt side by side
+  uint64_t* d_xteams = nullptr;  // their tagged words
 
   ~GridEngine();
   rt_status prepare(DmSampler& s);
   rt_status launch(DmSampler& s, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed, int64_t h0);
+  // As RunEngine::cftp, attempts [a0, a0 + n) side by side (n <= kGrTeams), where depth > 1.
+  rt_status cftp(DmSampler& s, int a0, int n, const std::vector<std::vector<RunEngine::Epoch>>& epochs,
+                 int64_t first_sweeps, uint64_t fast_seed, int* attempts_run, bool* coalesced);
   rt_status check_error(DmSampler& s);
 };
 

@@ -574,7 +574,7 @@ rt_status DmSampler::use_persistent(bool* yes) {
     eff_threads = tuned ? t : 0;
     return tuned;
   };
-  // A coupling runs its attempts side by side in clusters, where one holds the domain.
+  // A coupling runs its attempts side by side, whatever shape the table has for one walk.
   if (ask_table && !couple) take_entry(0);
   if (engine == 1 || opts.rng_mode == RT_RNG_MTGP) return RT_OK;
   if (plan_dirty) {
@@ -611,7 +611,7 @@ rt_status DmSampler::use_persistent(bool* yes) {
     *yes = true;
     return RT_OK;
   };
-  if (!couple && !explicit_engine && (engine == 0 || engine == 4) && (eff_bands == 0 || eff_bands > kClMaxCtas)) {
+  if (!explicit_engine && (engine == 0 || engine == 4) && (eff_bands == 0 || eff_bands > kClMaxCtas)) {
     if (rt_status st = try_grid(true)) return st;
     if (on_grid) return RT_OK;
   }
@@ -1019,17 +1019,19 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
   // that, or a sampler the run kernel does not take, runs attempt by attempt from the host.
   const int64_t kLaunchHalfSweeps = (int64_t)1 << 21;
   // TinyMT colours are drawn on the host for every attempt of a group, needed or not (5 ns a half-sweep): the
-  // first groups are short (order 15, first look-back 372: 1.6 ms, with one group 11.4).
+  // first groups are short (order 15, first look-back 372: 1.6 ms against 11.4 with one group).
   int64_t group_half_sweeps = fast ? kLaunchHalfSweeps : (int64_t)1 << 14;
   bool pers = false;
   if (rt_status st = s->use_persistent(&pers)) return st;
-  const bool one_launch = pers && !s->on_grid && (s->resident == 2 || s->resident == 4) && o.rng_mode != RT_RNG_MTGP;
+  const bool side_by_side = pers && s->on_grid && s->grid->plan.depth > 1;
+  const bool one_launch =
+      pers && (!s->on_grid || side_by_side) && (s->resident == 2 || s->resident == 4) && o.rng_mode != RT_RNG_MTGP;
   int att = 0;
   bool coalesced = false;
   while (att < max_attempts && !coalesced) {
     int n = 0;
     int64_t tot = 0;
-    while (one_launch && att + n < max_attempts &&
+    while (one_launch && att + n < max_attempts && !(side_by_side && n == kGrTeams) &&
            tot + look_back(att + n) <= (n ? group_half_sweeps : kLaunchHalfSweeps))
       tot += look_back(att + n++);
     group_half_sweeps = std::min(8 * group_half_sweeps, kLaunchHalfSweeps);
@@ -1039,7 +1041,9 @@ RT_API rt_status rt_domino_cftp(const int32_t* tmax, const int32_t* tmin, int32_
         for (int k = att + q; k >= 0; --k) epochs[(size_t)q].push_back({ep_seed[(size_t)k], &colours_of(k)});
       cudaEventRecord(s->ev0, s->stream);
       int ran = 0;
-      if (s->in_cluster) {
+      if (side_by_side) {
+        if (rt_status st = s->grid->cftp(*s, att, n, epochs, first_steps, (uint64_t)driver_seed, &ran, &coalesced)) return st;
+      } else if (s->in_cluster) {
         if (rt_status st =
                 s->cluster->cftp(*s, att, n, epochs, first_steps, (uint64_t)driver_seed, &ran, &coalesced))
           return st;
