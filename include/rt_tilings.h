@@ -78,11 +78,15 @@ typedef struct rt_walk_opts {
                            kernel (the run kernel, which rebuilds the passive colour only where
                            the colour switches, else k_persist); 3: k_persist, the resident
                            kernel that exchanges band rows every half-sweep; 4: the bit-plane
-                           kernel (one bit per lattice edge, TinyMT mode, 1 or 2 swept chains,
-                           tilings whose flip candidates keep off the array's outer cells; 0
-                           prefers it where it applies).  Lozenges: 0
-                           automatic, 1 per-step kernels, 2 the resident band kernel (TinyMT
-                           without MTGP, or fast mode); the same tilings from every engine */
+                           kernel with polled deltas (one bit per lattice edge, TinyMT mode, 1
+                           or 2 swept chains, tilings whose flip candidates keep off the
+                           array's outer cells).  0 prefers the bit-plane kernels in one
+                           cluster or with draw warps of their own, where they apply.
+                           Lozenges: 0 automatic (bit planes where they apply), 1 per-step
+                           kernels, 2 the resident kernel of bytes (TinyMT without MTGP, or
+                           fast mode).  Six-vertex: 0 automatic, 1 one kernel per sub-sweep, 2
+                           the resident kernel wherever it holds the chains (refused where 16
+                           CTAs could not).  The same tilings from every engine */
   void* cuda_stream;    /* cudaStream_t to run on; NULL = the library's own stream */
 } rt_walk_opts;
 
@@ -498,7 +502,7 @@ RT_API rt_status rt_dm_sampler_engine_info(rt_dm_sampler* s, int64_t* out4);
    multiple of 32 up to 1024, 0: 1024) of the run kernel.
    Results do not depend on the shape: every draw is keyed by its site.  Without this call,
    and with rt_walk_opts.engine 0, the autotuner's table (rt_tune_load) chooses when it has an
-   entry.  out6 of rt_dm_sampler_launch_info = {engine, units, bands, units per thread,
+   entry (couplings from the past run attempts side by side and choose for themselves).  out6 of rt_dm_sampler_launch_info = {engine, units, bands, units per thread,
    threads per band, 1 when the table chose}. */
 RT_API rt_status rt_dm_sampler_set_launch(rt_dm_sampler* s, int32_t engine, int32_t bands, int32_t threads);
 RT_API rt_status rt_dm_sampler_launch_info(rt_dm_sampler* s, int64_t* out6);

@@ -456,9 +456,9 @@ class LozengeTiler(_TinyMTTable):
 
     def __init__(self, rng: str = "tinymt", fast_stream: int = 0, q: float | None = None, engine: int = 0):
         """q: None for the reference's uniform rotation (lozengekernel.cl), else the q^volume
-        rotation of qlozengekernel.cl (down-move rescaling corrected).  engine: 0 automatic (the
-        resident band kernel where it holds the size), 1 the per-step kernels, 2 the resident
-        band kernel (an error where it does not hold the size); every engine gives the same
+        rotation of qlozengekernel.cl (down-move rescaling corrected).  engine: 0 automatic (bit
+        planes where they apply, else the resident kernel of bytes where it holds the size), 1 the
+        per-step kernels, 2 the resident kernel of bytes (an error where it does not hold the size); every engine gives the same
         tilings."""
         self.rng = rng
         self.fast_stream = int(fast_stream)
