@@ -32,8 +32,8 @@
 namespace rt {
 namespace {
 
-// 512 threads, two CTAs an SM: 512 mixed instances 61 ms; 384 threads and three CTAs 69, 512 and three (40
-// registers) 98, 256 and four 86; one hexagon of side 32 30 ms, with 256 threads 37.
+// 512 threads, two CTAs an SM: 512 mixed instances 59-64 ms (the call); 384 threads and two CTAs 61, three 72, 640 and two
+// 70; one hexagon of side 32 22.5 ms, 23.6, 28.3, 26.6.
 constexpr int kBatchThreads = 512;
 
 #define BT_CUDA(expr)                                                                   \
@@ -670,7 +670,7 @@ RT_API rt_status rt_cftp_batch(rt_cftp_instance* inst, int32_t count, void* cuda
       int per_sm = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_cftp, kBatchThreads, smem_max);
       // Few instances: the SMs left over run attempts ahead of the instances' own CTAs (one hexagon of side 32:
-      // 55 -> 30 ms; 64 mixed instances 49 -> 37 ms).
+      // 55 -> 30 ms; 64 mixed instances 49 -> 37 ms, when measured alone).
       grid = std::max(1, std::min(std::max(n_small, std::min(sms, 4 * n_small)), std::max(1, per_sm) * sms));
       BatchArgs ba{d_inst, d_state, n_small, d_tilings, d_queue, d_queue + 1, reinterpret_cast<int*>(d_queue + 2),
                    1L << 24, smem_max};

@@ -6,14 +6,14 @@
 // inputs whose edges agree at both ends and whose flip candidates border no cell that the reference
 // never rebuilds are held this way (bp_load tells); the others keep the byte kernels (batch_cftp.cuh).
 //
-// A half-sweep (step) is one interval between CTA barriers: every warp applies its words' moves, then
-// makes draws for the next one.  Draws are made for bytes of eight cells that hold a candidate, one
+// Warps of their own draw, a few half-sweeps (steps) ahead; the others apply the moves.  Draws are made for bytes of eight cells that hold a candidate, one
 // lane a Philox block (four cells), so a diamond draws for half of its bounding box.
 //
 // Bound: the issue of the draws, about 220 cycles of a scheduler for 32 blocks (160 of them Philox's
-// products), and in a CTA alone on its SM the latency of one such block and one update, about 1100
-// cycles.  Measured (GB300, hexagon of side 32, one CTA): 0.56 us a step, bytes of both chains with a
-// rebuild pass 2.58 us; 512 mixed diamonds (orders 16-48) and hexagons (sides 8-32): 61 ms, before 245.
+// products), and in a CTA alone on its SM an update's latency.  Measured (GB300): hexagon of side 32, one CTA,
+// attempts side by side, 23.1 ms (bytes of both chains with a rebuild pass: 253 ms, attempts in turn); 64 mixed
+// diamonds (orders 16-48) and hexagons (sides 8-32) 34 ms (226), 512 of them 65 (246).  Every warp drawing and updating
+// in turn, a barrier a step: 29.5, 39.4 and 73-82 ms; 192 or 256 update threads of the 512: 27.6 and 25.4 ms for the hexagon.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -27,9 +27,11 @@ namespace rt {
 // Shared memory of one instance, offsets in 32-bit words.
 struct BpLayout {
   int W;                                           // 32-cell words a row
+  int period;                                      // steps between the barriers of the whole CTA
   int planes, valid, moves, items, units, stage;  // stage shares its words with moves, items and units
   int words;                                       // all
 };
+constexpr int kBpUpdate = 128;      // threads that update, of a CTA; the others draw
 constexpr int kBpDominoWord = 8;    // [2 chains]{VD0, VD1, HE, HO}
 constexpr int kBpLozengeWord = 24;  // [2 chains]{E0-2, NE0-2, N0-2, three of padding}
 
@@ -40,7 +42,10 @@ __host__ __device__ inline BpLayout bp_layout(int model, int N, int P) {
   L.planes = PW;  // a word of padding in front, one after each row
   L.valid = L.planes + (N + (model == 0 ? 0 : 1)) * (L.W + 1) * PW;
   L.moves = L.stage = (L.valid + N * L.W + 3) & ~3;
-  L.items = L.moves + 4 * N * L.W;  // two sets of a pair of words each
+  // As many steps a period as 32 KB of moves hold, but 2 to 8: a hexagon of side 32 alone 29.5 ms with 1, 24.0 with 4, 23.1
+  // with 8.
+  L.period = N * L.W <= 256 ? 8 : N * L.W <= 512 ? 4 : 2;
+  L.items = L.moves + 2 * L.period * 2 * N * L.W;  // [period parity][step][word] pairs of words
   L.units = L.items + N * L.W;
   const int staged = L.stage + (model == 0 ? 2 : 3) * N * P / 4;
   L.words = L.units + 4 * N * L.W;
@@ -181,7 +186,6 @@ __device__ bool bp_load(uint32_t* sm, const BpLayout& L, const DevInstance& in, 
 
 // Draws of half-sweep h into one set of moves: bit k of x (y) set where cell k, in state 3 or 25 (12 or 38), is in
 // it (in the other) after the half-sweep.
-// The unit of a lane in its warp's first 16 is held in registers.
 struct BpUnit {
   uint32_t row, quad, to;  // to: byte offset in a set of moves
 };
@@ -193,12 +197,10 @@ __device__ __forceinline__ BpUnit bp_unit(const uint32_t* sm, const BpLayout& L,
   b.to = (b.row * (uint32_t)L.W + (byte >> 2)) * 8 + (byte & 3);
   return b;
 }
-__device__ __forceinline__ void bp_draw_unit(uint64_t seed, uint32_t stream, int64_t h, uint8_t* moves, const BpUnit& b,
-                                             bool on, uint32_t w_up, uint32_t lo_dn, uint32_t w_dn) {
-  const uint4 d = fast_quad(seed, stream, h, b.row, b.quad);
+__device__ __forceinline__ void bp_moves_of(const uint4& d, uint8_t* moves, const BpUnit& b, bool on, uint3 t) {
   auto nib = [](bool p, bool q, bool r, bool s) { return (p ? 1u : 0u) | (q ? 2u : 0u) | (r ? 4u : 0u) | (s ? 8u : 0u); };
-  const uint32_t up = nib(d.x < w_up, d.y < w_up, d.z < w_up, d.w < w_up);
-  const uint32_t dn = nib(d.x - lo_dn < w_dn, d.y - lo_dn < w_dn, d.z - lo_dn < w_dn, d.w - lo_dn < w_dn);
+  const uint32_t up = nib(d.x < t.x, d.y < t.x, d.z < t.x, d.w < t.x);
+  const uint32_t dn = nib(d.x - t.y < t.z, d.y - t.y < t.z, d.z - t.y < t.z, d.w - t.y < t.z);
   const uint32_t mine = (up ^ 15u) | (dn << 16);
   const uint32_t pair = mine | (__shfl_down_sync(~0u, mine, 1) << 4);
   if (on && !(threadIdx.x & 1)) {
@@ -207,53 +209,67 @@ __device__ __forceinline__ void bp_draw_unit(uint64_t seed, uint32_t stream, int
   }
 }
 
-// Half-sweeps [-look, 0) of a loaded domino instance; stop(step) is asked (by every thread, after a
-// barrier) every 256 steps.  False where it stopped.
+// The steps [-look, 0) of an attempt: the first kBpUpdate threads update, the others draw, a period of
+// L.period steps ahead, two steps' Philox blocks side by side; the update warps alone meet after every step.
+// update(k, step, moves): the moves of one set applied to item k (a word of a chain); test(row, step): {width up,
+// low down, width down}; stop() is asked (by every thread, after a barrier) every 256 steps.  False where it stopped.
+template <int kThreads, int period, class Update, class Test, class Stop>
+__device__ bool bp_steps_of(uint32_t* sm, const BpLayout& L, const DevInstance& in, int64_t look, int units, Update update,
+                         Test test, Stop stop) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int set = 2 * in.N * L.W;  // words of a set of moves
+  constexpr int ask = 256 / period - 1;
+  const int64_t periods = (look + period - 1) / period;
+  const uint64_t seed = in.seed;
+  const uint32_t stream = in.stream;
+  const int u_warp = ((tid - kBpUpdate) >> 5) * 16, u0 = u_warp + (lane >> 1);
+  const BpUnit unit0 = tid >= kBpUpdate ? bp_unit(sm, L, u0, units) : BpUnit{0, 0, 0};
+  auto draw = [&](int64_t q) {
+    uint8_t* const to = reinterpret_cast<uint8_t*>(sm + L.moves + (int)(q & 1) * period * set);
+    for (int u = u_warp; u < units; u += (kThreads - kBpUpdate) / 2) {
+      const BpUnit b = u == u_warp ? unit0 : bp_unit(sm, L, u + (lane >> 1), units);
+      const bool on = u + (lane >> 1) < units;
+#pragma unroll
+      for (int r = 0; r < period; r += 2) {
+        const int64_t h = -look + q * period + r;  // (draws of steps past the end are not used)
+        const uint4 d0 = fast_quad(seed, stream, h, b.row, b.quad), d1 = fast_quad(seed, stream, h + 1, b.row, b.quad);
+        bp_moves_of(d0, to + 4 * r * set, b, on, test(b.row, h));
+        bp_moves_of(d1, to + 4 * (r + 1) * set, b, on, test(b.row, h + 1));
+      }
+    }
+  };
+  if (tid >= kBpUpdate) draw(0);
+  __syncthreads();
+  for (int64_t q = 0; q < periods; ++q) {
+    if (tid < kBpUpdate) {
+      const uint32_t* moves = sm + L.moves + (int)(q & 1) * period * set;
+      const int len = (int)min((int64_t)period, look - q * period);
+      for (int r = 0; r < len; ++r, moves += set) {
+        update(-look + q * period + r, moves);
+        asm volatile("bar.sync 1, %0;" ::"n"(kBpUpdate) : "memory");
+      }
+    } else if (q + 1 < periods) {
+      draw(q + 1);
+    }
+    __syncthreads();
+    if ((q & ask) == ask && stop()) return false;
+  }
+  return true;
+}
+
+template <int kThreads, class Update, class Test, class Stop>
+__device__ __forceinline__ bool bp_steps(uint32_t* sm, const BpLayout& L, const DevInstance& in, int64_t look, int units,
+                                         Update update, Test test, Stop stop) {
+  return L.period == 8   ? bp_steps_of<kThreads, 8>(sm, L, in, look, units, update, test, stop)
+         : L.period == 4 ? bp_steps_of<kThreads, 4>(sm, L, in, look, units, update, test, stop)
+                         : bp_steps_of<kThreads, 2>(sm, L, in, look, units, update, test, stop);
+}
+
+// A loaded domino instance.
 template <int kThreads, class Stop>
 __device__ bool bp_domino(uint32_t* sm, const BpLayout& L, const DevInstance& in, int64_t look, int items, int units,
                           Stop stop) {
-  const int tid = threadIdx.x, W = L.W, lane = tid & 31, up_row = (W + 1) * kBpDominoWord;
-  const int move_set = 2 * in.N * W;
-  const uint64_t seed = in.seed;
-  const uint32_t stream = in.stream;
-  // the last warps draw first: the first ones have the words to update
-  const int u0 = (kThreads / 32 - 1 - (tid >> 5)) * 16 + (lane >> 1), u_warp = u0 - (lane >> 1);
-  const BpUnit unit0 = bp_unit(sm, L, u0, units);
-  auto draw = [&](int64_t h, int set) {
-    const int t = (h & 1) ? 0 : 2;
-    uint8_t* const moves = reinterpret_cast<uint8_t*>(sm + L.moves + set * move_set);
-    if (u_warp < units) {
-      const int c = (int)(unit0.row & 1u) | t;
-      bp_draw_unit(seed, stream, h, moves, unit0, u0 < units, in.w_up[c], in.lo_dn[c], in.w_dn[c]);
-    }
-    for (int u = u_warp + kThreads / 2; u < units; u += kThreads / 2) {
-      const BpUnit b = bp_unit(sm, L, u + (lane >> 1), units);
-      const int c = (int)(b.row & 1u) | t;
-      bp_draw_unit(seed, stream, h, moves, b, u + (lane >> 1) < units, in.w_up[c], in.lo_dn[c], in.w_dn[c]);
-    }
-  };
-  auto update = [&](int here_at, int move_at, bool odd, uint32_t valid, int t, const uint32_t* moves) {
-    uint32_t* const here = sm + here_at;
-    uint32_t* const above = here - up_row;
-    const uint2 move = *reinterpret_cast<const uint2*>(moves + move_at);
-    const uint4 me = *reinterpret_cast<const uint4*>(here);
-    const uint32_t U = above[1 - t], west = here[3 - kBpDominoWord];
-    const bool aligned = odd == (t != 0);  // left HE, right HO of the same word
-    const uint32_t D = t ? me.y : me.x;
-    const uint32_t lft = aligned ? me.z : __funnelshift_l(west, me.w, 1), rgt = aligned ? me.w : me.z;
-    // Flippable: up = down, left = right, up != left (states 3 and 12).
-    const uint32_t flip = ~(U ^ D) & ~(lft ^ rgt) & (U ^ lft) & valid;
-    const uint32_t T = flip & ((U & ~move.x) | (~U & move.y));
-    if (T) {
-      above[1 - t] = U ^ T;
-      here[t] = D ^ T;
-      here[2] = me.z ^ T;
-      // HO: the word itself, or bit k - 1 of this word and bit 31 of the word to the left, whose other bits belong
-      // to that word's cells.
-      atomicXor(here + 3, aligned ? T : T >> 1);
-      if (!aligned && (T & 1u)) atomicXor(here + 3 - kBpDominoWord, 0x80000000u);
-    }
-  };
+  const int tid = threadIdx.x, W = L.W, up_row = (W + 1) * kBpDominoWord;
   struct Item {
     int here, move;
     bool odd;
@@ -265,47 +281,65 @@ __device__ bool bp_domino(uint32_t* sm, const BpLayout& L, const DevInstance& in
     return Item{L.planes + (i * (W + 1) + x) * kBpDominoWord + 4 * (k & 1), 2 * (i * W + x), (i & 1) != 0,
                 k < 2 * items ? sm[L.valid + i * W + x] : 0u};
   };
-  const Item item0 = item(tid);
-  draw(-look, 0);
-  __syncthreads();
-  for (int64_t h = -look; h < 0; ++h) {
-    const int set = (int)(h & 1), t = set ? 0 : 1;
-    const uint32_t* const moves = sm + L.moves + set * move_set;
-    if (item0.valid) update(item0.here, item0.move, item0.odd, item0.valid, t, moves);
-    for (int k = tid + kThreads; k < 2 * items; k += kThreads) {
-      const Item it = item(k);
-      update(it.here, it.move, it.odd, it.valid, t, moves);
+  auto apply = [&](const Item& it, int t, const uint32_t* moves) {
+    uint32_t* const here = sm + it.here;
+    uint32_t* const above = here - up_row;
+    const uint2 move = *reinterpret_cast<const uint2*>(moves + it.move);
+    const uint4 me = *reinterpret_cast<const uint4*>(here);
+    const uint32_t U = above[1 - t], west = here[3 - kBpDominoWord];
+    const bool aligned = it.odd == (t != 0);  // left HE, right HO of the same word
+    const uint32_t D = t ? me.y : me.x;
+    const uint32_t lft = aligned ? me.z : __funnelshift_l(west, me.w, 1), rgt = aligned ? me.w : me.z;
+    // Flippable: up = down, left = right, up != left (states 3 and 12).
+    const uint32_t flip = ~(U ^ D) & ~(lft ^ rgt) & (U ^ lft) & it.valid;
+    const uint32_t T = flip & ((U & ~move.x) | (~U & move.y));
+    if (T) {
+      above[1 - t] = U ^ T;
+      here[t] = D ^ T;
+      here[2] = me.z ^ T;
+      // HO: the word itself, or bit k - 1 of this word and bit 31 of the word to the left, whose other bits belong
+      // to that word's cells.
+      atomicXor(here + 3, aligned ? T : T >> 1);
+      if (!aligned && (T & 1u)) atomicXor(here + 3 - kBpDominoWord, 0x80000000u);
     }
-    if (h + 1 < 0) draw(h + 1, set ^ 1);
-    __syncthreads();
-    if (((h + look) & 255) == 255 && stop()) return false;
-  }
-  return true;
+  };
+  const Item item0 = item(tid < kBpUpdate ? tid : 2 * items), item1 = item(tid < kBpUpdate ? tid + kBpUpdate : 2 * items);
+  return bp_steps<kThreads>(
+      sm, L, in, look, units,
+      [&](int64_t h, const uint32_t* moves) {
+        const int t = (h & 1) ? 0 : 1;
+        if (item0.valid) apply(item0, t, moves);
+        if (item1.valid) apply(item1, t, moves);
+        for (int k = tid + 2 * kBpUpdate; k < 2 * items; k += kBpUpdate) apply(item(k), t, moves);
+      },
+      [&](uint32_t row, int64_t h) {
+        const int c = (int)(row & 1u) | ((h & 1) ? 0 : 2);
+        return make_uint3(in.w_up[c], in.lo_dn[c], in.w_dn[c]);
+      },
+      stop);
 }
 
 template <int kThreads, class Stop>
 __device__ bool bp_lozenge(uint32_t* sm, const BpLayout& L, const DevInstance& in, int64_t look, uint32_t c4, uint32_t c8,
                            int items, int units, Stop stop) {
-  const int tid = threadIdx.x, W = L.W, left = kBpLozengeWord, lane = tid & 31, dn_row = (W + 1) * kBpLozengeWord;
-  const int move_set = 2 * in.N * W;
-  const uint64_t seed = in.seed;
-  const uint32_t stream = in.stream;
-  const int u0 = (kThreads / 32 - 1 - (tid >> 5)) * 16 + (lane >> 1), u_warp = u0 - (lane >> 1);
-  const BpUnit unit0 = bp_unit(sm, L, u0, units);
-  auto draw = [&](int64_t h, int set) {
-    uint8_t* const moves = reinterpret_cast<uint8_t*>(sm + L.moves + set * move_set);
-    if (u_warp < units) bp_draw_unit(seed, stream, h, moves, unit0, u0 < units, c4, c4, c8 - c4);
-    for (int u = u_warp + kThreads / 2; u < units; u += kThreads / 2)
-      bp_draw_unit(seed, stream, h, moves, bp_unit(sm, L, u + (lane >> 1), units), u + (lane >> 1) < units, c4, c4, c8 - c4);
+  const int tid = threadIdx.x, W = L.W, left = kBpLozengeWord, dn_row = (W + 1) * kBpLozengeWord;
+  struct Item {
+    int here, move, q;
+    uint32_t valid;
   };
-  auto update = [&](int here_at, int move_at, int q, uint32_t valid, const uint32_t* moves) {
-    if (q >= 3) q -= 3;
-    const int qw = q == 0 ? 2 : q - 1;
-    uint32_t* const own = sm + here_at + q;
-    uint32_t* const west = sm + here_at + qw;
+  auto item = [&](int k) {
+    const uint32_t e = k < 2 * items ? sm[L.items + (k >> 1)] : 0u;
+    const int i = (int)(e >> 16), x = (int)(e & 0xffffu);
+    return Item{L.planes + (i * (W + 1) + x) * kBpLozengeWord + 12 * (k & 1), 2 * (i * W + x), i % 3,
+                k < 2 * items ? sm[L.valid + i * W + x] : 0u};
+  };
+  auto apply = [&](const Item& it, int r, const uint32_t* moves) {
+    const int q = it.q + r >= 3 ? it.q + r - 3 : it.q + r, qw = q == 0 ? 2 : q - 1;
+    uint32_t* const own = sm + it.here + q;
+    uint32_t* const west = sm + it.here + qw;
     uint32_t* const south = own + dn_row + 6;
     uint32_t* const sw = west + dn_row + 3;
-    const uint2 move = *reinterpret_cast<const uint2*>(moves + move_at);
+    const uint2 move = *reinterpret_cast<const uint2*>(moves + it.move);
     const uint32_t e = own[0], ne = own[3], n = own[6], s = south[0], w_l = west[-left], ws_l = sw[-left];
     uint32_t w = west[0], ws = sw[0];
     if (q == 0) {
@@ -313,7 +347,7 @@ __device__ bool bp_lozenge(uint32_t* sm, const BpLayout& L, const DevInstance& i
       ws = __funnelshift_l(ws_l, ws, 1);
     }
     // Flippable: E, N, SW equal, NE, W, S their complement.
-    const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
+    const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & it.valid;
     const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
     if (T) {
       own[0] = e ^ T;
@@ -329,34 +363,17 @@ __device__ bool bp_lozenge(uint32_t* sm, const BpLayout& L, const DevInstance& i
       }
     }
   };
-  struct Item {
-    int here, move, q;
-    uint32_t valid;
-  };
-  auto item = [&](int k) {
-    const uint32_t e = k < 2 * items ? sm[L.items + (k >> 1)] : 0u;
-    const int i = (int)(e >> 16), x = (int)(e & 0xffffu);
-    return Item{L.planes + (i * (W + 1) + x) * kBpLozengeWord + 12 * (k & 1), 2 * (i * W + x), i % 3,
-                k < 2 * items ? sm[L.valid + i * W + x] : 0u};
-  };
-  const Item item0 = item(tid);
-  draw(-look, (int)(look & 1));
-  __syncthreads();
+  const Item item0 = item(tid < kBpUpdate ? tid : 2 * items), item1 = item(tid < kBpUpdate ? tid + kBpUpdate : 2 * items);
   int r = 0;  // the step's colour: look is a multiple of three
-  for (int64_t h = -look; h < 0; ++h) {
-    const int set = (int)(h & 1);
-    const uint32_t* const moves = sm + L.moves + set * move_set;
-    if (item0.valid) update(item0.here, item0.move, item0.q + r, item0.valid, moves);
-    for (int k = tid + kThreads; k < 2 * items; k += kThreads) {
-      const Item it = item(k);
-      update(it.here, it.move, it.q + r, it.valid, moves);
-    }
-    r = r == 2 ? 0 : r + 1;
-    if (h + 1 < 0) draw(h + 1, set ^ 1);
-    __syncthreads();
-    if (((h + look) & 255) == 255 && stop()) return false;
-  }
-  return true;
+  return bp_steps<kThreads>(
+      sm, L, in, look, units,
+      [&](int64_t, const uint32_t* moves) {
+        if (item0.valid) apply(item0, r, moves);
+        if (item1.valid) apply(item1, r, moves);
+        for (int k = tid + 2 * kBpUpdate; k < 2 * items; k += kBpUpdate) apply(item(k), r, moves);
+        r = r == 2 ? 0 : r + 1;
+      },
+      [&](uint32_t, int64_t) { return make_uint3(c4, c4, c8 - c4); }, stop);
 }
 
 // Words in which the two chains differ, of this thread's share.
