@@ -495,7 +495,9 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
     const uint32_t above = (uint32_t)__cvta_generic_to_shared(valid ? sm + (((i - 1 - i0) * wn + w - wlo) * NCH + c) * 4 : pad + 8);
     const uint32_t here = valid ? above + pitch : above;
     // Exchange words: of row i those that its own, the row above's or the row below's candidates change, and the
-    // word to the left (its last HO bit).  Per lane, the same every time; ~0: none.
+    // word to the left (its last HO bit); and of every row its first element, whatever it holds (a scratch word
+    // outside the window), so that two bands wait for each other or not at all, also where a gap in the domain leaves
+    // one of them nothing to change.  Per lane, the same every time; ~0: none.
     const bool silent = band + 1 == a.silent_band_plus1;  // test hook: publishes nothing
     const uint32_t parity = (uint32_t)((a.last - a.first + 1) * a.xn * NCH * 4);
     uint32_t send_at[kGrMove], send_to[kGrMove], take_at[kGrMove], take_to[kGrMove];
@@ -507,8 +509,10 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_dee
         const int n = row_words(r, &first);
         if (n) lo = min(lo, first - 1), hi = max(hi, first + n - 1);
       }
-      if (row < a.first || row > a.last || row < i0 || row >= u1 || ww < lo || ww > hi || ww < wlo || ww >= wlo + wn) return;
-      *local = (uint32_t)__cvta_generic_to_shared(sm + (((row - i0) * wn + ww - wlo) * NCH + cc) * 4 + p);
+      if (row < a.first || row > a.last || row < i0 || row >= u1) return;
+      const bool held = ww >= lo && ww <= hi && ww >= wlo && ww < wlo + wn;
+      if (!held && q != 0) return;
+      *local = (uint32_t)__cvta_generic_to_shared(held ? sm + (((row - i0) * wn + ww - wlo) * NCH + cc) * 4 + p : pad);
       *global = (uint32_t)((row - a.first) * a.xn * NCH * 4 + q);
     };
     const int per_row = a.xn * NCH * 4, own = r1 - r0, edge_rows = min(own, 2 * depth);

@@ -136,3 +136,28 @@ def test_automatic_depth_equals_per_half_sweep_kernels(rt, rng, shape):
         want, _ = _chains(rt, tiler, starts, (1, 0, 0), steps)
         for g, w in zip(got, want):
             assert np.array_equal(g, w), (shape, rng)
+
+
+@pytest.mark.parametrize("rng", ["tinymt", "fast"])
+@pytest.mark.parametrize("gap", [3, 8, 14, 40])
+def test_components_apart(rt, rng, gap):
+    # Two diamonds one above the other, of different columns, with rows between them that hold nothing that can flip
+    blocks = [_start(rt, order) for order in (9, 14)]
+    sides = [rt.side_of(b[0]) for b in blocks]
+    n = sum(sides) + gap + 60
+    n += n % 2
+    starts = []
+    for which in (0, 1):
+        g = np.zeros((n, n), np.int32)
+        row = 2
+        for (pair, side, col) in zip(blocks, sides, (40, 4)):
+            g[row:row + side, col:col + side] = pair[which].reshape(side, side)
+            row += side + gap - gap % 2
+        starts.append(g.ravel().copy())
+    tiler = rt.DominoTiler(rule="cftp", rng=rng, fast_stream=1)
+    steps = [(90, 3), (31, 4)]
+    for use in (starts[:1], starts):
+        got, info = _chains(rt, tiler, use, (0, 0, 0), steps)
+        assert info["engine"] == 4
+        want, _ = _chains(rt, tiler, use, (1, 0, 0), steps)
+        assert all(np.array_equal(g, w) for g, w in zip(got, want))
