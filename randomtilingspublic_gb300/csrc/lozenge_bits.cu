@@ -128,6 +128,9 @@ __device__ __forceinline__ void lb_cta_sync() { asm volatile("barrier.sync 0;" :
 
 constexpr int kLbWord = 12;  // words per (row, word, chain): E0-2, NE0-2, N0-2, three of padding
 constexpr int kLbPad = 3 * kLbWord * 2;
+// Runs that the draw warps are ahead: one, but a period in one CTA in fast mode, where a run is one step of one Philox
+// block's latency: there two blocks go side by side, and only the update warps meet after every step.
+constexpr int lb_ahead(bool fast, int form) { return fast && form == kLbOne ? 8 : 1; }
 
 // KS: words per draw warp.
 template <int NCH, int kMode, int KS, int kForm>
@@ -138,6 +141,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   __shared__ int s_failed;
   __shared__ int s_stop;  // a smaller attempt coalesced
   constexpr bool kFast = kMode == kLbFast, kParams = kMode == kLbTmtParams;
+  constexpr int kAhead = lb_ahead(kFast, kForm);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)(blockDim.x >> 5);
   const int ndraw = a.draw_warps, nslots = ndraw * KS, band = kForm == kLbOne ? 0 : (int)blockIdx.x;
   const bool cftp = kForm == kLbOne && NCH == 2 && a.attempts > 0;
@@ -288,6 +292,19 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       if (__any_sync(~0u, e != ~0u)) n_mine = g + 1;
     }
   }
+  // Fast mode: the moves of four words from their Philox blocks.
+  auto put = [&](const uint4& d, uint2* out) {
+    auto nib = [](bool p, bool q, bool r, bool s) { return (p ? 1u : 0u) | (q ? 2u : 0u) | (r ? 4u : 0u) | (s ? 8u : 0u); };
+    const uint32_t u = nib(d.x - a.lo_up < a.w_up, d.y - a.lo_up < a.w_up, d.z - a.lo_up < a.w_up, d.w - a.lo_up < a.w_up);
+    const uint32_t v = nib(d.x - a.lo_dn < a.w_dn, d.y - a.lo_dn < a.w_dn, d.z - a.lo_dn < a.w_dn, d.w - a.lo_dn < a.w_dn);
+    const uint32_t mine = (u ^ 15u) | (v << 16);
+    const uint32_t pair = mine | (__shfl_down_sync(~0u, mine, 1) << 4);
+    if (!(lane & 1)) {
+      uint8_t* to = reinterpret_cast<uint8_t*>(out + (lane >> 3)) + ((lane & 7) >> 1);
+      to[0] = (uint8_t)pair;
+      to[4] = (uint8_t)(pair >> 16);
+    }
+  };
   auto draw_run = [&](uint32_t run, int64_t h, uint32_t reseed_to, uint2* out) {
     if constexpr (!kFast) {
       const int L = (int)(run & 0x1fffffffu);
@@ -349,17 +366,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
 #pragma unroll
       for (int g = 0; g < KS / 4; ++g) {
         if (g > 0 && g >= n_mine) break;
-        const uint4 d = fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]);
-        auto nib = [](bool p, bool q, bool r, bool s) { return (p ? 1u : 0u) | (q ? 2u : 0u) | (r ? 4u : 0u) | (s ? 8u : 0u); };
-        const uint32_t u = nib(d.x - a.lo_up < a.w_up, d.y - a.lo_up < a.w_up, d.z - a.lo_up < a.w_up, d.w - a.lo_up < a.w_up);
-        const uint32_t v = nib(d.x - a.lo_dn < a.w_dn, d.y - a.lo_dn < a.w_dn, d.z - a.lo_dn < a.w_dn, d.w - a.lo_dn < a.w_dn);
-        const uint32_t mine = (u ^ 15u) | (v << 16);
-        const uint32_t pair = mine | (__shfl_down_sync(~0u, mine, 1) << 4);
-        if (!(lane & 1)) {
-          uint8_t* to = reinterpret_cast<uint8_t*>(out + warp * KS + 4 * g + (lane >> 3)) + ((lane & 7) >> 1);
-          to[0] = (uint8_t)pair;
-          to[4] = (uint8_t)(pair >> 16);
-        }
+        put(fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]), out + warp * KS + 4 * g);
       }
     }
   };
@@ -389,8 +396,27 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   auto seed_of = [&](uint32_t run) -> uint32_t {
     return !kFast && ((run >> 29) & 1u) ? __ldg(&a.epoch_seeds[epoch++]) : 0u;
   };
+  // A period's steps, two at a time (those past the end are not used).
+  auto draw_period = [&](int q) {
+    if constexpr (kAhead > 1) {
+      uint2* const out = smove + (q & 1) * kAhead * nslots + warp * KS;
+#pragma unroll
+      for (int g = 0; g < KS / 4; ++g) {
+        if (g > 0 && g >= n_mine) break;
+        for (int r = 0; r < kAhead; r += 2) {
+          const int64_t h = h0 + q * kAhead + r;
+          const uint4 d0 = fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]);
+          const uint4 d1 = fast_quad(a.seed, a.stream, h + 1, f_row[g], f_quad[g]);
+          put(d0, out + r * nslots + 4 * g);
+          put(d1, out + (r + 1) * nslots + 4 * g);
+        }
+      }
+    }
+  };
   uint32_t next = run_at(1);
-  if (!updates && nruns > 0) {
+  if (kAhead > 1) {
+    if (!updates) draw_period(0);
+  } else if (!updates && nruns > 0) {
     const uint32_t run = run_at(0);
     draw_run(run, h0, seed_of(run), smove);
     if (tid == 0) s_colour[0] = run >> 30;
@@ -459,7 +485,48 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
     }
     __syncwarp();
   };
-  if (updates) {
+  if constexpr (kAhead > 1) {
+    const int periods = (nruns + kAhead - 1) / kAhead;
+    int r = c0;  // the step's colour
+    for (int p = 0; p < periods; ++p) {
+      if (updates) {
+        uint32_t at = move_at + (uint32_t)((p & 1) * kAhead) * move_bytes;
+        const int len = min(kAhead, nruns - p * kAhead);
+        for (int k = 0; k < len; ++k, at += move_bytes) {
+          const uint2 move = lb_lds2(at);
+          const int q = i3 + r >= 3 ? i3 + r - 3 : i3 + r, qw = q == 0 ? 2 : q - 1;
+          const uint32_t own = here + 4u * q, west = here + 4u * qw, south = below + 4u * (6 + q), sw = below + 4u * (3 + qw);
+          const uint32_t e = lb_lds(own), ne = lb_lds(own + 12u), n = lb_lds(own + 24u);
+          uint32_t w = lb_lds(west), ws = lb_lds(sw);
+          const uint32_t s = lb_lds(south), w_l = lb_lds(west - left), ws_l = lb_lds(sw - left);
+          if (q == 0) {
+            w = __funnelshift_l(w_l, w, 1);
+            ws = __funnelshift_l(ws_l, ws, 1);
+          }
+          const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
+          const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
+          lb_sts(own, e ^ T);
+          lb_sts(own + 12u, ne ^ T);
+          lb_sts(own + 24u, n ^ T);
+          lb_sts(south, s ^ T);
+          const uint32_t tw = q == 0 ? T >> 1 : T, tl = q == 0 ? T << 31 : 0u;
+          lb_xor_if(west, tw);
+          lb_xor_if(sw, tw);
+          lb_xor_if(west - left, tl);
+          lb_xor_if(sw - left, tl);
+          r = r == 2 ? 0 : r + 1;
+          asm volatile("bar.sync 1, %0;" ::"r"(32 * (nwarps - ndraw)) : "memory");
+        }
+      } else if (p + 1 < periods) {
+        draw_period(p + 1);
+      }
+      lb_cta_sync();
+      if (told_stop(p * kAhead + kAhead - 1)) {
+        stopped = true;
+        break;
+      }
+    }
+  } else if (updates) {
     const bool edge_warp = __any_sync(~0u, is_first || is_last);
     const bool arms = kForm == kLbCluster && warp == ndraw && lane == 0;
     for (int j = 0; j < nruns; ++j) {
@@ -731,7 +798,7 @@ LbPlan lb_plan(const LzResidentGeom& g, const LzResidentRule& rule, const std::v
   if (!p.slots) return p;
   const int nslots = p.draw_warps * p.slots;
   p.smem = ((size_t)(rows_max + 1) * p.wn * g.nch * kLbWord + kLbPad + 4 * p.words * g.nch + nslots + 4) * sizeof(uint32_t) +
-           2 * (size_t)nslots * sizeof(uint2);
+           2 * (size_t)lb_ahead(!tinymt, p.form) * nslots * sizeof(uint2);
   const int mode = tinymt ? (params ? kLbTmtParams : kLbTmt) : kLbFast;
   p.kernel = g.nch == 1 ? lb_kernel<1>(p.form, mode, p.slots) : lb_kernel<2>(p.form, mode, p.slots);
   if (p.smem > 200 * 1024 ||
