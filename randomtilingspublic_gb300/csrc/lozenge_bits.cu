@@ -26,7 +26,8 @@
 //
 // What bounds it: the exchange of each run, 0.5 us in a cluster and 0.85 us through L2.  The byte kernel
 // (lozenge_resident.cu) spent its step on the rotation and rebuild of bytes: hexagon 512 0.73 us a step
-// (TinyMT; before 2.20) and 0.91 us (fast mode; 2.14), hexagon 20 0.36 (1.39) and 0.35 (1.36).  It stays for inputs whose edges disagree or whose candidates
+// (TinyMT; before 2.20) and 0.91 us (fast mode; 2.14), hexagon 20 0.36 (1.39) and 0.27 (1.36).  It
+// stays for inputs whose edges disagree or whose candidates
 // border vertices that the reference never rebuilds, and for sizes without a plan here.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -129,7 +130,8 @@ __device__ __forceinline__ void lb_cta_sync() { asm volatile("barrier.sync 0;" :
 constexpr int kLbWord = 12;  // words per (row, word, chain): E0-2, NE0-2, N0-2, three of padding
 constexpr int kLbPad = 3 * kLbWord * 2;
 // Runs that the draw warps are ahead: one, but a period in one CTA in fast mode, where a run is one step of one Philox
-// block's latency: there two blocks go side by side, and only the update warps meet after every step.
+// block's latency: there two blocks go side by side, and only the update warps meet after every step (hexagon 20:
+// 0.35 -> 0.27 us a step, exact sample 5.9 -> 4.0 ms; hexagon 8: 0.15).
 constexpr int lb_ahead(bool fast, int form) { return fast && form == kLbOne ? 8 : 1; }
 
 // KS: words per draw warp.
@@ -697,7 +699,7 @@ void* lb_kernel(LbForm form, int mode, int ks) {
 // (us per step, hexagon of side s, one CTA / cluster / one band per SM; the byte kernel):
 //   TinyMT  s = 12 (23 words) 0.28 / 0.34 / 0.42; 1.39    s = 20 (39) 0.41 / 0.36 / 0.53; 1.39
 //           s = 100 (500) - / 0.45 / 0.57; 1.51           s = 150 (964) - / 0.68 / 0.56; 1.53
-//   fast    s = 28 (55) 0.41 / 0.53 / 0.82; 1.51          s = 56 (120) 0.93 / 0.56 / 0.86; 1.51
+//   fast    s = 28 (55) 0.34 / 0.53 / 0.82; 1.51          s = 56 (120) 0.93 / 0.56 / 0.86; 1.51
 //           s = 150 (964) - / 0.67 / 0.84; 1.47           s = 256 (2300) - / 0.99 / 0.86; 1.56
 // (TinyMT runs of one colour last 1.5 steps, fast-mode runs one.)
 constexpr int lb_one_words(bool tinymt) { return tinymt ? 28 : 79; }
