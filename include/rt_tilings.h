@@ -527,6 +527,11 @@ RT_API rt_status rt_tune_lookup(int32_t model, int32_t n_side, int32_t chains, i
    or store) returns RT_ERR_TIMEOUT, with the CUDA context intact.  Nothing faults. */
 RT_API rt_status rt_dm_sampler_test_silent_band(rt_dm_sampler* s, int32_t band, int64_t max_spin);
 
+/* The same for the calling thread's walks and couplings, which make their own sampler: from now on band `band`
+   publishes nothing in launches [from, from + count) of a resident kernel (counted from this call), and waits
+   give up after max_spin polls.  band < 0 ends it. */
+RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count);
+
 /* ---- allocation-free sweep -------------------------------------------------------------
    No counterpart in the reference.  For callers that cannot allocate device memory (a
    host application that hands the library a fixed device arena up front, or code that must

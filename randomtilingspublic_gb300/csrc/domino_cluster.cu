@@ -711,8 +711,8 @@ ClArgs cl_args(const ClusterEngine& e, DmSampler& s) {
   a.stream = s.opts.fast_stream;
   a.best = e.d_result;
   a.error = e.d_result + 1;
-  a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : 1L << 22;
-  a.silent_cta_plus1 = s.test_silent_band + 1;
+  a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : test_silence().spin(1L << 22);
+  a.silent_cta_plus1 = s.test_silent_band >= 0 ? s.test_silent_band + 1 : test_silence().next_plus1();
   return a;
 }
 

@@ -949,8 +949,12 @@ rt_status GridEngine::prepare(DmSampler& s) {
   ready = false;
   plan.ok = false;
   nch = s.active;
-  bands_asked = s.eff_bands;
   stream = s.stream;
+  int dev = 0, coop = 0;
+  RT_CUDA_G(cudaGetDevice(&dev));
+  RT_CUDA_G(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  RT_CUDA_G(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  bands_max = s.eff_bands > 0 ? std::min(s.eff_bands, sms) : sms;
   const bool fast = s.opts.rng_mode == RT_RNG_FAST;
   if (s.opts.rng_mode == RT_RNG_MTGP || (nch != 1 && nch != 2)) {
     plan.why = "TinyMT or fast mode with 1 or 2 swept chains";
@@ -968,15 +972,10 @@ rt_status GridEngine::prepare(DmSampler& s) {
       return RT_OK;
     }
   }
-  int dev = 0, sms = 0, coop = 0;
-  RT_CUDA_G(cudaGetDevice(&dev));
-  RT_CUDA_G(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  RT_CUDA_G(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (!coop) {
     plan.why = "device lacks cooperative launch";
     return RT_OK;
   }
-  const int bands_max = s.eff_bands > 0 ? std::min(s.eff_bands, sms) : sms;
   const int deep_bands = s.couple ? std::max(1, sms / kGrTeams) : bands_max;
   plan.depth = 1;
   plan.build(s.cand_lo, s.cand_hi, s.N, nch, fast, bands_max);
@@ -1034,8 +1033,8 @@ GrArgs gr_args(const GridEngine& e, DmSampler& s) {
   a.stream = s.opts.fast_stream;
   a.xbuf = e.d_xbuf;
   a.error = e.d_rows + 3 * kGrMaxBands + 1;
-  a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : 1L << 22;
-  a.silent_band_plus1 = s.test_silent_band + 1;
+  a.max_spin = s.test_max_spin > 0 ? s.test_max_spin : test_silence().spin(1L << 22);
+  a.silent_band_plus1 = s.test_silent_band >= 0 ? s.test_silent_band + 1 : test_silence().next_plus1();
   return a;
 }
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -37,7 +38,7 @@ struct GrPlan {
 struct GridEngine {
   GrPlan plan;
   bool ready = false;
-  int nch = 0, bands_asked = 0;
+  int nch = 0, bands_max = 0, sms = 0;  // the plan's most bands: those asked for, else the device's SMs
   void* kernel = nullptr;
   cudaStream_t stream = nullptr;
   int* d_rows = nullptr;       // the plan's row_start and windows, then the error word
@@ -52,6 +53,8 @@ struct GridEngine {
 
   ~GridEngine();
   rt_status prepare(DmSampler& s);
+  // Is this the plan for `asked` bands (0: one per SM)?
+  bool serves(int asked) const { return bands_max == (asked > 0 ? std::min(asked, sms) : sms); }
   rt_status launch(DmSampler& s, const uint8_t* colours_host, int64_t steps, uint64_t fast_seed, int64_t h0);
   // As RunEngine::cftp, attempts [a0, a0 + n) side by side (n <= kGrTeams), where depth > 1.
   rt_status cftp(DmSampler& s, int a0, int n, const std::vector<std::vector<RunEngine::Epoch>>& epochs,

@@ -585,14 +585,24 @@ rt_status DmSampler::use_persistent(bool* yes) {
       return fail(RT_ERR_INVALID_ARGUMENT, "persistent engine needs consistent loaded tilings");
     return RT_OK;
   }
+  // An engine goes with its error word read: a wait of its launches that gave up is reported by the
+  // run after, not lost with the engine.
+  rt_status lost = RT_OK;
+  auto retire = [&](auto& engine_ptr) {
+    if (!engine_ptr) return;
+    if (rt_status st = engine_ptr->check_error(*this)) lost = st;
+    engine_ptr.reset();
+  };
   if (plan_dirty) {
-    cluster.reset();
-    grid.reset();
-    bits.reset();
-    runs.reset();
-    persist.reset();
+    retire(cluster);
+    retire(grid);
+    retire(bits);
+    retire(runs);
+    retire(persist);
+    not_deep = 0;
+    plan_dirty = false;
+    if (lost) return lost;
   }
-  plan_dirty = false;
   // The bit-plane kernel in one thread-block cluster: where 1..16 bands are asked for (they are
   // the cluster's CTAs), or automatically up to the size at which more SMs pay for the slower
   // exchange (cl_auto_words).  A table entry that asks for it gives way to the next where the
@@ -600,7 +610,8 @@ rt_status DmSampler::use_persistent(bool* yes) {
   const bool fast = opts.rng_mode == RT_RNG_FAST;
   // With an exchange every few runs one band per SM is faster than a cluster (domino_grid.cu).
   auto try_grid = [&](bool deep_only) -> rt_status {
-    if (grid && (grid->nch != active || grid->bands_asked != eff_bands)) grid.reset();
+    if (grid && (grid->nch != active || !grid->serves(eff_bands))) retire(grid);
+    if (lost) return lost;
     if (!grid) {
       grid = std::make_unique<GridEngine>();
       if (rt_status st = grid->prepare(*this)) return st;
@@ -611,13 +622,17 @@ rt_status DmSampler::use_persistent(bool* yes) {
     *yes = true;
     return RT_OK;
   };
-  if (!explicit_engine && (engine == 0 || engine == 4) && (eff_bands == 0 || eff_bands > kClMaxCtas)) {
+  // (A coupling asks once: its table entry may want other bands of the grid below.)
+  if (!explicit_engine && (engine == 0 || engine == 4) && (eff_bands == 0 || eff_bands > kClMaxCtas) &&
+      !(couple && not_deep == active)) {
     if (rt_status st = try_grid(true)) return st;
     if (on_grid) return RT_OK;
+    not_deep = active;
   }
   for (int skip = 0; (engine == 0 || (engine == 4 && !(fast && explicit_engine))) && eff_bands <= kClMaxCtas &&
                      (eff_bands > 0 || engine == 0);) {
-    if (cluster && (cluster->nch != active || cluster->bands_asked != eff_bands)) cluster.reset();
+    if (cluster && (cluster->nch != active || cluster->bands_asked != eff_bands)) retire(cluster);
+    if (lost) return lost;
     if (!cluster) {
       cluster = std::make_unique<ClusterEngine>();
       if (rt_status st = cluster->prepare(*this)) return st;
@@ -642,9 +657,10 @@ rt_status DmSampler::use_persistent(bool* yes) {
   // kernel alone; 2: the run kernel, else k_persist; 3: k_persist alone.
   if ((runs && (runs->nch != active || runs->bands_asked != eff_bands || runs->threads_asked != eff_threads)) ||
       (persist && persist->nch != active) || (bits && bits->nch != active)) {
-    bits.reset();
-    runs.reset();
-    persist.reset();
+    retire(bits);
+    retire(runs);
+    retire(persist);
+    if (lost) return lost;
   }
   if (engine == 1) return RT_OK;
   std::string why;

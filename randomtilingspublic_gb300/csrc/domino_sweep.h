@@ -90,6 +90,7 @@ struct DmSampler {
   bool in_cluster = false;  // resident 4: in one thread-block cluster (cluster),
   bool on_grid = false;     // or on every SM (grid), else bits
   bool couple = false;      // coupling from the past: attempts side by side
+  int not_deep = 0;         // the swept chains that k_deep was found not to hold
   int last_engine = 0;  // engine of the last run: 1 per-half-sweep kernels, 2-4 as resident
   // Launch shape: an explicit choice (rt_dm_sampler_set_launch; 0 = none), and the shape in
   // force, from that choice, else the autotuner's table, else the defaults (0).

@@ -11,6 +11,11 @@ thread_local std::string g_last_error;
 }
 void set_error(const std::string& msg) { g_last_error = msg; }
 void clear_error() { g_last_error.clear(); }
+
+TestSilence& test_silence() {
+  static thread_local TestSilence t;
+  return t;
+}
 }  // namespace rt
 
 extern "C" {
@@ -40,6 +45,18 @@ RT_API const char* rt_status_string(rt_status s) {
 }
 
 RT_API const char* rt_last_error(void) { return rt::g_last_error.c_str(); }
+
+RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count) {
+  rt::clear_error();
+  if (max_spin < 0 || from < 0 || count < 0) return rt::fail(RT_ERR_INVALID_ARGUMENT, "test_silent_band: negative argument");
+  rt::TestSilence t;
+  t.band = band < 0 ? -1 : band;
+  t.max_spin = (long)max_spin;
+  t.from = from;
+  t.count = count;
+  rt::test_silence() = t;
+  return RT_OK;
+}
 
 RT_API const char* rt_version(void) { return "rt_tilings 0.1 (sm_103a)"; }
 

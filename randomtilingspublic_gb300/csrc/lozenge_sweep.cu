@@ -403,7 +403,12 @@ struct LzSampler {
   rt_status resident(LzResidentState** out) {
     *out = nullptr;
     if (opts.engine == 1 || opts.rng_mode == RT_RNG_MTGP) return RT_OK;
-    if (!res || res_nch != active) {
+    if (res && res_nch != active) {
+      const rt_status st = lz_resident_error(*res, stream);
+      res.reset();
+      if (st) return st;
+    }
+    if (!res) {
       res = std::make_unique<LzResidentState>();
       res->plan = lz_resident_plan(geom(), opts.rng_mode == RT_RNG_TINYMT);
       res_nch = active;
@@ -426,6 +431,11 @@ struct LzSampler {
   rt_status bit_engine(LbState** out) {
     *out = nullptr;
     if (opts.engine != 0 || opts.rng_mode == RT_RNG_MTGP || !consistent || border) return RT_OK;
+    if (bits && (cand_dirty || bits->nch != active)) {  // it goes with its error word read
+      const rt_status st = lb_error(*bits, stream);
+      bits.reset();
+      if (st) return st;
+    }
     if (cand_dirty) {
       std::vector<int> both(2 * (size_t)N);
       LZ_CUDA(cudaMemcpyAsync(both.data(), d_cand, both.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -434,9 +444,8 @@ struct LzSampler {
       cand_hi.assign(both.begin() + N, both.end());
       for (int& v : cand_lo) v = v == INT_MAX ? -1 : v;
       cand_dirty = false;
-      bits.reset();
     }
-    if (!bits || bits->nch != active) {
+    if (!bits) {
       bits = std::make_unique<LbState>();
       bits->nch = active;
       bits->plan = lb_plan(geom(), LzResidentRule{rule.lo_up, rule.w_up, rule.lo_dn, rule.w_dn}, cand_lo, cand_hi,

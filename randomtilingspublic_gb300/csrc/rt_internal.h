@@ -29,6 +29,22 @@ inline rt_status dev_alloc(T** p, size_t bytes, cudaStream_t s) {
   return st;
 }
 
+// Test hook of the bounded waits (rt_test_silent_band), of the calling thread: in its launches [from, from + count)
+// of a resident kernel band `band` publishes nothing, and every wait gives up after max_spin polls (0: the default).
+struct TestSilence {
+  int band = -1, from = 0, count = 0;
+  long max_spin = 0;
+  // Of the launch that asks: the silent band plus 1, 0 for none.
+  int next_plus1() {
+    if (band < 0) return 0;
+    const int at = launch++;
+    return at >= from && at - from < count ? band + 1 : 0;
+  }
+  long spin(long usual) const { return band >= 0 && max_spin > 0 ? max_spin : usual; }
+  int launch = 0;
+};
+TestSilence& test_silence();
+
 // cuRAND MTGP32 generators in the reference's CUDA geometry (domino_mtgp.cu): 8 x 8 thread
 // blocks over a rows x cols grid of sites (row from the x index, column from the y index),
 // block (bx, by) drawing from generator bx * gy + by.
