@@ -622,6 +622,11 @@ void ClPlan::build(const std::vector<int>& lo, const std::vector<int>& hi, int N
   update_warps = (items + 32 * per_lane - 1) / (32 * per_lane);
   smem_bytes = ((size_t)(rows_max + 1) * 4 * wn * nch + kClPad) * sizeof(uint32_t) +
                3 * (size_t)draw_warps * slots * sizeof(uint2);
+  // Every CTA's window spans all the domain's words, so a long bent domain of few words a row needs much of it.
+  if (smem_bytes > kClMaxSmem) {
+    why = "band window exceeds shared memory";
+    return;
+  }
   ok = true;
 }
 
@@ -662,8 +667,13 @@ rt_status ClusterEngine::prepare(DmSampler& s) {
   if (!plan.ok) return RT_OK;
   const int mode = fast ? kClFast : (s.tmt_params ? kClTmtParams : kClTmt);
   kernel = nch == 1 ? cl_kernel<1>(mode, plan.slots, plan.per_lane) : cl_kernel<2>(mode, plan.slots, plan.per_lane);
-  RT_CUDA_C(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
-  RT_CUDA_C(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    plan.ok = false;
+    plan.why = "the device does not allow the launch";
+    return RT_OK;
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

@@ -15,6 +15,7 @@ namespace rt {
 struct DmSampler;
 
 constexpr int kClMaxCtas = 16;   // CTAs of the cluster
+constexpr size_t kClMaxSmem = 200 * 1024;  // dynamic shared memory of a CTA, at most
 constexpr int kClUpdateWarps = 8;  // warps that update the words, at most
 // Threads per CTA, at most: 64 registers a thread, 80 where the generators of 8 words need them.
 constexpr int cl_max_threads(bool fast, int slots) { return !fast && slots > 4 ? 768 : 1024; }
