@@ -666,7 +666,7 @@ RT_API rt_status rt_cftp_batch(rt_cftp_instance* inst, int32_t count, void* cuda
     const uint32_t c4 = (uint32_t)std::ceil(0.4 * 4294967296.0), c8 = (uint32_t)std::ceil(0.8 * 4294967296.0);
     cudaEventRecord(e0, stream);
     if (n_small > 0) {
-      cudaFuncSetAttribute(k_batch_cftp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+      dev_allow_smem((const void*)k_batch_cftp, smem_max);
       int per_sm = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_cftp, kBatchThreads, smem_max);
       // Few instances: the SMs left over run attempts ahead of the instances' own CTAs (one hexagon of side 32:
@@ -871,7 +871,7 @@ RT_API rt_status rt_server_create(const rt_server_opts* o, rt_server** out) {
     s->own_stream = true;
   }
   BT_CUDA(cudaEventCreateWithFlags(&s->ev_exit, cudaEventDisableTiming));
-  BT_CUDA(cudaFuncSetAttribute(k_serve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem));
+  BT_CUDA(dev_allow_smem((const void*)k_serve, s->smem));
   int per_sm = 0;
   BT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_serve, kBatchThreads, s->smem));
   s->grid = std::max(1, per_sm) * sms;

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 
 rt_status set_cluster_attrs(size_t smem) {
   if (cudaFuncSetAttribute(k_batch_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(k_batch_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+      dev_allow_smem((const void*)k_batch_cluster, smem) != cudaSuccess) {
     const cudaError_t e = cudaGetLastError();
     return fail(RT_ERR_CUDA, std::string("cftp_batch: cluster kernel attributes: ") + cudaGetErrorString(e));
   }

@@ -662,7 +662,7 @@ TdClPlan td_plan_of(const TdScan& sc, bool fast, bool params, int bands, int dep
   p.kernel = td_kernel(fast, params, p.K);
   int per_sm = 0;
   if (p.smem > 200 * 1024 ||
-      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      dev_allow_smem(p.kernel, p.smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.threads, p.smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return p;

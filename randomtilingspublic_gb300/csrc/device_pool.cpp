@@ -5,8 +5,11 @@
 // synchronisation.  Blocks are allocated and freed in the order of the stream that uses them.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 
 #include "rt_internal.h"
 
@@ -60,6 +63,25 @@ rt_status dev_alloc(void** p, size_t bytes, cudaStream_t s) {
                 std::string("device allocation: ") + cudaGetErrorString(e));
   }
   return RT_OK;
+}
+
+cudaError_t dev_allow_smem(const void* kernel, size_t bytes) {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limits;
+  std::lock_guard<std::mutex> lock(mu);
+  auto at = limits.find({dev, kernel});
+  if (at == limits.end()) {
+    cudaFuncAttributes a{};
+    if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+    if ((e = cudaFuncGetAttributes(&a, kernel)) != cudaSuccess) return e;
+    const size_t limit = (size_t)optin - std::min((size_t)optin, a.sharedSizeBytes);
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit)) != cudaSuccess) return e;
+    at = limits.emplace(std::make_pair(dev, kernel), limit).first;
+  }
+  return bytes <= at->second ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 void dev_free(void* p, cudaStream_t s) {

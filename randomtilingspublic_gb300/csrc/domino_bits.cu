@@ -849,7 +849,7 @@ rt_status BitEngine::prepare(DmSampler& s) {
     plan.why = "no bit-plane kernel for this chain count";
     return RT_OK;
   }
-  RT_CUDA_B(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
+  RT_CUDA_B(dev_allow_smem(kernel, plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_B(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, plan.warps * 32, plan.smem_bytes));
   if ((int64_t)per_sm * sms < (int64_t)plan.bands.size()) {

@@ -667,7 +667,7 @@ rt_status ClusterEngine::prepare(DmSampler& s) {
   if (!plan.ok) return RT_OK;
   const int mode = fast ? kClFast : (s.tmt_params ? kClTmtParams : kClTmt);
   kernel = nch == 1 ? cl_kernel<1>(mode, plan.slots, plan.per_lane) : cl_kernel<2>(mode, plan.slots, plan.per_lane);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes) != cudaSuccess ||
+  if (dev_allow_smem(kernel, plan.smem_bytes) != cudaSuccess ||
       cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     plan.ok = false;

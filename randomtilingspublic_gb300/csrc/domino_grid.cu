@@ -987,7 +987,7 @@ rt_status GridEngine::prepare(DmSampler& s) {
   }
   kernel = plan.depth > 1 ? (nch == 1 ? gr_deep_kernel<1>(mode, plan.slots) : gr_deep_kernel<2>(mode, plan.slots))
                           : gr_kernel(nch, mode, plan.slots, plan.per_lane);
-  RT_CUDA_G(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
+  RT_CUDA_G(dev_allow_smem(kernel, plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_G(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, plan.threads(), plan.smem_bytes));
   if ((int64_t)per_sm * sms < plan.bands * (s.couple && plan.depth > 1 ? kGrTeams : 1)) {

@@ -121,7 +121,7 @@ extern "C" RT_API rt_status rt_dm_sweep_noalloc(uint8_t* dev_chains, void* dev_g
     return st;
   if (!plan.ok) return fail(RT_ERR_INVALID_ARGUMENT, "sweep_noalloc: " + plan.why);
   void* kernel = dm_persist_kernel_ptr(o.rng_mode, plan.K, false, n_chains, false);
-  NOALLOC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
+  NOALLOC_CUDA(dev_allow_smem(kernel, plan.smem_bytes));
   int per_sm = 0;
   NOALLOC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPersistThreads, plan.smem_bytes));
   const int nbands = (int)plan.bands.size();

@@ -645,7 +645,7 @@ rt_status PersistEngine::prepare(DmSampler& s) {
     return RT_OK;
   }
   kernel = dm_persist_kernel_ptr(s.opts.rng_mode, plan.K, params, s.active, true);
-  RT_CUDA_P(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
+  RT_CUDA_P(dev_allow_smem(kernel, plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_P(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, plan.smem_bytes));
   if ((int64_t)per_sm * sms < (int64_t)plan.bands.size()) {

@@ -883,7 +883,7 @@ rt_status RunEngine::prepare(DmSampler& s) {
     plan.why = "no run kernel for this mode";
     return RT_OK;
   }
-  RT_CUDA_R(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem_bytes));
+  RT_CUDA_R(dev_allow_smem(kernel, plan.smem_bytes));
   int per_sm = 0;
   RT_CUDA_R(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, plan.threads, plan.smem_bytes));
   if ((int64_t)per_sm * sms < (int64_t)plan.bands.size()) {

@@ -804,7 +804,7 @@ LbPlan lb_plan(const LzResidentGeom& g, const LzResidentRule& rule, const std::v
   const int mode = tinymt ? (params ? kLbTmtParams : kLbTmt) : kLbFast;
   p.kernel = g.nch == 1 ? lb_kernel<1>(p.form, mode, p.slots) : lb_kernel<2>(p.form, mode, p.slots);
   if (p.smem > 200 * 1024 ||
-      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      dev_allow_smem(p.kernel, p.smem) != cudaSuccess ||
       (p.form == kLbCluster &&
        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
     cudaGetLastError();

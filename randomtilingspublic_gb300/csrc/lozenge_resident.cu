@@ -294,7 +294,7 @@ LzResidentPlan lz_resident_plan(const LzResidentGeom& g, bool tinymt) {
   const size_t smem = (size_t)g.nch * 3 * (rows_max + 2) * g.P;
   if (smem > (size_t)optin - 1024) return p;
   void* kern = kernel_for(tinymt, std::max(1, K), g.nch);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (dev_allow_smem(kern, smem) != cudaSuccess) {
     cudaGetLastError();
     return p;
   }

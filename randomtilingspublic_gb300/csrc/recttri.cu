@@ -702,7 +702,7 @@ RtClPlan rt_cluster_plan(const int* lo, const int* hi, int N, int Np, bool fast,
   p.smem = (size_t)2 * (rows_max + 1) * Np + (size_t)(rows_max + 1) * sizeof(int) + (fast ? (size_t)units * 4 : 0) + 16;
   p.kernel = rt_cluster_kernel(fast, params, p.K);
   if (p.smem > 200 * 1024 ||
-      cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      dev_allow_smem(p.kernel, p.smem) != cudaSuccess ||
       cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return p;

@@ -29,6 +29,11 @@ inline rt_status dev_alloc(T** p, size_t bytes, cudaStream_t s) {
   return st;
 }
 
+// Lets launches of `kernel` on the current device ask for `bytes` of dynamic shared memory.  The limit is the
+// kernel's own attribute, shared by all threads and samplers, so it is set once, to all the device allows: a plan
+// that set it to its own bytes would have the launches of larger plans refused.
+cudaError_t dev_allow_smem(const void* kernel, size_t bytes);
+
 // Test hook of the bounded waits (rt_test_silent_band), of the calling thread: in its launches [from, from + count)
 // of a resident kernel band `band` publishes nothing, and every wait gives up after max_spin polls (0: the default).
 struct TestSilence {

@@ -745,7 +745,7 @@ SvBandPlan sv_band_plan(const SvGeom& G, int chains, const std::vector<uint32_t>
   p.kernel = chains == 1 ? (p.sum ? (void*)k_sv_bands<1, true> : (void*)k_sv_bands<1, false>)
                          : (p.sum ? (void*)k_sv_bands<2, true> : (void*)k_sv_bands<2, false>);
   int per_sm = 0;
-  if (cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+  if (dev_allow_smem(p.kernel, p.smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.threads, p.smem) != cudaSuccess) {
     cudaGetLastError();
     return p;
