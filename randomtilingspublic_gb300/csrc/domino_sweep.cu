@@ -541,11 +541,13 @@ rt_status DmSampler::accumulate_heights(int ch, long long* sums, int32_t* height
   k_merge<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(v, ch, scratch);
   launches++;
   if (rt_status st = check_launch()) return st;
-  int32_t* const h = heights ? heights : d_h;
-  if (rt_status st = dm_heights_device(scratch, d_hf, N, hf_start, h, d_hflags, stream)) return st;
+  if (rt_status st = dm_heights_device(scratch, d_hf, N, hf_start, d_h, d_hflags, stream)) return st;
   if (sums) {
-    if (rt_status st = dm_heights_accumulate(h, N, sums, stream)) return st;
+    if (rt_status st = dm_heights_accumulate(d_h, N, sums, stream)) return st;
   }
+  // The caller's buffer is written once, when the heights are whole (4 us of copy at order 1024); it may lie at any
+  // address that a copy takes.
+  if (heights) RT_CUDA(cudaMemcpyAsync(heights, d_h, (size_t)N * N * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
   return RT_OK;
 }
 
