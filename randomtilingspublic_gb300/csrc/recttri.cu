@@ -909,29 +909,29 @@ RT_API rt_status rt_recttri_walk(int32_t* tiling, int32_t n_side, int64_t steps,
   const int N = n_side, M = N / 3, P = (M + 3) / 4 * 4;
   const RtWeights W = make_weights(weights9);
   cudaStream_t stream = (cudaStream_t)o.cuda_stream;
-  if (o.rng_mode != RT_RNG_MTGP && steps > 0) {
+  // The cluster kernel's set-up (packing, a wait for the candidates, a plan) is longer than what a few steps take on a
+  // small array (us a call, fast mode, per-step kernels / cluster kernel: N = 12, 1 step 36 / 66, 7 steps 64 / 66; N = 48,
+  // 1 step 44 / 72, 7 steps 74 / 72; N = 93, 1 step 68 / 90, 4 steps 87 / 90; N = 144 the cluster at any number).
+  const bool few = steps < (N <= 48 ? 8 : N <= 96 ? 4 : 0);
+  if (o.rng_mode != RT_RNG_MTGP && steps > 0 && !few) {
     bool done = false;
     if (rt_status st = rt_cluster_walk(tiling, N, steps, seed, W, o, stream, &done)) return st;
     if (done) return RT_OK;
   }
-  int32_t *base = nullptr, *scratch = nullptr;
+  int32_t* base = nullptr;
   uint4 *tmt = nullptr, *tmt_params = nullptr;
   void* mtgp = nullptr;
   const MtgpGrid mg = mtgp_grid(N, M);
   auto cleanup = [&]() {
-    if (base) cudaFree(base);
-    if (scratch) cudaFree(scratch);
-    if (tmt) cudaFree(tmt);
+    for (void* p : {(void*)base, (void*)tmt, mtgp}) dev_free(p, stream);
     if (tmt_params) cudaFree(tmt_params);
-    if (mtgp) cudaFree(mtgp);
   };
   const size_t cs = (size_t)N * P;
   rt_status status = RT_OK;
   do {
-    if (cudaMalloc(&base, 3 * cs * sizeof(int32_t)) != cudaSuccess || cudaMalloc(&scratch, (size_t)N * N * sizeof(int32_t)) != cudaSuccess ||
-        (o.rng_mode == RT_RNG_TINYMT && cudaMalloc(&tmt, (size_t)N * M * sizeof(uint4)) != cudaSuccess) ||
-        (o.rng_mode == RT_RNG_MTGP && cudaMalloc(&mtgp, mtgp_state_bytes(mg.count())) != cudaSuccess)) {
-      cudaGetLastError();
+    if (dev_alloc(&base, 3 * cs * sizeof(int32_t), stream) ||
+        (o.rng_mode == RT_RNG_TINYMT && dev_alloc(&tmt, (size_t)N * M * sizeof(uint4), stream)) ||
+        (o.rng_mode == RT_RNG_MTGP && dev_alloc(&mtgp, mtgp_state_bytes(mg.count()), stream))) {
       status = fail(RT_ERR_OUT_OF_MEMORY, "recttri walk: device allocation failed");
       break;
     }
