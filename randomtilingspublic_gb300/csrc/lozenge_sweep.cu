@@ -211,6 +211,12 @@ __global__ void k_lz_scan(const int32_t* t, int N, int* cand, unsigned long long
   if (threadIdx.x < 3 && inside[threadIdx.x]) atomicAdd(&scan[1 + threadIdx.x], (unsigned long long)inside[threadIdx.x]);
 }
 
+// No candidates yet.
+__global__ void k_lz_scan_init(int* cand, int N) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < 2 * N) cand[k] = k < N ? INT_MAX : -1;
+}
+
 __global__ void k_lz_split(LzView v, int ch, const int32_t* t) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
   if (j >= v.N) return;
@@ -318,15 +324,18 @@ struct LzSampler {
   std::unique_ptr<LzResidentState> res;  // the resident engine for `res_nch` swept chains
   int res_nch = 0;
   std::unique_ptr<LbState> bits;  // the bit-plane engine for its nch swept chains
-  int* d_cand = nullptr;          // [2][N]: first (INT_MAX: none) and last slot that can flip, over the loaded chains
+  // The scan's flags and counts, then `counter`, then d_cand: one copy brings them to the host after a load.
   unsigned long long* d_scan = nullptr;
+  int* d_cand = nullptr;          // [2][N]: first (INT_MAX: none) and last slot that can flip, over the loaded chains
+  static constexpr int kScanWords = 6;
+  std::vector<unsigned long long> scanned;  // d_scan's block after the last load
   bool consistent = true, border = false, cand_dirty = true;
   std::vector<int> cand_lo, cand_hi;
 
   ~LzSampler() {
     res.reset();
     bits.reset();
-    for (void* p : {(void*)base, (void*)tmt, mtgp, (void*)scratch, (void*)counter, (void*)d_cand, (void*)d_scan})
+    for (void* p : {(void*)base, (void*)tmt, mtgp, (void*)scratch, (void*)d_scan})
       dev_free(p, stream);
     if (tmt_params) cudaFree(tmt_params);
     if (ev0) cudaEventDestroy(ev0);
@@ -373,20 +382,14 @@ struct LzSampler {
       LZ_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
       s->own_stream = true;
     }
-    LZ_CUDA(cudaEventCreate(&s->ev0));
-    LZ_CUDA(cudaEventCreate(&s->ev1));
     // pool allocations, ordered on the sampler's stream (device_pool.cpp)
     if (rt_status st = dev_alloc(&s->base, s->chain_stride * chains, s->stream)) return st;
     LZ_CUDA(cudaMemsetAsync(s->base, 0, s->chain_stride * chains, s->stream));
     if (rt_status st = dev_alloc(&s->scratch, (size_t)s->N * s->N * sizeof(int32_t), s->stream)) return st;
-    if (rt_status st = dev_alloc(&s->counter, sizeof(unsigned long long), s->stream)) return st;
-    if (rt_status st = dev_alloc(&s->d_scan, 4 * sizeof(unsigned long long), s->stream)) return st;
-    if (rt_status st = dev_alloc(&s->d_cand, 2 * (size_t)s->N * sizeof(int), s->stream)) return st;
-    {
-      std::vector<int> init(2 * (size_t)s->N, -1);
-      std::fill(init.begin(), init.begin() + s->N, INT_MAX);
-      LZ_CUDA(cudaMemcpyAsync(s->d_cand, init.data(), init.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
-    }
+    if (rt_status st = dev_alloc(&s->d_scan, (kScanWords + (size_t)s->N) * sizeof(unsigned long long), s->stream)) return st;
+    s->counter = s->d_scan + 4;
+    s->d_cand = reinterpret_cast<int*>(s->d_scan + kScanWords);
+    k_lz_scan_init<<<(2 * s->N + 255) / 256, 256, 0, s->stream>>>(s->d_cand, s->N);
     if (o.rng_mode == RT_RNG_TINYMT) {
       if (rt_status st = dev_alloc(&s->tmt, (size_t)s->N * s->M * sizeof(uint4), s->stream)) return st;
       if (rt_status st = tmt_param_table(o, (int64_t)s->N * s->M, &s->tmt_params, s->stream)) return st;
@@ -437,11 +440,10 @@ struct LzSampler {
       if (st) return st;
     }
     if (cand_dirty) {
-      std::vector<int> both(2 * (size_t)N);
-      LZ_CUDA(cudaMemcpyAsync(both.data(), d_cand, both.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      LZ_CUDA(cudaStreamSynchronize(stream));
-      cand_lo.assign(both.begin(), both.begin() + N);
-      cand_hi.assign(both.begin() + N, both.end());
+      if (scanned.empty()) return RT_OK;  // nothing loaded
+      const int* both = reinterpret_cast<const int*>(scanned.data() + kScanWords);
+      cand_lo.assign(both, both + N);
+      cand_hi.assign(both + N, both + 2 * N);
       for (int& v : cand_lo) v = v == INT_MAX ? -1 : v;
       cand_dirty = false;
     }
@@ -463,9 +465,10 @@ struct LzSampler {
     LZ_CUDA(cudaMemcpyAsync(scratch, t, (size_t)N * N * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
     LZ_CUDA(cudaMemsetAsync(d_scan, 0, 4 * sizeof(unsigned long long), stream));
     k_lz_scan<<<dim3((N + 255) / 256, N), 256, 0, stream>>>(scratch, N, d_cand, d_scan, ch == 0);
-    unsigned long long h[4] = {0, 0, 0, 0};
-    LZ_CUDA(cudaMemcpyAsync(h, d_scan, sizeof h, cudaMemcpyDeviceToHost, stream));
+    scanned.resize(kScanWords + (size_t)N);
+    LZ_CUDA(cudaMemcpyAsync(scanned.data(), d_scan, scanned.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     LZ_CUDA(cudaStreamSynchronize(stream));
+    const unsigned long long* h = scanned.data();
     if (h[0] & 1u) return fail(RT_ERR_INVALID_ARGUMENT, "lozenge tiling values must be edge masks in [0, 63]");
     consistent = consistent && !(h[0] & 2u);
     border = border || (h[0] & 4u);
@@ -663,6 +666,8 @@ RT_API rt_status rt_lozenge_cftp(const int32_t* tmax, const int32_t* tmin, int32
   if (rt_status st = s->copy_chain(2, 0)) return st;
   if (rt_status st = s->load(3, tmax)) return st;
   s->active = 2;
+  LZ_CUDA(cudaEventCreate(&s->ev0));
+  LZ_CUDA(cudaEventCreate(&s->ev1));
   const bool fast = o.rng_mode == RT_RNG_FAST;
   // Epoch k is created by attempt k with the driver's k-th draw as its seed; attempt a runs epochs a, a-1, ..., 0,
   // each one reference Walk(t, steps_k, seed_k) on both chains.

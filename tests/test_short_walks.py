@@ -24,3 +24,18 @@ def test_recttri(rt, orc, side, steps, mode):
         orc.rt_walk_tinymt(want, n, steps, 11, None)
     tiler.Walk(got, steps, 11)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("mode", ["tinymt", "fast"])
+@pytest.mark.parametrize("side", [1, 2, 9, 30, 60])
+@pytest.mark.parametrize("steps", [0, 1, 2, 9])
+def test_lozenge(rt, orc, side, steps, mode):
+    L = rt.LozengeTiler
+    start = L.MinTiling(L.Hexagon(side))
+    got, want = start.copy(), start.copy()
+    if mode == "fast":
+        orc.lz_walk_fast(want, rt.side_of(start), 0, steps, 11, 7)
+    else:
+        orc.lz_walk_tinymt(want, rt.side_of(start), steps, 11)
+    L(rng=mode, fast_stream=7).Walk(got, steps, 11)
+    assert np.array_equal(got, want)
