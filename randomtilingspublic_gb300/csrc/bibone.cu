@@ -546,6 +546,13 @@ struct TdScan {
   unsigned long long by_residue[36];
 };
 
+inline TdScan td_no_scan(int M) {
+  TdScan scan{};
+  scan.row_lo = scan.col_lo = M;
+  scan.row_hi = scan.col_hi = -1;
+  return scan;
+}
+
 __device__ __forceinline__ uint32_t td_byte(const int32_t* t, int N, int M, int a, int b) {
   if (a < 0 || b < 0 || a >= M || b >= M) return 0u;
   const int eR = t[(size_t)(2 * a + 1) * N + 2 * b + 1], eH = t[(size_t)(2 * a) * N + 2 * b + 1];
@@ -772,17 +779,41 @@ std::vector<int> td_cover(const uint8_t* D, int M) {
   return c;
 }
 
-// The checks of k_td_pack on the host, for an input refused before a missing device is.
-rt_status td_check_host(const int32_t* tiling, int N) {
+// Side of the vertex array up to which a walk's conversions are made on the host: two launches, a wait and two pool
+// blocks less, 10 ns a vertex more (walk of one step, fast mode, host / device: side 10 47 / 74 us, 46 72 / 81, 70
+// 115 / 106, 106 169 / 110).
+constexpr int kTdHostSide = 48;
+
+// k_td_pack on the host.
+TdScan td_pack_host(const int32_t* tiling, int N, std::vector<uint8_t>* bytes) {
   const int M = N / 2;
-  std::vector<uint8_t> D((size_t)M * M);
+  std::vector<uint8_t>& D = *bytes;
+  D.resize((size_t)M * M);
   td_from_tiling(tiling, N, D.data());
+  TdScan scan = td_no_scan(M);
   std::vector<int32_t> back(tiling, tiling + (size_t)N * N);
   td_to_tiling(D.data(), N, back.data());
-  if (!std::equal(back.begin(), back.end(), tiling))
+  if (!std::equal(back.begin(), back.end(), tiling)) scan.flags |= 1u;
+  const std::vector<int> cover = td_cover(D.data(), M);
+  for (int a = 0; a < M; ++a)
+    for (int b = 0; b < M; ++b) {
+      const uint8_t v = D[(size_t)a * M + b];
+      if ((a == 0 && (v & (kL | kR))) || (b == M - 1 && (v & (kH | kR)))) scan.flags |= 4u;
+      if (!cover[(size_t)a * M + b]) continue;
+      if (cover[(size_t)a * M + b] > 1) scan.flags |= 2u;
+      scan.row_lo = std::min(scan.row_lo, a);
+      scan.row_hi = std::max(scan.row_hi, a);
+      scan.col_lo = std::min(scan.col_lo, b);
+      scan.col_hi = std::max(scan.col_hi, b);
+      ++scan.by_residue[(a % 6) * 6 + b % 6];
+    }
+  return scan;
+}
+
+rt_status td_check(const TdScan& scan) {
+  if (scan.flags & 1u)
     return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: tiling states are not those of a dimer configuration");
-  for (int v : td_cover(D.data(), M))
-    if (v > 1) return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: two dimers share a vertex");
+  if (scan.flags & 2u) return fail(RT_ERR_INVALID_ARGUMENT, "bibone walk: two dimers share a vertex");
   return RT_OK;
 }
 
@@ -1026,7 +1057,8 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   int devs = 0;
   if (cudaGetDeviceCount(&devs) != cudaSuccess || devs == 0) {
     cudaGetLastError();
-    if (rt_status cs = td_check_host(tiling, N)) return cs;
+    std::vector<uint8_t> bytes;
+    if (rt_status cs = td_check(td_pack_host(tiling, N, &bytes))) return cs;  // an input is refused before a missing device
     return fail(RT_ERR_CUDA, "no CUDA device: the sweep has no CPU fallback");
   }
   cudaStream_t st = (cudaStream_t)o.cuda_stream;
@@ -1050,26 +1082,35 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
     cleanup();
     return fail(RT_ERR_OUT_OF_MEMORY, "bibone walk: device allocation failed");
   };
-  if (dev_alloc(&d_t, cells * sizeof(int32_t), st) || dev_alloc(&dD, (size_t)M * M, st) ||
-      dev_alloc(&d_scan, sizeof(TdScan), st))
-    return out_of_memory();
-  TdScan scan{};
-  scan.row_lo = scan.col_lo = M;
-  scan.row_hi = scan.col_hi = -1;
-  cudaMemcpyAsync(d_t, tiling, cells * sizeof(int32_t), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_scan, &scan, sizeof scan, cudaMemcpyHostToDevice, st);
+  TdScan scan = td_no_scan(M);
+  std::vector<uint8_t> bytes;
   const dim3 g_all((M + 127) / 128, M), g_quad(((M + 3) / 4 + 31) / 32, (M + 7) / 8);
-  k_td_pack<<<g_all, 128, 0, st>>>(d_t, N, dD, d_scan);
-  cudaMemcpyAsync(&scan, d_scan, sizeof scan, cudaMemcpyDeviceToHost, st);
-  const cudaError_t pe = cudaStreamSynchronize(st);
-  if (pe != cudaSuccess) {
-    cleanup();
-    return fail(RT_ERR_CUDA, std::string("bibone walk: ") + cudaGetErrorString(pe));
+  const bool on_device = M > kTdHostSide;
+  if (!on_device) {
+    scan = td_pack_host(tiling, N, &bytes);
+    if (rt_status cs = td_check(scan)) {
+      cleanup();
+      return cs;
+    }
   }
-  if (scan.flags & 3u) {
-    cleanup();
-    return fail(RT_ERR_INVALID_ARGUMENT, (scan.flags & 1u) ? "bibone walk: tiling states are not those of a dimer configuration"
-                                                           : "bibone walk: two dimers share a vertex");
+  if (dev_alloc(&dD, (size_t)M * M, st)) return out_of_memory();
+  if (on_device) {
+    if (dev_alloc(&d_t, cells * sizeof(int32_t), st) || dev_alloc(&d_scan, sizeof(TdScan), st)) return out_of_memory();
+    cudaMemcpyAsync(d_t, tiling, cells * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(d_scan, &scan, sizeof scan, cudaMemcpyHostToDevice, st);
+    k_td_pack<<<g_all, 128, 0, st>>>(d_t, N, dD, d_scan);
+    cudaMemcpyAsync(&scan, d_scan, sizeof scan, cudaMemcpyDeviceToHost, st);
+    const cudaError_t pe = cudaStreamSynchronize(st);
+    if (pe != cudaSuccess) {
+      cleanup();
+      return fail(RT_ERR_CUDA, std::string("bibone walk: ") + cudaGetErrorString(pe));
+    }
+    if (rt_status cs = td_check(scan)) {
+      cleanup();
+      return cs;
+    }
+  } else {
+    cudaMemcpyAsync(dD, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, st);
   }
   TdClPlan plan;
   if (o.rng_mode != RT_RNG_MTGP && steps > 0) {
@@ -1170,7 +1211,7 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
       pdl_launch(k_td_step_fast, g_quad, dim3(32, 8), st, dD, M, sched[(size_t)h], (uint64_t)seed, o.fast_stream, h);
   }
   cudaEventRecord(e1, st);
-  k_td_unpack<<<g_all, 128, 0, st>>>(dD, N, d_t);
+  if (on_device) k_td_unpack<<<g_all, 128, 0, st>>>(dD, N, d_t);
   if (le == cudaSuccess) le = cudaGetLastError();
   int gave_up = 0;
   if (exchanges && le == cudaSuccess) {  // before the caller's tiling changes
@@ -1183,7 +1224,8 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
       return fail(RT_ERR_TIMEOUT, "bibone walk: a band gave up waiting for a neighbour's rows");
     }
   }
-  if (le == cudaSuccess) cudaMemcpyAsync(tiling, d_t, cells * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  if (le == cudaSuccess && on_device) cudaMemcpyAsync(tiling, d_t, cells * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  if (le == cudaSuccess && !on_device) cudaMemcpyAsync(bytes.data(), dD, bytes.size(), cudaMemcpyDeviceToHost, st);
   const cudaError_t se = cudaStreamSynchronize(st);
   float ms = 0.f;
   if (se == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -1192,6 +1234,7 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   cleanup();
   if (le != cudaSuccess || se != cudaSuccess)
     return fail(RT_ERR_CUDA, std::string("bibone walk: ") + cudaGetErrorString(le != cudaSuccess ? le : se));
+  if (!on_device) td_to_tiling(bytes.data(), N, tiling);
   if (stats) {
     std::memset(stats, 0, sizeof *stats);
     // per class, the sites whose anchor vertex is covered: the classes have periods 2 and 3

@@ -39,3 +39,25 @@ def test_lozenge(rt, orc, side, steps, mode):
         orc.lz_walk_tinymt(want, rt.side_of(start), steps, 11)
     L(rng=mode, fast_stream=7).Walk(got, steps, 11)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("mode", ["tinymt", "fast"])
+@pytest.mark.parametrize("rows,cols", [(4, 4), (20, 12), (41, 40), (42, 42), (43, 40), (44, 44)])
+@pytest.mark.parametrize("steps", [0, 1, 12])
+def test_bibone(rt, orc, rows, cols, steps, mode):
+    T = rt.TriangleDimerTiler
+    start = T.RhombusBrick(rows, cols)
+    n = rt.side_of(start)
+    got, want = start.copy(), start.copy()
+    if mode == "fast":
+        orc.td_walk_fast(want, n, 0, steps, 11, 7)
+    else:
+        orc.td_walk_tinymt(want, n, steps, 11)
+    stats = T(rng=mode, fast_stream=7).Walk(got, steps, 11)
+    assert np.array_equal(got, want)
+    assert stats["total_steps"] == steps
+    bad = start.copy()
+    bad[n + 1] ^= 4  # no dimer configuration
+    with pytest.raises(rt.RTError) as err:
+        T(rng=mode).Walk(bad, steps, 11)
+    assert err.value.status == rt.RT_ERR_INVALID_ARGUMENT
