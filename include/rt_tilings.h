@@ -530,6 +530,8 @@ RT_API rt_status rt_dm_sampler_test_silent_band(rt_dm_sampler* s, int32_t band, 
 /* The same for the calling thread's walks and couplings, which make their own sampler: from now on band `band`
    publishes nothing in launches [from, from + count) of a resident kernel (counted from this call), and waits
    give up after max_spin polls.  band < 0 ends it. */
+/* Test hook: in the calling thread device blocks above `bytes` fail as if memory had run out (0: no limit). */
+RT_API rt_status rt_test_alloc_limit(int64_t bytes);
 RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count);
 
 /* ---- allocation-free sweep -------------------------------------------------------------

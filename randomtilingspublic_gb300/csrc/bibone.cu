@@ -1085,7 +1085,10 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   TdScan scan = td_no_scan(M);
   std::vector<uint8_t> bytes;
   const dim3 g_all((M + 127) / 128, M), g_quad(((M + 3) / 4 + 31) / 32, (M + 7) / 8);
-  const bool on_device = M > kTdHostSide;
+  // (on the host too where the device has no room for the tiling's words, 16 times the bytes)
+  const bool on_device = M > kTdHostSide && !dev_alloc(&d_t, cells * sizeof(int32_t), st) &&
+                         !dev_alloc(&d_scan, sizeof(TdScan), st);
+  clear_error();
   if (!on_device) {
     scan = td_pack_host(tiling, N, &bytes);
     if (rt_status cs = td_check(scan)) {
@@ -1095,7 +1098,6 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
   }
   if (dev_alloc(&dD, (size_t)M * M, st)) return out_of_memory();
   if (on_device) {
-    if (dev_alloc(&d_t, cells * sizeof(int32_t), st) || dev_alloc(&d_scan, sizeof(TdScan), st)) return out_of_memory();
     cudaMemcpyAsync(d_t, tiling, cells * sizeof(int32_t), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_scan, &scan, sizeof scan, cudaMemcpyHostToDevice, st);
     k_td_pack<<<g_all, 128, 0, st>>>(d_t, N, dD, d_scan);

@@ -20,6 +20,8 @@ constexpr int kMaxDevices = 128;
 // Bytes a pool keeps reserved while idle: enough for the samplers of an order-2048 domain.
 constexpr uint64_t kPoolKeepBytes = 2ull << 30;
 
+thread_local size_t g_alloc_limit = 0;  // test hook: larger blocks fail in this thread (0: none)
+
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 
@@ -53,6 +55,7 @@ rt_status pool_of(cudaMemPool_t* out) {
 
 rt_status dev_alloc(void** p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
+  if (g_alloc_limit > 0 && bytes > g_alloc_limit) return fail(RT_ERR_OUT_OF_MEMORY, "device allocation: above the test's limit");
   cudaMemPool_t pool = nullptr;
   if (rt_status st = pool_of(&pool)) return st;
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
@@ -89,3 +92,10 @@ void dev_free(void* p, cudaStream_t s) {
 }
 
 }  // namespace rt
+
+extern "C" RT_API rt_status rt_test_alloc_limit(int64_t bytes) {
+  rt::clear_error();
+  if (bytes < 0) return rt::fail(RT_ERR_INVALID_ARGUMENT, "test_alloc_limit: negative limit");
+  rt::g_alloc_limit = (size_t)bytes;
+  return RT_OK;
+}

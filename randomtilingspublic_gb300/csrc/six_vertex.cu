@@ -976,9 +976,13 @@ RT_API rt_status rt_sv_walk(int32_t* h, int32_t n, int64_t sweeps, int64_t seed,
     if (on_device && !sv_valid_heights(h, n)) return fail(RT_ERR_INVALID_ARGUMENT, invalid);
     return e;
   }
+  if (on_device && dev_alloc(&R.dev.heights, points * sizeof(int32_t), st)) {  // no room for them: on the host
+    clear_error();
+    on_device = false;
+    if (!sv_valid_heights(h, n)) return fail(RT_ERR_INVALID_ARGUMENT, invalid);
+  }
   std::vector<uint32_t> bits;
   if (on_device) {
-    if (rt_status e = dev_alloc(&R.dev.heights, points * sizeof(int32_t), st)) return e;
     int bad = 0;
     cudaMemcpyAsync(R.dev.heights, h, points * sizeof(int32_t), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(R.dev.chains, 0, G.chain_words * sizeof(uint32_t), st);  // the guard words
