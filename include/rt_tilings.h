@@ -416,6 +416,9 @@ typedef struct rt_server_opts {
 
 RT_API rt_status rt_server_create(const rt_server_opts* opts, rt_server** out);
 /* Copies the request (its tmax / tmin) and returns its ticket; req->out is not used here. */
+/* Test hook: steps between the barriers of the bit-plane kernel for a request of this model and side (which draws
+   that many steps ahead), 0 where the server's CTAs run it as bytes. */
+RT_API int32_t rt_server_test_period(rt_server* s, int32_t model, int32_t n_side);
 RT_API rt_status rt_server_submit(rt_server* s, const rt_cftp_instance* req, int64_t* ticket);
 RT_API rt_status rt_server_poll(rt_server* s, int64_t ticket, int32_t* done);
 /* Waits up to timeout_s, writes the sample to result->out (N x N) and result->attempts /

@@ -151,6 +151,7 @@ _SIGNATURES = {
     "rt_dm_sweep_noalloc": (C.c_int32, [_P, _P, C.c_int32, C.c_int32, _P, C.c_int64, C.c_uint64, C.c_int64, _P]),
     "rt_cftp_batch": (C.c_int32, [_P, C.c_int32, _P, _P]),
     "rt_server_create": (C.c_int32, [_P, _P]),
+    "rt_server_test_period": (C.c_int32, [_P, C.c_int32, C.c_int32]),
     "rt_server_submit": (C.c_int32, [_P, _P, _P]),
     "rt_server_poll": (C.c_int32, [_P, C.c_int64, _P]),
     "rt_server_wait": (C.c_int32, [_P, C.c_int64, C.c_double, _P]),

@@ -106,7 +106,7 @@ __device__ int run_attempt(uint8_t* sm, size_t smem, const DevInstance& in, int 
   const uint32_t* gmin = reinterpret_cast<const uint32_t*>(tmin);
   uint32_t* s32 = reinterpret_cast<uint32_t*>(sm);
   const int64_t look = ncol * (in.first_sweeps << att);
-  const BpLayout L = bp_layout(in.model, in.N, in.P);
+  const BpLayout L = bp_layout(in.model, in.N, in.P, smem);
   // the plane kernels' first interval is [0, width up)
   *planes = (size_t)L.words * 4 <= smem &&
             (in.model != 0 || (in.lo_up[0] | in.lo_up[1] | in.lo_up[2] | in.lo_up[3]) == 0) &&
@@ -879,6 +879,13 @@ RT_API rt_status rt_server_create(const rt_server_opts* o, rt_server** out) {
   s->footprint.assign(s->slots, 0);
   *out = s.release();
   return RT_OK;
+}
+
+RT_API int32_t rt_server_test_period(rt_server* s, int32_t model, int32_t n_side) {
+  if (!s || n_side < 1 || n_side > s->max_side) return -1;
+  const int P = (n_side / (model == RT_MODEL_DOMINO ? 2 : 3) + 15) / 16 * 16;
+  const BpLayout L = bp_layout(model, n_side, P, s->smem);
+  return (size_t)L.words * 4 <= s->smem ? L.period : 0;
 }
 
 RT_API rt_status rt_server_submit(rt_server* s, const rt_cftp_instance* req, int64_t* ticket) {

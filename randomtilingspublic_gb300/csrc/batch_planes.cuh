@@ -35,7 +35,9 @@ constexpr int kBpUpdate = 128;      // threads that update, of a CTA; the others
 constexpr int kBpDominoWord = 8;    // [2 chains]{VD0, VD1, HE, HO}
 constexpr int kBpLozengeWord = 24;  // [2 chains]{E0-2, NE0-2, N0-2, three of padding}
 
-__host__ __device__ inline BpLayout bp_layout(int model, int N, int P) {
+// smem: bytes to keep within, if fewer steps a period do (a smaller side may ask for more than a larger one, whose
+// period is shorter).
+__host__ __device__ inline BpLayout bp_layout(int model, int N, int P, size_t smem = ~(size_t)0) {
   BpLayout L;
   const int PW = model == 0 ? kBpDominoWord : kBpLozengeWord;
   L.W = ((model == 0 ? N / 2 : N / 3) + 31) / 32;
@@ -44,13 +46,14 @@ __host__ __device__ inline BpLayout bp_layout(int model, int N, int P) {
   L.moves = L.stage = (L.valid + N * L.W + 3) & ~3;
   // As many steps a period as 32 KB of moves hold, but 2 to 8: a hexagon of side 32 alone 29.5 ms with 1, 24.0 with 4, 23.1
   // with 8.
-  L.period = N * L.W <= 256 ? 8 : N * L.W <= 512 ? 4 : 2;
-  L.items = L.moves + 2 * L.period * 2 * N * L.W;  // [period parity][step][word] pairs of words
-  L.units = L.items + N * L.W;
   const int staged = L.stage + (model == 0 ? 2 : 3) * N * P / 4;
-  L.words = L.units + 4 * N * L.W;
-  if (L.words < staged) L.words = staged;
-  return L;
+  for (L.period = N * L.W <= 256 ? 8 : N * L.W <= 512 ? 4 : 2;; L.period /= 2) {
+    L.items = L.moves + 2 * L.period * 2 * N * L.W;  // [period parity][step][word] pairs of words
+    L.units = L.items + N * L.W;
+    L.words = L.units + 4 * N * L.W;
+    if (L.words < staged) L.words = staged;
+    if (L.period == 2 || (size_t)L.words * 4 <= smem) return L;
+  }
 }
 inline size_t bp_bytes(int model, int N, int P) { return (size_t)bp_layout(model, N, P).words * 4; }
 
