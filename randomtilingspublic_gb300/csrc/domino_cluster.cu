@@ -365,9 +365,9 @@ __global__ void __launch_bounds__(cl_max_threads(kMode == kClFast, KS), 1) k_clu
         uint2 move[UI];
 #pragma unroll
         for (int u = 0; u < UI; ++u) move[u] = cl_lds2(move_at[u] + b * move_bytes);
-        if (waits && j > 0 && live) {
+        if (waits && j > 0) {  // (the vote wants all the warp's lanes, whatever each has read of s_failed)
           const uint32_t last = seq - 1, at = 8u * (last & 1u), phase = (last >> 1) & 1u;
-          if (wait_up && !cl_bar_wait(bar0 + at, phase, a.max_spin)) live = false;
+          if (wait_up && live && !cl_bar_wait(bar0 + at, phase, a.max_spin)) live = false;
           if (wait_dn && live && !cl_bar_wait(bar1 + at, phase, a.max_spin)) live = false;
           if (!__all_sync(~0u, live)) {
             live = false;

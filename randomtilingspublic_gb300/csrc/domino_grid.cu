@@ -220,11 +220,12 @@ __global__ void __launch_bounds__(gr_max_threads(kMode == kClFast, KS), 1) k_gri
         const uint32_t west = cl_lds(here - 16u * NCH + 12u);
         const bool aligned = ((flags[u] & kOdd) != 0u) == (t != 0u);  // left HE, right HO of the same word
         uint32_t U = t ? ab.x : ab.y, D = t ? me.y : me.x;
-        if (edge[u] && j > 0 && live) {
-          // the neighbours' words of the run before, which changed these planes
+        if (edge[u] && j > 0) {
+          // the neighbours' words of the run before, which changed these planes (the vote wants all the warp's lanes,
+          // whatever each has read of s_failed)
           const int xi = (int)(flags[u] >> 8);
-          bool ok = true;
-          if (flags[u] & kLinkUp) ok = gr_recv(xel(b ^ 1u, band - 1, 1, xi), (uint32_t)j, U, a.max_spin, a.error);
+          bool ok = live;
+          if (ok && (flags[u] & kLinkUp)) ok = gr_recv(xel(b ^ 1u, band - 1, 1, xi), (uint32_t)j, U, a.max_spin, a.error);
           if (ok && (flags[u] & kLinkDn)) ok = gr_recv(xel(b ^ 1u, band + 1, 0, xi), (uint32_t)j, D, a.max_spin, a.error);
           if (!__all_sync(~0u, ok)) {
             live = false;

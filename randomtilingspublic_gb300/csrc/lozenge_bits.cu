@@ -436,7 +436,8 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   bool failed = false;
   uint32_t r_last = 0u;  // colour of the run before
   // The neighbours' toggles of run `last` (colour r_last) into this CTA's copies of the planes.
-  // Each boundary row is one warp, so a word of its left neighbour is patched after the __syncwarp.
+  // Each boundary row is one warp, so a word of its left neighbour is patched after the __syncwarp.  All its lanes come
+  // here whatever they read of s_failed (another warp may just be setting it): the votes want them all.
   auto patch = [&](uint32_t last, bool& live) {
     const uint32_t par = last & 1u;
     uint32_t tu = 0u, td = 0u;
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
         }
         return (uint32_t)v;
       };
-      if (is_first) tu = poll(xel(par, band - 1, 1));
+      if (is_first && live) tu = poll(xel(par, band - 1, 1));
       if (is_last && live) td = poll(xel(par, band + 1, 0));
     }
     if (!__all_sync(~0u, live)) {
@@ -541,7 +542,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       }
       const uint32_t r = s_colour[b];
       const uint2 move = lb_lds2(move_at + b * move_bytes);
-      if (kForm != kLbOne && edge_warp && j > 0 && live) {
+      if (kForm != kLbOne && edge_warp && j > 0) {
         patch((uint32_t)j - 1u, live);
         if (!live) {
           failed = true;
@@ -612,10 +613,10 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   }
   if constexpr (kForm != kLbOne) {
     // the neighbours' last toggles
-    if (nruns > 0 && !failed && !*static_cast<volatile int*>(&s_failed) && updates) {
-      bool live = true;
+    if (nruns > 0 && updates) {
+      bool live = !failed && !*static_cast<volatile int*>(&s_failed);
       if (__any_sync(~0u, is_first || is_last)) patch((uint32_t)nruns - 1u, live);
-      failed = !live;
+      failed = failed || !live;
     }
     if (__syncthreads_or(failed ? 1 : 0) && tid == 0) {
       *static_cast<volatile int*>(a.error) = 1;
