@@ -184,6 +184,7 @@ struct TdClArgs {
   uint64_t* xbuf;  // [period parity][row from row_lo - 2][word][plane H, L, R], tags cleared
   int* error;
   long max_spin;
+  int silent_plus1;  // test hook: this band, less one, publishes nothing
 };
 
 // First site row of band b.
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(kTdThreads, 1) k_td_bands(const __grid_constan
       send_at[m] = take_at[m] = -1;
       send_to[m] = take_to[m] = 0;
       const int e = tid + m * T, y = e / row_elements, q = e - y * row_elements, x = q / 3, p = q - 3 * x;
-      if (y < mine) {
+      if (y < mine && rank + 1 != a.silent_plus1) {
         const int row = v1 - v0 <= 2 * reach || y < reach ? v0 + y : v1 - 2 * reach + y;
         send_at[m] = ((row - r0 + 2) * Wp + x) * 4 + p;
         send_to[m] = (row - a.row_lo + 2) * row_elements + q;
@@ -1195,7 +1196,8 @@ RT_API rt_status rt_td_walk(int32_t* tiling, int32_t n_side, int64_t steps, int6
     a.row_hi = scan.row_hi;
     a.xbuf = xbuf;
     a.error = d_error;
-    a.max_spin = 1L << 22;
+    a.max_spin = test_silence().spin(1L << 22);
+    a.silent_plus1 = test_silence().next_plus1();
     if (exchanges) {
       if (s0 == 0) cudaMemsetAsync(d_error, 0, sizeof(int), st);
       cudaMemsetAsync(xbuf, 0, plan.xbuf_words * sizeof(uint64_t), st);  // no stale tags

@@ -65,6 +65,7 @@ struct LbArgs {
   uint64_t* xbuf;  // [2 parities][band][to above, to below][word][chain]
   int* error;
   long max_spin;
+  int silent_plus1;  // test hook: this band, less one, publishes nothing
   // Coupling from the past (attempts > 0, two chains, kLbOne): CTA `team` runs attempts team, team + teams, ...
   // from the chains at start, into chains of its own at base + team * team_stride.
   int attempts;
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   }
   const bool is_last = updates && uw == 0 && my_y >= 0 && has_dn;                      // faces the band below
   const bool is_first = updates && my_y == 0 && has_up && (uw == 1 || (uw == 0 && R == 1));  // the band above
+  const bool tells_dn = is_last && band + 1 != a.silent_plus1, tells_up = is_first && band + 1 != a.silent_plus1;
   const uint32_t here = lb_addr(my_y >= 0 ? PL(my_y, my_x, my_c) : pad + kLbWord * NCH);
   const uint32_t below = lb_addr(my_y >= 0 ? PL(my_y + 1, my_x, my_c) : pad + 2 * kLbWord * NCH);
   const uint32_t left = (uint32_t)(NCH * kLbWord * 4);  // bytes to the word on the left
@@ -563,12 +565,12 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
       const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
       const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
       if constexpr (kForm == kLbCluster) {
-        lb_send_if(is_first && live, send_up + b * recv_bytes, T, rbar_up + 8u * b);
-        lb_send_if(is_last && live, send_dn + b * recv_bytes, T, rbar_dn + 8u * b);
+        lb_send_if(tells_up && live, send_up + b * recv_bytes, T, rbar_up + 8u * b);
+        lb_send_if(tells_dn && live, send_dn + b * recv_bytes, T, rbar_dn + 8u * b);
       } else if constexpr (kForm == kLbGrid) {
         const uint64_t tagged = ((uint64_t)((uint32_t)j + 1u) << 32) | T;
-        if (is_first && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 0)), "l"(tagged) : "memory");
-        if (is_last && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 1)), "l"(tagged) : "memory");
+        if (tells_up && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 0)), "l"(tagged) : "memory");
+        if (tells_dn && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 1)), "l"(tagged) : "memory");
       }
       lb_sts(own, e ^ T);
       lb_sts(own + 12u, ne ^ T);
@@ -897,7 +899,7 @@ LbArgs lb_args(const LbState& st, const LzResidentGeom& g, uint8_t* base, const 
   a.stream = fast_stream;
   a.xbuf = st.d_xbuf;
   a.error = st.d_error;
-  a.max_spin = 1L << 22;
+  a.max_spin = test_silence().spin(1L << 22);
   return a;
 }
 
@@ -996,6 +998,7 @@ rt_status lb_run(LbState& st, const LzResidentGeom& g, uint8_t* base, const LzRe
     LbArgs a = lb_args(st, g, base, rule, tinymt, tmt, params, d_cand, fast_seed, fast_stream);
     a.h0 = h0 + done;
     a.nruns = (int)n;
+    a.silent_plus1 = test_silence().next_plus1();
     if (tinymt) {
       runs.clear();
       lb_runs(colours_host + done, n, false, &runs);

@@ -185,6 +185,7 @@ struct SvBandArgs {
   uint64_t* xbuf;       // [period parity][band][to above, to below][chain][row][class][word], tags cleared
   int* error;
   long max_spin;
+  int silent_plus1;     // test hook: this band, less one, publishes nothing
   // Coupling from the past (couple, two chains): blockIdx.y = k runs attempt attempt0 + k, sub-sweeps
   // [-4 first << attempt, 0), into the k-th pair of chains at dst, and leaves once a smaller one has coalesced.
   int couple, attempt0;
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(kSvBandThreads, 1) k_sv_bands(const __grid_con
   for (int py = 0; py < 2; ++py) {
     const int2 ph = phase_tab[2 + py];
     const int row = ph.x + my_row;
-    if (!updates || ut >= ph.y || row < r0 || row >= r1) continue;
+    if (!updates || ut >= ph.y || row < r0 || row >= r1 || band + 1 == A.silent_plus1) continue;
     if (band > 0 && row < r0 + A.depth) send_up[py] = slot(band, 0) + ((row - r0) * 4 + 2 * py) * words + my_word;
     if (band + 1 < A.bands && row >= r1 - A.depth)
       send_dn[py] = slot(band, 1) + ((row - (r1 - A.depth)) * 4 + 2 * py) * words + my_word;
@@ -810,7 +811,8 @@ struct SvRun {
     A.stream = stream;
     A.xbuf = dev.xbuf;
     A.error = dev.flag + 1;
-    A.max_spin = 1L << 22;
+    A.max_spin = test_silence().spin(1L << 22);
+    A.silent_plus1 = test_silence().next_plus1();
     return A;
   }
 
