@@ -535,6 +535,9 @@ RT_API rt_status rt_dm_sampler_test_silent_band(rt_dm_sampler* s, int32_t band, 
    give up after max_spin polls.  band < 0 ends it. */
 /* Test hook: in the calling thread device blocks above `bytes` fail as if memory had run out (0: no limit). */
 RT_API rt_status rt_test_alloc_limit(int64_t bytes);
+/* Test hook: out4 = {engine, form of engine 4: 1 one thread-block cluster, 2 one band per SM, 0 other, bands, colour
+   runs between exchanges} that the calling thread's last domino run or coupling was planned on. */
+RT_API rt_status rt_test_route(int32_t* out4);
 RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count);
 
 /* ---- allocation-free sweep -------------------------------------------------------------

@@ -137,6 +137,7 @@ _SIGNATURES = {
     "rt_tune_clear": (C.c_int32, []),
     "rt_tune_lookup": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P]),
     "rt_dm_sampler_test_silent_band": (C.c_int32, [_P, C.c_int32, C.c_int64]),
+    "rt_test_route": (C.c_int32, [_P]),
     "rt_test_alloc_limit": (C.c_int32, [C.c_int64]),
     "rt_test_silent_band": (C.c_int32, [C.c_int32, C.c_int64, C.c_int32, C.c_int32]),
     "rt_walk": (C.c_int32, [C.c_int32, _P, C.c_int32, C.c_int64, C.c_int64, _P, _P]),

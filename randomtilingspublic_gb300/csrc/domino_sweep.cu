@@ -557,6 +557,15 @@ rt_status DmSampler::sync() {
 }
 
 rt_status DmSampler::use_persistent(bool* yes) {
+  const rt_status st = choose_engine(yes);
+  if (st == RT_OK)
+    test_route() = in_cluster ? TestRoute{4, 1, cluster->plan.ctas, 1}
+                   : on_grid  ? TestRoute{4, 2, grid->plan.bands, grid->plan.depth}
+                              : TestRoute{*yes ? resident : 1, 0, 0, 0};
+  return st;
+}
+
+rt_status DmSampler::choose_engine(bool* yes) {
   *yes = false;
   resident = 0;
   in_cluster = on_grid = false;

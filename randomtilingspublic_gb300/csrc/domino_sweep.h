@@ -127,6 +127,7 @@ struct DmSampler {
   rt_status sync();
   // Picks the engine for the next run: true when a resident kernel (see `resident`) will run it.
   rt_status use_persistent(bool* yes);
+  rt_status choose_engine(bool* yes);
   rt_status check_resident_error();
   rt_status launch_resident(const uint8_t* colours, int64_t steps, uint64_t fast_seed, int64_t h0);
 };

@@ -16,6 +16,11 @@ TestSilence& test_silence() {
   static thread_local TestSilence t;
   return t;
 }
+
+TestRoute& test_route() {
+  static thread_local TestRoute t;
+  return t;
+}
 }  // namespace rt
 
 extern "C" {
@@ -55,6 +60,17 @@ RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t fro
   t.from = from;
   t.count = count;
   rt::test_silence() = t;
+  return RT_OK;
+}
+
+RT_API rt_status rt_test_route(int32_t* out4) {
+  rt::clear_error();
+  if (!out4) return rt::fail(RT_ERR_INVALID_ARGUMENT, "test_route: out is NULL");
+  const rt::TestRoute& t = rt::test_route();
+  out4[0] = t.engine;
+  out4[1] = t.form;
+  out4[2] = t.bands;
+  out4[3] = t.depth;
   return RT_OK;
 }
 

@@ -50,6 +50,13 @@ struct TestSilence {
 };
 TestSilence& test_silence();
 
+// What the calling thread's last domino run or coupling was planned on (rt_test_route): the engine, the form of
+// engine 4 (1 one cluster, 2 one band per SM, 0 other), its bands and the runs between its exchanges.
+struct TestRoute {
+  int engine = 0, form = 0, bands = 0, depth = 0;
+};
+TestRoute& test_route();
+
 // cuRAND MTGP32 generators in the reference's CUDA geometry (domino_mtgp.cu): 8 x 8 thread
 // blocks over a rows x cols grid of sites (row from the x index, column from the y index),
 // block (bx, by) drawing from generator bx * gy + by.
