@@ -17,6 +17,7 @@ result: every draw is keyed by its site, whichever thread makes it.
 from __future__ import annotations
 
 import argparse
+import tempfile
 import time
 from pathlib import Path
 
@@ -25,12 +26,13 @@ THREADS = (512, 640, 768, 896, 960, 992, 1024)
 
 def candidates(sms: int) -> list[tuple[int, int, int]]:
     """(engine, bands, threads): the per-half-sweep kernels, k_persist, the run kernel over
-    bands and threads per band, the band form of the bit-plane kernel with polled
-    deltas (engine 4, TinyMT only), and the bit-plane kernel in one thread-block cluster or
-    with one band per SM (engine 0 with the bands asked for)."""
-    out = [(1, 0, 0), (3, 0, 0), (0, 1, 0), (0, 4, 0), (0, 16, 0), (0, sms, 0)]
+    bands and threads per band, and the bit-plane kernels in one thread-block cluster (1..16
+    bands) or on many SMs (engine 0 with the bands: what a table entry of engine 4 asks
+    for).  (Engine 4 asked for explicitly is the kernel with polled deltas, which an entry
+    only reaches where the others do not hold the domain.)"""
+    out = [(1, 0, 0), (3, 0, 0), (0, 1, 0), (0, 4, 0), (0, 16, 0)]
     for bands in sorted({sms, (3 * sms) // 4, sms // 2}, reverse=True):
-        out.append((4, bands, 0))
+        out.append((0, bands, 0))
         for threads in THREADS:
             out.append((2, bands, threads))
     return out
@@ -49,17 +51,21 @@ def measure(rt, n, chains, rng, tmax, tmin, shape, half_sweeps: int = 256, reps:
     """(microseconds per half-sweep, the shape the sampler used) for `shape` on this domain,
     or None when the sampler does not take it (no such plan, e.g. too many quads per thread
     for register generators).  A plan has at most one band per row, so on small domains the
-    bands used can be fewer than asked."""
+    bands used can be fewer than asked.  A shape of engine 0 runs as the table entry that it
+    becomes (the loaded table goes)."""
     s = _sampler(rt, n, chains, rng, tmax, tmin)
+    engine, bands, threads = shape
     try:
-        s.set_launch(*shape)
+        if engine == 0:
+            _load_entry(rt, n, chains, rng, bands)
+        else:
+            s.set_launch(*shape)
         try:
             info = s.engine_info()
         except rt.RTError:
             return None
-        engine, bands, threads = shape
-        if engine == 0:  # the cluster and grid forms, reported as the bit-plane kernel
-            if info["engine"] != 4 or info["bands"] > bands or (bands > 16) != (info["bands"] > 16):
+        if engine == 0:
+            if not info["tuned"] or info["bands"] > bands or (bands > 16) != (info["bands"] > 16):
                 return None
             engine = 4
         if info["engine"] != engine or (engine == 2 and info["threads"] != threads):
@@ -86,6 +92,16 @@ def measure(rt, n, chains, rng, tmax, tmin, shape, half_sweeps: int = 256, reps:
         return best / half_sweeps * 1e6, used
     finally:
         s.close()
+        if shape[0] == 0:
+            rt.tune_clear()
+
+
+def _load_entry(rt, n, chains, rng, bands) -> None:
+    """Loads a table of one entry of engine 4 for this size."""
+    with tempfile.TemporaryDirectory() as d:
+        path = Path(d) / "entry.txt"
+        path.write_text(f"domino {n} {n} {chains} {rng} 4 {bands} 0\n")
+        rt.tune_load(path)
 
 
 def tune_domino(rt, orders, chains_list=(2,), rngs=("tinymt",), half_sweeps: int = 256, log=print) -> list[dict]:
@@ -135,6 +151,7 @@ def write_table(entries, path) -> None:
     path = Path(path)
     path.parent.mkdir(parents=True, exist_ok=True)
     lines = ["# rt_tilings launch shapes measured by randomtilingspublic_gb300.autotune",
+             "# engine 4: the bit-plane kernels, in one cluster of 1..16 bands (else the next entry) or on more SMs",
              "# model n_lo n_hi chains rng engine bands threads us_per_half_sweep (measured at order, N)"]
     for e in entries:
         lines.append(f"domino {e['n_lo']} {e['n_hi']} {e['chains']} {e['rng']} {e['engine']} {e['bands']} "

@@ -648,7 +648,7 @@ rt_status DmSampler::choose_engine(bool* yes) {
       cluster = std::make_unique<ClusterEngine>();
       if (rt_status st = cluster->prepare(*this)) return st;
     }
-    if (cluster->ready && (launch_bands > 0 || cluster->plan.words <= cl_auto_words(fast))) {
+    if (cluster->ready && (launch_bands > 0 || tuned || cluster->plan.words <= cl_auto_words(fast))) {
       resident = 4;
       in_cluster = true;
       *yes = true;
