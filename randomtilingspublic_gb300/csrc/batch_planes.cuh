@@ -6,8 +6,9 @@
 // inputs whose edges agree at both ends and whose flip candidates border no cell that the reference
 // never rebuilds are held this way (bp_load tells); the others keep the byte kernels (batch_cftp.cuh).
 //
-// Warps of their own draw, a few half-sweeps (steps) ahead; the others apply the moves.  Draws are made for bytes of eight cells that hold a candidate, one
-// lane a Philox block (four cells), so a diamond draws for half of its bounding box.
+// Warps of their own draw, a few half-sweeps (steps) ahead; the others apply the moves.  Draws are made for bytes of
+// eight cells that hold a candidate, one lane a Philox block (four cells), so a diamond draws for half of its bounding
+// box.
 //
 // Bound: the issue of the draws, about 220 cycles of a scheduler for 32 blocks (160 of them Philox's
 // products), and in a CTA alone on its SM an update's latency.  Measured (GB300): hexagon of side 32, one CTA,

@@ -933,6 +933,14 @@ GridEngine::~GridEngine() {
 //           150: 4 0.45, 6 0.37, 8 0.37, 12 0.48    200: 1 1.06, 3 0.52, 4 0.45, 6 0.44, 8 0.50
 //           300: 1 1.08, 3 0.57, 4 0.56, 6 0.60    400: 2 0.72, 3 0.76    512: 2 0.95, 3 1.23
 // (rows of 1, 2, 3, 4, 5, 7, 8, 10, 13 and 17 words).  Wider rows than the last ones: d = 1.
+// The same lines serve two chains on a quarter of the SMs (couplings; ms of a call whose longest attempt is 8192
+// half-sweeps):
+//   TinyMT  order 16: d = 5 4.10, 6 3.91, 7 3.77    40: 4 5.18, 6 5.42, 8 6.37    64: 3 6.42, 4 5.89, 5 5.81
+//           100: 2 7.92, 3 7.50, 4 7.96    128: 1 12.40, 2 8.70, 3 9.05    160: 1 12.84, 2 11.86
+//   fast    order 24: d = 8 4.52, 12 4.26    64: 8 5.37, 11 5.13, 12 5.19    100: 6 6.86, 8 6.60, 10 7.11
+//           128: 7 7.33, 8 7.69    160: 4 8.84, 5 9.05, 6 10.10    200: 2 13.98, 4 12.63
+// within a tenth of the best for diamonds.  Few rows of many words are further off: 20 x 400 in TinyMT mode 2 8.65 and
+// one cluster 6.25, in fast mode 6 7.26 and 7, the choice, 9.63.
 static int gr_depth(const GrPlan& p, bool fast, int bands) {
   const int rows = p.row_start[p.bands] - p.row_start[0], used = std::min(bands, rows), rho = (rows + used - 1) / used;
   const auto words = [&](int d) { return (rho + 2 * d - 1) * p.xn; };

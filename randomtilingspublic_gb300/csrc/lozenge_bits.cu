@@ -22,7 +22,7 @@
 // steps into one pair of move words per 32 slots (as domino_cluster.cu).
 //
 // Coupling from the past where one CTA holds the chains: four CTAs run attempts side by side, as in
-// domino_cluster.cu (exact sample of the hexagon of side 20 in fast mode: 7.3 -> 5.9 ms).
+// domino_cluster.cu (exact sample of the hexagon of side 20 in fast mode: 7.3 -> 5.9 ms, and 4.0 with draws a period ahead).
 //
 // What bounds it: the exchange of each run, 0.5 us in a cluster and 0.85 us through L2.  The byte kernel
 // (lozenge_resident.cu) spent its step on the rotation and rebuild of bytes: hexagon 512 0.73 us a step
@@ -377,269 +377,269 @@ __global__ void __launch_bounds__(lb_max_threads(KS, kMode == kLbFast), 1) k_lz_
   const int n_att = cftp ? a.attempts : 1, teams = (int)gridDim.x;
   bool stopped = false;
   for (int att = cftp ? (int)blockIdx.x : 0; att < n_att; att += teams) {
-  int nruns = a.nruns, epoch = 0;
-  const uint32_t* runs = a.runs;
-  int64_t h0 = a.h0;
-  if (cftp) {
-    if (kFast) {
-      nruns = (int)(3 * (a.first_sweeps << att));
-      h0 = -(int64_t)nruns;
-    } else {
-      const int4 d = a.attempt_desc[att];
-      runs += d.x;
-      nruns = d.y;
-      epoch = d.z;
+    int nruns = a.nruns, epoch = 0;
+    const uint32_t* runs = a.runs;
+    int64_t h0 = a.h0;
+    if (cftp) {
+      if (kFast) {
+        nruns = (int)(3 * (a.first_sweeps << att));
+        h0 = -(int64_t)nruns;
+      } else {
+        const int4 d = a.attempt_desc[att];
+        runs += d.x;
+        nruns = d.y;
+        epoch = d.z;
+      }
+      load_planes(a.start);
     }
-    load_planes(a.start);
-  }
-  const int c0 = kFast ? (int)(((h0 % 3) + 3) % 3) : 0;
-  auto run_at = [&](int j) -> uint32_t {
-    if (kFast) return (uint32_t)((c0 + j) % 3) << 30 | 1u;
-    return j < nruns ? __ldg(&runs[j]) : 0u;
-  };
-  auto seed_of = [&](uint32_t run) -> uint32_t {
-    return !kFast && ((run >> 29) & 1u) ? __ldg(&a.epoch_seeds[epoch++]) : 0u;
-  };
-  // A period's steps, two at a time (those past the end are not used).
-  auto draw_period = [&](int q) {
-    if constexpr (kAhead > 1) {
-      uint2* const out = smove + (q & 1) * kAhead * nslots + warp * KS;
-#pragma unroll
-      for (int g = 0; g < KS / 4; ++g) {
-        if (g > 0 && g >= n_mine) break;
-        for (int r = 0; r < kAhead; r += 2) {
-          const int64_t h = h0 + q * kAhead + r;
-          const uint4 d0 = fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]);
-          const uint4 d1 = fast_quad(a.seed, a.stream, h + 1, f_row[g], f_quad[g]);
-          put(d0, out + r * nslots + 4 * g);
-          put(d1, out + (r + 1) * nslots + 4 * g);
+    const int c0 = kFast ? (int)(((h0 % 3) + 3) % 3) : 0;
+    auto run_at = [&](int j) -> uint32_t {
+      if (kFast) return (uint32_t)((c0 + j) % 3) << 30 | 1u;
+      return j < nruns ? __ldg(&runs[j]) : 0u;
+    };
+    auto seed_of = [&](uint32_t run) -> uint32_t {
+      return !kFast && ((run >> 29) & 1u) ? __ldg(&a.epoch_seeds[epoch++]) : 0u;
+    };
+    // A period's steps, two at a time (those past the end are not used).
+    auto draw_period = [&](int q) {
+      if constexpr (kAhead > 1) {
+        uint2* const out = smove + (q & 1) * kAhead * nslots + warp * KS;
+  #pragma unroll
+        for (int g = 0; g < KS / 4; ++g) {
+          if (g > 0 && g >= n_mine) break;
+          for (int r = 0; r < kAhead; r += 2) {
+            const int64_t h = h0 + q * kAhead + r;
+            const uint4 d0 = fast_quad(a.seed, a.stream, h, f_row[g], f_quad[g]);
+            const uint4 d1 = fast_quad(a.seed, a.stream, h + 1, f_row[g], f_quad[g]);
+            put(d0, out + r * nslots + 4 * g);
+            put(d1, out + (r + 1) * nslots + 4 * g);
+          }
         }
       }
+    };
+    uint32_t next = run_at(1);
+    if (kAhead > 1) {
+      if (!updates) draw_period(0);
+    } else if (!updates && nruns > 0) {
+      const uint32_t run = run_at(0);
+      draw_run(run, h0, seed_of(run), smove);
+      if (tid == 0) s_colour[0] = run >> 30;
     }
-  };
-  uint32_t next = run_at(1);
-  if (kAhead > 1) {
-    if (!updates) draw_period(0);
-  } else if (!updates && nruns > 0) {
-    const uint32_t run = run_at(0);
-    draw_run(run, h0, seed_of(run), smove);
-    if (tid == 0) s_colour[0] = run >> 30;
-  }
-  // Every 256 runs: has a smaller attempt coalesced?
-  auto told_stop = [&](int j) {
-    if (!cftp || (j & 255) != 255) return false;
-    if (tid == 0) s_stop = *static_cast<volatile int*>(a.best) < att;
-    __syncthreads();
-    return *static_cast<volatile int*>(&s_stop) != 0;
-  };
-  if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
-  else __syncthreads();
+    // Every 256 runs: has a smaller attempt coalesced?
+    auto told_stop = [&](int j) {
+      if (!cftp || (j & 255) != 255) return false;
+      if (tid == 0) s_stop = *static_cast<volatile int*>(a.best) < att;
+      __syncthreads();
+      return *static_cast<volatile int*>(&s_stop) != 0;
+    };
+    if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
 
-  bool failed = false;
-  uint32_t r_last = 0u;  // colour of the run before
-  // The neighbours' toggles of run `last` (colour r_last) into this CTA's copies of the planes.
-  // Each boundary row is one warp, so a word of its left neighbour is patched after the __syncwarp.  All its lanes come
-  // here whatever they read of s_failed (another warp may just be setting it): the votes want them all.
-  auto patch = [&](uint32_t last, bool& live) {
-    const uint32_t par = last & 1u;
-    uint32_t tu = 0u, td = 0u;
-    if constexpr (kForm == kLbCluster) {
-      const uint32_t phase = (last >> 1) & 1u;
-      if (__any_sync(~0u, is_first)) live = live && lb_bar_wait(bar_up + 8u * par, phase, a.max_spin);
-      if (__any_sync(~0u, is_last)) live = live && lb_bar_wait(bar_dn + 8u * par, phase, a.max_spin);
-      if (is_first && live) tu = lb_lds(recv_up + par * recv_bytes);
-      if (is_last && live) td = lb_lds(recv_dn + par * recv_bytes);
-    } else if constexpr (kForm == kLbGrid) {
-      auto poll = [&](const uint64_t* g) -> uint32_t {
-        uint64_t v = 0;
-        for (long it = 0;; ++it) {
-          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(g) : "memory");
-          if ((uint32_t)(v >> 32) == last + 1u) break;
-          if (it > a.max_spin) {
-            live = false;
+    bool failed = false;
+    uint32_t r_last = 0u;  // colour of the run before
+    // The neighbours' toggles of run `last` (colour r_last) into this CTA's copies of the planes.
+    // Each boundary row is one warp, so a word of its left neighbour is patched after the __syncwarp.  All its lanes come
+    // here whatever they read of s_failed (another warp may just be setting it): the votes want them all.
+    auto patch = [&](uint32_t last, bool& live) {
+      const uint32_t par = last & 1u;
+      uint32_t tu = 0u, td = 0u;
+      if constexpr (kForm == kLbCluster) {
+        const uint32_t phase = (last >> 1) & 1u;
+        if (__any_sync(~0u, is_first)) live = live && lb_bar_wait(bar_up + 8u * par, phase, a.max_spin);
+        if (__any_sync(~0u, is_last)) live = live && lb_bar_wait(bar_dn + 8u * par, phase, a.max_spin);
+        if (is_first && live) tu = lb_lds(recv_up + par * recv_bytes);
+        if (is_last && live) td = lb_lds(recv_dn + par * recv_bytes);
+      } else if constexpr (kForm == kLbGrid) {
+        auto poll = [&](const uint64_t* g) -> uint32_t {
+          uint64_t v = 0;
+          for (long it = 0;; ++it) {
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(g) : "memory");
+            if ((uint32_t)(v >> 32) == last + 1u) break;
+            if (it > a.max_spin) {
+              live = false;
+              break;
+            }
+          }
+          return (uint32_t)v;
+        };
+        if (is_first && live) tu = poll(xel(par, band - 1, 1));
+        if (is_last && live) td = poll(xel(par, band + 1, 0));
+      }
+      if (!__all_sync(~0u, live)) {
+        live = false;
+        return;
+      }
+      const int q = (i3 + (int)r_last) % 3;  // this row's residue in that run
+      // from above: row r0 - 1 (residue q - 1) toggled N(r0, q - 1) and NE(r0, q - 2), one slot to the
+      // left where its residue is 0
+      const uint32_t tu_right = __shfl_down_sync(~0u, tu, NCH);  // the word on the right's
+      if (is_first) {
+        const int qa = q == 0 ? 2 : q - 1, qb = qa == 0 ? 2 : qa - 1;
+        const uint32_t right = my_x - (a.w0 - wlo) + 1 < W ? tu_right : 0u;
+        const uint32_t n_at = here + 4u * (6 + qa), ne_at = here + 4u * (3 + qb);
+        lb_sts(n_at, lb_lds(n_at) ^ tu);
+        lb_sts(ne_at, lb_lds(ne_at) ^ (qa == 0 ? __funnelshift_r(tu, right, 1) : tu));
+        if (qa == 0 && my_x == a.w0 - wlo) lb_xor_if(ne_at - left, tu << 31);  // into the word left of all
+      }
+      // from below: row r1 (residue q + 1) toggled NE and N of its own vertices
+      if (is_last) {
+        const int qc = q == 2 ? 0 : q + 1;
+        const uint32_t n_at = below + 4u * (6 + qc), ne_at = below + 4u * (3 + qc);
+        lb_sts(n_at, lb_lds(n_at) ^ td);
+        lb_sts(ne_at, lb_lds(ne_at) ^ td);
+      }
+      __syncwarp();
+    };
+    if constexpr (kAhead > 1) {
+      const int periods = (nruns + kAhead - 1) / kAhead;
+      int r = c0;  // the step's colour
+      for (int p = 0; p < periods; ++p) {
+        if (updates) {
+          uint32_t at = move_at + (uint32_t)((p & 1) * kAhead) * move_bytes;
+          const int len = min(kAhead, nruns - p * kAhead);
+          for (int k = 0; k < len; ++k, at += move_bytes) {
+            const uint2 move = lb_lds2(at);
+            const int q = i3 + r >= 3 ? i3 + r - 3 : i3 + r, qw = q == 0 ? 2 : q - 1;
+            const uint32_t own = here + 4u * q, west = here + 4u * qw, south = below + 4u * (6 + q), sw = below + 4u * (3 + qw);
+            const uint32_t e = lb_lds(own), ne = lb_lds(own + 12u), n = lb_lds(own + 24u);
+            uint32_t w = lb_lds(west), ws = lb_lds(sw);
+            const uint32_t s = lb_lds(south), w_l = lb_lds(west - left), ws_l = lb_lds(sw - left);
+            if (q == 0) {
+              w = __funnelshift_l(w_l, w, 1);
+              ws = __funnelshift_l(ws_l, ws, 1);
+            }
+            const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
+            const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
+            lb_sts(own, e ^ T);
+            lb_sts(own + 12u, ne ^ T);
+            lb_sts(own + 24u, n ^ T);
+            lb_sts(south, s ^ T);
+            const uint32_t tw = q == 0 ? T >> 1 : T, tl = q == 0 ? T << 31 : 0u;
+            lb_xor_if(west, tw);
+            lb_xor_if(sw, tw);
+            lb_xor_if(west - left, tl);
+            lb_xor_if(sw - left, tl);
+            r = r == 2 ? 0 : r + 1;
+            asm volatile("bar.sync 1, %0;" ::"r"(32 * (nwarps - ndraw)) : "memory");
+          }
+        } else if (p + 1 < periods) {
+          draw_period(p + 1);
+        }
+        lb_cta_sync();
+        if (told_stop(p * kAhead + kAhead - 1)) {
+          stopped = true;
+          break;
+        }
+      }
+    } else if (updates) {
+      const bool edge_warp = __any_sync(~0u, is_first || is_last);
+      const bool arms = kForm == kLbCluster && warp == ndraw && lane == 0;
+      for (int j = 0; j < nruns; ++j) {
+        const uint32_t b = (uint32_t)j & 1u;
+        bool live = true;
+        if constexpr (kForm != kLbOne) live = !*static_cast<volatile int*>(&s_failed);
+        if constexpr (kForm == kLbCluster) {
+          lb_expect_if(arms && has_up && live, bar_up + 8u * b, recv_bytes);
+          lb_expect_if(arms && has_dn && live, bar_dn + 8u * b, recv_bytes);
+        }
+        const uint32_t r = s_colour[b];
+        const uint2 move = lb_lds2(move_at + b * move_bytes);
+        if (kForm != kLbOne && edge_warp && j > 0) {
+          patch((uint32_t)j - 1u, live);
+          if (!live) {
+            failed = true;
+            s_failed = 1;
+          }
+        }
+        const int q = i3 + (int)r >= 3 ? i3 + (int)r - 3 : i3 + (int)r, qw = q == 0 ? 2 : q - 1;
+        const uint32_t own = here + 4u * q, west = here + 4u * qw, south = below + 4u * (6 + q), sw = below + 4u * (3 + qw);
+        const uint32_t e = lb_lds(own), ne = lb_lds(own + 12u), n = lb_lds(own + 24u);
+        uint32_t w = lb_lds(west), ws = lb_lds(sw);
+        const uint32_t s = lb_lds(south), w_l = lb_lds(west - left), ws_l = lb_lds(sw - left);
+        if (q == 0) {
+          w = __funnelshift_l(w_l, w, 1);
+          ws = __funnelshift_l(ws_l, ws, 1);
+        }
+        // Flippable: E, N, SW equal, NE, W, S their complement; T: slots whose state differs at the
+        // end of the run (x: what becomes of 25, y: of 38).
+        const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
+        const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
+        if constexpr (kForm == kLbCluster) {
+          lb_send_if(tells_up && live, send_up + b * recv_bytes, T, rbar_up + 8u * b);
+          lb_send_if(tells_dn && live, send_dn + b * recv_bytes, T, rbar_dn + 8u * b);
+        } else if constexpr (kForm == kLbGrid) {
+          const uint64_t tagged = ((uint64_t)((uint32_t)j + 1u) << 32) | T;
+          if (tells_up && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 0)), "l"(tagged) : "memory");
+          if (tells_dn && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 1)), "l"(tagged) : "memory");
+        }
+        lb_sts(own, e ^ T);
+        lb_sts(own + 12u, ne ^ T);
+        lb_sts(own + 24u, n ^ T);
+        lb_sts(south, s ^ T);
+        const uint32_t tw = q == 0 ? T >> 1 : T, tl = q == 0 ? T << 31 : 0u;
+        lb_xor_if(west, tw);
+        lb_xor_if(sw, tw);
+        lb_xor_if(west - left, tl);
+        lb_xor_if(sw - left, tl);
+        r_last = r;
+        if (kForm == kLbOne || (j & 63) != 63) {
+          lb_cta_sync();
+          if (told_stop(j)) {
+            stopped = true;
             break;
           }
-        }
-        return (uint32_t)v;
-      };
-      if (is_first && live) tu = poll(xel(par, band - 1, 1));
-      if (is_last && live) td = poll(xel(par, band + 1, 0));
-    }
-    if (!__all_sync(~0u, live)) {
-      live = false;
-      return;
-    }
-    const int q = (i3 + (int)r_last) % 3;  // this row's residue in that run
-    // from above: row r0 - 1 (residue q - 1) toggled N(r0, q - 1) and NE(r0, q - 2), one slot to the
-    // left where its residue is 0
-    const uint32_t tu_right = __shfl_down_sync(~0u, tu, NCH);  // the word on the right's
-    if (is_first) {
-      const int qa = q == 0 ? 2 : q - 1, qb = qa == 0 ? 2 : qa - 1;
-      const uint32_t right = my_x - (a.w0 - wlo) + 1 < W ? tu_right : 0u;
-      const uint32_t n_at = here + 4u * (6 + qa), ne_at = here + 4u * (3 + qb);
-      lb_sts(n_at, lb_lds(n_at) ^ tu);
-      lb_sts(ne_at, lb_lds(ne_at) ^ (qa == 0 ? __funnelshift_r(tu, right, 1) : tu));
-      if (qa == 0 && my_x == a.w0 - wlo) lb_xor_if(ne_at - left, tu << 31);  // into the word left of all
-    }
-    // from below: row r1 (residue q + 1) toggled NE and N of its own vertices
-    if (is_last) {
-      const int qc = q == 2 ? 0 : q + 1;
-      const uint32_t n_at = below + 4u * (6 + qc), ne_at = below + 4u * (3 + qc);
-      lb_sts(n_at, lb_lds(n_at) ^ td);
-      lb_sts(ne_at, lb_lds(ne_at) ^ td);
-    }
-    __syncwarp();
-  };
-  if constexpr (kAhead > 1) {
-    const int periods = (nruns + kAhead - 1) / kAhead;
-    int r = c0;  // the step's colour
-    for (int p = 0; p < periods; ++p) {
-      if (updates) {
-        uint32_t at = move_at + (uint32_t)((p & 1) * kAhead) * move_bytes;
-        const int len = min(kAhead, nruns - p * kAhead);
-        for (int k = 0; k < len; ++k, at += move_bytes) {
-          const uint2 move = lb_lds2(at);
-          const int q = i3 + r >= 3 ? i3 + r - 3 : i3 + r, qw = q == 0 ? 2 : q - 1;
-          const uint32_t own = here + 4u * q, west = here + 4u * qw, south = below + 4u * (6 + q), sw = below + 4u * (3 + qw);
-          const uint32_t e = lb_lds(own), ne = lb_lds(own + 12u), n = lb_lds(own + 24u);
-          uint32_t w = lb_lds(west), ws = lb_lds(sw);
-          const uint32_t s = lb_lds(south), w_l = lb_lds(west - left), ws_l = lb_lds(sw - left);
-          if (q == 0) {
-            w = __funnelshift_l(w_l, w, 1);
-            ws = __funnelshift_l(ws_l, ws, 1);
-          }
-          const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
-          const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
-          lb_sts(own, e ^ T);
-          lb_sts(own + 12u, ne ^ T);
-          lb_sts(own + 24u, n ^ T);
-          lb_sts(south, s ^ T);
-          const uint32_t tw = q == 0 ? T >> 1 : T, tl = q == 0 ? T << 31 : 0u;
-          lb_xor_if(west, tw);
-          lb_xor_if(sw, tw);
-          lb_xor_if(west - left, tl);
-          lb_xor_if(sw - left, tl);
-          r = r == 2 ? 0 : r + 1;
-          asm volatile("bar.sync 1, %0;" ::"r"(32 * (nwarps - ndraw)) : "memory");
-        }
-      } else if (p + 1 < periods) {
-        draw_period(p + 1);
-      }
-      lb_cta_sync();
-      if (told_stop(p * kAhead + kAhead - 1)) {
-        stopped = true;
-        break;
-      }
-    }
-  } else if (updates) {
-    const bool edge_warp = __any_sync(~0u, is_first || is_last);
-    const bool arms = kForm == kLbCluster && warp == ndraw && lane == 0;
-    for (int j = 0; j < nruns; ++j) {
-      const uint32_t b = (uint32_t)j & 1u;
-      bool live = true;
-      if constexpr (kForm != kLbOne) live = !*static_cast<volatile int*>(&s_failed);
-      if constexpr (kForm == kLbCluster) {
-        lb_expect_if(arms && has_up && live, bar_up + 8u * b, recv_bytes);
-        lb_expect_if(arms && has_dn && live, bar_dn + 8u * b, recv_bytes);
-      }
-      const uint32_t r = s_colour[b];
-      const uint2 move = lb_lds2(move_at + b * move_bytes);
-      if (kForm != kLbOne && edge_warp && j > 0) {
-        patch((uint32_t)j - 1u, live);
-        if (!live) {
+        } else if (__syncthreads_or(failed ? 1 : 0)) {  // a band that gave up leaves within 64 runs
           failed = true;
-          s_failed = 1;
-        }
-      }
-      const int q = i3 + (int)r >= 3 ? i3 + (int)r - 3 : i3 + (int)r, qw = q == 0 ? 2 : q - 1;
-      const uint32_t own = here + 4u * q, west = here + 4u * qw, south = below + 4u * (6 + q), sw = below + 4u * (3 + qw);
-      const uint32_t e = lb_lds(own), ne = lb_lds(own + 12u), n = lb_lds(own + 24u);
-      uint32_t w = lb_lds(west), ws = lb_lds(sw);
-      const uint32_t s = lb_lds(south), w_l = lb_lds(west - left), ws_l = lb_lds(sw - left);
-      if (q == 0) {
-        w = __funnelshift_l(w_l, w, 1);
-        ws = __funnelshift_l(ws_l, ws, 1);
-      }
-      // Flippable: E, N, SW equal, NE, W, S their complement; T: slots whose state differs at the
-      // end of the run (x: what becomes of 25, y: of 38).
-      const uint32_t flip = ~(n ^ e) & ~(n ^ ws) & (n ^ ne) & (n ^ w) & (n ^ s) & valid;
-      const uint32_t T = flip & ((n & ~move.x) | (~n & move.y));
-      if constexpr (kForm == kLbCluster) {
-        lb_send_if(tells_up && live, send_up + b * recv_bytes, T, rbar_up + 8u * b);
-        lb_send_if(tells_dn && live, send_dn + b * recv_bytes, T, rbar_dn + 8u * b);
-      } else if constexpr (kForm == kLbGrid) {
-        const uint64_t tagged = ((uint64_t)((uint32_t)j + 1u) << 32) | T;
-        if (tells_up && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 0)), "l"(tagged) : "memory");
-        if (tells_dn && live) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(xel(b, band, 1)), "l"(tagged) : "memory");
-      }
-      lb_sts(own, e ^ T);
-      lb_sts(own + 12u, ne ^ T);
-      lb_sts(own + 24u, n ^ T);
-      lb_sts(south, s ^ T);
-      const uint32_t tw = q == 0 ? T >> 1 : T, tl = q == 0 ? T << 31 : 0u;
-      lb_xor_if(west, tw);
-      lb_xor_if(sw, tw);
-      lb_xor_if(west - left, tl);
-      lb_xor_if(sw - left, tl);
-      r_last = r;
-      if (kForm == kLbOne || (j & 63) != 63) {
-        lb_cta_sync();
-        if (told_stop(j)) {
-          stopped = true;
           break;
         }
-      } else if (__syncthreads_or(failed ? 1 : 0)) {  // a band that gave up leaves within 64 runs
-        failed = true;
-        break;
       }
-    }
-  } else {
-    for (int j = 0; j < nruns; ++j) {
-      const uint32_t after = run_at(j + 2);
-      if (j + 1 < nruns) {
-        if (tid == 0) s_colour[(j + 1) & 1] = next >> 30;
-        draw_run(next, h0 + j + 1, seed_of(next), smove + ((j + 1) & 1) * nslots);
-      }
-      next = after;
-      if (kForm == kLbOne || (j & 63) != 63) {
-        lb_cta_sync();
-        if (told_stop(j)) {
-          stopped = true;
+    } else {
+      for (int j = 0; j < nruns; ++j) {
+        const uint32_t after = run_at(j + 2);
+        if (j + 1 < nruns) {
+          if (tid == 0) s_colour[(j + 1) & 1] = next >> 30;
+          draw_run(next, h0 + j + 1, seed_of(next), smove + ((j + 1) & 1) * nslots);
+        }
+        next = after;
+        if (kForm == kLbOne || (j & 63) != 63) {
+          lb_cta_sync();
+          if (told_stop(j)) {
+            stopped = true;
+            break;
+          }
+        } else if (__syncthreads_or(0)) {
+          failed = true;
           break;
         }
-      } else if (__syncthreads_or(0)) {
-        failed = true;
-        break;
       }
     }
-  }
-  if constexpr (kForm != kLbOne) {
-    // the neighbours' last toggles
-    if (nruns > 0 && updates) {
-      bool live = !failed && !*static_cast<volatile int*>(&s_failed);
-      if (__any_sync(~0u, is_first || is_last)) patch((uint32_t)nruns - 1u, live);
-      failed = failed || !live;
+    if constexpr (kForm != kLbOne) {
+      // the neighbours' last toggles
+      if (nruns > 0 && updates) {
+        bool live = !failed && !*static_cast<volatile int*>(&s_failed);
+        if (__any_sync(~0u, is_first || is_last)) patch((uint32_t)nruns - 1u, live);
+        failed = failed || !live;
+      }
+      if (__syncthreads_or(failed ? 1 : 0) && tid == 0) {
+        *static_cast<volatile int*>(a.error) = 1;
+        if (kForm == kLbCluster)
+          for (int k = 0; k < 64; ++k) __nanosleep(1000);  // what is in flight to this CTA lands
+      }
+      if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
     }
-    if (__syncthreads_or(failed ? 1 : 0) && tid == 0) {
-      *static_cast<volatile int*>(a.error) = 1;
-      if (kForm == kLbCluster)
-        for (int k = 0; k < 64; ++k) __nanosleep(1000);  // what is in flight to this CTA lands
+    __syncthreads();
+    if (!cftp) break;
+    if (stopped) return;
+    uint32_t differ = 0u;
+    if (NCH == 2)
+      for (int k = tid; k < (R + 1) * wn * kLbWord; k += (int)blockDim.x) {
+        const uint32_t* p = lsm + (size_t)(k / kLbWord) * 2 * kLbWord + k % kLbWord;
+        differ |= p[0] ^ p[kLbWord];
+      }
+    if (!__syncthreads_or(differ != 0u)) {
+      if (tid == 0) atomicMin(a.best, att);
+      break;
     }
-    if constexpr (kForm == kLbCluster) cooperative_groups::this_cluster().sync();
-  }
-  __syncthreads();
-  if (!cftp) break;
-  if (stopped) return;
-  uint32_t differ = 0u;
-  if (NCH == 2)
-    for (int k = tid; k < (R + 1) * wn * kLbWord; k += (int)blockDim.x) {
-      const uint32_t* p = lsm + (size_t)(k / kLbWord) * 2 * kLbWord + k % kLbWord;
-      differ |= p[0] ^ p[kLbWord];
-    }
-  if (!__syncthreads_or(differ != 0u)) {
-    if (tid == 0) atomicMin(a.best, att);
-    break;
-  }
   }
   __syncthreads();
   // Rows r0 .. r1 - 1 back to the chains: slots [1, M - 2] of the window's inner words.

@@ -529,7 +529,7 @@ struct LzSampler {
         pdl_launch(k_lz_rotate_mtgp, dim3(g.gx, g.gy), dim3(kMtgpBlock, kMtgpBlock), stream, v, r, rule,
                    static_cast<curandStateMtgp32*>(mtgp));
         pdl_launch(k_lz_update_w, gu, dim3(32, 8), stream, v, r);
-        }
+      }
       return check();
     }
     LbState* lb = nullptr;
