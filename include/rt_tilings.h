@@ -416,10 +416,10 @@ typedef struct rt_server_opts {
 
 RT_API rt_status rt_server_create(const rt_server_opts* opts, rt_server** out);
 /* Copies the request (its tmax / tmin) and returns its ticket; req->out is not used here. */
+RT_API rt_status rt_server_submit(rt_server* s, const rt_cftp_instance* req, int64_t* ticket);
 /* Test hook: steps between the barriers of the bit-plane kernel for a request of this model and side (which draws
    that many steps ahead), 0 where the server's CTAs run it as bytes. */
 RT_API int32_t rt_server_test_period(rt_server* s, int32_t model, int32_t n_side);
-RT_API rt_status rt_server_submit(rt_server* s, const rt_cftp_instance* req, int64_t* ticket);
 RT_API rt_status rt_server_poll(rt_server* s, int64_t ticket, int32_t* done);
 /* Waits up to timeout_s, writes the sample to result->out (N x N) and result->attempts /
    final_steps, and frees the ticket's slot. */
@@ -533,12 +533,12 @@ RT_API rt_status rt_dm_sampler_test_silent_band(rt_dm_sampler* s, int32_t band, 
 /* The same for the calling thread's walks and couplings, which make their own sampler: from now on band `band`
    publishes nothing in launches [from, from + count) of a resident kernel (counted from this call), and waits
    give up after max_spin polls.  band < 0 ends it. */
+RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count);
 /* Test hook: in the calling thread device blocks above `bytes` fail as if memory had run out (0: no limit). */
 RT_API rt_status rt_test_alloc_limit(int64_t bytes);
 /* Test hook: out4 = {engine, form of engine 4: 1 one thread-block cluster, 2 one band per SM, 0 other, bands, colour
    runs between exchanges} that the calling thread's last domino run or coupling was planned on. */
 RT_API rt_status rt_test_route(int32_t* out4);
-RT_API rt_status rt_test_silent_band(int32_t band, int64_t max_spin, int32_t from, int32_t count);
 
 /* ---- allocation-free sweep -------------------------------------------------------------
    No counterpart in the reference.  For callers that cannot allocate device memory (a
